@@ -295,14 +295,14 @@ typedef struct SoupTuneResult {
                                      particle), 1 each warp's in-range pairs compacted and evaluated with
                                      every lane busy (one lane per particle; the same result bits as
                                      variant 0 with tpp 1) */
-  uint32_t list_cells;            /* list build: 0 a thread per particle, 1 a group of lanes per cell */
+  uint32_t list_cells;            /* accepted and ignored (0 from soup_autotune): there is one list build, a warp
+                                     per particle */
 } SoupTuneResult;
 int soup_autotune(SoupHandle* h, uint32_t steps, SoupTuneResult* out);
 /* Apply a tuning found before (by soup_autotune on a system of the same shape) without timing
  * anything: lanes per particle, the list-force variant, list-walk radius, and the current skin scaled
  * by skin_scale (at most 1: the list capacity was sized for it; drift-triggered rebuilds only).  The
- * lists are rebuilt and the force recomputed.  Only tpp, queued, walk, skin_scale and list_cells are
- * read. */
+ * lists are rebuilt and the force recomputed.  Only tpp, queued, walk and skin_scale are read. */
 int soup_apply_tuning(SoupHandle* h, const SoupTuneResult* tuning);
 /* soup_step runs chunks of chunkSteps steps (at least 4) as captured CUDA graphs, captured on first
  * use; this captures every chunk graph of the current schedule now, without stepping. */

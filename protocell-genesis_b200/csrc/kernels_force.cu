@@ -52,18 +52,19 @@ __device__ __forceinline__ void bonded_term(const Shared& S, const SysParams& P,
 }
 
 // The end of the part of particle k's row a force pass must read.  The row is grouped by build
-// distance (k_group_rows): shell 0 within the force's reach r0 = sqrt(rmax2), shells 1..4 the rest of the
-// list range in four widths w.  No bead has moved more than dm since the build (the replica's largest
-// drift), so a pair of shell s is at least r0 + (s - 1) w - 2 dm apart now, and shell s can hold an
-// in-range pair only if (s - 1) w < 2 dm (a margin of 1e-3 sigma covers rounding).  Skipped entries are
-// beyond the reach, so the force is the same bits as over the whole row.
+// distance (k_build_list): shell 0 within the force's reach r0 = sqrt(rmax2), shells 1..4 the rest of the
+// list range in four widths w2 of r^2.  No bead has moved more than dm since the build (the replica's largest
+// drift), so a pair of shell s is at least sqrt(r0^2 + (s - 1) w2) - 2 dm apart now, and shell s can hold
+// an in-range pair only if r0^2 + (s - 1) w2 < (r0 + 2 dm)^2 (a margin of 1e-3 sigma covers rounding).
+// Skipped entries are beyond the reach, so the force is the same bits as over the whole row.
 __device__ __forceinline__ uint32_t list_force_end(uint32_t k, const uint32_t* __restrict__ nl_cnt,
                                                    const uint4* __restrict__ nl_shell, float drift2, float rmax2,
                                                    float list_range) {
   const uint32_t cnt = nl_cnt[k];
-  const float r0 = sqrtf(rmax2), w = (list_range - r0) * 0.25f;
-  if (!nl_shell || !(drift2 >= 0.f && drift2 < 1e30f) || !(w > 0.f)) return cnt;
-  const float x = (2.0f * sqrtf(drift2) + 1e-3f) / w;
+  const float w2 = list_shell_width2(rmax2, list_range);
+  if (!nl_shell || !(drift2 >= 0.f && drift2 < 1e30f) || !(w2 > 0.f)) return cnt;
+  const float d = 2.0f * sqrtf(drift2) + 1e-3f;
+  const float x = d * (2.0f * sqrtf(rmax2) + d) / w2;   // (r0 + d)^2 - r0^2 in shells
   if (x >= 3.0f) return cnt;
   const uint4 e = nl_shell[k];
   return x < 1.0f ? e.y : (x < 2.0f ? e.z : e.w);

@@ -173,20 +173,10 @@ __global__ void k_copy_back(uint32_t N, const float4* __restrict__ pos2, const f
   id[k] = id2[k];
 }
 
-// Distinct wrapped cell coordinates of a +-R walk along one axis, as at most two [lo,hi] intervals.
+// At most two [lo,hi] intervals of cells along one axis.
 struct AxisRange { int lo[2], hi[2], n; };
-__device__ __forceinline__ AxisRange axis_ranges(int q, int R, int dim) {
-  AxisRange a;
-  int lo = q - R, hi = q + R;
-  if (hi - lo + 1 >= dim) { a.n = 1; a.lo[0] = 0; a.hi[0] = dim - 1; }
-  else if (lo < 0) { a.n = 2; a.lo[0] = lo + dim; a.hi[0] = dim - 1; a.lo[1] = 0; a.hi[1] = hi; }
-  else if (hi >= dim) { a.n = 2; a.lo[0] = lo; a.hi[0] = dim - 1; a.lo[1] = 0; a.hi[1] = hi - dim; }
-  else { a.n = 1; a.lo[0] = lo; a.hi[0] = hi; }
-  return a;
-}
 
-// The cells lo..hi (unwrapped, hi - lo + 1 < dim) as at most two wrapped [lo,hi] intervals, in the
-// order axis_ranges gives them.
+// The cells lo..hi (unwrapped, hi - lo + 1 <= dim) as at most two wrapped [lo,hi] intervals.
 __device__ __forceinline__ AxisRange span_ranges(int lo, int hi, int dim) {
   AxisRange a;
   if (lo < 0) { a.n = 2; a.lo[0] = lo + dim; a.hi[0] = dim - 1; a.lo[1] = 0; a.hi[1] = hi; }
@@ -203,271 +193,205 @@ __device__ __forceinline__ float gap_to_cell(float p, int c, float cs) {
   return fmaxf(0.f, fmaxf(lo, -hi) - 1e-4f);
 }
 
-// The build-distance shell of a list entry, carried in its top three bits until k_group_rows groups
-// the row: 0 inside the force's reach (sqrt(rmax2)), 1..4 the rest of the list range in four equal
-// widths.  A force pass needs shell k > 0 only once the largest displacement since the build can have
-// closed (k - 1) widths (list_force_end).
+// The build-distance shell of a list entry, carried in its top three bits until its row is grouped: 0
+// inside the force's reach, 1..4 the rest of the list range (list_shell_width2).  A force pass needs shell
+// s > 0 only once the largest displacement since the build can have closed the distance from the reach to
+// that shell's inner edge (list_force_end).
 struct Shells {
-  float reach2, e1, e2, e3;
+  float reach2, scale;
   __device__ __forceinline__ static Shells of(float rmax2, float list_range) {
     Shells s;
-    const float r0 = sqrtf(rmax2), w = fmaxf(list_range - r0, 0.f) * 0.25f;
     s.reach2 = rmax2;
-    s.e1 = (r0 + w) * (r0 + w); s.e2 = (r0 + 2.f * w) * (r0 + 2.f * w); s.e3 = (r0 + 3.f * w) * (r0 + 3.f * w);
+    s.scale = 1.0f / fmaxf(list_shell_width2(rmax2, list_range), 1e-12f);
     return s;
   }
   __device__ __forceinline__ uint32_t tag(float r2) const {
-    const uint32_t k = r2 < reach2 ? 0u : 1u + (r2 >= e1) + (r2 >= e2) + (r2 >= e3);
-    return k << 29;
+    return (uint32_t)(min(max(__float2int_rd((r2 - reach2) * scale), -1), 3) + 1) << 29;
   }
 };
 
-// soup/wgsl/verlet.wgsl:53-92, thread per particle, rows of cells as contiguous slot ranges.  When
-// the walk does not wrap onto itself, each (y, z) row of cells is trimmed to the x cells that can
-// reach the list sphere (with a margin) and rows wholly outside it are skipped; the accept test is
-// unchanged, so the list is the same set.
+// ---- the neighbour walk of one particle by a warp -------------------------------------------------
+// The cells within the walk radius of a particle's cell form rows along x, and the beads of a row (they are
+// in cell order) one or two contiguous runs.  The lanes take a row each: the runs trimmed to the x cells that
+// can reach the list sphere, rows wholly beyond it dropped, and an axis on which the walk would wrap onto
+// itself visited once, whole.  The runs then make one flat sequence of candidates, and the warp takes 32 of
+// them at a time whatever run they lie in, so every lane has work but in the last 32.  (A run holds about 20
+// candidates: run by run, half the lanes would idle; a thread per particle diverges at every accepted
+// candidate and leaves a small system's chain of dependent loads uncovered.)
+constexpr uint32_t kWalkRuns = 128;                    // runs: two per row, (2 * 3 + 1)^2 rows at walk 3
+constexpr uint32_t kWalkSpan = 4096;                   // candidates whose run starts are marked at a time
+constexpr uint32_t kWalkWords = 2 * kWalkRuns + kWalkSpan / 32;   // shared words a warp's walk needs
+
+struct WalkGrid { int dims[3]; int walk; uint32_t cell_off; float range; };
+
+// take(j, valid): warp-wide, 2 x 32 candidates j (indices into the cell-ordered array) per round
+template <class Take>
+__device__ __forceinline__ void warp_walk(const float4& xi, const float* box, const WalkGrid& G,
+                                          const uint32_t* __restrict__ start, uint32_t* __restrict__ sm, Take&& take) {
+  uint32_t* shift = sm;                                // candidate q of run s is bead q + shift[s]
+  uint32_t* first = sm + kWalkRuns;                    // its first candidate
+  uint32_t* mark = sm + 2 * kWalkRuns;                 // bit per candidate: a run starts here
+  const uint32_t lane = threadIdx.x & 31u, lt = (1u << lane) - 1u, le = lt | (1u << lane);
+  const int R = G.walk, D = 2 * R + 1;
+  const int dx = G.dims[0], dy = G.dims[1], dz = G.dims[2];
+  const int qx = ex_cell_axis(xi.x, box[0], dx), qy = ex_cell_axis(xi.y, box[1], dy), qz = ex_cell_axis(xi.z, box[2], dz);
+  const bool fx = dx < D, fy = dy < D, fz = dz < D;    // this axis is visited whole
+  const int ny = fy ? dy : D, nz = fz ? dz : D;
+  const float csx = box[0] / (float)dx, csy = box[1] / (float)dy, csz = box[2] / (float)dz;
+  const float lrm = G.range * (1.0f + 1e-5f) + 1e-3f, lrm2 = lrm * lrm;
+  uint32_t runs = 0, total = 0;
+  for (int r0 = 0; r0 < ny * nz; r0 += 32) {
+    const int rr = r0 + (int)lane;
+    uint32_t a0 = 0, l0 = 0, a1 = 0, l1 = 0;
+    if (rr < ny * nz) {
+      const int iy = rr % ny, iz = rr / ny;
+      const int y = fy ? iy : qy - R + iy, z = fz ? iz : qz - R + iz;
+      const float gy = fy ? 0.f : gap_to_cell(xi.y, y, csy), gz = fz ? 0.f : gap_to_cell(xi.z, z, csz);
+      const float g2 = gy * gy + gz * gz;
+      if (g2 < lrm2) {
+        const uint32_t row = G.cell_off + (uint32_t)(dx * ((y + dy) % dy + dy * ((z + dz) % dz)));
+        if (fx) {
+          a0 = start[row];
+          l0 = start[row + (uint32_t)dx] - a0;
+        } else {
+          const float ext = sqrtf(lrm2 - g2);
+          const int xlo = max(qx - R, (int)floorf((xi.x - ext) / csx)), xhi = min(qx + R, (int)floorf((xi.x + ext) / csx));
+          if (xlo <= xhi) {
+            const AxisRange xr = span_ranges(xlo, xhi, dx);
+            a0 = start[row + (uint32_t)xr.lo[0]];
+            l0 = start[row + (uint32_t)xr.hi[0] + 1] - a0;
+            if (xr.n == 2) {
+              a1 = start[row + (uint32_t)xr.lo[1]];
+              l1 = start[row + (uint32_t)xr.hi[1] + 1] - a1;
+            }
+          }
+        }
+      }
+    }
+    uint32_t incl = l0 + l1;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const uint32_t v = __shfl_up_sync(0xffffffffu, incl, o);
+      if (lane >= (uint32_t)o) incl += v;
+    }
+    const uint32_t at = total + incl - (l0 + l1);
+    const uint32_t b0 = __ballot_sync(0xffffffffu, l0 != 0), b1 = __ballot_sync(0xffffffffu, l1 != 0);
+    uint32_t s = runs + __popc(b0 & lt) + __popc(b1 & lt);
+    if (l0) { shift[s] = a0 - at; first[s] = at; ++s; }
+    if (l1) { shift[s] = a1 - (at + l0); first[s] = at + l0; }
+    runs += __popc(b0) + __popc(b1);
+    total += __shfl_sync(0xffffffffu, incl, 31);
+  }
+  __syncwarp();
+  for (uint32_t w0 = 0; w0 < total; w0 += kWalkSpan) {
+    const uint32_t n = min(total - w0, kWalkSpan);
+    for (uint32_t i = lane; i < (n + 63u) / 64u * 2u; i += 32u) mark[i] = 0;
+    __syncwarp();
+    uint32_t before = 0;
+    for (uint32_t s0 = 0; s0 < runs; s0 += 32u) {
+      const uint32_t p = s0 + lane < runs ? first[s0 + lane] : 0xFFFFFFFFu;
+      if (p >= w0 && p - w0 < n) atomicOr(&mark[(p - w0) >> 5], 1u << (p & 31u));
+      before += __popc(__ballot_sync(0xffffffffu, p < w0));
+    }
+    __syncwarp();
+    for (uint32_t c = 0; c < n; c += 64u) {
+      const uint2 m = *reinterpret_cast<const uint2*>(&mark[c >> 5]);
+      const uint32_t q0 = w0 + c + lane, q1 = q0 + 32u;
+      const bool v0 = q0 < total, v1 = q1 < total;
+      const uint32_t s0 = before + __popc(m.x & le) - 1u;
+      before += __popc(m.x);
+      const uint32_t s1 = before + __popc(m.y & le) - 1u;
+      before += __popc(m.y);
+      take(v0 ? shift[s0] + q0 : 0u, v0, v1 ? shift[s1] + q1 : 0u, v1);
+    }
+    __syncwarp();
+  }
+}
+
+__device__ __forceinline__ uint32_t field12(unsigned long long w, uint32_t t) {
+  return (uint32_t)(w >> (12u * t)) & 0xFFFu;
+}
+constexpr uint32_t kGRegs = 17;                        // entries a lane can hold while a row is grouped
+
+// soup/wgsl/verlet.wgsl:53-92, a warp per particle (warp_walk).  The fast squared distance decides unless it
+// lies within 1e-5 of the range, where the reference's arithmetic decides (the minimum image cannot differ
+// there: range < box/2), so the list is the reference's set.  The accepted entries are compacted into the
+// warp's shared row with ballots, then the row is grouped by build-distance shell, keeping its order inside
+// a shell, and written once, coalesced.
+//
+// Bound: instruction issue (about 17 rounds of 32 candidates, some 35 instructions each, and 200 to group the
+// row).  Grouping in shared memory takes the place of a second pass that read and rewrote every row.
 __global__ void __launch_bounds__(128) k_build_list(
     const float4* __restrict__ pos, const uint8_t* __restrict__ sysid, const SysParams* __restrict__ sp,
-    const uint32_t* __restrict__ cell_of, const uint32_t* __restrict__ start, uint32_t N, uint32_t cap,
-    float rmax2, uint32_t* __restrict__ nl, uint32_t* __restrict__ nl_cnt, uint32_t* __restrict__ flags) {
-  uint32_t k = blockIdx.x * blockDim.x + threadIdx.x;
-  if (k >= N) return;
+    const uint32_t* __restrict__ start, uint32_t N, uint32_t cap, float rmax2, uint32_t* __restrict__ nl,
+    uint32_t* __restrict__ nl_cnt, uint4* __restrict__ shell_end, uint32_t* __restrict__ flags) {
+  extern __shared__ __align__(16) uint32_t sm[];
+  const uint32_t wib = threadIdx.x >> 5, lane = threadIdx.x & 31u, lt = (1u << lane) - 1u;
+  uint32_t* row = sm + (size_t)wib * (cap + kWalkWords);   // cap is a multiple of 8
+  const uint32_t k = blockIdx.x * (blockDim.x >> 5) + wib;
+  if (k >= N) return;   // whole warps
   const SysParams& P = sp[sysid[k]];
-  const Shells sh = Shells::of(rmax2, P.list_range);
   const float4 xi = pos[k];
   const float box[3] = {P.box[0], P.box[1], P.box[2]};
   const float inv[3] = {P.inv_box[0], P.inv_box[1], P.inv_box[2]};
   const float lr = P.list_range;
-  // fast squared distance decides unless it lies within 1e-5 of the range, where the exact
-  // reference arithmetic decides (the minimum image cannot differ there: range < box/2)
-  const float lr2_lo = lr * lr * (1.0f - 1e-5f), lr2_hi = lr * lr * (1.0f + 1e-5f);
-  uint32_t c = cell_of[k] - P.cell_off;
-  int qx = (int)(c % (uint32_t)P.dims[0]);
-  int qy = (int)((c / (uint32_t)P.dims[0]) % (uint32_t)P.dims[1]);
-  int qz = (int)(c / ((uint32_t)P.dims[0] * (uint32_t)P.dims[1]));
-  const int R = P.walk;
-  AxisRange ax = axis_ranges(qx, R, P.dims[0]);
-  // distinct y and z coordinates in walk order
-  int ys[16], zs[16], ny = 0, nz = 0;
-  for (int d = -R; d <= R; ++d) {
-    int y = ((qy + d) % P.dims[1] + P.dims[1]) % P.dims[1];
-    bool dup = false;
-    for (int t = 0; t < ny; ++t) dup |= ys[t] == y;
-    if (!dup) ys[ny++] = y;
-    int z = ((qz + d) % P.dims[2] + P.dims[2]) % P.dims[2];
-    dup = false;
-    for (int t = 0; t < nz; ++t) dup |= zs[t] == z;
-    if (!dup) zs[nz++] = z;
-  }
-  uint32_t cnt = 0;
-  uint32_t* row = nl + (size_t)k * cap;
-  // a warp whose particles lie at least the list range inside every face screens with plain
-  // differences: a candidate within the range sits at its stored coordinates (fast_mi would return the
-  // same difference), and one beyond it by the plain difference is beyond it by the minimum image too
-  const float rm = lr * (1.0f + 1e-5f) + 1e-3f;
-  const bool direct = __all_sync(__activemask(), xi.x >= rm && xi.x <= box[0] - rm && xi.y >= rm &&
-                                                   xi.y <= box[1] - rm && xi.z >= rm && xi.z <= box[2] - rm);
-  auto take = [&](uint32_t a, uint32_t e) {
-    for (uint32_t j = a; j < e; ++j) {
-      if (j == k) continue;
-      const float4 xj = pos[j];
-      float dx = xi.x - xj.x, dy = xi.y - xj.y, dz = xi.z - xj.z;
-      if (!direct) {
-        dx = fast_mi(dx, box[0], inv[0]);
-        dy = fast_mi(dy, box[1], inv[1]);
-        dz = fast_mi(dz, box[2], inv[2]);
-      }
-      const float r2 = dx * dx + dy * dy + dz * dz;
-      if (r2 > lr2_hi) continue;
-      if (r2 >= lr2_lo && !(ex_dist(xi, xj, box) < lr)) continue;
-      if (cnt < cap) row[cnt] = j | sh.tag(r2);
-      ++cnt;
-    }
-  };
-  if (P.dims[0] >= 2 * R + 1 && P.dims[1] >= 2 * R + 1 && P.dims[2] >= 2 * R + 1) {
-    const float cs[3] = {box[0] / (float)P.dims[0], box[1] / (float)P.dims[1], box[2] / (float)P.dims[2]};
-    const float lrm = lr * (1.0f + 1e-5f) + 1e-3f, lrm2 = lrm * lrm;
-    for (int oz = -R; oz <= R; ++oz) {
-      const float gz = gap_to_cell(xi.z, qz + oz, cs[2]);
-      const int cz = (qz + oz + P.dims[2]) % P.dims[2];
-      for (int oy = -R; oy <= R; ++oy) {
-        const float gy = gap_to_cell(xi.y, qy + oy, cs[1]);
-        const float g2 = gy * gy + gz * gz;
-        if (g2 >= lrm2) continue;
-        const float ext = sqrtf(lrm2 - g2);
-        const int xlo = max(qx - R, (int)floorf((xi.x - ext) / cs[0]));
-        const int xhi = min(qx + R, (int)floorf((xi.x + ext) / cs[0]));
-        if (xlo > xhi) continue;
-        const int cy = (qy + oy + P.dims[1]) % P.dims[1];
-        const uint32_t rowbase = P.cell_off + (uint32_t)(P.dims[0] * (cy + P.dims[1] * cz));
-        const AxisRange xr = span_ranges(xlo, xhi, P.dims[0]);
-        for (int sgi = 0; sgi < xr.n; ++sgi) take(start[rowbase + xr.lo[sgi]], start[rowbase + xr.hi[sgi] + 1]);
-      }
-    }
-    if (cnt > cap) { flags[0] = 1u; cnt = cap; }
-    nl_cnt[k] = cnt;
-    return;
-  }
-  for (int iz = 0; iz < nz; ++iz) {
-    for (int iy = 0; iy < ny; ++iy) {
-      uint32_t rowbase = P.cell_off + (uint32_t)(P.dims[0] * (ys[iy] + P.dims[1] * zs[iz]));
-      for (int s = 0; s < ax.n; ++s) {
-        uint32_t a = start[rowbase + ax.lo[s]], e = start[rowbase + ax.hi[s] + 1];
-        for (uint32_t j = a; j < e; ++j) {
-          if (j == k) continue;
-          const float4 xj = pos[j];
-          const float dx = fast_mi(xi.x - xj.x, box[0], inv[0]);
-          const float dy = fast_mi(xi.y - xj.y, box[1], inv[1]);
-          const float dz = fast_mi(xi.z - xj.z, box[2], inv[2]);
-          const float r2 = dx * dx + dy * dy + dz * dz;
-          if (r2 > lr2_hi) continue;
-          if (r2 >= lr2_lo && !(ex_dist(xi, xj, box) < lr)) continue;
-          if (cnt < cap) row[cnt] = j | sh.tag(r2);
-          ++cnt;
-        }
-      }
-    }
-  }
-  if (cnt > cap) { flags[0] = 1u; cnt = cap; }
-  nl_cnt[k] = cnt;
-}
-
-// The same list build with the neighbour cells staged, for replicas whose walk does not wrap onto
-// itself (every grid side at least 2 walk + 1 cells).  A group of 8 lanes takes one cell; its lanes
-// hold up to 8 of the cell's particles at a time.  The group walks the cell's neighbour rows in
-// k_build_list's order (z, then y, then the x cells of the row as at most two wrapped segments) and
-// stages each segment 8 particles at a time in shared memory, shifted by the periodic image of the
-// segment, so that the separation is a plain difference; every lane then tests the 8 staged beads
-// against its particle.  A particle's accepted neighbours therefore come in k_build_list's order and
-// pass its test (the fast squared distance away from the range, the exact reference arithmetic on
-// the unshifted positions within 1e-5 of it), and the rows are the same lists.  Four groups in a warp
-// take four consecutive cells of one x row, whose neighbour rows coincide.
-constexpr int kGroup = 8;
-constexpr int kGBlock = 128;
-__global__ void __launch_bounds__(kGBlock) k_build_list_cells(
-    const float4* __restrict__ pos, const SysParams* __restrict__ sp, const uint8_t* __restrict__ cell_sys,
-    const uint32_t* __restrict__ start, uint32_t ncells, uint32_t cap, float rmax2, uint32_t* __restrict__ nl,
-    uint32_t* __restrict__ nl_cnt, uint32_t* __restrict__ flags) {
-  __shared__ float4 stage[kGBlock];
-  // every loop below runs the same trip count on the whole warp (the maximum over its four groups,
-  // with the shorter groups predicated off): groups that branched apart would run one after another
-  const uint32_t cg = (blockIdx.x * blockDim.x + threadIdx.x) / kGroup;
-  const bool have = cg < ncells;
-  const uint32_t c = have ? cg : 0u;
-  const uint32_t l8 = threadIdx.x & (kGroup - 1);
-  float4* st = stage + (threadIdx.x & ~(kGroup - 1));
-  const SysParams& P = sp[cell_sys[c]];
-  const float bx = P.box[0], by = P.box[1], bz = P.box[2];
-  const float lr = P.list_range;
-  const float lr2_lo = lr * lr * (1.0f - 1e-5f), lr2_hi = lr * lr * (1.0f + 1e-5f);
   const Shells sh = Shells::of(rmax2, lr);
-  const uint32_t cl = c - P.cell_off;
-  const int dx = P.dims[0], dy = P.dims[1], dz = P.dims[2];
-  const int qx = (int)(cl % (uint32_t)dx), qy = (int)((cl / (uint32_t)dx) % (uint32_t)dy),
-            qz = (int)(cl / ((uint32_t)dx * (uint32_t)dy));
-  const int R = P.walk;
-  // the row's x cells as at most two wrapped segments, in axis_ranges' order (qx - R .. qx + R does
-  // not wrap onto itself here), and the image shift of each: cells wrapped round a face sit one box
-  // beyond it
-  const bool wrap_lo = qx - R < 0, wrap_hi = qx + R >= dx;
-  const int nseg = (wrap_lo || wrap_hi) ? 2 : 1;
-  const int s0lo = wrap_lo ? qx - R + dx : qx - R, s0hi = (wrap_lo || wrap_hi) ? dx - 1 : qx + R;
-  const int s1hi = wrap_lo ? qx + R : qx + R - dx;
-  const float xs0 = wrap_lo ? -bx : 0.f;
-  const float xs1 = wrap_hi ? bx : 0.f;
-  const uint32_t a_i = have ? start[c] : 0u, e_i = have ? start[c + 1] : 0u;
-  const uint32_t nib = __reduce_max_sync(0xffffffffu, (e_i - a_i + kGroup - 1) / kGroup);
-  for (uint32_t ib = 0; ib < nib; ++ib) {
-    const uint32_t k = a_i + ib * kGroup + l8;
-    const bool mine = k < e_i;
-    const float4 xi = mine ? pos[k] : make_float4(0.f, 0.f, 0.f, 0.f);
-    uint32_t cnt = 0;
-    uint32_t* row = nl + (size_t)(mine ? k : 0u) * cap;
-    // R is the replica's walk; a warp spans one x row of one replica, so every bound is warp-uniform
-    for (int oz = -R; oz <= R; ++oz) {
-      const int z = qz + oz;
-      const int cz = (z + dz) % dz;
-      const float sz = z < 0 ? -bz : (z >= dz ? bz : 0.f);
-      for (int oy = -R; oy <= R; ++oy) {
-        const int y = qy + oy;
-        const int cy = (y + dy) % dy;
-        const float sy = y < 0 ? -by : (y >= dy ? by : 0.f);
-        const uint32_t rowbase = P.cell_off + (uint32_t)(dx * (cy + dy * cz));
-#pragma unroll
-        for (int sgi = 0; sgi < 2; ++sgi) {
-          uint32_t a = 0, len = 0;
-          if (have && sgi < nseg) {
-            a = start[rowbase + (sgi == 0 ? s0lo : 0)];
-            len = start[rowbase + (sgi == 0 ? s0hi : s1hi) + 1] - a;
-          }
-          const float xs = sgi == 0 ? xs0 : xs1;
-          const uint32_t mlen = __reduce_max_sync(0xffffffffu, len);
-          for (uint32_t t0 = 0; t0 < mlen; t0 += kGroup) {
-            if (t0 + l8 < len) {
-              const uint32_t j = a + t0 + l8;
-              const float4 p = pos[j];
-              st[l8] = make_float4(p.x + xs, p.y + sy, p.z + sz, __uint_as_float(j));
-            }
-            __syncwarp();
-#pragma unroll
-            for (uint32_t u = 0; u < (uint32_t)kGroup; ++u) {
-              const float4 q = st[u];
-              const uint32_t jj = __float_as_uint(q.w);
-              const float ddx = xi.x - q.x, ddy = xi.y - q.y, ddz = xi.z - q.z;
-              const float r2 = ddx * ddx + ddy * ddy + ddz * ddz;
-              if (!mine || t0 + u >= len || jj == k || r2 > lr2_hi) continue;
-              if (r2 >= lr2_lo) {
-                const float4 pj = pos[jj];
-                const float ex = ex_len(ex_mi(__fsub_rn(xi.x, pj.x), bx), ex_mi(__fsub_rn(xi.y, pj.y), by),
-                                        ex_mi(__fsub_rn(xi.z, pj.z), bz));
-                if (!(ex < lr)) continue;
-              }
-              if (cnt < cap) row[cnt] = jj | sh.tag(r2);
-              ++cnt;
-            }
-            __syncwarp();
-          }
-        }
-      }
+  const float lr2_lo = lr * lr * (1.0f - 1e-5f), lr2_hi = lr * lr * (1.0f + 1e-5f);
+  // a particle at least the list range inside every face screens with plain differences: a candidate within
+  // the range sits at its stored coordinates, and one beyond it by the plain difference is beyond it by
+  // the minimum image too
+  const float rm = lr * (1.0f + 1e-5f) + 1e-3f;
+  const bool direct = xi.x >= rm && xi.x <= box[0] - rm && xi.y >= rm && xi.y <= box[1] - rm && xi.z >= rm &&
+                      xi.z <= box[2] - rm;
+  const WalkGrid G{{P.dims[0], P.dims[1], P.dims[2]}, P.walk, P.cell_off, lr};
+  uint32_t cnt = 0;
+  auto test = [&](uint32_t j, bool v, const float4& xj) -> uint32_t {   // the tagged entry, or NONE
+    float dx = xi.x - xj.x, dy = xi.y - xj.y, dz = xi.z - xj.z;
+    if (!direct) {
+      dx = fast_mi(dx, box[0], inv[0]);
+      dy = fast_mi(dy, box[1], inv[1]);
+      dz = fast_mi(dz, box[2], inv[2]);
     }
-    if (mine) {
-      if (cnt > cap) { flags[0] = 1u; cnt = cap; }
-      nl_cnt[k] = cnt;
-    }
+    const float r2 = dx * dx + dy * dy + dz * dz;
+    bool in = v && j != k && r2 <= lr2_hi;
+    if (in && r2 >= lr2_lo) in = ex_dist(xi, xj, box) < lr;
+    return in ? (j | sh.tag(r2)) : SOUP_NONE_U32;
+  };
+  auto put = [&](uint32_t e) {
+    const bool in = e != SOUP_NONE_U32;
+    const uint32_t m = __ballot_sync(0xffffffffu, in);
+    const uint32_t at = cnt + __popc(m & lt);
+    if (in && at < cap) row[at] = e;
+    cnt += __popc(m);
+  };
+  warp_walk(xi, box, G, start, row + cap, [&](uint32_t j0, bool v0, uint32_t j1, bool v1) {
+    const float4 x0 = pos[j0], x1 = pos[j1];
+    const uint32_t e0 = test(j0, v0, x0), e1 = test(j1, v1, x1);
+    put(e0);
+    put(e1);
+  });
+  if (cnt > cap) {
+    if (lane == 0) flags[0] = 1u;
+    cnt = cap;
   }
-}
-
-// Group every row by build-distance shell, strip the tags, and record where shells 0..3 end.  A warp
-// per row.  A row of up to 32 * kGRegs entries is read in one go into registers, lane l holding
-// entries l, l + 32, ..; each lane counts its entries per shell (five 12-bit fields of one 64-bit word:
-// a row holds fewer than 4096 entries), one warp scan of those words gives every lane the place of its
-// entries, and each shell receives its entries lane by lane (lane 0's first, each lane's in row order),
-// a deterministic order.  A longer row (dense aggregates) is grouped in shared memory, shell by shell
-// with ballots, keeping the build's order inside a shell.
-constexpr uint32_t kGRegs = 16;
-__device__ __forceinline__ uint32_t field12(unsigned long long w, uint32_t t) {
-  return (uint32_t)(w >> (12u * t)) & 0xFFFu;
-}
-__global__ void k_group_rows(uint32_t N, uint32_t cap, uint32_t* __restrict__ nl, const uint32_t* __restrict__ nl_cnt,
-                             uint4* __restrict__ shell_end) {
-  extern __shared__ uint32_t gbuf[];
-  const uint32_t wib = threadIdx.x >> 5, lane = threadIdx.x & 31u;
-  const uint32_t k = blockIdx.x * (blockDim.x >> 5) + wib;
-  if (k >= N) return;   // whole warps
-  uint32_t* row = nl + (size_t)k * cap;
-  const uint32_t cnt = min(nl_cnt[k], cap);
+  __syncwarp();
+  // group the row by shell.  Up to 32 * 16 entries: lane l holds a contiguous piece, counts its entries per
+  // shell (five 12-bit fields of one 64-bit word), one warp scan of those words gives every lane its places,
+  // and the pieces are written back in lane order.  A longer row (dense aggregates) goes out shell by
+  // shell with ballots.  Both keep the walk's order inside a shell.
+  uint32_t* out = nl + (size_t)k * cap;
   uint32_t e[4];
-  if (cnt <= 32u * kGRegs) {
+  if (cnt <= 32u * (kGRegs - 1u)) {
+    const uint32_t piece = ((cnt + 31u) >> 5) | 1u;    // odd: no bank conflicts
+    const uint32_t s0 = lane * piece, s1 = min(s0 + piece, cnt);
     uint32_t v[kGRegs];
     unsigned long long mine = 0;
 #pragma unroll
     for (uint32_t c = 0; c < kGRegs; ++c) {
-      const uint32_t s = 32u * c + lane;
-      v[c] = s < cnt ? row[s] : 0xFFFFFFFFu;
+      if (c >= piece) break;
+      v[c] = s0 + c < s1 ? row[s0 + c] : SOUP_NONE_U32;
+      if (v[c] != SOUP_NONE_U32) mine += 1ull << (12u * (v[c] >> 29));
     }
-#pragma unroll
-    for (uint32_t c = 0; c < kGRegs; ++c)
-      if (v[c] != 0xFFFFFFFFu) mine += 1ull << (12u * (v[c] >> 29));
     unsigned long long incl = mine;
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
@@ -475,8 +399,7 @@ __global__ void k_group_rows(uint32_t N, uint32_t cap, uint32_t* __restrict__ nl
       if (lane >= (uint32_t)o) incl += y;
     }
     const unsigned long long tot = __shfl_sync(0xffffffffu, incl, 31);
-    // the shells' first places, packed like the counts
-    unsigned long long bases = 0;
+    unsigned long long bases = 0;                      // the shells' first places, packed like the counts
     uint32_t run = 0;
 #pragma unroll
     for (uint32_t t = 0; t < 5; ++t) {
@@ -484,35 +407,37 @@ __global__ void k_group_rows(uint32_t N, uint32_t cap, uint32_t* __restrict__ nl
       run += field12(tot, t);
       if (t < 4) e[t] = run;
     }
-    unsigned long long at = bases + (incl - mine);   // this lane's first place in every shell
-    __syncwarp();                                     // every lane has read its entries
+    unsigned long long at = bases + (incl - mine);     // this lane's next place in every shell
 #pragma unroll
     for (uint32_t c = 0; c < kGRegs; ++c) {
-      if (v[c] == 0xFFFFFFFFu) continue;
+      if (c >= piece) break;
+      if (v[c] == SOUP_NONE_U32) continue;
       const uint32_t t = v[c] >> 29;
       row[field12(at, t)] = v[c] & 0x1FFFFFFFu;
       at += 1ull << (12u * t);
     }
-  } else {
-    uint32_t* sb = gbuf + (size_t)wib * cap;
-    for (uint32_t s = lane; s < cnt; s += 32u) sb[s] = row[s];
     __syncwarp();
-    const uint32_t lt = (1u << lane) - 1u;
-    uint32_t out = 0;
+    for (uint32_t s = 4u * lane; s < cnt; s += 128u)   // rows are 32-byte aligned; the tail up to 4 is unread
+      *reinterpret_cast<uint4*>(out + s) = *reinterpret_cast<const uint4*>(row + s);
+  } else {
+    uint32_t o = 0;
 #pragma unroll
     for (uint32_t b = 0; b < 5; ++b) {
       for (uint32_t s0 = 0; s0 < cnt; s0 += 32u) {
         const uint32_t s = s0 + lane;
-        const uint32_t v = s < cnt ? sb[s] : 0xFFFFFFFFu;
+        const uint32_t v = s < cnt ? row[s] : SOUP_NONE_U32;
         const bool hit = (v >> 29) == b;
         const uint32_t m = __ballot_sync(0xffffffffu, hit);
-        if (hit) row[out + __popc(m & lt)] = v & 0x1FFFFFFFu;
-        out += __popc(m);
+        if (hit) out[o + __popc(m & lt)] = v & 0x1FFFFFFFu;
+        o += __popc(m);
       }
-      if (b < 4) e[b] = out;
+      if (b < 4) e[b] = o;
     }
   }
-  if (lane == 0) shell_end[k] = make_uint4(e[0], e[1], e[2], e[3]);
+  if (lane == 0) {
+    nl_cnt[k] = cnt;
+    shell_end[k] = make_uint4(e[0], e[1], e[2], e[3]);
+  }
 }
 
 // heads: bin into the coarse head grid (replica-local cells), deterministic order inside a cell
@@ -564,89 +489,47 @@ __global__ void k_head_gather_sorted(const uint32_t* __restrict__ hsorted, uint3
   xg[t] = make_float4(p.x, p.y, p.z, __uint_as_float(g));
 }
 
-// soup/wgsl/electrostatics-long.wgsl:31-56 head list at rc_es + skin, via the head grid, a warp per
-// head: lanes test 32 candidates at a time, hits are compacted with a ballot.  Entries are the
+// soup/wgsl/electrostatics-long.wgsl:31-56 head list at rc_es + skin, via the head grid, a warp per head
+// (warp_walk over the heads in head-cell order); hits are compacted with a ballot.  Entries are the
 // neighbours' HEAD indices (head_slot maps them to slots); membership uses the exact test near the
 // range, so the set equals the reference's.
-__global__ void __launch_bounds__(256) k_build_es_list(const uint32_t* __restrict__ head_sys, uint32_t H,
+__global__ void __launch_bounds__(128) k_build_es_list(const uint32_t* __restrict__ head_sys, uint32_t H,
                                                        const uint32_t* __restrict__ head_slot, const float4* __restrict__ pos,
-                                                       const SysParams* __restrict__ sp, const uint32_t* __restrict__ hcell_of,
-                                                       const uint32_t* __restrict__ hstart, const float4* __restrict__ hxg,
-                                                       uint32_t cap, uint32_t* __restrict__ es_nl, uint32_t* __restrict__ es_cnt,
+                                                       const SysParams* __restrict__ sp, const uint32_t* __restrict__ hstart,
+                                                       const float4* __restrict__ hxg, uint32_t cap,
+                                                       uint32_t* __restrict__ es_nl, uint32_t* __restrict__ es_cnt,
                                                        uint32_t* __restrict__ flags) {
-  const uint32_t h = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  const int lane = threadIdx.x & 31;
-  if (h >= H) return;   // warp-uniform
+  __shared__ __align__(16) uint32_t sm[4][kWalkWords];
+  const uint32_t wib = threadIdx.x >> 5, lane = threadIdx.x & 31u, lt = (1u << lane) - 1u;
+  const uint32_t h = blockIdx.x * 4u + wib;
+  if (h >= H) return;   // whole warps
   const SysParams& P = sp[head_sys[h]];
   const float4 xi = pos[head_slot[h]];
   const float box[3] = {P.box[0], P.box[1], P.box[2]};
   const float inv[3] = {P.inv_box[0], P.inv_box[1], P.inv_box[2]};
   const float lr = P.es_list_range;
   const float lo = lr * lr * (1.0f - 1e-5f), hi = lr * lr * (1.0f + 1e-5f);
-  const uint32_t c = hcell_of[h] - P.hcell_off;
-  const int q[3] = {(int)(c % (uint32_t)P.hdims[0]), (int)((c / (uint32_t)P.hdims[0]) % (uint32_t)P.hdims[1]),
-                    (int)(c / ((uint32_t)P.hdims[0] * (uint32_t)P.hdims[1]))};
-  const int R = P.hwalk;
-  int ax[3][8], na[3] = {0, 0, 0};
-  for (int a = 0; a < 3; ++a)
-    for (int d = -R; d <= R; ++d) {
-      int v = ((q[a] + d) % P.hdims[a] + P.hdims[a]) % P.hdims[a];
-      bool dup = false;
-      for (int t = 0; t < na[a]; ++t) dup |= ax[a][t] == v;
-      if (!dup) ax[a][na[a]++] = v;
-    }
+  const WalkGrid G{{P.hdims[0], P.hdims[1], P.hdims[2]}, P.hwalk, P.hcell_off, lr};
   uint32_t cnt = 0;
   uint32_t* row = es_nl + (size_t)h * cap;
-  const uint32_t lt = (1u << lane) - 1u;
-  auto scan_cell = [&](uint32_t cc) {
-    const uint32_t a0 = hstart[cc], e0 = hstart[cc + 1];
-    for (uint32_t b0 = a0; b0 < e0; b0 += 32) {
-      const uint32_t t = b0 + lane;
-      bool hit = false;
-      uint32_t g = 0;
-      if (t < e0) {
-        const float4 xj = hxg[t];
-        g = __float_as_uint(xj.w);
-        if (g != h) {
-          const float dx = fast_mi(xi.x - xj.x, box[0], inv[0]);
-          const float dy = fast_mi(xi.y - xj.y, box[1], inv[1]);
-          const float dz = fast_mi(xi.z - xj.z, box[2], inv[2]);
-          const float r2 = dx * dx + dy * dy + dz * dz;
-          hit = r2 < lo || (r2 <= hi && ex_dist(xi, xj, box) < lr);
-        }
-      }
-      const uint32_t m = __ballot_sync(0xffffffffu, hit);
-      if (hit) {
-        const uint32_t at = cnt + __popc(m & lt);
-        if (at < cap) row[at] = g;
-      }
-      cnt += __popc(m);
-    }
+  auto put = [&](const float4& xj, bool v) {
+    const uint32_t g = __float_as_uint(xj.w);
+    const float dx = fast_mi(xi.x - xj.x, box[0], inv[0]);
+    const float dy = fast_mi(xi.y - xj.y, box[1], inv[1]);
+    const float dz = fast_mi(xi.z - xj.z, box[2], inv[2]);
+    const float r2 = dx * dx + dy * dy + dz * dz;
+    bool hit = v && g != h && r2 <= hi;
+    if (hit && r2 >= lo) hit = ex_dist(xi, xj, box) < lr;
+    const uint32_t m = __ballot_sync(0xffffffffu, hit);
+    const uint32_t at = cnt + __popc(m & lt);
+    if (hit && at < cap) row[at] = g;
+    cnt += __popc(m);
   };
-  if (P.hdims[0] >= 2 * R + 1 && P.hdims[1] >= 2 * R + 1 && P.hdims[2] >= 2 * R + 1) {
-    // the walk does not wrap onto itself: cells wholly beyond the list sphere (with a margin) are
-    // skipped, which leaves the list the same set
-    const float cs[3] = {box[0] / (float)P.hdims[0], box[1] / (float)P.hdims[1], box[2] / (float)P.hdims[2]};
-    const float lrm = lr * (1.0f + 1e-5f) + 1e-3f, lrm2 = lrm * lrm;
-    for (int oz = -R; oz <= R; ++oz) {
-      const float gz = gap_to_cell(xi.z, q[2] + oz, cs[2]);
-      for (int oy = -R; oy <= R; ++oy) {
-        const float gy = gap_to_cell(xi.y, q[1] + oy, cs[1]);
-        for (int ox = -R; ox <= R; ++ox) {
-          const float gx = gap_to_cell(xi.x, q[0] + ox, cs[0]);
-          if (gx * gx + gy * gy + gz * gz >= lrm2) continue;
-          const int cx = (q[0] + ox + P.hdims[0]) % P.hdims[0], cy = (q[1] + oy + P.hdims[1]) % P.hdims[1],
-                    cz = (q[2] + oz + P.hdims[2]) % P.hdims[2];
-          scan_cell(P.hcell_off + (uint32_t)(cx + P.hdims[0] * (cy + P.hdims[1] * cz)));
-        }
-      }
-    }
-  } else {
-    for (int iz = 0; iz < na[2]; ++iz)
-      for (int iy = 0; iy < na[1]; ++iy)
-        for (int ix = 0; ix < na[0]; ++ix)
-          scan_cell(P.hcell_off + (uint32_t)(ax[0][ix] + P.hdims[0] * (ax[1][iy] + P.hdims[1] * ax[2][iz])));
-  }
+  warp_walk(xi, box, G, hstart, sm[wib], [&](uint32_t j0, bool v0, uint32_t j1, bool v1) {
+    const float4 x0 = hxg[j0], x1 = hxg[j1];
+    put(x0, v0);
+    put(x1, v1);
+  });
   if (lane == 0) {
     if (cnt > cap) { flags[1] = 1u; cnt = cap; }
     es_cnt[h] = cnt;
@@ -677,32 +560,23 @@ void launch_sort_and_gather(Batch& b) {
                                                       b.held2, b.brng2, b.trng2, b.frozen2, b.id2, b.pos, b.vel, b.force,
                                                       b.charge, b.slots, b.center, b.held, b.brng, b.trng, b.frozen,
                                                       b.id);
-  // the cell of every new slot: cell_start is monotone, so recompute from the sorted positions
-  cudaMemsetAsync(b.cell_count, 0, sizeof(uint32_t) * (b.ncells + 1), b.stream);
-  k_cell_index<<<nblocks(b.N), kBlock, 0, b.stream>>>(b.pos, b.sysid, b.sp, b.N, b.cell_of_slot, b.cell_count);
-  b.launches += 6 + scans;
+  b.launches += 4 + scans;
   prof_end(b);
 }
 
 void launch_build_lists(Batch& b) {
   b.launches += 1;
   prof_begin(b, SOUP_K_LIST);
-  if (b.list_by_cell && b.list_cells)
-    k_build_list_cells<<<nblocks((uint64_t)b.ncells * kGroup, kGBlock), kGBlock, 0, b.stream>>>(
-        b.pos, b.sp, b.cell_sys, b.cell_start, b.ncells, b.list_cap, b.hs.rmax2, b.nl, b.nl_cnt, b.flags);
-  else
-    k_build_list<<<nblocks(b.N, 128), 128, 0, b.stream>>>(b.pos, b.sysid, b.sp, b.cell_of_slot, b.cell_start, b.N,
-                                                          b.list_cap, b.hs.rmax2, b.nl, b.nl_cnt, b.flags);
-  // rows grouped by shell: four warps per block while four staged rows fit the shared memory
-  const uint32_t wpb = 16u * b.list_cap <= 200u * 1024u ? 4u : 1u;
-  const size_t smem = (size_t)wpb * b.list_cap * 4u;
-  if (smem > 48u * 1024u && b.group_smem_set < smem) {
-    SOUP_CUDA_TRY(cudaFuncSetAttribute(k_group_rows, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    b.group_smem_set = smem;
+  // a row of shared memory per warp: four warps per block while they fit
+  const size_t per = sizeof(uint32_t) * ((size_t)b.list_cap + kWalkWords);
+  const uint32_t wpb = 4u * per <= 200u * 1024u ? 4u : 1u;
+  const size_t smem = wpb * per;
+  if (smem > 48u * 1024u && b.list_smem_set < smem) {
+    SOUP_CUDA_TRY(cudaFuncSetAttribute(k_build_list, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    b.list_smem_set = smem;
   }
-  k_group_rows<<<(unsigned)((b.N + wpb - 1) / wpb), 32u * wpb, smem, b.stream>>>(b.N, b.list_cap, b.nl, b.nl_cnt,
-                                                                                b.nl_shell);
-  b.launches += 1;
+  k_build_list<<<(unsigned)((b.N + wpb - 1) / wpb), 32u * wpb, smem, b.stream>>>(
+      b.pos, b.sysid, b.sp, b.cell_start, b.N, b.list_cap, b.hs.rmax2, b.nl, b.nl_cnt, b.nl_shell, b.flags);
   prof_end(b);
 }
 
@@ -717,9 +591,8 @@ void launch_build_es_lists(Batch& b) {
   k_head_scatter<<<nblocks(b.H), kBlock, 0, b.stream>>>(b.hcell_of, b.hcell_start, b.H, b.hcell_cursor, b.hsorted);
   k_head_sort_cells<<<nblocks(b.nhcells), kBlock, 0, b.stream>>>(b.hcell_start, b.nhcells, b.hsorted);
   k_head_gather_sorted<<<nblocks(b.H), kBlock, 0, b.stream>>>(b.hsorted, b.H, b.head_slot, b.pos, b.hsorted_xg);
-  k_build_es_list<<<nblocks((uint64_t)b.H * 32, 256), 256, 0, b.stream>>>(b.head_sys, b.H, b.head_slot, b.pos, b.sp,
-                                                                         b.hcell_of, b.hcell_start, b.hsorted_xg,
-                                                                         b.es_cap, b.es_nl, b.es_cnt, b.flags);
+  k_build_es_list<<<nblocks(b.H, 4), 128, 0, b.stream>>>(b.head_sys, b.H, b.head_slot, b.pos, b.sp, b.hcell_start,
+                                                        b.hsorted_xg, b.es_cap, b.es_nl, b.es_cnt, b.flags);
   b.launches += 6 + scans;
   prof_end(b);
 }

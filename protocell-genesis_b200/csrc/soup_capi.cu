@@ -181,7 +181,7 @@ namespace {
 
 // ---- batch construction ----------------------------------------------------------------------
 void alloc_grids(Batch& b) {
-  dfree(b.cell_count); dfree(b.cell_start); dfree(b.cell_cursor); dfree(b.scan_tmp); dfree(b.cell_sys);
+  dfree(b.cell_count); dfree(b.cell_start); dfree(b.cell_cursor); dfree(b.scan_tmp);
   dfree(b.hcell_count); dfree(b.hcell_start); dfree(b.hcell_cursor);
   uint64_t nc = 0, nh = 0;
   for (uint32_t r = 0; r < b.R; ++r) {
@@ -196,17 +196,6 @@ void alloc_grids(Batch& b) {
   b.cell_count = dalloc<uint32_t>(nc + 1);
   b.cell_start = dalloc<uint32_t>(nc + 1);
   b.cell_cursor = dalloc<uint32_t>(nc + 1);
-  {
-    std::vector<uint8_t> cs((size_t)nc);
-    b.list_by_cell = true;
-    for (uint32_t r = 0; r < b.R; ++r) {
-      const SysParams& p = b.hsp[r];
-      std::fill(cs.begin() + p.cell_off, cs.begin() + p.cell_off + cells_of(p.dims), (uint8_t)r);
-      for (int a = 0; a < 3; ++a) b.list_by_cell = b.list_by_cell && p.dims[a] >= 2 * p.walk + 1;
-    }
-    b.cell_sys = dalloc<uint8_t>(nc);
-    SOUP_CUDA_TRY(cudaMemcpy(b.cell_sys, cs.data(), nc, cudaMemcpyHostToDevice));
-  }
   b.hcell_count = dalloc<uint32_t>(nh + 1);
   b.hcell_start = dalloc<uint32_t>(nh + 1);
   b.hcell_cursor = dalloc<uint32_t>(nh + 1);
@@ -443,7 +432,6 @@ Batch* make_batch(const SoupConfig* cfgs, const SoupInitState* inits, uint32_t R
   b.tpp = 4;
   if (const char* e = std::getenv("SOUP_TPP")) b.tpp = std::atoi(e);
   if (const char* e = std::getenv("SOUP_FORCE_QUEUED")) b.queued = std::atoi(e) != 0;
-  if (const char* e = std::getenv("SOUP_LIST_BY_CELL")) b.list_cells = std::atoi(e) != 0;
   if (const char* e = std::getenv("SOUP_FULL_ROWS")) b.prune = std::atoi(e) == 0;
   force_pass(b);   // priming pass (soup/src/sim.ts:396-408)
   SOUP_CUDA_TRY(cudaStreamSynchronize(b.stream));
@@ -466,7 +454,7 @@ void destroy_batch(Batch* b) {
   if (b->cap_stream) cudaStreamDestroy(b->cap_stream);
   void* ptrs[] = {b->rebuild_count, b->pos, b->vel, b->force, b->pos_ref, b->charge, b->slots, b->center, b->held, b->brng, b->trng,
                   b->frozen, b->id, b->slot_of, b->pos2, b->vel2, b->force2, b->charge2, b->slots2, b->center2,
-                  b->held2, b->brng2, b->trng2, b->frozen2, b->id2, b->cell_of_slot, b->cell_count, b->cell_start, b->cell_sys,
+                  b->held2, b->brng2, b->trng2, b->frozen2, b->id2, b->cell_of_slot, b->cell_count, b->cell_start,
                   b->cell_cursor, b->perm, b->scan_tmp, b->nl, b->nl_cnt, b->nl_shell, b->heads, b->head_sys, b->es_nl,
                   b->es_cnt, b->head_slot, b->head_e, b->head_pos, b->head_xq, b->head_d, b->head_flag, b->draw_site, b->sweep_band, b->hcell_count, b->hcell_start, b->hcell_cursor, b->hsorted, b->hsorted_xg, b->hcell_of, b->flags,
                   b->events, b->desorb, b->drift_bits, b->bond_items, b->bond_nitems, b->bond_sel, b->uf_parent, b->comp_min,
@@ -1451,27 +1439,18 @@ int soup_autotune(SoupHandle* h, uint32_t steps, SoupTuneResult* out) {
     b.tpp = (int)res.tpp;
     b.queued = res.queued != 0;
     drop_graphs(b);
-    // cell size (the list-walk radius: cell = list range / walk) and the list build (a thread per
-    // particle, or a group of lanes per cell), timed on the list build
+    // cell size (the list-walk radius: cell = list range / walk), timed on the list build and, as the walk
+    // sets the slot order the force gathers in, the ten force passes of a typical rebuild interval
     best = 1e30;
-    bool cells_best = false;
-    for (int w : {2, 3})
-      for (int lc = 0; lc < 2; ++lc) {
-        tune_plan(b, planned, w);
-        if (lc && !b.list_by_cell) continue;
-        b.list_cells = lc != 0;
-        force_pass(b);
-        // the walk sets the slot order the force gathers in: a rebuild and the ten force passes of a
-        // typical rebuild interval
-        const double ms = tune_time(b, 3, [&] {
-          launch_cell_index(b);
-          launch_build_lists(b);
-          for (int f = 0; f < 10; ++f) launch_force_list(b);
-        });
-        if (ms < best) { best = ms; res.walk = (uint32_t)w; cells_best = lc != 0; }
-      }
-    b.list_cells = cells_best;
-    res.list_cells = cells_best ? 1u : 0u;
+    for (int w : {2, 3}) {
+      tune_plan(b, planned, w);
+      force_pass(b);
+      const double ms = tune_time(b, 3, [&] {
+        launch_build_lists(b);
+        for (int f = 0; f < 10; ++f) launch_force_list(b);
+      });
+      if (ms < best) { best = ms; res.walk = (uint32_t)w; }
+    }
     // skin (drift-triggered rebuilds only): at most the planned one, which sized the list capacity;
     // timed on whole steps, rebuilds and sweeps included
     res.skin_scale = 1.0;
@@ -1512,7 +1491,6 @@ int soup_apply_tuning(SoupHandle* h, const SoupTuneResult* t) {
       fail(SOUP_E_ARG, "tuning: the skin can only be scaled with drift-triggered rebuilds");
     b.tpp = (int)t->tpp;
     b.queued = t->queued != 0;
-    b.list_cells = t->list_cells != 0;
     std::vector<double> sk(b.R);
     for (uint32_t r = 0; r < b.R; ++r) sk[r] = b.cfg[r].skin * t->skin_scale;
     tune_plan(b, sk, (int)t->walk);

@@ -144,6 +144,12 @@ struct PairP {
   }
 };
 
+// The width in r^2 of a list row's outer build-distance shells: shell 0 lies within the force's reach
+// (rmax2), shell s = 1..4 between rmax2 + (s - 1) w2 and rmax2 + s w2, where the list range ends.
+__device__ __forceinline__ float list_shell_width2(float rmax2, float list_range) {
+  return fmaxf(list_range * list_range - rmax2, 0.f) * 0.25f;
+}
+
 // The pair loop's constants of one replica, held in registers (batch-wide numbers from Shared, the
 // replica's acid-soap depth and screened-Coulomb numbers from its SysParams).
 struct PairLean {

@@ -13,7 +13,7 @@
 //   pos_ref float4 positions at the last rebuild (drift reference)
 //   nl     u32 [slot][list_cap] Verlet neighbours as SLOT indices; nl_cnt u32 [slot]; each row is
 //          grouped by build distance (shell 0: inside the force's reach; shells 1-4: the skin in four
-//          equal widths), nl_shell uint4 [slot] the ends of shells 0..3
+//          widths equal in r^2), nl_shell uint4 [slot] the ends of shells 0..3 (shell 4 ends at nl_cnt)
 //   heads  u32 original ids of titratable beads (ascending; static);  es_nl [head][es_cap] slots
 #pragma once
 #include <algorithm>
@@ -90,17 +90,14 @@ struct Batch {
   // grid + list
   uint32_t ncells = 0;               // total list-build cells over the batch
   uint32_t *cell_of_slot = nullptr, *cell_count = nullptr, *cell_start = nullptr, *cell_cursor = nullptr;
-  uint8_t* cell_sys = nullptr;       // replica of each list-build cell
-  bool list_by_cell = false;         // every replica's walk fits its grid: the cell-group build can run
-  bool list_cells = false;           // use it (the autotuner's choice; SOUP_LIST_BY_CELL=1)
   uint32_t* perm = nullptr;          // new slot -> old slot
   uint32_t* scan_tmp = nullptr;
   uint32_t list_cap = 0;             // row stride of nl (max over replicas, rounded to 32)
   uint32_t* nl = nullptr;
   uint32_t* nl_cnt = nullptr;
   uint4* nl_shell = nullptr;
-  size_t group_smem_set = 0;         // dynamic shared memory k_group_rows was opened to
-  bool prune = true;                 // force passes read only the shells the drift can have brought in range         // per slot: ends of the row's build-distance shells 0..3 (shell 4 ends at nl_cnt)
+  size_t list_smem_set = 0;          // dynamic shared memory k_build_list was opened to
+  bool prune = true;                 // force passes read only the shells the drift can have brought in range
 
   // heads / long-range electrostatics
   uint32_t H = 0;                    // total heads
