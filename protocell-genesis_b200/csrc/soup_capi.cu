@@ -135,6 +135,12 @@ SysParams make_sys(const SoupConfig& c) {
   grid_of(c.box, es ? c.es_list_range : c.list_range, p.hwalk, p.hdims);
   p.list_cap = c.list_capacity;
   p.es_cap = c.es_list_capacity;
+  // draws of a block of the walk: a round pulls, per draw, the flips among the earlier draws of its block that
+  // lie within the cutoff, so a cutoff that fills more of the box takes the smaller blocks (twice the handoffs).
+  // Measured, 512 against 256 draws: share 0.034 of the box 0.91 / 1.00 ms a sweep, 0.13 0.55 / 0.36 ms,
+  // 0.38 0.29 / 0.10 ms
+  const double vol = c.wall_radius > 0 ? c.wall_radius * c.wall_radius * c.wall_radius : c.box[0] * c.box[1] * c.box[2] / 4.18879;
+  p.sweep_draws = es && c.es_cutoff * c.es_cutoff * c.es_cutoff < 0.06 * vol ? 512u : 256u;
   p.charged_kind = c.charged_kind;
   p.d_A = es ? c.es_coeff_a : 0.0; p.d_kappa = c.es_kappa; p.d_rc = c.es_cutoff; p.d_shiftU = c.es_shift_u;
   p.d_shiftF = c.es_shift_f; p.d_pka = c.pka_intrinsic; p.d_ph = c.ph; p.d_kT = c.kT; p.d_q = c.charge_deprotonated;
@@ -414,9 +420,9 @@ Batch* make_batch(const SoupConfig* cfgs, const SoupInitState* inits, uint32_t R
   b.head_e = dalloc<long long>(b.H);
   b.head_pos = dalloc<float4>(b.H);
   b.head_xq = dalloc<float4>(b.H);
-  b.head_flag = dalloc<uint8_t>(b.H);
-  b.draw_site = dalloc<uint32_t>(std::max<size_t>(sweep_draw_sites(b), 1));
-  b.sweep_band = dalloc<long long>(std::max<size_t>(sweep_band_rows(b) * 64, 1));
+  b.draw_site = dalloc<uint32_t>(sweep_draws(b)); b.pair_cnt = dalloc<uint32_t>(sweep_draws(b));
+  b.walk_shared = dalloc<char>(sweep_shared_bytes(b));
+  b.pair_idx = dalloc<uint16_t>(sweep_pairs(b)); b.pair_del = dalloc<long long>(sweep_pairs(b));
   sweep_prepare(b);
   b.es_nl = dalloc<uint32_t>((size_t)b.H * std::max<uint32_t>(b.es_cap, 1)); b.es_cnt = dalloc<uint32_t>(b.H);
   b.head_d = dalloc<long long>((size_t)b.H * std::max<uint32_t>(b.es_cap, 1));
@@ -456,7 +462,7 @@ void destroy_batch(Batch* b) {
                   b->frozen, b->id, b->slot_of, b->pos2, b->vel2, b->force2, b->charge2, b->slots2, b->center2,
                   b->held2, b->brng2, b->trng2, b->frozen2, b->id2, b->cell_of_slot, b->cell_count, b->cell_start,
                   b->cell_cursor, b->perm, b->scan_tmp, b->nl, b->nl_cnt, b->nl_shell, b->heads, b->head_sys, b->es_nl,
-                  b->es_cnt, b->head_slot, b->head_e, b->head_pos, b->head_xq, b->head_d, b->head_flag, b->draw_site, b->sweep_band, b->hcell_count, b->hcell_start, b->hcell_cursor, b->hsorted, b->hsorted_xg, b->hcell_of, b->flags,
+                  b->es_cnt, b->head_slot, b->head_e, b->head_pos, b->head_xq, b->head_d, b->draw_site, b->pair_cnt, b->pair_idx, b->pair_del, b->walk_shared, b->hcell_count, b->hcell_start, b->hcell_cursor, b->hsorted, b->hsorted_xg, b->hcell_of, b->flags,
                   b->events, b->desorb, b->drift_bits, b->bond_items, b->bond_nitems, b->bond_sel, b->uf_parent, b->comp_min,
                   b->item_done, b->has_item, b->sweep_out, b->prot_rng_dev, b->sp, b->shared, b->sysid, b->an_buf[0],
                   b->an_buf[1]};
@@ -560,7 +566,7 @@ void sweep_all(Batch& b, std::vector<SoupSweepResult>* out) {
   SOUP_CUDA_TRY(cudaStreamSynchronize(b.stream));
   for (uint32_t r = 0; r < b.R; ++r)
     if (so[4 * r] < 0)
-      fail(SOUP_E_TIMEOUT, "constant-pH sweep: a handoff between the cluster's CTAs did not arrive within its "
+      fail(SOUP_E_TIMEOUT, "constant-pH sweep: a handoff between the walk's CTAs did not arrive within its "
                            "poll limit; the charges of this sweep are not valid");
   b.sweeps++;
   if (out) {
@@ -1509,7 +1515,7 @@ int soup_protonation_sweep(SoupHandle* h, SoupSweepResult* out) {
     force_pass(b);
     SOUP_CUDA_TRY(cudaStreamSynchronize(b.stream));
     if (so[0] < 0)
-      fail(SOUP_E_TIMEOUT, "constant-pH sweep: a handoff between the cluster's CTAs did not arrive within its "
+      fail(SOUP_E_TIMEOUT, "constant-pH sweep: a handoff between the walk's CTAs did not arrive within its "
                            "poll limit; the charges of this sweep are not valid");
     b.sweeps++;
     b.next_sweep[r] = b.step[r] + b.cfg[r].sweep_every;

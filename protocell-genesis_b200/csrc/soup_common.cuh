@@ -39,6 +39,7 @@ struct SysParams {
   int hwalk;                 // head-grid walk radius (cells)
   uint32_t hcell_off;
   uint32_t list_cap, es_cap; // capacities (overflow threshold)
+  uint32_t sweep_draws;      // draws of a block of the constant-pH walk: 512 or 256
   uint32_t es_on;            // electrostatics enabled
   int32_t charged_kind;
   // FP64 host-style numbers for the constant-pH sweep

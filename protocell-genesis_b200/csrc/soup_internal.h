@@ -105,13 +105,16 @@ struct Batch {
   uint32_t* head_sys = nullptr;      // replica of each head
   uint32_t* head_slot = nullptr;     // current slot of each head (refreshed at every rebuild)
   long long* head_e = nullptr;       // constant-pH site energy per head, fixed point 2^-40 (sweep scratch)
-  float4* head_pos = nullptr;        // head positions gathered for the sweep
+  float4* head_pos = nullptr;        // head positions and charges gathered for the sweep
   float4* head_xq = nullptr;         // head positions and charges by head index, for the far half
   long long* head_d = nullptr;       // [head][es_cap] change of a list neighbour's energy when the head
                                      // deprotonates, fixed point 2^-40 (sweep scratch)
-  uint8_t* head_flag = nullptr;      // charge state per head when the sweep cannot keep it in shared memory
   uint32_t* draw_site = nullptr;     // the site each draw of a sweep's stream selects (sweep scratch)
-  long long* sweep_band = nullptr;   // [draw][64] changes of the next 63 draws' site energies (sweep scratch)
+  uint32_t* pair_cnt = nullptr;      // per draw: the earlier draws of its block with a site near its own
+  uint16_t* pair_idx = nullptr;      // [block][entry][place] which (k_sweep_pairs)
+  long long* pair_del = nullptr;     // [block][entry][place] the change of the draw's site energy when that one flips
+  void* walk_shared = nullptr;       // per replica: what the CTAs of a walk share (WalkShared)
+  int sms = 0;                       // of the device
   uint32_t es_cap = 0;
   uint32_t* es_nl = nullptr;
   uint32_t* es_cnt = nullptr;
@@ -223,9 +226,10 @@ void launch_nonfinite(Batch& b);
 void launch_relax_step(Batch& b, float d);
 void launch_bonds(Batch& b);
 void launch_sweep(Batch& b, uint32_t replica);
-size_t sweep_band_rows(const Batch& b);
+size_t sweep_shared_bytes(const Batch& b);
+size_t sweep_pairs(const Batch& b);   // entries of the sweep's pair arrays
 uint32_t sweep_max_heads();   // heads one replica may hold for the device constant-pH sweep
-size_t sweep_draw_sites(const Batch& b);
+size_t sweep_draws(const Batch& b);   // draws of every replica, in whole blocks
 void adj_unpermute(Batch& b, float4* dst);
 void adj_scatter_pos(Batch& b, const float4* src);
 void adj_hvp(Batch& b, const float4* g, float4* jg, double* partial_dev);
