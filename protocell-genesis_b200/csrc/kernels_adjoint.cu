@@ -325,7 +325,7 @@ void adj_hvp(Batch& b, const float4* g, float4* jg, double* partial_dev) {
   const unsigned g2 = b.H ? nblocks((uint64_t)b.H * 32, kBlock) : 0;
   b.launches += 1 + (g2 ? 1 : 0);
   k_hvp<<<g1, kBlock, 0, b.stream>>>(b.shared, b.sp, b.sysid, b.N, b.pos, b.charge, b.slots, b.center, b.id, b.slot_of,
-                                     b.nl, b.nl_cnt, b.list_cap, g, jg, partial_dev);
+                                     b.nl, b.nl_cnt, b.list_stride, g, jg, partial_dev);
   if (g2)
     k_hvp_far<<<g2, kBlock, 0, b.stream>>>(b.sp, b.head_slot, b.head_sys, b.H, b.pos, b.charge, b.id, b.es_nl,
                                            b.es_cnt, b.es_cap, g, jg, partial_dev + (size_t)g1 * SOUP_DIFF_NPARAM);

@@ -468,7 +468,7 @@ void launch_bonds(Batch& b) {
   k_bond_select<<<nblocks(b.N, 256), 256, 0, b.stream>>>(b.shared, b.N, b.pos, b.center, b.bond_sel,
                                                          b.bond_nitems + 2);
   k_bond_walk<<<nblocks(b.N, 128), 128, 0, b.stream>>>(b.shared, b.sp, b.sysid, b.bond_sel, b.bond_nitems + 2, b.pos,
-                                                       b.id, b.slots, b.center, b.nl, b.nl_cnt, b.list_cap, b.brng,
+                                                       b.id, b.slots, b.center, b.nl, b.nl_cnt, b.list_stride, b.brng,
                                                        b.bond_items, b.bond_nitems, has_item);
   cudaMemcpyAsync(b.bond_nitems + 1, b.bond_nitems, sizeof(uint32_t), cudaMemcpyDeviceToDevice, b.stream);
   k_bond_partners<<<std::max(1u, std::min(nblocks(b.N, 256) / 8u, 592u)), 256, 0, b.stream>>>(

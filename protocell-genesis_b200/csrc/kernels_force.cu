@@ -5,17 +5,11 @@
 // nonbondedSoup), soup/wgsl/step.wgsl:152-193 bondedForce, soup/wgsl/electrostatics-long.wgsl:63-103
 // (far half, accumulated), soup/wgsl/wall.wgsl:42-56 (wall, accumulated), step.wgsl:277-292 brute.
 //
-// TPP threads cooperate on one particle: lane t takes list entries t, t+TPP, ... and bonded terms
-// t, t+TPP, ...; the group reduces with shuffles and lane 0 writes the force.  No atomics: every
-// particle's force is produced by exactly one group (full list, no Newton-3), so the sum order is
-// fixed and the result is run-to-run deterministic.
+// TPP threads (4, 8 or 16) cooperate on one particle.  A particle's force is summed in sixteen partial sums:
+// list entry e and bonded term t go to sums e mod 16 and t, each in ascending order, and the sums are added
+// in a fixed tree, so the result is the same bits for every TPP and run to run.  No atomics: every
+// particle's force is produced by exactly one group (full list, no Newton-3).
 #include "soup_internal.h"
-
-// four 256-thread blocks per SM (64 registers): the force is latency-bound on its gathers, and the
-// fourth block hides more of it than the registers it costs (a few bytes of spill)
-#ifndef SOUP_FORCE_MINB
-#define SOUP_FORCE_MINB 4
-#endif
 
 namespace soup {
 
@@ -52,275 +46,166 @@ __device__ __forceinline__ void bonded_term(const Shared& S, const SysParams& P,
 }
 
 // The end of the part of particle k's row a force pass must read.  The row is grouped by build
-// distance (k_build_list): shell 0 within the force's reach r0 = sqrt(rmax2), shells 1..4 the rest of the
-// list range in four widths w2 of r^2.  No bead has moved more than dm since the build (the replica's largest
+// distance (k_build_list): shell 0 within the force's reach r0 (a plain bead's or a wide one's, list_wide), shells
+// 1..7 the rest of the list range in widths w2 of r^2.  No bead has moved more than dm since the build (the replica's largest
 // drift), so a pair of shell s is at least sqrt(r0^2 + (s - 1) w2) - 2 dm apart now, and shell s can hold
 // an in-range pair only if r0^2 + (s - 1) w2 < (r0 + 2 dm)^2 (a margin of 1e-3 sigma covers rounding).
 // Skipped entries are beyond the reach, so the force is the same bits as over the whole row.
 __device__ __forceinline__ uint32_t list_force_end(uint32_t k, const uint32_t* __restrict__ nl_cnt,
-                                                   const uint4* __restrict__ nl_shell, float drift2, float rmax2,
-                                                   float list_range) {
-  const uint32_t cnt = nl_cnt[k];
-  const float w2 = list_shell_width2(rmax2, list_range);
-  if (!nl_shell || !(drift2 >= 0.f && drift2 < 1e30f) || !(w2 > 0.f)) return cnt;
+                                                   const uint32_t* __restrict__ nl_shell, float drift2,
+                                                   const SysParams& P, bool wide) {
+  const float scale = P.shell_scale[wide];
+  if (!nl_shell || !(drift2 >= 0.f && drift2 < 1e30f) || !(scale > 0.f)) return nl_cnt[k];
   const float d = 2.0f * sqrtf(drift2) + 1e-3f;
-  const float x = d * (2.0f * sqrtf(rmax2) + d) / w2;   // (r0 + d)^2 - r0^2 in shells
-  if (x >= 3.0f) return cnt;
-  const uint4 e = nl_shell[k];
-  return x < 1.0f ? e.y : (x < 2.0f ? e.z : e.w);
+  const float x = d * (2.0f * P.reach[wide] + d) * scale;   // (r0 + d)^2 - r0^2 in shells
+  return nl_shell[(size_t)kShells * k + 1u + (uint32_t)fminf(x, (float)(kShells - 2))];
 }
 
+// One group's pass over its particle's row up to `end`: four entries a lane and iteration, the next
+// iteration's indices loaded before this one's pairs.  Rows are padded to 16 entries with the particle
+// itself, and what a chunk holds beyond `end` is beyond the reach: neither adds anything.
+// INSIDE: the warp's particles lie at least the reach inside every face, so their in-range neighbours are at
+// their stored (wrapped) coordinates and the minimum image is the plain difference (fast_mi returns it
+// unchanged; an entry beyond the reach by the plain difference is beyond it by the minimum image too).
+// CHARGED: some particle of the warp is charged or of the polar class.
+__device__ __forceinline__ uint4 ld_stream(const uint4* p) {   // read once: keeps the L1 for the neighbours
+  uint4 v;
+  asm("ld.global.nc.L1::no_allocate.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p));
+  return v;
+}
+template <int TPP, bool INSIDE, bool CHARGED>
+__device__ __forceinline__ void list_sum(uint32_t k, int lane, uint32_t end, const uint32_t* __restrict__ row,
+                                         const float4* __restrict__ pos, const float* __restrict__ charge,
+                                         const float4& xi, float qi, bool needq, uint32_t polar,
+                                         const PairW* __restrict__ prow, const PairLean& L, const SysParams& P,
+                                         float (&f)[16 / TPP][3]) {
+  constexpr int E = 16 / TPP, C = 4 / E;          // a lane's entries of a chunk of 16, chunks an iteration
+  const float bx = P.box[0], by = P.box[1], bz = P.box[2];
+  const float ix = P.inv_box[0], iy = P.inv_box[1], iz = P.inv_box[2];
+  const bool qi_nz = qi != 0.f;
+  uint32_t nj[4];
+  auto fetch = [&](uint32_t base) {
+#pragma unroll
+    for (int c = 0; c < C; ++c) {
+      const uint32_t at = base + 16u * c;
+      const uint32_t* p = row + at + E * lane;
+      const bool in = C == 1 || at < end;
+      if (E == 4) {
+        const uint4 v = in ? ld_stream(reinterpret_cast<const uint4*>(p)) : make_uint4(k, k, k, k);
+        nj[0] = v.x; nj[1] = v.y; nj[2] = v.z; nj[3] = v.w;
+      } else if (E == 2) {
+        const uint2 v = in ? __ldg(reinterpret_cast<const uint2*>(p)) : make_uint2(k, k);
+        nj[2 * c] = v.x; nj[2 * c + 1] = v.y;
+      } else {
+        nj[c] = in ? __ldg(p) : k;
+      }
+    }
+  };
+  if (end > 0) fetch(0);
+  for (uint32_t base = 0; base < end; base += 16u * C) {
+    uint32_t j[4];
+    float4 xj[4];
+#pragma unroll
+    for (int u = 0; u < 4; ++u) { j[u] = nj[u]; xj[u] = __ldg(pos + j[u]); }
+    if (base + 16u * C < end) fetch(base + 16u * C);
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      float dx = xi.x - xj[u].x, dy = xi.y - xj[u].y, dz = xi.z - xj[u].z;
+      if (!INSIDE) {
+        dx = fast_mi(dx, bx, ix);
+        dy = fast_mi(dy, by, iy);
+        dz = fast_mi(dz, bz, iz);
+      }
+      const float r2 = dx * dx + dy * dy + dz * dz;
+      // the kind, a small whole number held as a float, from the low bits of its sum with 2^23
+      const uint32_t kj = __float_as_uint(xj[u].w + 8388608.0f) & (SOUP_KMAX - 1u);
+      const float qj = CHARGED && needq ? __ldg(charge + j[u]) : 0.f;
+      const float s = pair_lean<CHARGED>(prow[kj], L, r2, CHARGED && ((polar >> kj) & 1u), qi_nz, qi, qj);
+      float (&a)[3] = f[u % E];
+      a[0] += s * dx; a[1] += s * dy; a[2] += s * dz;
+    }
+  }
+}
+
+// eight 128-thread blocks per SM (64 registers): small blocks even out rows of unequal length (256 threads: 192
+// against 183 us at 483k beads); fewer registers spill, fewer blocks hide less of the gathers' latency
+constexpr int kForceBlock = 128;
+
 // SEL: the particles are the nsel slots sel[] (the heads, after a charge sweep) instead of all N
+//
+// Bound: instruction issue and the neighbour gathers.  %FORCE%
 template <int TPP, bool SEL>
-__global__ void __launch_bounds__(256, SOUP_FORCE_MINB) k_force(
+__global__ void __launch_bounds__(kForceBlock, 8) k_force(
     const Shared* __restrict__ Sg, const SysParams* __restrict__ sp, const uint8_t* __restrict__ sysid, uint32_t N,
     const float4* __restrict__ pos, const float* __restrict__ charge, const uint32_t* __restrict__ slots,
     const uint32_t* __restrict__ center, const uint32_t* __restrict__ id, const uint32_t* __restrict__ slot_of,
-    const uint32_t* __restrict__ nl, const uint32_t* __restrict__ nl_cnt, const uint4* __restrict__ nl_shell,
-    const uint32_t* __restrict__ drift_bits, uint32_t cap, float4* __restrict__ force,
+    const uint32_t* __restrict__ nl, const uint32_t* __restrict__ nl_cnt, const uint32_t* __restrict__ nl_shell,
+    const uint32_t* __restrict__ drift_bits, uint32_t stride, float4* __restrict__ force,
     const uint32_t* __restrict__ sel, uint32_t nsel) {
-  __shared__ Shared S;
-  for (int w = threadIdx.x; w < (int)(sizeof(Shared) / 4); w += blockDim.x)
-    reinterpret_cast<uint32_t*>(&S)[w] = reinterpret_cast<const uint32_t*>(Sg)[w];
+  __shared__ PairW pw[SOUP_KMAX * SOUP_KMAX];
+  for (int w = threadIdx.x; w < (int)(sizeof(pw) / 4); w += kForceBlock)
+    reinterpret_cast<uint32_t*>(pw)[w] = reinterpret_cast<const uint32_t*>(Sg->pw)[w];
   __syncthreads();
-  const uint32_t gtid = blockIdx.x * blockDim.x + threadIdx.x;
+  constexpr int E = 16 / TPP;
+  const Shared& S = *Sg;
+  const uint32_t gtid = blockIdx.x * (uint32_t)kForceBlock + threadIdx.x;
   const uint32_t g = gtid / TPP;
   const int lane = (int)(gtid % TPP);
   const bool active = SEL ? g < nsel : g < N;
-  const uint32_t k = SEL ? (active ? sel[g] : 0u) : g;
-  float fx = 0.f, fy = 0.f, fz = 0.f;
-  if (active) {
-    const uint32_t rs = sysid[k];
-    const SysParams& Pg = sp[rs];
-    const PairP P = PairP::of(Pg);
-    const PairLean L = PairLean::of(S, Pg);
-    const float4 xi = pos[k];
-    const int ki = (int)xi.w;
-    const float qi = charge[k];
-    const bool qi_nz = qi != 0.f;
-    const bool needq = qi_nz || (S.cls[ki] == 1u && P.acid > 0.f);
-    const float rmax2 = S.rmax2;
-    const uint32_t cnt = list_force_end(k, nl_cnt, nl_shell, __uint_as_float(drift_bits[rs]), rmax2, Pg.list_range);
-    const uint32_t* row = nl + (size_t)k * cap;
-    const PairW* prow = &S.pw[ki * SOUP_KMAX];
-    // a particle at least the interaction reach inside every face has its in-range neighbours at
-    // their stored (wrapped) coordinates: the minimum image is the plain difference there (fast_mi
-    // returns it unchanged), and an entry beyond the reach by the plain difference is beyond it by the
-    // minimum image too.  Decided per warp, so that whole warps skip the image.
-    const float reach = sqrtf(rmax2) + 1e-3f;
-    const bool inside = __all_sync(__activemask(), xi.x >= reach && xi.x <= P.box[0] - reach && xi.y >= reach &&
-                                                   xi.y <= P.box[1] - reach && xi.z >= reach && xi.z <= P.box[2] - reach);
-    // lane takes entries [c*4*TPP + 4*lane, +4): one 16-byte load (rows are 32-byte aligned); the
-    // next chunk's load is issued before the current chunk is evaluated
-    constexpr uint32_t CH = 4 * TPP;
-    uint32_t base = 4u * (uint32_t)lane;
-    uint4 nxt = base < cnt ? __ldg(reinterpret_cast<const uint4*>(row + base)) : make_uint4(k, k, k, k);
-    for (; base < cnt; base += CH) {
-      const uint4 jj = nxt;
-      if (base + CH < cnt) nxt = __ldg(reinterpret_cast<const uint4*>(row + base + CH));
-      const uint32_t jv[4] = {jj.x, base + 1 < cnt ? jj.y : k, base + 2 < cnt ? jj.z : k, base + 3 < cnt ? jj.w : k};
-      float4 xj[4];
-#pragma unroll
-      for (int e = 0; e < 4; ++e) xj[e] = __ldg(pos + jv[e]);
-#pragma unroll
-      for (int e = 0; e < 4; ++e) {
-        float dx = xi.x - xj[e].x, dy = xi.y - xj[e].y, dz = xi.z - xj[e].z;
-        if (!inside) {
-          dx = fast_mi(dx, P.box[0], P.inv_box[0]);
-          dy = fast_mi(dy, P.box[1], P.inv_box[1]);
-          dz = fast_mi(dz, P.box[2], P.inv_box[2]);
-        }
-        const float r2 = dx * dx + dy * dy + dz * dz;
-        if (r2 >= rmax2 || r2 < 1e-12f) continue;
-        const int kj = (int)xj[e].w;
-        const float qj = needq ? __ldg(charge + jv[e]) : 0.f;
-        const float sc = pair_lean(prow[kj], L, r2, qi_nz, qi, qj);
-        fx += sc * dx; fy += sc * dy; fz += sc * dz;
-      }
-    }
-    // bonded terms (bondedForce), spread over the group
+  const uint32_t k = SEL ? (active ? sel[g] : 0u) : (active ? g : 0u);
+  const uint32_t rs = sysid[k];
+  const SysParams& P = sp[rs];
+  const float4 xi = pos[k];
+  const int ki = (int)xi.w & (SOUP_KMAX - 1);
+  const float qi = charge[k];
+  const bool needq = qi != 0.f || (S.cls[ki] == 1u && P.acid > 0.f);
+  const PairLean L = PairLean::of(S, P);
+  const uint32_t end = active ? list_force_end(k, nl_cnt, nl_shell, __uint_as_float(drift_bits[rs]), P, list_wide(S, P, ki, qi))
+                              : 0u;
+  const float reach = P.reach[1] + 1e-3f;
+  const bool in = xi.x >= reach && xi.x <= P.box[0] - reach && xi.y >= reach && xi.y <= P.box[1] - reach &&
+                  xi.z >= reach && xi.z <= P.box[2] - reach;
+  const bool inside = __all_sync(0xffffffffu, in || !active), charged = __any_sync(0xffffffffu, needq && active);
+  const uint32_t polar = (S.polar >> ki) & 1u ? S.polar : 0u;   // the kinds of the polar class, for an owner of it
+  const uint32_t* row = nl + (size_t)k * stride;
+  const PairW* prow = pw + ki * SOUP_KMAX;
+  float f[E][3] = {};
+  if (inside) {
+    if (charged) list_sum<TPP, true, true>(k, lane, end, row, pos, charge, xi, qi, needq, polar, prow, L, P, f);
+    else list_sum<TPP, true, false>(k, lane, end, row, pos, charge, xi, qi, needq, polar, prow, L, P, f);
+  } else {
+    if (charged) list_sum<TPP, false, true>(k, lane, end, row, pos, charge, xi, qi, needq, polar, prow, L, P, f);
+    else list_sum<TPP, false, false>(k, lane, end, row, pos, charge, xi, qi, needq, polar, prow, L, P, f);
+  }
+  if (active) {   // bonded terms (bondedForce), spread over the sums
     uint32_t sl[3] = {slots[3 * k], slots[3 * k + 1], slots[3 * k + 2]};
-    uint32_t owner = center[k];
+    const uint32_t owner = center[k];
     if ((sl[0] & sl[1] & sl[2] & owner) != SOUP_NONE_U32) {
       const uint32_t gi = id[k];
-      for (int t = lane; t < 13; t += TPP) bonded_term(S, Pg, t, gi, xi, sl, owner, slots, slot_of, pos, fx, fy, fz);
+#pragma unroll
+      for (int e = 0; e < E; ++e) {
+        const int t = E * lane + e;
+        if (t < 13) bonded_term(S, P, t, gi, xi, sl, owner, slots, slot_of, pos, f[e][0], f[e][1], f[e][2]);
+      }
     }
   }
+  // the tree over the sums: neighbours first, inside the lane and then across the group
 #pragma unroll
-  for (int o = TPP / 2; o > 0; o >>= 1) {
-    fx += __shfl_xor_sync(0xffffffffu, fx, o);
-    fy += __shfl_xor_sync(0xffffffffu, fy, o);
-    fz += __shfl_xor_sync(0xffffffffu, fz, o);
+  for (int a = 0; a < 3; ++a) {
+#pragma unroll
+    for (int o = 1; o < E; o <<= 1)
+#pragma unroll
+      for (int e = 0; e < E; e += 2 * o) f[e][a] += f[e + o][a];
+#pragma unroll
+    for (int o = 1; o < TPP; o <<= 1) f[0][a] += __shfl_xor_sync(0xffffffffu, f[0][a], o);
   }
   if (active && lane == 0) {
-    const SysParams& P = sp[sysid[k]];
+    float fx = f[0][0], fy = f[0][1], fz = f[0][2];
     if (P.wall_r > 0.f) {   // wall.wgsl:42-56
-      const float4 xi = pos[k];
       float d0 = xi.x - P.box[0] * 0.5f, d1 = xi.y - P.box[1] * 0.5f, d2 = xi.z - P.box[2] * 0.5f;
       float r = sqrtf(d0 * d0 + d1 * d1 + d2 * d2);
       if (r > P.wall_r) {
         float w = -P.wall_k * (r - P.wall_r) / fmaxf(r, 1e-6f);
-        fx += w * d0; fy += w * d1; fz += w * d2;
-      }
-    }
-    force[k] = make_float4(fx, fy, fz, 0.f);
-  }
-}
-
-// The list force with the pair maths evaluated only on in-range entries, every lane busy.  In k_force
-// a warp runs the pair maths whenever any of its lanes holds an in-range entry, which at the skins in
-// use is nearly every entry, with about half the lanes idle.  Here each lane owns one particle (its
-// list row) and works in rounds: it screens its next four entries (index, gather, minimum image,
-// squared distance), the warp compacts the in-range ones owner-major (lane 0's first, each lane's in
-// list order) into shared memory, every lane evaluates pairs lane, lane + 32, .. of the compacted
-// set, and each owner then adds sc * d for its own pairs in list order with its own separations.  So
-// every particle accumulates exactly the terms k_force<1>'s lane does, in the same order and with the
-// same arithmetic, and the force is bit-identical to k_force<1>'s.
-//
-// A warp whose particles all lie at least the interaction reach inside every face of one replica's box
-// skips the minimum image: for such a particle every neighbour within the reach has its stored
-// (wrapped) coordinates within the reach too, and an entry whose direct separation is beyond the
-// reach is beyond it under the minimum image as well.  Per-pair numbers that depend on the replica are
-// the owner's: a warp whose particles span replicas evaluates each owner's pairs on the owner's lane.
-constexpr int kWBlock = 128;
-constexpr int kWRound = 4;                      // entries a lane screens per round
-constexpr int kWPairs = 32 * kWRound;           // in-range pairs of one warp round, at most
-struct WarpPairs {
-  float r2[kWPairs];
-  float qj[kWPairs];
-  uint32_t ko[kWPairs];                         // neighbour kind | owner lane << 8
-  float sc[kWPairs];
-  float oq[32];                                 // owner charge
-  uint32_t okind[32];                           // owner kind | owner charge nonzero << 8
-};
-
-// six 128-thread blocks per SM: 80 registers, no spills (64 registers spill the round's arrays)
-#ifndef SOUP_FORCE_W_MINB
-#define SOUP_FORCE_W_MINB 6
-#endif
-template <bool SEL>
-__global__ void __launch_bounds__(kWBlock, SOUP_FORCE_W_MINB) k_force_w(
-    const Shared* __restrict__ Sg, const SysParams* __restrict__ sp, const uint8_t* __restrict__ sysid, uint32_t N,
-    const float4* __restrict__ pos, const float* __restrict__ charge, const uint32_t* __restrict__ slots,
-    const uint32_t* __restrict__ center, const uint32_t* __restrict__ id, const uint32_t* __restrict__ slot_of,
-    const uint32_t* __restrict__ nl, const uint32_t* __restrict__ nl_cnt, const uint4* __restrict__ nl_shell,
-    const uint32_t* __restrict__ drift_bits, uint32_t cap, float4* __restrict__ force,
-    const uint32_t* __restrict__ sel, uint32_t nsel) {
-  __shared__ Shared S;
-  __shared__ WarpPairs W[kWBlock / 32];
-  for (int w = threadIdx.x; w < (int)(sizeof(Shared) / 4); w += blockDim.x)
-    reinterpret_cast<uint32_t*>(&S)[w] = reinterpret_cast<const uint32_t*>(Sg)[w];
-  __syncthreads();
-  WarpPairs& wp = W[threadIdx.x >> 5];
-  const uint32_t lane = threadIdx.x & 31u;
-  const uint32_t lt = (1u << lane) - 1u;
-  const uint32_t g = blockIdx.x * blockDim.x + threadIdx.x;
-  const bool active = SEL ? g < nsel : g < N;
-  const uint32_t k = SEL ? (active ? sel[g] : 0u) : (active ? g : 0u);
-  const uint32_t rs = sysid[k];
-  const SysParams& Pg = sp[rs];
-  const PairP P = PairP::of(Pg);
-  const PairLean L = PairLean::of(S, Pg);
-  const float4 xi = pos[k];
-  const int ki = (int)xi.w;
-  const float qi = charge[k];
-  const bool qi_nz = qi != 0.f;
-  const bool needq = qi_nz || (S.cls[ki] == 1u && P.acid > 0.f);
-  const float rmax2 = S.rmax2;
-  const uint32_t cnt =
-      active ? list_force_end(k, nl_cnt, nl_shell, __uint_as_float(drift_bits[rs]), rmax2, Pg.list_range) : 0u;
-  const uint32_t* row = nl + (size_t)k * cap;
-  wp.oq[lane] = qi;
-  wp.okind[lane] = (uint32_t)ki | (qi_nz ? 0x100u : 0u);
-  const bool uni = __all_sync(0xffffffffu, rs == __shfl_sync(0xffffffffu, rs, 0));
-  const float reach = sqrtf(rmax2) + 1e-3f;
-  const bool inside = !active || (xi.x >= reach && xi.x <= P.box[0] - reach && xi.y >= reach &&
-                                  xi.y <= P.box[1] - reach && xi.z >= reach && xi.z <= P.box[2] - reach);
-  const bool direct = uni && __all_sync(0xffffffffu, inside);
-  float fx = 0.f, fy = 0.f, fz = 0.f;
-  uint4 nxt = cnt > 0 ? __ldg(reinterpret_cast<const uint4*>(row)) : make_uint4(k, k, k, k);
-  for (uint32_t base = 0;; base += kWRound) {
-    if (!__any_sync(0xffffffffu, base < cnt)) break;
-    const uint4 jj = nxt;
-    if (base + kWRound < cnt) nxt = __ldg(reinterpret_cast<const uint4*>(row + base + kWRound));
-    const uint32_t jv[4] = {base < cnt ? jj.x : k, base + 1 < cnt ? jj.y : k, base + 2 < cnt ? jj.z : k,
-                            base + 3 < cnt ? jj.w : k};
-    float4 xj[4];
-#pragma unroll
-    for (int e = 0; e < 4; ++e) xj[e] = __ldg(pos + jv[e]);
-    float dx[4], dy[4], dz[4], r2[4];
-    bool in[4];
-    uint32_t c = 0;
-#pragma unroll
-    for (int e = 0; e < 4; ++e) {
-      if (direct) {
-        dx[e] = xi.x - xj[e].x; dy[e] = xi.y - xj[e].y; dz[e] = xi.z - xj[e].z;
-      } else {
-        dx[e] = fast_mi(xi.x - xj[e].x, P.box[0], P.inv_box[0]);
-        dy[e] = fast_mi(xi.y - xj[e].y, P.box[1], P.inv_box[1]);
-        dz[e] = fast_mi(xi.z - xj[e].z, P.box[2], P.inv_box[2]);
-      }
-      r2[e] = dx[e] * dx[e] + dy[e] * dy[e] + dz[e] * dz[e];
-      in[e] = base + e < cnt && r2[e] < rmax2 && r2[e] >= 1e-12f;
-      c += in[e] ? 1u : 0u;
-    }
-    // owner-major offsets of this round's in-range pairs
-    uint32_t incl = c;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-      const uint32_t t = __shfl_up_sync(0xffffffffu, incl, o);
-      if (lane >= (uint32_t)o) incl += t;
-    }
-    const uint32_t first = incl - c;
-    const uint32_t total = __shfl_sync(0xffffffffu, incl, 31);
-    uint32_t p = first;
-#pragma unroll
-    for (int e = 0; e < 4; ++e) {
-      if (in[e]) {
-        wp.r2[p] = r2[e];
-        wp.qj[p] = needq ? __ldg(charge + jv[e]) : 0.f;
-        wp.ko[p] = (uint32_t)xj[e].w | (lane << 8);
-        ++p;
-      }
-    }
-    __syncwarp();
-    if (uni) {
-      for (uint32_t q = lane; q < total; q += 32u) {
-        const uint32_t ko = wp.ko[q];
-        const uint32_t o = ko >> 8, kj = ko & 0xffu;
-        const uint32_t ok = wp.okind[o];
-        const uint32_t kio = ok & 0xffu;
-        wp.sc[q] = pair_lean(S.pw[kio * SOUP_KMAX + kj], L, wp.r2[q], (ok >> 8) != 0u, wp.oq[o], wp.qj[q]);
-      }
-    } else {
-      const PairW* prow = &S.pw[ki * SOUP_KMAX];
-      for (uint32_t q = first; q < incl; ++q)
-        wp.sc[q] = pair_lean(prow[wp.ko[q] & 0xffu], L, wp.r2[q], qi_nz, qi, wp.qj[q]);
-    }
-    __syncwarp();
-    p = first;
-#pragma unroll
-    for (int e = 0; e < 4; ++e) {
-      if (in[e]) {
-        const float sc = wp.sc[p++];
-        fx += sc * dx[e]; fy += sc * dy[e]; fz += sc * dz[e];
-      }
-    }
-    __syncwarp();
-  }
-  if (active) {
-    // bonded terms (bondedForce), all on the particle's lane
-    uint32_t sl[3] = {slots[3 * k], slots[3 * k + 1], slots[3 * k + 2]};
-    uint32_t owner = center[k];
-    if ((sl[0] & sl[1] & sl[2] & owner) != SOUP_NONE_U32) {
-      const uint32_t gi = id[k];
-      for (int t = 0; t < 13; ++t) bonded_term(S, Pg, t, gi, xi, sl, owner, slots, slot_of, pos, fx, fy, fz);
-    }
-    if (Pg.wall_r > 0.f) {   // wall.wgsl:42-56
-      float d0 = xi.x - Pg.box[0] * 0.5f, d1 = xi.y - Pg.box[1] * 0.5f, d2 = xi.z - Pg.box[2] * 0.5f;
-      float r = sqrtf(d0 * d0 + d1 * d1 + d2 * d2);
-      if (r > Pg.wall_r) {
-        float w = -Pg.wall_k * (r - Pg.wall_r) / fmaxf(r, 1e-6f);
         fx += w * d0; fy += w * d1; fz += w * d2;
       }
     }
@@ -411,7 +296,8 @@ __global__ void __launch_bounds__(128) k_force_brute(
     const int kj = (int)xj.w;
     const float qj = charge[j];
     if (r2 < S.rmax2) {
-      const float sc = pair_lean(S.pw[ki * SOUP_KMAX + kj], L, r2, qi != 0.f, qi, qj);
+      const float sc = pair_lean<true>(S.pw[ki * SOUP_KMAX + kj], L, r2, (S.polar >> ki) & (S.polar >> kj) & 1u, qi != 0.f,
+                                       qi, qj);
       fx += sc * dx; fy += sc * dy; fz += sc * dz;
     }
     const float qq = qi * qj;
@@ -439,31 +325,19 @@ __global__ void __launch_bounds__(128) k_force_brute(
   force[k] = make_float4(fx, fy, fz, 0.f);
 }
 
-void launch_force_w(Batch& b, bool heads) {
-  if (heads) {
-    if (b.H == 0) return;
-    k_force_w<true><<<nblocks(b.H, kWBlock), kWBlock, 0, b.stream>>>(
-        b.shared, b.sp, b.sysid, b.N, b.pos, b.charge, b.slots, b.center, b.id, b.slot_of, b.nl, b.nl_cnt, b.prune ? b.nl_shell : nullptr, b.drift_bits, b.list_cap,
-        b.force, b.head_slot, b.H);
-    return;
-  }
-  k_force_w<false><<<nblocks(b.N, kWBlock), kWBlock, 0, b.stream>>>(
-      b.shared, b.sp, b.sysid, b.N, b.pos, b.charge, b.slots, b.center, b.id, b.slot_of, b.nl, b.nl_cnt, b.prune ? b.nl_shell : nullptr, b.drift_bits, b.list_cap,
-      b.force, nullptr, 0u);
-}
-
 template <int TPP>
 void launch_force_tpp(Batch& b, bool heads) {
-  if (heads) {
-    if (b.H == 0) return;
-    k_force<TPP, true><<<nblocks((uint64_t)b.H * TPP, 256), 256, 0, b.stream>>>(
-        b.shared, b.sp, b.sysid, b.N, b.pos, b.charge, b.slots, b.center, b.id, b.slot_of, b.nl, b.nl_cnt, b.prune ? b.nl_shell : nullptr, b.drift_bits, b.list_cap,
-        b.force, b.head_slot, b.H);
-    return;
-  }
-  k_force<TPP, false><<<nblocks((uint64_t)b.N * TPP, 256), 256, 0, b.stream>>>(
-      b.shared, b.sp, b.sysid, b.N, b.pos, b.charge, b.slots, b.center, b.id, b.slot_of, b.nl, b.nl_cnt, b.prune ? b.nl_shell : nullptr, b.drift_bits, b.list_cap,
-      b.force, nullptr, 0u);
+  const uint32_t n = heads ? b.H : b.N;
+  const unsigned blocks = nblocks((uint64_t)n * TPP, kForceBlock);
+  const uint32_t* shells = b.prune ? b.nl_shell : nullptr;
+  if (heads)
+    k_force<TPP, true><<<blocks, kForceBlock, 0, b.stream>>>(b.shared, b.sp, b.sysid, b.N, b.pos, b.charge, b.slots, b.center, b.id,
+                                                     b.slot_of, b.nl, b.nl_cnt, shells, b.drift_bits, b.list_stride,
+                                                     b.force, b.head_slot, b.H);
+  else
+    k_force<TPP, false><<<blocks, kForceBlock, 0, b.stream>>>(b.shared, b.sp, b.sysid, b.N, b.pos, b.charge, b.slots, b.center, b.id,
+                                                      b.slot_of, b.nl, b.nl_cnt, shells, b.drift_bits, b.list_stride,
+                                                      b.force, nullptr, 0u);
 }
 
 }  // namespace
@@ -479,19 +353,21 @@ void launch_force(Batch& b) {
   }
 }
 
+// Lanes per particle: the result is the same bits, so the launch's size decides.  Few particles need the lanes
+// to cover the gathers' latency; many need the fewest instructions.  %TPP%
+int force_lanes(const Batch& b, uint32_t n) {
+  if (b.tpp) return b.tpp <= 4 ? 4 : (b.tpp <= 8 ? 8 : 16);
+  return n >= 80000u ? 4 : (n >= 40000u ? 8 : 16);
+}
+
 void launch_force_list(Batch& b, bool heads) {
+  const uint32_t n = heads ? b.H : b.N;
+  if (n == 0) return;
   b.launches += 1;
-  if (b.queued) {   // the warp-compacted kernel: one lane per particle whatever tpp says
-    launch_force_w(b, heads);
-    return;
-  }
-  switch (b.tpp) {
-    case 1: launch_force_tpp<1>(b, heads); break;
-    case 2: launch_force_tpp<2>(b, heads); break;
-    case 16: launch_force_tpp<16>(b, heads); break;
-    case 32: launch_force_tpp<32>(b, heads); break;
+  switch (force_lanes(b, n)) {
+    case 4: launch_force_tpp<4>(b, heads); break;
     case 8: launch_force_tpp<8>(b, heads); break;
-    default: launch_force_tpp<4>(b, heads); break;
+    default: launch_force_tpp<16>(b, heads); break;
   }
 }
 

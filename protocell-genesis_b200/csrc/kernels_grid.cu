@@ -194,19 +194,19 @@ __device__ __forceinline__ float gap_to_cell(float p, int c, float cs) {
 }
 
 // The build-distance shell of a list entry, carried in its top three bits until its row is grouped: 0
-// inside the force's reach, 1..4 the rest of the list range (list_shell_width2).  A force pass needs shell
+// inside the force's reach, 1..7 the rest of the list range (list_shell_width2).  A force pass needs shell
 // s > 0 only once the largest displacement since the build can have closed the distance from the reach to
 // that shell's inner edge (list_force_end).
 struct Shells {
   float reach2, scale;
-  __device__ __forceinline__ static Shells of(float rmax2, float list_range) {
+  __device__ __forceinline__ static Shells of(float reach2, float list_range) {
     Shells s;
-    s.reach2 = rmax2;
-    s.scale = 1.0f / fmaxf(list_shell_width2(rmax2, list_range), 1e-12f);
+    s.reach2 = reach2;
+    s.scale = 1.0f / fmaxf(list_shell_width2(reach2, list_range), 1e-12f);
     return s;
   }
   __device__ __forceinline__ uint32_t tag(float r2) const {
-    return (uint32_t)(min(max(__float2int_rd((r2 - reach2) * scale), -1), 3) + 1) << 29;
+    return (uint32_t)(min(max(__float2int_rd((r2 - reach2) * scale), -1), kShells - 2) + 1) << 29;
   }
 };
 
@@ -308,26 +308,37 @@ __device__ __forceinline__ void warp_walk(const float4& xi, const float* box, co
   }
 }
 
-__device__ __forceinline__ uint32_t field12(unsigned long long w, uint32_t t) {
-  return (uint32_t)(w >> (12u * t)) & 0xFFFu;
-}
+// eight 12-bit counters, five to a word
+struct Count8 {
+  unsigned long long a, b;
+  __device__ __forceinline__ uint32_t at(uint32_t t) const {
+    return (uint32_t)(t < 5u ? a >> (12u * t) : b >> (12u * (t - 5u))) & 0xFFFu;
+  }
+  __device__ __forceinline__ void add(uint32_t t, unsigned long long n) {
+    if (t < 5u) a += n << (12u * t);
+    else b += n << (12u * (t - 5u));
+  }
+};
 constexpr uint32_t kGRegs = 17;                        // entries a lane can hold while a row is grouped
 
 // soup/wgsl/verlet.wgsl:53-92, a warp per particle (warp_walk).  The fast squared distance decides unless it
 // lies within 1e-5 of the range, where the reference's arithmetic decides (the minimum image cannot differ
 // there: range < box/2), so the list is the reference's set.  The accepted entries are compacted into the
 // warp's shared row with ballots, then the row is grouped by build-distance shell, keeping its order inside
-// a shell, and written once, coalesced.
+// a shell, and written once, coalesced.  Every whole chunk of 16 entries is stored transposed (entry 4 e + l at
+// place 4 l + e), so that the force's four lanes of a particle, which read four places each, gather four
+// successive entries at a time: beads of one run, which share cache lines.
 //
 // Bound: instruction issue (about 17 rounds of 32 candidates, some 35 instructions each, and 200 to group the
 // row).  Grouping in shared memory takes the place of a second pass that read and rewrote every row.
 __global__ void __launch_bounds__(128) k_build_list(
-    const float4* __restrict__ pos, const uint8_t* __restrict__ sysid, const SysParams* __restrict__ sp,
-    const uint32_t* __restrict__ start, uint32_t N, uint32_t cap, float rmax2, uint32_t* __restrict__ nl,
-    uint32_t* __restrict__ nl_cnt, uint4* __restrict__ shell_end, uint32_t* __restrict__ flags) {
+    const Shared* __restrict__ Sg, const float4* __restrict__ pos, const float* __restrict__ charge,
+    const uint8_t* __restrict__ sysid, const SysParams* __restrict__ sp, const uint32_t* __restrict__ start, uint32_t N,
+    uint32_t cap, uint32_t stride, uint32_t* __restrict__ nl, uint32_t* __restrict__ nl_cnt,
+    uint32_t* __restrict__ shell_end, uint32_t* __restrict__ flags) {
   extern __shared__ __align__(16) uint32_t sm[];
   const uint32_t wib = threadIdx.x >> 5, lane = threadIdx.x & 31u, lt = (1u << lane) - 1u;
-  uint32_t* row = sm + (size_t)wib * (cap + kWalkWords);   // cap is a multiple of 8
+  uint32_t* row = sm + (size_t)wib * (stride + kWalkWords);   // stride: cap rounded up to 16
   const uint32_t k = blockIdx.x * (blockDim.x >> 5) + wib;
   if (k >= N) return;   // whole warps
   const SysParams& P = sp[sysid[k]];
@@ -335,7 +346,7 @@ __global__ void __launch_bounds__(128) k_build_list(
   const float box[3] = {P.box[0], P.box[1], P.box[2]};
   const float inv[3] = {P.inv_box[0], P.inv_box[1], P.inv_box[2]};
   const float lr = P.list_range;
-  const Shells sh = Shells::of(rmax2, lr);
+  const Shells sh = Shells::of(list_wide(*Sg, P, (int)xi.w & (SOUP_KMAX - 1), charge[k]) ? Sg->rmax2 : Sg->rplain2, lr);
   const float lr2_lo = lr * lr * (1.0f - 1e-5f), lr2_hi = lr * lr * (1.0f + 1e-5f);
   // a particle at least the list range inside every face screens with plain differences: a candidate within
   // the range sits at its stored coordinates, and one beyond it by the plain difference is beyond it by
@@ -364,7 +375,7 @@ __global__ void __launch_bounds__(128) k_build_list(
     if (in && at < cap) row[at] = e;
     cnt += __popc(m);
   };
-  warp_walk(xi, box, G, start, row + cap, [&](uint32_t j0, bool v0, uint32_t j1, bool v1) {
+  warp_walk(xi, box, G, start, row + stride, [&](uint32_t j0, bool v0, uint32_t j1, bool v1) {
     const float4 x0 = pos[j0], x1 = pos[j1];
     const uint32_t e0 = test(j0, v0, x0), e1 = test(j1, v1, x1);
     put(e0);
@@ -376,53 +387,57 @@ __global__ void __launch_bounds__(128) k_build_list(
   }
   __syncwarp();
   // group the row by shell.  Up to 32 * 16 entries: lane l holds a contiguous piece, counts its entries per
-  // shell (five 12-bit fields of one 64-bit word), one warp scan of those words gives every lane its places,
+  // shell (12-bit counters), one warp scan of them gives every lane its places,
   // and the pieces are written back in lane order.  A longer row (dense aggregates) goes out shell by
   // shell with ballots.  Both keep the walk's order inside a shell.
-  uint32_t* out = nl + (size_t)k * cap;
-  uint32_t e[4];
+  uint32_t* out = nl + (size_t)k * stride;
+  const uint32_t full = (cnt + 15u) & ~15u;          // rows are padded with the particle itself
+  uint32_t e[kShells - 1];
   if (cnt <= 32u * (kGRegs - 1u)) {
     const uint32_t piece = ((cnt + 31u) >> 5) | 1u;    // odd: no bank conflicts
     const uint32_t s0 = lane * piece, s1 = min(s0 + piece, cnt);
     uint32_t v[kGRegs];
-    unsigned long long mine = 0;
+    Count8 mine{0, 0};
 #pragma unroll
     for (uint32_t c = 0; c < kGRegs; ++c) {
       if (c >= piece) break;
       v[c] = s0 + c < s1 ? row[s0 + c] : SOUP_NONE_U32;
-      if (v[c] != SOUP_NONE_U32) mine += 1ull << (12u * (v[c] >> 29));
+      if (v[c] != SOUP_NONE_U32) mine.add(v[c] >> 29, 1ull);
     }
-    unsigned long long incl = mine;
+    Count8 incl = mine;
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
-      const unsigned long long y = __shfl_up_sync(0xffffffffu, incl, o);
-      if (lane >= (uint32_t)o) incl += y;
+      const unsigned long long ya = __shfl_up_sync(0xffffffffu, incl.a, o), yb = __shfl_up_sync(0xffffffffu, incl.b, o);
+      if (lane >= (uint32_t)o) { incl.a += ya; incl.b += yb; }
     }
-    const unsigned long long tot = __shfl_sync(0xffffffffu, incl, 31);
-    unsigned long long bases = 0;                      // the shells' first places, packed like the counts
+    const Count8 tot{__shfl_sync(0xffffffffu, incl.a, 31), __shfl_sync(0xffffffffu, incl.b, 31)};
+    Count8 at{incl.a - mine.a, incl.b - mine.b};       // this lane's next place in every shell
     uint32_t run = 0;
 #pragma unroll
-    for (uint32_t t = 0; t < 5; ++t) {
-      bases |= (unsigned long long)run << (12u * t);
-      run += field12(tot, t);
-      if (t < 4) e[t] = run;
+    for (uint32_t t = 0; t < (uint32_t)kShells; ++t) {
+      at.add(t, run);
+      run += tot.at(t);
+      if (t + 1u < (uint32_t)kShells) e[t] = run;
     }
-    unsigned long long at = bases + (incl - mine);     // this lane's next place in every shell
 #pragma unroll
     for (uint32_t c = 0; c < kGRegs; ++c) {
       if (c >= piece) break;
       if (v[c] == SOUP_NONE_U32) continue;
       const uint32_t t = v[c] >> 29;
-      row[field12(at, t)] = v[c] & 0x1FFFFFFFu;
-      at += 1ull << (12u * t);
+      row[at.at(t)] = v[c] & 0x1FFFFFFFu;
+      at.add(t, 1ull);
     }
+    if (cnt + lane < full) row[cnt + lane] = k;
     __syncwarp();
-    for (uint32_t s = 4u * lane; s < cnt; s += 128u)   // rows are 32-byte aligned; the tail up to 4 is unread
-      *reinterpret_cast<uint4*>(out + s) = *reinterpret_cast<const uint4*>(row + s);
+    for (uint32_t s = 4u * lane; s < full; s += 128u) {
+      const uint32_t c = s & ~15u, l = (s >> 2) & 3u;
+      *reinterpret_cast<uint4*>(out + s) = c + 16u <= cnt ? make_uint4(row[c + l], row[c + 4u + l], row[c + 8u + l], row[c + 12u + l])
+                                                         : *reinterpret_cast<const uint4*>(row + s);
+    }
   } else {
     uint32_t o = 0;
 #pragma unroll
-    for (uint32_t b = 0; b < 5; ++b) {
+    for (uint32_t b = 0; b < (uint32_t)kShells; ++b) {
       for (uint32_t s0 = 0; s0 < cnt; s0 += 32u) {
         const uint32_t s = s0 + lane;
         const uint32_t v = s < cnt ? row[s] : SOUP_NONE_U32;
@@ -431,12 +446,15 @@ __global__ void __launch_bounds__(128) k_build_list(
         if (hit) out[o + __popc(m & lt)] = v & 0x1FFFFFFFu;
         o += __popc(m);
       }
-      if (b < 4) e[b] = o;
+      if (b + 1u < (uint32_t)kShells) e[b] = o;
     }
+    if (cnt + lane < full) out[cnt + lane] = k;
   }
   if (lane == 0) {
     nl_cnt[k] = cnt;
-    shell_end[k] = make_uint4(e[0], e[1], e[2], e[3]);
+    uint4* se = reinterpret_cast<uint4*>(shell_end + (size_t)kShells * k);
+    se[0] = make_uint4(e[0], e[1], e[2], e[3]);
+    se[1] = make_uint4(e[4], e[5], e[6], cnt);
   }
 }
 
@@ -568,7 +586,7 @@ void launch_build_lists(Batch& b) {
   b.launches += 1;
   prof_begin(b, SOUP_K_LIST);
   // a row of shared memory per warp: four warps per block while they fit
-  const size_t per = sizeof(uint32_t) * ((size_t)b.list_cap + kWalkWords);
+  const size_t per = sizeof(uint32_t) * ((size_t)b.list_stride + kWalkWords);
   const uint32_t wpb = 4u * per <= 200u * 1024u ? 4u : 1u;
   const size_t smem = wpb * per;
   if (smem > 48u * 1024u && b.list_smem_set < smem) {
@@ -576,7 +594,8 @@ void launch_build_lists(Batch& b) {
     b.list_smem_set = smem;
   }
   k_build_list<<<(unsigned)((b.N + wpb - 1) / wpb), 32u * wpb, smem, b.stream>>>(
-      b.pos, b.sysid, b.sp, b.cell_start, b.N, b.list_cap, b.hs.rmax2, b.nl, b.nl_cnt, b.nl_shell, b.flags);
+      b.shared, b.pos, b.charge, b.sysid, b.sp, b.cell_start, b.N, b.list_cap, b.list_stride, b.nl, b.nl_cnt, b.nl_shell,
+      b.flags);
   prof_end(b);
 }
 

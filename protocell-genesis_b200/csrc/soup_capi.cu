@@ -80,6 +80,7 @@ Shared make_shared(const SoupConfig& c) {
   for (uint32_t k = 0; k < SOUP_KMAX; ++k) {
     s.radius[k] = (float)c.radius[k];
     s.cls[k] = c.kind_class[k] & 3u;
+    s.polar |= (s.cls[k] == 1u ? 1u : 0u) << k;
   }
   for (uint32_t i = 0; i < SOUP_KMAX; ++i)
     for (uint32_t j = 0; j < SOUP_KMAX; ++j) {
@@ -90,10 +91,10 @@ Shared make_shared(const SoupConfig& c) {
       p.wcut = w; p.wcut2 = w * w; p.b2 = b * b;
       p.attr = (float)c.attr_scale[s.cls[i]][s.cls[j]];
       PairW& q = s.pw[i * SOUP_KMAX + j];
-      q.b2 = p.b2; q.wcut2 = p.wcut2; q.amp = p.attr * s.attr_amp;
-      q.polar = (s.cls[i] == 1u && s.cls[j] == 1u) ? 1.f : 0.f;
+      q.b2 = p.b2; q.amp = p.attr * s.attr_amp;
       if (i < c.n_kinds && j < c.n_kinds) rmax = std::max(rmax, (float)w);
     }
+  s.rplain2 = rmax * rmax * 1.0001f;
   if (c.es_enabled) rmax = std::max(rmax, (float)c.es_split_radius);
   s.rmax2 = rmax * rmax * 1.0001f;
   for (uint32_t r = 0; r < SOUP_RMAX; ++r) {
@@ -210,6 +211,14 @@ void alloc_grids(Batch& b) {
 }
 
 void upload_params(Batch& b) {
+  for (uint32_t r = 0; r < b.R; ++r) {
+    SysParams& p = b.hsp[r];
+    for (int wide = 0; wide < 2; ++wide) {
+      const float reach2 = wide ? b.hs.rmax2 : b.hs.rplain2, w2 = list_shell_width2(reach2, p.list_range);
+      p.reach[wide] = std::sqrt(reach2);
+      p.shell_scale[wide] = w2 > 0.f ? 1.0f / w2 : 0.f;
+    }
+  }
   SOUP_CUDA_TRY(cudaMemcpyAsync(b.sp, b.hsp.data(), sizeof(SysParams) * b.R, cudaMemcpyHostToDevice, b.stream));
   SOUP_CUDA_TRY(cudaMemcpyAsync(b.shared, &b.hs, sizeof(Shared), cudaMemcpyHostToDevice, b.stream));
 }
@@ -344,6 +353,7 @@ Batch* make_batch(const SoupConfig* cfgs, const SoupInitState* inits, uint32_t R
   if (N > 0xFFFFFFF0ull) fail(SOUP_E_ARG, "too many particles");
   b.N = (uint32_t)N;
   b.list_cap = (b.list_cap + 7u) & ~7u;
+  b.list_stride = (b.list_cap + 15u) & ~15u;
   b.prot_rng.assign(R, 0);
   for (uint32_t r = 0; r < R; ++r) {
     b.wall_r0.push_back(b.cfg[r].wall_radius);
@@ -367,7 +377,7 @@ Batch* make_batch(const SoupConfig* cfgs, const SoupInitState* inits, uint32_t R
   b.slots2 = dalloc<uint32_t>(3 * n); b.center2 = dalloc<uint32_t>(n); b.held2 = dalloc<uint32_t>(n);
   b.brng2 = dalloc<uint32_t>(n); b.trng2 = dalloc<uint32_t>(n); b.frozen2 = dalloc<uint8_t>(n); b.id2 = dalloc<uint32_t>(n);
   b.cell_of_slot = dalloc<uint32_t>(n); b.perm = dalloc<uint32_t>(n);
-  b.nl = dalloc<uint32_t>(n * (size_t)b.list_cap); b.nl_cnt = dalloc<uint32_t>(n); b.nl_shell = dalloc<uint4>(n);
+  b.nl = dalloc<uint32_t>(n * (size_t)b.list_stride); b.nl_cnt = dalloc<uint32_t>(n); b.nl_shell = dalloc<uint32_t>(kShells * n);
   b.sysid = dalloc<uint8_t>(n);
   b.sp = dalloc<SysParams>(R); b.shared = dalloc<Shared>(1);
   b.flags = dalloc<uint32_t>(FLAG_WORDS + 2 * (size_t)R);
@@ -433,11 +443,9 @@ Batch* make_batch(const SoupConfig* cfgs, const SoupInitState* inits, uint32_t R
   }
   alloc_grids(b);
   upload_params(b);
-  // lanes per particle in the list force: 4 measured fastest at 483k beads (2: same, 8: +5%,
-  // 16: +16%); SOUP_TPP in the environment overrides it for tuning (1, 2, 4, 8, 16 or 32)
-  b.tpp = 4;
+  // lanes per particle in the list force by the launch's size (force_lanes); SOUP_TPP in the environment
+  // overrides it (up to 4: 4, up to 8: 8, else 16)
   if (const char* e = std::getenv("SOUP_TPP")) b.tpp = std::atoi(e);
-  if (const char* e = std::getenv("SOUP_FORCE_QUEUED")) b.queued = std::atoi(e) != 0;
   if (const char* e = std::getenv("SOUP_FULL_ROWS")) b.prune = std::atoi(e) == 0;
   force_pass(b);   // priming pass (soup/src/sim.ts:396-408)
   SOUP_CUDA_TRY(cudaStreamSynchronize(b.stream));
@@ -1183,10 +1191,10 @@ int soup_read_checkpoint(SoupHandle* h, void* dst, size_t bytes, SoupCheckpointS
 int soup_read_verlet(SoupHandle* h, uint32_t* counts, uint32_t* lists, size_t lists_cap) {
   return guarded(h, [&](Batch& b, uint32_t r) {
     const uint32_t n = b.cfg[r].n, off = b.hsp[r].slot_off;
-    std::vector<uint32_t> cnt(n), ids(b.N), rows((size_t)n * b.list_cap);
+    std::vector<uint32_t> cnt(n), ids(b.N), rows((size_t)n * b.list_stride);
     SOUP_CUDA_TRY(cudaMemcpyAsync(cnt.data(), b.nl_cnt + off, 4 * (size_t)n, cudaMemcpyDeviceToHost, b.stream));
     SOUP_CUDA_TRY(cudaMemcpyAsync(ids.data(), b.id, 4 * (size_t)b.N, cudaMemcpyDeviceToHost, b.stream));
-    SOUP_CUDA_TRY(cudaMemcpyAsync(rows.data(), b.nl + (size_t)off * b.list_cap, 4 * rows.size(), cudaMemcpyDeviceToHost, b.stream));
+    SOUP_CUDA_TRY(cudaMemcpyAsync(rows.data(), b.nl + (size_t)off * b.list_stride, 4 * rows.size(), cudaMemcpyDeviceToHost, b.stream));
     SOUP_CUDA_TRY(cudaStreamSynchronize(b.stream));
     std::vector<uint32_t> slot_of_local(n);
     for (uint32_t k = 0; k < n; ++k) slot_of_local[ids[off + k] - off] = k;
@@ -1198,7 +1206,7 @@ int soup_read_verlet(SoupHandle* h, uint32_t* counts, uint32_t* lists, size_t li
     for (uint32_t i = 0; i < n; ++i) {
       const uint32_t k = slot_of_local[i];
       uint32_t* o = lists + at;
-      for (uint32_t s = 0; s < cnt[k]; ++s) o[s] = ids[rows[(size_t)k * b.list_cap + s]] - off;
+      for (uint32_t s = 0; s < cnt[k]; ++s) o[s] = ids[rows[(size_t)k * b.list_stride + s]] - off;
       std::sort(o, o + cnt[k]);
       at += cnt[k];
     }
@@ -1423,7 +1431,7 @@ int soup_autotune(SoupHandle* h, uint32_t steps, SoupTuneResult* out) {
     std::vector<double> planned(b.R);
     for (uint32_t r = 0; r < b.R; ++r) planned[r] = b.cfg[r].skin;
     const int walk0 = b.hsp[0].walk;
-    const int tpp0 = b.tpp;
+    const int tpp0 = force_lanes(b, b.N);
     auto steps_ms = [&]() { return tune_time(b, 1, [&] { step_batch(b, steps); }) / steps; };
     SoupTuneResult res{};
     if (steps) {
@@ -1431,19 +1439,13 @@ int soup_autotune(SoupHandle* h, uint32_t steps, SoupTuneResult* out) {
       tune_restore(b, snap);
     }
     // block shape: lanes per particle of the list force, timed on the force alone
-    const int tpps[4] = {1, 2, 4, 8};
-    const bool queued0 = b.queued;
     double best = 1e30;
-    for (int q = 0; q < 2; ++q)
-      for (int t : tpps) {
-        if (q && t != 1) continue;   // the compacted kernel is one lane per particle
-        b.tpp = t;
-        b.queued = q != 0;
-        const double ms = tune_time(b, 5, [&] { launch_force_list(b); });
-        if (ms < best) { best = ms; res.tpp = (uint32_t)t; res.queued = (uint32_t)q; }
-      }
+    for (int t : {4, 8}) {
+      b.tpp = t;
+      const double ms = tune_time(b, 5, [&] { launch_force_list(b); });
+      if (ms < best) { best = ms; res.tpp = (uint32_t)t; }
+    }
     b.tpp = (int)res.tpp;
-    b.queued = res.queued != 0;
     drop_graphs(b);
     // cell size (the list-walk radius: cell = list range / walk), timed on the list build and, as the walk
     // sets the slot order the force gathers in, the ten force passes of a typical rebuild interval
@@ -1481,7 +1483,6 @@ int soup_autotune(SoupHandle* h, uint32_t steps, SoupTuneResult* out) {
     }
     b.prof = prof;
     res.tpp_before = (uint32_t)tpp0;
-    res.queued_before = queued0 ? 1u : 0u;
     res.walk_before = (uint32_t)walk0;
     if (out) *out = res;
   });
@@ -1496,7 +1497,6 @@ int soup_apply_tuning(SoupHandle* h, const SoupTuneResult* t) {
     if (t->skin_scale != 1.0 && !b.cfg[0].rebuild_on_drift)
       fail(SOUP_E_ARG, "tuning: the skin can only be scaled with drift-triggered rebuilds");
     b.tpp = (int)t->tpp;
-    b.queued = t->queued != 0;
     std::vector<double> sk(b.R);
     for (uint32_t r = 0; r < b.R; ++r) sk[r] = b.cfg[r].skin * t->skin_scale;
     tune_plan(b, sk, (int)t->walk);

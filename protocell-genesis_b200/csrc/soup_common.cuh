@@ -30,6 +30,9 @@ struct SysParams {
   float kT, gamma, dt, hdt, gdt, sigma_v;
   float acid;                // AttrScale.pair.x
   float skin_half2;          // (skin/2)^2 for the drift trigger
+  // the force's reach of a plain bead and of one that list_wide names, and 1 / list_shell_width2 for it (0: its
+  // row is read whole)
+  float reach[2], shell_scale[2];
   int dims[3];               // list-build grid
   uint32_t cell_off;         // first global cell of this system
   int walk;                  // list-build walk radius (cells)
@@ -55,12 +58,11 @@ struct PairConst {
   float b2;      // b^2
   float attr;    // class-table depth
 };
-// The list force's per-kind-pair numbers, premultiplied for the pair loop.
-struct PairW {
+// The list force's per-kind-pair numbers, premultiplied for the pair loop: two words, read from shared memory
+// once a pair (four of them took twice the L1 cycles).
+struct alignas(8) PairW {
   float b2;      // b^2
-  float wcut2;   // (c6 * b)^2
   float amp;     // class-table depth * eps * pi / (2 wc)
-  float polar;   // 1 when both kinds are of the polar class (the acid-soap depth applies), else 0
 };
 struct Shared {
   PairConst pair[SOUP_KMAX * SOUP_KMAX];
@@ -72,6 +74,8 @@ struct Shared {
   float attr_k;              // pi / (2 wc) (fast path)
   float attr_amp;            // eps * pi / (2 wc) (fast path)
   float rmax2;               // max squared pair reach of any nonbonded term (fast path skip)
+  uint32_t polar;            // bit k: kind k is of the polar class (the acid-soap depth applies between two)
+  float rplain2;             // the same of a bead with no charge and not of the polar class
   // bond rules (soup/wgsl/bond-common.wgsl:54-80 BondParams)
   float kindA[SOUP_RMAX], kindB[SOUP_RMAX];
   float att_form[SOUP_RMAX], att_break[SOUP_RMAX], acc_form[SOUP_RMAX], acc_break[SOUP_RMAX];
@@ -145,16 +149,23 @@ struct PairP {
   }
 };
 
-// The width in r^2 of a list row's outer build-distance shells: shell 0 lies within the force's reach
-// (rmax2), shell s = 1..4 between rmax2 + (s - 1) w2 and rmax2 + s w2, where the list range ends.
-__device__ __forceinline__ float list_shell_width2(float rmax2, float list_range) {
-  return fmaxf(list_range * list_range - rmax2, 0.f) * 0.25f;
+// The width w2 in r^2 of a list row's outer build-distance shells: shell 0 lies within the force's reach
+// (reach2), shell s = 1..7 between reach2 + (s - 1) w2 and reach2 + s w2, where the list range ends.
+constexpr int kShells = 8;
+__host__ __device__ __forceinline__ float list_shell_width2(float reach2, float list_range) {
+  return fmaxf(list_range * list_range - reach2, 0.f) * (1.0f / (kShells - 1));
+}
+// Whether a bead can take part in a term that reaches beyond the class attraction: it is charged, or a sweep
+// can charge it, or it is of the polar class.  A plain bead's force ends at rplain2.
+__device__ __forceinline__ bool list_wide(const Shared& S, const SysParams& P, int kind, float charge) {
+  return charge != 0.f || S.cls[kind] == 1u || kind == P.charged_kind;
 }
 
 // The pair loop's constants of one replica, held in registers (batch-wide numbers from Shared, the
 // replica's acid-soap depth and screened-Coulomb numbers from its SysParams).
 struct PairLean {
   float c48, c24;         // 48 eps, 24 eps
+  float c62;              // c6^2: WCA ends at c6^2 b^2
   float k2, k2rc;         // sin argument 2 (r - rc) pi / (2 wc) = r k2 - k2rc
   float rc2, rcw2;        // the attraction window [rc, rc + wc], squared
   float acid_amp;         // acid-soap depth * eps * pi / (2 wc), 0 without it
@@ -163,6 +174,7 @@ struct PairLean {
     PairLean L;
     L.c48 = 48.0f * S.eps;
     L.c24 = 24.0f * S.eps;
+    L.c62 = S.c6 * S.c6;
     L.k2 = 2.0f * S.attr_k;
     L.k2rc = L.k2 * S.rc_attr;
     L.rc2 = S.rc_attr * S.rc_attr;
@@ -176,30 +188,43 @@ struct PairLean {
   }
 };
 
+__device__ __forceinline__ float rsqrt_ftz(float x) {   // rsqrtf without its handling of denormals
+  float y;
+  asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+  return y;
+}
+
 // Scalar s such that the pair force on i is s * d (d = mi(xi - xj)), for every term the neighbour
 // list carries (soup/wgsl/pair.wgsl:168-204 nonbondedSoup): WCA below c6 b (forces.wgsl:19-23,
 // -wca_dv(r)/r = 24 eps (2 (b/r)^12 - (b/r)^6) / r^2), the class attraction on [rc, rc + wc] with the
 // acid-soap depth added between two polar beads of which exactly one is charged (forces.wgsl:32-37,
 // pair.wgsl:151-160, 188: -(A + acid) eps pi / (2 wc) sin(pi (r - rc) / wc) / r), and the near half of
-// the screened Coulomb force between charged beads (electrostatics.wgsl:65-83).  WCA and the
-// attraction are selected, not branched on; the windows are tested on r^2 (both forces vanish at
-// their edges).  The screened Coulomb term only exists between charged beads and stays a branch.
-// qi_nz: the owner's charge is nonzero.
-__device__ __forceinline__ float pair_lean(const PairW& pc, const PairLean& L, float r2, bool qi_nz, float qi,
-                                           float qj) {
-  const float rinv = rsqrtf(r2);
+// the screened Coulomb force between charged beads (electrostatics.wgsl:65-83).  Every term is selected by
+// its window on r^2 (the forces vanish at their edges), so s is 0 beyond all of them and for a bead with
+// itself (r2 = 0), and no lane waits for another's branch; the screened Coulomb term only exists
+// between charged beads and stays a branch.  CHARGED = false leaves out what needs a charge: the same bits
+// for an owner that is neither charged nor of the polar class.  qi_nz: the owner's charge is nonzero; polar: both
+// beads are of the polar class.
+template <bool CHARGED>
+__device__ __forceinline__ float pair_lean(const PairW& pc, const PairLean& L, float r2, bool polar, bool qi_nz,
+                                           float qi, float qj) {
+  const float rinv = rsqrt_ftz(r2);
   const float r = r2 * rinv;
   const float rinv2 = rinv * rinv;
   const float s2 = pc.b2 * rinv2;
   const float s6 = s2 * s2 * s2;
-  float s = (r2 < pc.wcut2) ? (L.c48 * s6 - L.c24) * s6 * rinv2 : 0.f;
-  const float amp = pc.amp + ((pc.polar != 0.f && (qi_nz != (qj != 0.f))) ? L.acid_amp : 0.f);
+  const bool apart = r2 >= 1e-12f;
+  float s = (apart && r2 < pc.b2 * L.c62) ? (L.c48 * s6 - L.c24) * s6 * rinv2 : 0.f;
+  float amp = pc.amp;
+  if (CHARGED) amp += (polar && (qi_nz != (qj != 0.f))) ? L.acid_amp : 0.f;
   const float sn = __sinf(fmaf(r, L.k2, -L.k2rc));
   s -= (r2 >= L.rc2 && r2 <= L.rcw2) ? amp * sn * rinv : 0.f;
-  const float qq = qi * qj;
-  if (qq != 0.f && r2 < L.es_lim2) {
-    const float u = L.es_A * __expf(-L.es_kappa * r) * rinv;
-    s += qq * (u * (rinv + L.es_kappa) - L.es_fc) * rinv;
+  if (CHARGED) {
+    const float qq = qi * qj;
+    if (qq != 0.f && apart && r2 < L.es_lim2) {
+      const float u = L.es_A * __expf(-L.es_kappa * r) * rinv;
+      s += qq * (u * (rinv + L.es_kappa) - L.es_fc) * rinv;
+    }
   }
   return s;
 }

@@ -11,9 +11,9 @@
 //   center u32 ORIGINAL id                held, bond_rng, thermo_rng u32;  frozen u8
 //   id     u32 slot -> original id        slot_of u32 original id -> slot
 //   pos_ref float4 positions at the last rebuild (drift reference)
-//   nl     u32 [slot][list_cap] Verlet neighbours as SLOT indices; nl_cnt u32 [slot]; each row is
-//          grouped by build distance (shell 0: inside the force's reach; shells 1-4: the skin in four
-//          widths equal in r^2), nl_shell uint4 [slot] the ends of shells 0..3 (shell 4 ends at nl_cnt)
+//   nl     u32 [slot][list_stride] Verlet neighbours as SLOT indices; nl_cnt u32 [slot]; each row is
+//          grouped by build distance (shell 0: inside the force's reach; shells 1-7: the rest of the range in
+//          widths equal in r^2), nl_shell u32 [slot][8] the shells' ends; padded to 16 with the slot itself
 //   heads  u32 original ids of titratable beads (ascending; static);  es_nl [head][es_cap] slots
 #pragma once
 #include <algorithm>
@@ -92,10 +92,11 @@ struct Batch {
   uint32_t *cell_of_slot = nullptr, *cell_count = nullptr, *cell_start = nullptr, *cell_cursor = nullptr;
   uint32_t* perm = nullptr;          // new slot -> old slot
   uint32_t* scan_tmp = nullptr;
-  uint32_t list_cap = 0;             // row stride of nl (max over replicas, rounded to 32)
+  uint32_t list_cap = 0;             // entries a row of nl may hold (max over replicas, rounded to 8)
+  uint32_t list_stride = 0;          // row stride of nl: list_cap rounded to 16
   uint32_t* nl = nullptr;
   uint32_t* nl_cnt = nullptr;
-  uint4* nl_shell = nullptr;
+  uint32_t* nl_shell = nullptr;      // per slot kShells words: where the row's build-distance shells end
   size_t list_smem_set = 0;          // dynamic shared memory k_build_list was opened to
   bool prune = true;                 // force passes read only the shells the drift can have brought in range
 
@@ -157,8 +158,7 @@ struct Batch {
   std::vector<uint64_t> next_sweep;
   uint64_t rebuilds = 0, sweeps = 0;
   bool force_fresh = false;          // force array matches positions+charges+lists
-  int tpp = 4;                       // threads per particle in the list force
-  bool queued = false;               // list force with the in-range pairs compacted per warp (k_force_w)
+  int tpp = 0;                       // threads per particle in the list force (0: by the launch's size)
   uint32_t wait_limit = 0;           // polls of a bounded device-side handoff before it gives up (0: default)
   DiffWindow diff;
   // captured step chunks (CUDA graphs), keyed by length and schedule phase; the drift-triggered
@@ -214,6 +214,7 @@ void launch_build_lists(Batch& b);
 void launch_build_es_lists(Batch& b);
 void launch_force(Batch& b);       // list force, then the far electrostatics half
 void launch_force_list(Batch& b, bool heads = false);
+int force_lanes(const Batch& b, uint32_t n);   // lanes per particle for n particles
 void launch_force_heads(Batch& b);  // the heads' list force and far half only (after a charge sweep)
 void launch_es_far(Batch& b);
 void launch_force_brute(Batch& b);
