@@ -9,6 +9,8 @@
 // every array is physically reordered into cell order at each rebuild (coalesced neighbour reads);
 // list membership uses the exact f32 test of the reference, so the lists equal the oracle's sets.
 // Walks are over x-rows of cells (contiguous slot ranges), a row at a time.
+#include <type_traits>
+
 #include "soup_internal.h"
 
 namespace soup {
@@ -198,15 +200,15 @@ __device__ __forceinline__ float gap_to_cell(float p, int c, float cs) {
 // s > 0 only once the largest displacement since the build can have closed the distance from the reach to
 // that shell's inner edge (list_force_end).
 struct Shells {
-  float reach2, scale;
+  float mul, add;                                        // r2 mul + add = (shell + fraction) / kShells
   __device__ __forceinline__ static Shells of(float reach2, float list_range) {
-    Shells s;
-    s.reach2 = reach2;
-    s.scale = 1.0f / fmaxf(list_shell_width2(reach2, list_range), 1e-12f);
-    return s;
+    const float scale = 1.0f / fmaxf(list_shell_width2(reach2, list_range), 1e-12f);
+    return Shells{scale * (1.0f / kShells), (1.0f - reach2 * scale) * (1.0f / kShells)};
   }
+  // (a shell edge may fall to either side by rounding: list_force_end's margin is far wider)
   __device__ __forceinline__ uint32_t tag(float r2) const {
-    return (uint32_t)(min(max(__float2int_rd((r2 - reach2) * scale), -1), kShells - 2) + 1) << 29;
+    const float x = __saturatef(fmaf(r2, mul, add));
+    return __float_as_uint(__fmaf_rz(x, (float)kShells * 0.999999f, 8388608.0f)) << 29;   // floor in the low bits
   }
 };
 
@@ -219,43 +221,51 @@ struct Shells {
 // candidates: run by run, half the lanes would idle; a thread per particle diverges at every accepted
 // candidate and leaves a small system's chain of dependent loads uncovered.)
 constexpr uint32_t kWalkRuns = 128;                    // runs: two per row, (2 * 3 + 1)^2 rows at walk 3
-constexpr uint32_t kWalkSpan = 4096;                   // candidates whose run starts are marked at a time
-constexpr uint32_t kWalkWords = 2 * kWalkRuns + kWalkSpan / 32;   // shared words a warp's walk needs
+constexpr uint32_t kWalkSpan = 2048;                   // candidates whose run starts are marked at a time
+constexpr uint32_t kWalkWords = 2 * kWalkRuns + 2 * kWalkSpan / 32;   // shared words a warp's walk needs
 
-struct WalkGrid { int dims[3]; int walk; uint32_t cell_off; float range; };
+struct WalkGrid { int dims[3]; int walk; uint32_t cell_off; float range; float cell[3]; float inv_cell_x; };
 
-// take(j, valid): warp-wide, 2 x 32 candidates j (indices into the cell-ordered array) per round
+__device__ __forceinline__ float sqrt_approx(float x) {   // under the walk's margins
+  float y;
+  asm("sqrt.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+  return y;
+}
+
+// take(j0, v0, j1, v1): warp-wide, 2 x 32 candidates j (indices into the cell-ordered array; v: one of the walk's)
 template <class Take>
 __device__ __forceinline__ void warp_walk(const float4& xi, const float* box, const WalkGrid& G,
                                           const uint32_t* __restrict__ start, uint32_t* __restrict__ sm, Take&& take) {
   uint32_t* shift = sm;                                // candidate q of run s is bead q + shift[s]
   uint32_t* first = sm + kWalkRuns;                    // its first candidate
-  uint32_t* mark = sm + 2 * kWalkRuns;                 // bit per candidate: a run starts here
+  uint2* mark = reinterpret_cast<uint2*>(sm + 2 * kWalkRuns);   // per 32 candidates: a bit where a run starts; the
+                                                       // runs that start before them, less one
   const uint32_t lane = threadIdx.x & 31u, lt = (1u << lane) - 1u, le = lt | (1u << lane);
   const int R = G.walk, D = 2 * R + 1;
   const int dx = G.dims[0], dy = G.dims[1], dz = G.dims[2];
   const int qx = ex_cell_axis(xi.x, box[0], dx), qy = ex_cell_axis(xi.y, box[1], dy), qz = ex_cell_axis(xi.z, box[2], dz);
   const bool fx = dx < D, fy = dy < D, fz = dz < D;    // this axis is visited whole
   const int ny = fy ? dy : D, nz = fz ? dz : D;
-  const float csx = box[0] / (float)dx, csy = box[1] / (float)dy, csz = box[2] / (float)dz;
+  const float csy = G.cell[1], csz = G.cell[2], icx = G.inv_cell_x;
   const float lrm = G.range * (1.0f + 1e-5f) + 1e-3f, lrm2 = lrm * lrm;
   uint32_t runs = 0, total = 0;
   for (int r0 = 0; r0 < ny * nz; r0 += 32) {
     const int rr = r0 + (int)lane;
     uint32_t a0 = 0, l0 = 0, a1 = 0, l1 = 0;
     if (rr < ny * nz) {
-      const int iy = rr % ny, iz = rr / ny;
+      const int iz = ny == 5 ? (rr * 205) >> 10 : rr / ny, iy = rr - iz * ny;   // rr < 51 where ny is 5
       const int y = fy ? iy : qy - R + iy, z = fz ? iz : qz - R + iz;
       const float gy = fy ? 0.f : gap_to_cell(xi.y, y, csy), gz = fz ? 0.f : gap_to_cell(xi.z, z, csz);
       const float g2 = gy * gy + gz * gz;
       if (g2 < lrm2) {
-        const uint32_t row = G.cell_off + (uint32_t)(dx * ((y + dy) % dy + dy * ((z + dz) % dz)));
+        const int wy = y < 0 ? y + dy : (y >= dy ? y - dy : y), wz = z < 0 ? z + dz : (z >= dz ? z - dz : z);
+        const uint32_t row = G.cell_off + (uint32_t)(dx * (wy + dy * wz));
         if (fx) {
           a0 = start[row];
           l0 = start[row + (uint32_t)dx] - a0;
         } else {
-          const float ext = sqrtf(lrm2 - g2);
-          const int xlo = max(qx - R, (int)floorf((xi.x - ext) / csx)), xhi = min(qx + R, (int)floorf((xi.x + ext) / csx));
+          const float ext = sqrt_approx(lrm2 - g2) + 1e-3f;
+          const int xlo = max(qx - R, (int)floorf((xi.x - ext) * icx)), xhi = min(qx + R, (int)floorf((xi.x + ext) * icx));
           if (xlo <= xhi) {
             const AxisRange xr = span_ranges(xlo, xhi, dx);
             a0 = start[row + (uint32_t)xr.lo[0]];
@@ -283,43 +293,40 @@ __device__ __forceinline__ void warp_walk(const float4& xi, const float* box, co
     total += __shfl_sync(0xffffffffu, incl, 31);
   }
   __syncwarp();
+  uint32_t before = 0xFFFFFFFFu;                       // the runs that start before the span, less one
   for (uint32_t w0 = 0; w0 < total; w0 += kWalkSpan) {
-    const uint32_t n = min(total - w0, kWalkSpan);
-    for (uint32_t i = lane; i < (n + 63u) / 64u * 2u; i += 32u) mark[i] = 0;
+    const uint32_t n = min(total - w0, kWalkSpan), words = (n + 63u) / 64u * 2u;
+    for (uint32_t i = lane; i < words; i += 32u) mark[i].x = 0;
     __syncwarp();
-    uint32_t before = 0;
-    for (uint32_t s0 = 0; s0 < runs; s0 += 32u) {
-      const uint32_t p = s0 + lane < runs ? first[s0 + lane] : 0xFFFFFFFFu;
-      if (p >= w0 && p - w0 < n) atomicOr(&mark[(p - w0) >> 5], 1u << (p & 31u));
-      before += __popc(__ballot_sync(0xffffffffu, p < w0));
+    for (uint32_t s = lane; s < runs; s += 32u) {
+      const uint32_t p = first[s] - w0;                // the spans ahead wrap round
+      if (p < n) atomicOr(&mark[p >> 5].x, 1u << (p & 31u));
+    }
+    __syncwarp();
+    for (uint32_t i0 = 0; i0 < words; i0 += 32u) {
+      const uint32_t own = i0 + lane < words ? __popc(mark[i0 + lane].x) : 0u;
+      uint32_t incl = own;
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const uint32_t v = __shfl_up_sync(0xffffffffu, incl, o);
+        if (lane >= (uint32_t)o) incl += v;
+      }
+      if (i0 + lane < words) mark[i0 + lane].y = before + incl - own;
+      before += __shfl_sync(0xffffffffu, incl, 31);
     }
     __syncwarp();
     for (uint32_t c = 0; c < n; c += 64u) {
-      const uint2 m = *reinterpret_cast<const uint2*>(&mark[c >> 5]);
-      const uint32_t q0 = w0 + c + lane, q1 = q0 + 32u;
-      const bool v0 = q0 < total, v1 = q1 < total;
-      const uint32_t s0 = before + __popc(m.x & le) - 1u;
-      before += __popc(m.x);
-      const uint32_t s1 = before + __popc(m.y & le) - 1u;
-      before += __popc(m.y);
-      take(v0 ? shift[s0] + q0 : 0u, v0, v1 ? shift[s1] + q1 : 0u, v1);
+      const uint4 m = *reinterpret_cast<const uint4*>(&mark[c >> 5]);
+      const uint32_t q0 = w0 + c + lane, q1 = q0 + 32u, c0 = min(q0, total - 1u), c1 = min(q1, total - 1u);
+      // (a place past the end reads the last run's last candidate, which its v leaves out)
+      const uint32_t s0 = min(m.y + __popc(m.x & le), runs - 1u), s1 = min(m.w + __popc(m.z & le), runs - 1u);
+      take(shift[s0] + c0, q0 < total, shift[s1] + c1, q1 < total);
     }
     __syncwarp();
   }
 }
 
-// eight 12-bit counters, five to a word
-struct Count8 {
-  unsigned long long a, b;
-  __device__ __forceinline__ uint32_t at(uint32_t t) const {
-    return (uint32_t)(t < 5u ? a >> (12u * t) : b >> (12u * (t - 5u))) & 0xFFFu;
-  }
-  __device__ __forceinline__ void add(uint32_t t, unsigned long long n) {
-    if (t < 5u) a += n << (12u * t);
-    else b += n << (12u * (t - 5u));
-  }
-};
-constexpr uint32_t kGRegs = 17;                        // entries a lane can hold while a row is grouped
+constexpr uint32_t kGRegs = 16;                        // entries a lane holds while a row is grouped
 
 // soup/wgsl/verlet.wgsl:53-92, a warp per particle (warp_walk).  The fast squared distance decides unless it
 // lies within 1e-5 of the range, where the reference's arithmetic decides (the minimum image cannot differ
@@ -354,11 +361,12 @@ __global__ void __launch_bounds__(128) k_build_list(
   const float rm = lr * (1.0f + 1e-5f) + 1e-3f;
   const bool direct = xi.x >= rm && xi.x <= box[0] - rm && xi.y >= rm && xi.y <= box[1] - rm && xi.z >= rm &&
                       xi.z <= box[2] - rm;
-  const WalkGrid G{{P.dims[0], P.dims[1], P.dims[2]}, P.walk, P.cell_off, lr};
+  const WalkGrid G{{P.dims[0], P.dims[1], P.dims[2]}, P.walk, P.cell_off, lr, {P.cell[0], P.cell[1], P.cell[2]}, P.inv_cell[0]};
   uint32_t cnt = 0;
-  auto test = [&](uint32_t j, bool v, const float4& xj) -> uint32_t {   // the tagged entry, or NONE
+  // 32 candidates: the accepted ones, tagged, behind the row
+  auto put = [&](auto image, uint32_t j, bool v, const float4& xj) {
     float dx = xi.x - xj.x, dy = xi.y - xj.y, dz = xi.z - xj.z;
-    if (!direct) {
+    if (decltype(image)::value) {
       dx = fast_mi(dx, box[0], inv[0]);
       dy = fast_mi(dy, box[1], inv[1]);
       dz = fast_mi(dz, box[2], inv[2]);
@@ -366,66 +374,62 @@ __global__ void __launch_bounds__(128) k_build_list(
     const float r2 = dx * dx + dy * dy + dz * dz;
     bool in = v && j != k && r2 <= lr2_hi;
     if (in && r2 >= lr2_lo) in = ex_dist(xi, xj, box) < lr;
-    return in ? (j | sh.tag(r2)) : SOUP_NONE_U32;
+    const uint32_t m = __ballot_sync(0xffffffffu, in), at = cnt + __popc(m & lt);
+    if (in && at < cap) row[at] = j | sh.tag(r2);
+    cnt = __shfl_sync(0xffffffffu, at + (in ? 1u : 0u), 31);
   };
-  auto put = [&](uint32_t e) {
-    const bool in = e != SOUP_NONE_U32;
-    const uint32_t m = __ballot_sync(0xffffffffu, in);
-    const uint32_t at = cnt + __popc(m & lt);
-    if (in && at < cap) row[at] = e;
-    cnt += __popc(m);
+  auto walk = [&](auto image) {
+    warp_walk(xi, box, G, start, row + stride, [&](uint32_t j0, bool v0, uint32_t j1, bool v1) {
+      const float4 x0 = pos[j0], x1 = pos[j1];
+      put(image, j0, v0, x0);
+      put(image, j1, v1, x1);
+    });
   };
-  warp_walk(xi, box, G, start, row + stride, [&](uint32_t j0, bool v0, uint32_t j1, bool v1) {
-    const float4 x0 = pos[j0], x1 = pos[j1];
-    const uint32_t e0 = test(j0, v0, x0), e1 = test(j1, v1, x1);
-    put(e0);
-    put(e1);
-  });
+  if (direct) walk(std::false_type{});
+  else walk(std::true_type{});
   if (cnt > cap) {
     if (lane == 0) flags[0] = 1u;
     cnt = cap;
   }
   __syncwarp();
-  // group the row by shell.  Up to 32 * 16 entries: lane l holds a contiguous piece, counts its entries per
-  // shell (12-bit counters), one warp scan of them gives every lane its places,
-  // and the pieces are written back in lane order.  A longer row (dense aggregates) goes out shell by
-  // shell with ballots.  Both keep the walk's order inside a shell.
+  // group the row by shell, keeping the walk's order inside a shell: 32 entries at a time, three ballots of the
+  // shell's bits give every lane the entries of its own shell (its place among them) and lane s those of shell s
+  // (the shells' running ends).  A longer row than the registers hold (dense aggregates) goes out shell by shell.
   uint32_t* out = nl + (size_t)k * stride;
   const uint32_t full = (cnt + 15u) & ~15u;          // rows are padded with the particle itself
   uint32_t e[kShells - 1];
-  if (cnt <= 32u * (kGRegs - 1u)) {
-    const uint32_t piece = ((cnt + 31u) >> 5) | 1u;    // odd: no bank conflicts
-    const uint32_t s0 = lane * piece, s1 = min(s0 + piece, cnt);
-    uint32_t v[kGRegs];
-    Count8 mine{0, 0};
+  if (cnt <= 32u * kGRegs) {
+    // lane l stands for shell l mod 8: a ballot of bit i xor this is ones where bit i is the shell's
+    const uint32_t y0 = (lane & 1u) - 1u, y1 = ((lane >> 1) & 1u) - 1u, y2 = ((lane >> 2) & 1u) - 1u;
+    uint32_t v[kGRegs], end = 0;
 #pragma unroll
     for (uint32_t c = 0; c < kGRegs; ++c) {
-      if (c >= piece) break;
-      v[c] = s0 + c < s1 ? row[s0 + c] : SOUP_NONE_U32;
-      if (v[c] != SOUP_NONE_U32) mine.add(v[c] >> 29, 1ull);
+      if (32u * c >= cnt) break;
+      v[c] = 32u * c + lane < cnt ? row[32u * c + lane] : SOUP_NONE_U32;   // beyond the row: the last shell
+      const uint32_t b0 = __ballot_sync(0xffffffffu, v[c] & 0x20000000u), b1 = __ballot_sync(0xffffffffu, v[c] & 0x40000000u),
+                     b2 = __ballot_sync(0xffffffffu, v[c] & 0x80000000u);
+      end += __popc((b0 ^ y0) & (b1 ^ y1) & (b2 ^ y2));
     }
-    Count8 incl = mine;
+    uint32_t incl = end;                               // the shells' ends
 #pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-      const unsigned long long ya = __shfl_up_sync(0xffffffffu, incl.a, o), yb = __shfl_up_sync(0xffffffffu, incl.b, o);
-      if (lane >= (uint32_t)o) { incl.a += ya; incl.b += yb; }
+    for (int o = 1; o < kShells; o <<= 1) {
+      const uint32_t y = __shfl_up_sync(0xffffffffu, incl, o);
+      if ((lane & 7u) >= (uint32_t)o) incl += y;
     }
-    const Count8 tot{__shfl_sync(0xffffffffu, incl.a, 31), __shfl_sync(0xffffffffu, incl.b, 31)};
-    Count8 at{incl.a - mine.a, incl.b - mine.b};       // this lane's next place in every shell
-    uint32_t run = 0;
+    uint32_t next = incl - end;                        // the shells' next places
 #pragma unroll
-    for (uint32_t t = 0; t < (uint32_t)kShells; ++t) {
-      at.add(t, run);
-      run += tot.at(t);
-      if (t + 1u < (uint32_t)kShells) e[t] = run;
-    }
+    for (uint32_t t = 0; t + 1u < (uint32_t)kShells; ++t) e[t] = __shfl_sync(0xffffffffu, incl, (int)t);
+    __syncwarp();
 #pragma unroll
     for (uint32_t c = 0; c < kGRegs; ++c) {
-      if (c >= piece) break;
-      if (v[c] == SOUP_NONE_U32) continue;
-      const uint32_t t = v[c] >> 29;
-      row[at.at(t)] = v[c] & 0x1FFFFFFFu;
-      at.add(t, 1ull);
+      if (32u * c >= cnt) break;
+      const uint32_t b0 = __ballot_sync(0xffffffffu, v[c] & 0x20000000u), b1 = __ballot_sync(0xffffffffu, v[c] & 0x40000000u),
+                     b2 = __ballot_sync(0xffffffffu, v[c] & 0x80000000u);
+      const uint32_t x0 = ~(uint32_t)((int)(v[c] << 2) >> 31), x1 = ~(uint32_t)((int)(v[c] << 1) >> 31),
+                     x2 = ~(uint32_t)((int)v[c] >> 31);
+      const uint32_t at = __shfl_sync(0xffffffffu, next, (int)(v[c] >> 29)) + __popc((b0 ^ x0) & (b1 ^ x1) & (b2 ^ x2) & lt);
+      if (32u * c + lane < cnt) row[at] = v[c] & 0x1FFFFFFFu;
+      next += __popc((b0 ^ y0) & (b1 ^ y1) & (b2 ^ y2));
     }
     if (cnt + lane < full) row[cnt + lane] = k;
     __syncwarp();
@@ -527,7 +531,8 @@ __global__ void __launch_bounds__(128) k_build_es_list(const uint32_t* __restric
   const float inv[3] = {P.inv_box[0], P.inv_box[1], P.inv_box[2]};
   const float lr = P.es_list_range;
   const float lo = lr * lr * (1.0f - 1e-5f), hi = lr * lr * (1.0f + 1e-5f);
-  const WalkGrid G{{P.hdims[0], P.hdims[1], P.hdims[2]}, P.hwalk, P.hcell_off, lr};
+  const WalkGrid G{{P.hdims[0], P.hdims[1], P.hdims[2]}, P.hwalk, P.hcell_off, lr, {P.hcell[0], P.hcell[1], P.hcell[2]},
+                   P.inv_hcell[0]};
   uint32_t cnt = 0;
   uint32_t* row = es_nl + (size_t)h * cap;
   auto put = [&](const float4& xj, bool v) {

@@ -213,6 +213,10 @@ void alloc_grids(Batch& b) {
 void upload_params(Batch& b) {
   for (uint32_t r = 0; r < b.R; ++r) {
     SysParams& p = b.hsp[r];
+    for (int a = 0; a < 3; ++a) {
+      p.cell[a] = p.box[a] / (float)p.dims[a]; p.inv_cell[a] = (float)p.dims[a] / p.box[a];
+      p.hcell[a] = p.box[a] / (float)p.hdims[a]; p.inv_hcell[a] = (float)p.hdims[a] / p.box[a];
+    }
     for (int wide = 0; wide < 2; ++wide) {
       const float reach2 = wide ? b.hs.rmax2 : b.hs.rplain2, w2 = list_shell_width2(reach2, p.list_range);
       p.reach[wide] = std::sqrt(reach2);

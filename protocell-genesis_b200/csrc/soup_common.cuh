@@ -41,6 +41,7 @@ struct SysParams {
   int hdims[3];              // head grid
   int hwalk;                 // head-grid walk radius (cells)
   uint32_t hcell_off;
+  float cell[3], inv_cell[3], hcell[3], inv_hcell[3];   // cell sides of the two grids and their inverses
   uint32_t list_cap, es_cap; // capacities (overflow threshold)
   uint32_t sweep_draws;      // draws of a block of the constant-pH walk: 512 or 256
   uint32_t es_on;            // electrostatics enabled
