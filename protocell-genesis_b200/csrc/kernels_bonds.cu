@@ -63,83 +63,104 @@ __global__ void __launch_bounds__(256) k_bond_select(const Shared* __restrict__ 
   if (act) sel[base + __popc(m & ((1u << lane) - 1u))] = k;
 }
 
-// a thread per active bead (k_bond_select), so that the warps walk full
+// A warp per active bead (k_bond_select): the lanes test 32 row entries at a time, up to where the row can hold a
+// pair in contact (list_force_end: contacts lie within the force's reach).  The few that qualify are kept by
+// all lanes alike, the SOUP_CAND_CAP smallest ids in order.  (A thread per bead walked its row entry by
+// entry, 200 us at 3k beads and 350 us at 483k, waiting on one gather after another.)
 __global__ void __launch_bounds__(128) k_bond_walk(
     const Shared* __restrict__ Sg, const SysParams* __restrict__ sp, const uint8_t* __restrict__ sysid,
     const uint32_t* __restrict__ sel, const uint32_t* __restrict__ nsel,
-    const float4* __restrict__ pos, const uint32_t* __restrict__ id, const uint32_t* __restrict__ slots,
-    const uint32_t* __restrict__ center, const uint32_t* __restrict__ nl, const uint32_t* __restrict__ nl_cnt,
-    uint32_t cap, uint32_t* __restrict__ brng, uint32_t* __restrict__ items, uint32_t* __restrict__ nitems,
+    const float4* __restrict__ pos, const float* __restrict__ charge, const uint32_t* __restrict__ id,
+    const uint32_t* __restrict__ slots, const uint32_t* __restrict__ center, const uint32_t* __restrict__ nl,
+    const uint32_t* __restrict__ nl_cnt, const uint32_t* __restrict__ nl_shell, const uint32_t* __restrict__ drift_bits,
+    uint32_t stride, uint32_t* __restrict__ brng, uint32_t* __restrict__ items, uint32_t* __restrict__ nitems,
     uint32_t* __restrict__ has_item) {
   const uint32_t ns = *nsel;
-  if (blockIdx.x * blockDim.x >= ns) return;   // the whole block: past the active beads
+  if (blockIdx.x * 4u >= ns) return;   // the whole block: past the active beads
   __shared__ Shared S;
   for (int w = threadIdx.x; w < (int)(sizeof(Shared) / 4); w += blockDim.x)
     reinterpret_cast<uint32_t*>(&S)[w] = reinterpret_cast<const uint32_t*>(Sg)[w];
   __syncthreads();
-  const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= ns) return;
-  const uint32_t k = sel[t];
-  const float4 xi = pos[k];
-  const float ti = xi.w;
-  const SysParams& P = sp[sysid[k]];
-  const float box[3] = {P.box[0], P.box[1], P.box[2]};
-  const uint32_t gi = id[k];
-  const uint32_t s0 = slots[3 * k], s1 = slots[3 * k + 1], s2 = slots[3 * k + 2];
-  const float cat_reach = ex_wcut(S, ex_pairB(S, ti, S.cat_kind));
-  uint32_t catId = NONE;
-  uint32_t cj[SOUP_CAND_CAP], cr[SOUP_CAND_CAP];
-  int nc = 0;
-  const uint32_t cnt = nl_cnt[k];
-  const uint32_t* row = nl + (size_t)k * cap;
-  for (uint32_t s = 0; s < cnt; ++s) {
-    const uint32_t js = row[s];
-    const float4 xj = pos[js];
-    const float tj = xj.w;
-    const bool isCat = tj == S.cat_kind;
-    const int rk = match_rule(S, ti, tj);        // by the kinds alone
-    if (!isCat && rk < 0) continue;
-    const uint32_t j = id[js];
-    int r = -1;
-    if (j > gi) {
-      r = rk;
-      if (r >= 0 && (s0 == j || s1 == j || s2 == j)) r = -1;          // hasBondTo
-      if (r >= 0 && nc == SOUP_CAND_CAP && j > cj[SOUP_CAND_CAP - 1]) r = -1;
+  const uint32_t lane = threadIdx.x & 31u;
+  for (uint32_t t = blockIdx.x * 4u + (threadIdx.x >> 5); t < ns; t += gridDim.x * 4u) {
+    const uint32_t k = sel[t];
+    const float4 xi = pos[k];
+    const float ti = xi.w;
+    const uint32_t rs = sysid[k];
+    const SysParams& P = sp[rs];
+    const float box[3] = {P.box[0], P.box[1], P.box[2]};
+    const uint32_t gi = id[k];
+    const uint32_t s0 = slots[3 * k], s1 = slots[3 * k + 1], s2 = slots[3 * k + 2];
+    const float cat_reach = ex_wcut(S, ex_pairB(S, ti, S.cat_kind));
+    uint32_t catId = NONE;
+    uint32_t cj[SOUP_CAND_CAP], cr[SOUP_CAND_CAP];
+#pragma unroll
+    for (int c = 0; c < SOUP_CAND_CAP; ++c) { cj[c] = NONE; cr[c] = 0; }
+    const uint32_t end = list_force_end(k, nl_cnt, nl_shell, __uint_as_float(drift_bits[rs]), P,
+                                        list_wide(S, P, (int)ti & (SOUP_KMAX - 1), charge[k]));
+    // the force reads whole chunks: entries of the next shells lie among those up to its end
+    const uint32_t last = min((end + 15u) & ~15u, nl_cnt[k]);
+    const uint32_t* row = nl + (size_t)k * stride;
+    for (uint32_t b = 0; b < last; b += 32u) {
+      const uint32_t s = b + lane;
+      const uint32_t js = s < last ? row[s] : k;
+      const float4 xj = pos[js];
+      const float tj = xj.w;
+      const bool isCat = js != k && tj == S.cat_kind;
+      const int rk = js != k ? match_rule(S, ti, tj) : -1;
+      uint32_t hit_j = NONE;
+      if (isCat || rk >= 0) {
+        const uint32_t j = id[js];
+        const float d = ex_dist(xi, xj, box);
+        if (isCat && d < cat_reach) catId = min(catId, j);                  // smallest catalyst in reach
+        if (rk >= 0 && j > gi && s0 != j && s1 != j && s2 != j && d < ex_wcut(S, ex_pairB(S, ti, tj))) hit_j = j;
+      }
+      for (uint32_t m = __ballot_sync(0xffffffffu, hit_j != NONE); m; m &= m - 1u) {
+        uint32_t j = __shfl_sync(0xffffffffu, hit_j, __ffs(m) - 1);
+        uint32_t r = (uint32_t)__shfl_sync(0xffffffffu, rk, __ffs(m) - 1);
+#pragma unroll
+        for (int c = 0; c < SOUP_CAND_CAP; ++c)      // insert, ascending; the largest drops out
+          if (j < cj[c]) {
+            const uint32_t oj = cj[c], orr = cr[c];
+            cj[c] = j; cr[c] = r;
+            j = oj; r = orr;
+          }
+      }
     }
-    if (!isCat && r < 0) continue;
-    const float d = ex_dist(xi, xj, box);
-    if (isCat && d < cat_reach && j < catId) catId = j;                // smallest catalyst in reach
-    if (r >= 0 && d < ex_wcut(S, ex_pairB(S, ti, tj))) {
-      // keep the SOUP_CAND_CAP smallest qualifying j, ascending
-      int p = nc < SOUP_CAND_CAP ? nc : SOUP_CAND_CAP - 1;
-      if (nc < SOUP_CAND_CAP) ++nc;
-      while (p > 0 && cj[p - 1] > j) { cj[p] = cj[p - 1]; cr[p] = cr[p - 1]; --p; }
-      cj[p] = j; cr[p] = (uint32_t)r;
+    catId = __reduce_min_sync(0xffffffffu, catId);
+    // draws (bondFormDecide's candidate loop up to the claims), on every lane alike
+    uint32_t rng = brng[k];
+    uint32_t pj[SOUP_CAND_CAP];
+    uint32_t meta = 0;
+    int np = 0;
+#pragma unroll
+    for (int c = 0; c < SOUP_CAND_CAP; ++c) {
+      pj[c] = NONE;
+      if (cj[c] == NONE) continue;
+      const uint32_t r = cr[c];
+      if (S.req_cat[r] > 0.5f && catId == NONE) continue;
+      rng = pcg_hash(rng);
+      if (u01(rng) >= S.att_form[r]) continue;
+      rng = pcg_hash(rng);
+      if (u01(rng) >= S.acc_form[r]) continue;
+      pj[c] = cj[c];
+      meta |= r << (8 + 2 * np);
+      ++np;
     }
-  }
-  // draws (bondFormDecide's candidate loop up to the claims)
-  uint32_t rng = brng[k];
-  uint32_t pj[SOUP_CAND_CAP];
-  uint32_t meta = 0;
-  int np = 0;
-  for (int c = 0; c < nc; ++c) {
-    const uint32_t r = cr[c];
-    if (S.req_cat[r] > 0.5f && catId == NONE) continue;
-    rng = pcg_hash(rng);
-    if (u01(rng) >= S.att_form[r]) continue;
-    rng = pcg_hash(rng);
-    if (u01(rng) >= S.acc_form[r]) continue;
-    pj[np] = cj[c];
-    meta |= r << (8 + 2 * np);
-    ++np;
-  }
-  brng[k] = rng;
-  if (np > 0 || ti == S.cat_kind || center[k] != NONE) {
-    const uint32_t at = atomicAdd(nitems, 1u);
-    uint32_t* rec = items + (size_t)at * REC;
-    rec[0] = gi; rec[1] = catId; rec[2] = meta | (uint32_t)np;
-    for (int c = 0; c < SOUP_CAND_CAP; ++c) rec[3 + c] = c < np ? pj[c] : NONE;
-    has_item[gi] = 1;
+    if (lane == 0) {
+      brng[k] = rng;
+      if (np > 0 || ti == S.cat_kind || center[k] != NONE) {
+        const uint32_t at = atomicAdd(nitems, 1u);
+        uint32_t* rec = items + (size_t)at * REC;
+        rec[0] = gi; rec[1] = catId; rec[2] = meta | (uint32_t)np;
+        int n = 0;
+#pragma unroll
+        for (int c = 0; c < SOUP_CAND_CAP; ++c)
+          if (pj[c] != NONE) rec[3 + n++] = pj[c];
+        for (; n < SOUP_CAND_CAP; ++n) rec[3 + n] = NONE;
+        has_item[gi] = 1;
+      }
+    }
   }
 }
 
@@ -401,6 +422,31 @@ __global__ void __launch_bounds__(1024) k_bond_claims(
   }
   __syncthreads();
   St st{S, sp, sysid, pos, slots, center, held, slot_of, events, desorb};
+  // the rounds behind the first one hold a few items: with at most 32 items a thread, its pending ones are bits
+  // of a word
+  if (L <= 32u * blockDim.x) {
+    uint32_t pend = 0;
+    for (uint32_t q = 0, u = threadIdx.x; u < L; ++q, u += blockDim.x) pend |= (item(u) != NONE ? 1u : 0u) << q;
+    while (__syncthreads_or(pend != 0)) {
+      for (uint32_t m = pend; m; m &= m - 1u) {
+        const uint32_t* rec = items + (size_t)item(threadIdx.x + (uint32_t)(__ffs(m) - 1) * blockDim.x) * REC;
+        atomicMin(&comp_min[rec[9]], rec[0]);
+      }
+      __syncthreads();
+      uint32_t left = 0;
+      for (uint32_t m = pend; m; m &= m - 1u) {
+        const uint32_t* rec = items + (size_t)item(threadIdx.x + (uint32_t)(__ffs(m) - 1) * blockDim.x) * REC;
+        if (comp_min[rec[9]] == rec[0]) st.run(rec);
+        else left |= m & (0u - m);
+      }
+      __syncthreads();
+      for (uint32_t m = left; m; m &= m - 1u)
+        comp_min[items[(size_t)item(threadIdx.x + (uint32_t)(__ffs(m) - 1) * blockDim.x) * REC + 9]] = NONE;
+      pend = left;
+      __syncthreads();
+    }
+    return;
+  }
   for (int round = 0;; ++round) {
     int pending = 0;
     for (uint32_t u = threadIdx.x; u < L; u += blockDim.x) {
@@ -467,9 +513,9 @@ void launch_bonds(Batch& b) {
   uint32_t* has_item = b.has_item;
   k_bond_select<<<nblocks(b.N, 256), 256, 0, b.stream>>>(b.shared, b.N, b.pos, b.center, b.bond_sel,
                                                          b.bond_nitems + 2);
-  k_bond_walk<<<nblocks(b.N, 128), 128, 0, b.stream>>>(b.shared, b.sp, b.sysid, b.bond_sel, b.bond_nitems + 2, b.pos,
-                                                       b.id, b.slots, b.center, b.nl, b.nl_cnt, b.list_stride, b.brng,
-                                                       b.bond_items, b.bond_nitems, has_item);
+  k_bond_walk<<<std::min(nblocks(b.N, 4), 148u * 16u), 128, 0, b.stream>>>(
+      b.shared, b.sp, b.sysid, b.bond_sel, b.bond_nitems + 2, b.pos, b.charge, b.id, b.slots, b.center, b.nl, b.nl_cnt,
+      b.prune ? b.nl_shell : nullptr, b.drift_bits, b.list_stride, b.brng, b.bond_items, b.bond_nitems, has_item);
   cudaMemcpyAsync(b.bond_nitems + 1, b.bond_nitems, sizeof(uint32_t), cudaMemcpyDeviceToDevice, b.stream);
   k_bond_partners<<<std::max(1u, std::min(nblocks(b.N, 256) / 8u, 592u)), 256, 0, b.stream>>>(
       b.center, b.slot_of, b.bond_items, b.bond_nitems, b.N, has_item, b.flags);

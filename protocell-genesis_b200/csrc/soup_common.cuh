@@ -162,6 +162,22 @@ __device__ __forceinline__ bool list_wide(const Shared& S, const SysParams& P, i
   return charge != 0.f || S.cls[kind] == 1u || kind == P.charged_kind;
 }
 
+// The end of the part of particle k's row a force pass must read.  The row is grouped by build
+// distance (k_build_list): shell 0 within the force's reach r0 (a plain bead's or a wide one's, list_wide), shells
+// 1..7 the rest of the list range in widths w2 of r^2.  No bead has moved more than dm since the build (the replica's largest
+// drift), so a pair of shell s is at least sqrt(r0^2 + (s - 1) w2) - 2 dm apart now, and shell s can hold
+// an in-range pair only if r0^2 + (s - 1) w2 < (r0 + 2 dm)^2 (a margin of 1e-3 sigma covers rounding).
+// Skipped entries are beyond the reach, so the force is the same bits as over the whole row.
+__device__ __forceinline__ uint32_t list_force_end(uint32_t k, const uint32_t* __restrict__ nl_cnt,
+                                                   const uint32_t* __restrict__ nl_shell, float drift2,
+                                                   const SysParams& P, bool wide) {
+  const float scale = P.shell_scale[wide];
+  if (!nl_shell || !(drift2 >= 0.f && drift2 < 1e30f) || !(scale > 0.f)) return nl_cnt[k];
+  const float d = 2.0f * sqrtf(drift2) + 1e-3f;
+  const float x = d * (2.0f * P.reach[wide] + d) * scale;   // (r0 + d)^2 - r0^2 in shells
+  return nl_shell[(size_t)kShells * k + 1u + (uint32_t)fminf(x, (float)(kShells - 2))];
+}
+
 // The pair loop's constants of one replica, held in registers (batch-wide numbers from Shared, the
 // replica's acid-soap depth and screened-Coulomb numbers from its SysParams).
 struct PairLean {
