@@ -345,10 +345,10 @@ int soup_aggregate_labels(SoupHandle* h, const uint32_t* member_idx, uint32_t n_
                           double cutoff, uint32_t* labels, uint32_t* n_components);
 
 /* The same labels as soup_aggregate_labels, computed without allocating device memory.  It has no
- * counterpart in the reference.  soup_aggregate_labels allocates its scratch with cudaMalloc and
- * frees it with cudaFree on every call; a caller whose device memory is held by another allocator
- * (a framework's caching allocator that reserved the GPU) may see that cudaMalloc fail, and the
- * cudaFree stalls every stream on the device.  This entry point keeps its scratch in one fixed
+ * counterpart in the reference.  soup_aggregate_labels keeps its scratch with the system and
+ * grows it (cudaMalloc, cudaFree) when a request is larger than any before; a caller whose device
+ * memory is held by another allocator (a framework's caching allocator that reserved the GPU) may see
+ * that cudaMalloc fail, and the cudaFree stalls every stream on the device.  This entry point keeps its scratch in one fixed
  * array that the library holds on each GPU it runs on (about 9.4 MB, for as long as the process
  * lives), so it needs no allocation and no free.
  *   Limits: n_members <= SOUP_NOALLOC_MAX_MEMBERS and floor(box_x/cutoff) * floor(box_y/cutoff)

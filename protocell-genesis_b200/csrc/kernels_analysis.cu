@@ -90,31 +90,83 @@ __global__ void k_seed_min_index(const uint8_t* __restrict__ occ, uint64_t nc, G
   if ((unsigned long long)__double_as_longlong(seed_d2(g, c, i)) + 1ull == *best) atomicMin(idx, (unsigned long long)i);
 }
 
-// floodOutsidePeriodic (water-closure.ts:154-189), one BFS level per launch
-__global__ void k_flood_level(const uint8_t* __restrict__ occ, uint32_t* __restrict__ vis, Grid g,
-                              const uint32_t* __restrict__ front, const uint32_t* __restrict__ nfront,
-                              uint32_t* __restrict__ next, uint32_t* __restrict__ nnext, uint32_t cap) {
-  const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= *nfront) return;
-  const uint32_t i = front[t];
-  const int z = (int)(i / ((uint32_t)g.nx * g.ny));
-  const uint32_t rem = i - (uint32_t)z * g.nx * g.ny;
-  const int y = (int)(rem / g.nx), x = (int)(rem - (uint32_t)y * g.nx);
-  const int nb[6][3] = {{(x + 1) % g.nx, y, z}, {(x - 1 + g.nx) % g.nx, y, z}, {x, (y + 1) % g.ny, z},
-                        {x, (y - 1 + g.ny) % g.ny, z}, {x, y, (z + 1) % g.nz}, {x, y, (z - 1 + g.nz) % g.nz}};
-  for (int q = 0; q < 6; ++q) {
-    const uint32_t ni = (uint32_t)nb[q][0] + (uint32_t)g.nx * ((uint32_t)nb[q][1] + (uint32_t)g.ny * nb[q][2]);
-    if (occ[ni]) continue;
-    if (atomicCAS(&vis[ni], 0u, 1u) == 0u) {
-      const uint32_t at = atomicAdd(nnext, 1u);
-      if (at < cap) next[at] = ni;
-    }
+// ---- union-find helpers (hook the larger root under the smaller: roots are component minima) ----
+__device__ __forceinline__ uint32_t uf_find(uint32_t* parent, uint32_t x) {
+  volatile uint32_t* vp = parent;
+  uint32_t p = vp[x];
+  while (p != x) { x = p; p = vp[x]; }
+  return x;
+}
+// the same, halving the path behind it (a parent is only ever replaced by an ancestor)
+__device__ __forceinline__ uint32_t uf_find_halve(uint32_t* parent, uint32_t x) {
+  volatile uint32_t* vp = parent;
+  uint32_t p = vp[x];
+  while (p != x) {
+    const uint32_t q = vp[p];
+    if (q != p) vp[x] = q;
+    x = p;
+    p = q;
   }
+  return x;
+}
+__device__ __forceinline__ void uf_union(uint32_t* parent, uint32_t a, uint32_t b) {
+  for (;;) {
+    a = uf_find_halve(parent, a);
+    b = uf_find_halve(parent, b);
+    if (a == b) return;
+    if (a > b) { const uint32_t t = a; a = b; b = t; }
+    if (atomicCAS(&parent[b], b, a) == b) return;
+  }
+}
+
+// floodOutsidePeriodic (water-closure.ts:154-189): the empty cells the flood from the seed reaches are the
+// seed's component under the six periodic neighbours, found by union-find in three launches whatever the
+// flood's depth (a breadth-first level per launch took a hundred launches and host waits, 4 ms a closure).
+// Every empty cell starts under the first cell of its run of 32 along x; a cell joins its left run only across
+// the runs' borders, and the row before it in y and z only where the pair one cell to the left does not do so
+// already.
+__global__ void k_flood_init(const uint8_t* __restrict__ occ, uint32_t nc, uint32_t nx, uint32_t* __restrict__ parent) {
+  const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x, lane = threadIdx.x & 31u;
+  const bool empty = i < nc && !occ[i];
+  const uint32_t em = __ballot_sync(0xffffffffu, empty);
+  const bool first = empty && (lane == 0 || !((em >> (lane - 1u)) & 1u) || i % nx == 0);
+  const uint32_t fm = __ballot_sync(0xffffffffu, first);
+  if (i >= nc) return;
+  parent[i] = empty ? i - lane + (31u - (uint32_t)__clz(fm & (0xFFFFFFFFu >> (31u - lane)))) : i;
+}
+__global__ void k_flood_union(const uint8_t* __restrict__ occ, uint32_t nc, Grid g, uint32_t* __restrict__ parent) {
+  const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= nc || occ[i]) return;
+  const uint32_t nx = (uint32_t)g.nx, ny = (uint32_t)g.ny, nz = (uint32_t)g.nz;
+  const uint32_t row = i / nx, x = i - row * nx, z = row / ny, y = row - z * ny;
+  const bool left = x > 0 && !occ[i - 1];
+  if (left && (i & 31u) == 0) uf_union(parent, i, i - 1);
+  if (x == 0 && !occ[i + nx - 1]) uf_union(parent, i, i + nx - 1);
+  const uint32_t by = y > 0 ? i - nx : i + (ny - 1) * nx, bz = z > 0 ? i - nx * ny : i + (nz - 1) * nx * ny;
+  if (!occ[by] && !(left && !occ[by - 1])) uf_union(parent, i, by);
+  if (!occ[bz] && !(left && !occ[bz - 1])) uf_union(parent, i, bz);
+}
+__global__ void k_flood_mark(const uint8_t* __restrict__ occ, uint32_t nc, const unsigned long long* __restrict__ seed,
+                             uint32_t* __restrict__ parent, uint8_t* __restrict__ vis) {
+  const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= nc) return;
+  vis[i] = *seed < nc && !occ[i] && uf_find_halve(parent, i) == uf_find(parent, (uint32_t)*seed) ? 1 : 0;
+}
+
+// a block's sum of three counts added to out[0..2], one atomic each (whole blocks; every thread calls it)
+__device__ __forceinline__ void add_counts(uint32_t a, uint32_t b, uint32_t c, unsigned long long* out) {
+  __shared__ uint32_t tot[3];
+  if (threadIdx.x < 3) tot[threadIdx.x] = 0;
+  __syncthreads();
+  a = __reduce_add_sync(0xffffffffu, a); b = __reduce_add_sync(0xffffffffu, b); c = __reduce_add_sync(0xffffffffu, c);
+  if ((threadIdx.x & 31) == 0) { atomicAdd(&tot[0], a); atomicAdd(&tot[1], b); atomicAdd(&tot[2], c); }
+  __syncthreads();
+  if (threadIdx.x < 3 && tot[threadIdx.x]) atomicAdd(&out[threadIdx.x], (unsigned long long)tot[threadIdx.x]);
 }
 
 // cell counts and water classification (water-closure.ts:297-327)
 // reachedEmpty counts only cells whose centre lies in the parcel when pr2 >= 0 (water-closure.ts:323-337)
-__global__ void k_cell_counts(const uint8_t* __restrict__ occ, const uint32_t* __restrict__ vis, uint64_t nc, Grid g,
+__global__ void k_cell_counts(const uint8_t* __restrict__ occ, const uint8_t* __restrict__ vis, uint64_t nc, Grid g,
                               double pcx, double pcy, double pcz, double pr2,
                               unsigned long long* __restrict__ out /* totalEmpty, unreached, reachedEmpty */) {
   const uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
@@ -134,40 +186,20 @@ __global__ void k_cell_counts(const uint8_t* __restrict__ occ, const uint32_t* _
       c = sq3(ex, ey, ez) > pr2 ? 0u : 1u;
     }
   }
-  for (int o = 16; o > 0; o >>= 1) {
-    a += __shfl_xor_sync(0xffffffffu, a, o); b += __shfl_xor_sync(0xffffffffu, b, o); c += __shfl_xor_sync(0xffffffffu, c, o);
-  }
-  if ((threadIdx.x & 31) == 0) { atomicAdd(&out[0], a); atomicAdd(&out[1], b); atomicAdd(&out[2], c); }
+  add_counts(a, b, c, out);
 }
 __global__ void k_water(const float4* __restrict__ pos, const uint32_t* __restrict__ slot_of, uint32_t off,
                         const uint32_t* __restrict__ wat, uint32_t nw, Grid g, const uint8_t* __restrict__ occ,
-                        const uint32_t* __restrict__ vis, unsigned long long* __restrict__ out /* enc, reachedWater */) {
+                        const uint8_t* __restrict__ vis, unsigned long long* __restrict__ out /* enc, reachedWater, - */) {
   const uint32_t k = blockIdx.x * blockDim.x + threadIdx.x;
-  if (k >= nw) return;
-  const float4 p = pos[slot_of[off + wat[k]]];
+  const bool mine = k < nw;
+  const float4 p = pos[mine ? slot_of[off + wat[k]] : off];
   const int gx = min(g.nx - 1, (int)floor(__ddiv_rn(wrap1((double)p.x, g.box[0]), g.cell)));
   const int gy = min(g.ny - 1, (int)floor(__ddiv_rn(wrap1((double)p.y, g.box[1]), g.cell)));
   const int gz = min(g.nz - 1, (int)floor(__ddiv_rn(wrap1((double)p.z, g.box[2]), g.cell)));
   const size_t c = (size_t)gx + (size_t)g.nx * ((size_t)gy + (size_t)g.ny * gz);
-  if (occ[c]) return;
-  atomicAdd(&out[vis[c] ? 1 : 0], 1ull);
-}
-
-// ---- union-find helpers (hook the larger root under the smaller: roots are component minima) ----
-__device__ __forceinline__ uint32_t uf_find(uint32_t* parent, uint32_t x) {
-  volatile uint32_t* vp = parent;
-  uint32_t p = vp[x];
-  while (p != x) { x = p; p = vp[x]; }
-  return x;
-}
-__device__ __forceinline__ void uf_union(uint32_t* parent, uint32_t a, uint32_t b) {
-  for (;;) {
-    a = uf_find(parent, a);
-    b = uf_find(parent, b);
-    if (a == b) return;
-    if (a > b) { const uint32_t t = a; a = b; b = t; }
-    if (atomicCAS(&parent[b], b, a) == b) return;
-  }
+  const bool in = mine && !occ[c];
+  add_counts(in && !vis[c], in && vis[c], 0, out);
 }
 
 // findAmphiphiles (amphiphile.ts:55-141) on the bond graph, indices local to the replica
@@ -231,40 +263,65 @@ __global__ void k_agg_bin(const float4* __restrict__ pos, const uint32_t* __rest
   cell[k] = c;
   atomicAdd(&count[c], 1u);
 }
-__global__ void k_agg_scatter(const uint32_t* __restrict__ cell, uint32_t m, const uint32_t* __restrict__ start,
-                              uint32_t* __restrict__ cursor, uint32_t* __restrict__ sorted) {
+__global__ void k_agg_scatter(const float4* __restrict__ pos, const uint32_t* __restrict__ slot_of, uint32_t off,
+                              const uint32_t* __restrict__ mem, const uint32_t* __restrict__ cell, uint32_t m,
+                              const uint32_t* __restrict__ start, uint32_t* __restrict__ cursor,
+                              float4* __restrict__ sorted) {
   const uint32_t k = blockIdx.x * blockDim.x + threadIdx.x;
   if (k >= m) return;
   const uint32_t c = cell[k];
-  sorted[start[c] + atomicAdd(&cursor[c], 1u)] = k;
+  const float4 p = pos[slot_of[off + mem[k]]];
+  sorted[start[c] + atomicAdd(&cursor[c], 1u)] = make_float4(p.x, p.y, p.z, __uint_as_float(k));   // w: the member
 }
-__global__ void k_agg_union(const float4* __restrict__ pos, const uint32_t* __restrict__ slot_of, uint32_t off,
-                            const uint32_t* __restrict__ mem, uint32_t m, Grid g, const uint32_t* __restrict__ cell,
-                            const uint32_t* __restrict__ start, const uint32_t* __restrict__ sorted, double c2,
-                            int periodic_z, uint32_t* __restrict__ parent) {
-  const uint32_t k = blockIdx.x * blockDim.x + threadIdx.x;
-  if (k >= m) return;
-  const float4 pi = pos[slot_of[off + mem[k]]];
-  const uint32_t c = cell[k];
-  const int cz = (int)(c / ((uint32_t)g.nx * g.ny)), cy = (int)((c / g.nx) % g.ny), cx = (int)(c % g.nx);
-  for (int dx = -1; dx <= 1; ++dx) {
-    const int ax = ((cx + dx) % g.nx + g.nx) % g.nx;
-    for (int dy = -1; dy <= 1; ++dy) {
-      const int ay = ((cy + dy) % g.ny + g.ny) % g.ny;
-      for (int dz = -1; dz <= 1; ++dz) {
-        const int az = ((cz + dz) % g.nz + g.nz) % g.nz;
-        const uint32_t nc = (uint32_t)ax + (uint32_t)g.nx * ((uint32_t)ay + (uint32_t)g.ny * az);
-        for (uint32_t t = start[nc]; t < start[nc + 1]; ++t) {
-          const uint32_t l = sorted[t];
-          if (l <= k) continue;
-          const float4 pj = pos[slot_of[off + mem[l]]];
-          const double ddx = mi1(__dsub_rn((double)pi.x, (double)pj.x), g.box[0]);
-          const double ddy = mi1(__dsub_rn((double)pi.y, (double)pj.y), g.box[1]);
-          const double rz = __dsub_rn((double)pi.z, (double)pj.z);
-          const double ddz = periodic_z ? mi1(rz, g.box[2]) : rz;
-          if (sq3(ddx, ddy, ddz) <= c2) uf_union(parent, k, l);
-        }
+// A warp per member, over the members in cell order: a run of candidates per (y, z) row and wrapped x piece, a
+// lane each.  The reference's FP64 test decides only where the FP32 distance lies within a margin of the
+// cutoff ten times its error (roundings of coordinates and box: a few 1e-7 of the box).  (A thread per member, with three dependent loads and three FP64
+// divisions a candidate: 826 us at 16,500 members.)
+__global__ void k_agg_union(const float4* __restrict__ sorted, uint32_t m, Grid g, double wx, double wy, double wz,
+                            const uint32_t* __restrict__ start, double c2, int periodic_z, uint32_t* __restrict__ parent) {
+  const uint32_t w = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31u;
+  if (w >= m) return;   // whole warps
+  const float4 pi = sorted[w];
+  const uint32_t k = __float_as_uint(pi.w);
+  const float lx = (float)g.box[0], ly = (float)g.box[1], lz = (float)g.box[2];
+  const float c = sqrtf((float)c2), margin = 1e-4f * c + 1e-6f * fmaxf(lx, fmaxf(ly, lz));
+  const float lo = c > margin ? (c - margin) * (c - margin) : 0.f, hi = (c + margin) * (c + margin);
+  const int cx = min(g.nx - 1, (int)floor(__ddiv_rn(wrap1((double)pi.x, g.box[0]), wx)));
+  const int cy = min(g.ny - 1, (int)floor(__ddiv_rn(wrap1((double)pi.y, g.box[1]), wy)));
+  const int cz = min(g.nz - 1, (int)floor(__ddiv_rn(wrap1((double)pi.z, g.box[2]), wz)));
+  // x - 1 .. x + 1 as at most two pieces of a row; axes of up to three cells are visited whole
+  const int x0 = g.nx <= 3 ? 0 : cx - 1, x1 = g.nx <= 3 ? g.nx - 1 : cx + 1;
+  const int ylo = g.ny <= 3 ? 0 : cy - 1, yhi = g.ny <= 3 ? g.ny - 1 : cy + 1;
+  const int zlo = g.nz <= 3 ? 0 : cz - 1, zhi = g.nz <= 3 ? g.nz - 1 : cz + 1;
+  auto scan = [&](uint32_t a, uint32_t e) {
+    for (uint32_t t = a + lane; t < e; t += 32u) {
+      const float4 pj = sorted[t];
+      const uint32_t l = __float_as_uint(pj.w);
+      if (l <= k) continue;
+      float dx = pi.x - pj.x, dy = pi.y - pj.y, dz = pi.z - pj.z;
+      dx -= rintf(dx / lx) * lx;
+      dy -= rintf(dy / ly) * ly;
+      if (periodic_z) dz -= rintf(dz / lz) * lz;
+      const float r2 = dx * dx + dy * dy + dz * dz;
+      if (r2 > hi) continue;
+      if (r2 >= lo) {
+        const double ddx = mi1(__dsub_rn((double)pi.x, (double)pj.x), g.box[0]);
+        const double ddy = mi1(__dsub_rn((double)pi.y, (double)pj.y), g.box[1]);
+        const double rz = __dsub_rn((double)pi.z, (double)pj.z);
+        const double ddz = periodic_z ? mi1(rz, g.box[2]) : rz;
+        if (!(sq3(ddx, ddy, ddz) <= c2)) continue;
       }
+      uf_union(parent, k, l);
+    }
+  };
+  for (int z = zlo; z <= zhi; ++z) {
+    const int az = z < 0 ? z + g.nz : (z >= g.nz ? z - g.nz : z);
+    for (int y = ylo; y <= yhi; ++y) {
+      const int ay = y < 0 ? y + g.ny : (y >= g.ny ? y - g.ny : y);
+      const uint32_t row = (uint32_t)g.nx * ((uint32_t)ay + (uint32_t)g.ny * az);
+      scan(start[row + (uint32_t)max(x0, 0)], start[row + (uint32_t)min(x1, g.nx - 1) + 1u]);
+      if (x0 < 0) scan(start[row + (uint32_t)(g.nx - 1)], start[row + (uint32_t)g.nx]);
+      if (x1 >= g.nx) scan(start[row], start[row + 1u]);
     }
   }
 }
@@ -290,19 +347,6 @@ __global__ void k_fill(uint32_t* __restrict__ a, uint32_t n, uint32_t v) {
   const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i < n) a[i] = v;
 }
-
-// scratch that lives for one call of the aggregate labels (soup_aggregate_labels allocates and
-// frees per call, as its declaration states; the other analysis calls use the batch's scratch)
-struct Scratch {
-  std::vector<void*> ptrs;
-  ~Scratch() { for (void* p : ptrs) cudaFree(p); }
-  template <class T> T* get(size_t n) {
-    T* p = nullptr;
-    SOUP_CUDA_TRY(cudaMalloc(&p, std::max<size_t>(n, 1) * sizeof(T)));
-    ptrs.push_back(p);
-    return p;
-  }
-};
 
 }  // namespace
 
@@ -338,21 +382,18 @@ int run_closure(Batch& b, uint32_t r, const uint32_t* mem, uint32_t nm, const ui
   if (nc >= 0xFFFFFFF0ull) { err = "closure: grid too large"; return SOUP_E_ARG; }
   const int reach = std::max(1, (int)std::ceil(radius / cell));
   ScratchLayout L;
-  const size_t o_occ = L.add<uint8_t>(nc), o_vis = L.add<uint32_t>(nc), o_mem = L.add<uint32_t>(nm),
-               o_wat = L.add<uint32_t>(nw), o_fa = L.add<uint32_t>(nc), o_fb = L.add<uint32_t>(nc),
-               o_cnt = L.add<uint32_t>(2), o_u64 = L.add<unsigned long long>(8);
+  const size_t o_occ = L.add<uint8_t>(nc), o_vis = L.add<uint8_t>(nc), o_mem = L.add<uint32_t>(nm),
+               o_wat = L.add<uint32_t>(nw), o_par = L.add<uint32_t>(nc), o_u64 = L.add<unsigned long long>(8);
   char* base = analysis_scratch(b, L.used);
   uint8_t* occ = reinterpret_cast<uint8_t*>(base + o_occ);
-  uint32_t* vis = reinterpret_cast<uint32_t*>(base + o_vis);
+  uint8_t* vis = reinterpret_cast<uint8_t*>(base + o_vis);
   uint32_t* dmem = reinterpret_cast<uint32_t*>(base + o_mem);
   uint32_t* dwat = reinterpret_cast<uint32_t*>(base + o_wat);
-  uint32_t* fa = reinterpret_cast<uint32_t*>(base + o_fa);
-  uint32_t* fb = reinterpret_cast<uint32_t*>(base + o_fb);
-  uint32_t* cnt = reinterpret_cast<uint32_t*>(base + o_cnt);
+  uint32_t* parent = reinterpret_cast<uint32_t*>(base + o_par);
+  // [0] the seed's distance, [1] its cell, [2..4] cell counts, [5..7] water counts
   unsigned long long* u64 = reinterpret_cast<unsigned long long*>(base + o_u64);
   cudaStream_t st = b.stream;
   SOUP_CUDA_TRY(cudaMemsetAsync(occ, 0, nc, st));
-  SOUP_CUDA_TRY(cudaMemsetAsync(vis, 0, 4 * nc, st));
   SOUP_CUDA_TRY(cudaMemsetAsync(u64, 0, 64, st));
   if (nm) SOUP_CUDA_TRY(cudaMemcpyAsync(dmem, mem, 4 * (size_t)nm, cudaMemcpyHostToDevice, st));
   if (nw) SOUP_CUDA_TRY(cudaMemcpyAsync(dwat, wat, 4 * (size_t)nw, cudaMemcpyHostToDevice, st));
@@ -362,33 +403,18 @@ int run_closure(Batch& b, uint32_t r, const uint32_t* mem, uint32_t nm, const ui
   const unsigned long long init_idx = ~0ull;
   SOUP_CUDA_TRY(cudaMemcpyAsync(u64 + 1, &init_idx, 8, cudaMemcpyHostToDevice, st));
   k_seed_min_index<<<nblocks(nc), kBlock, 0, st>>>(occ, nc, g, centre[0], centre[1], centre[2], u64, u64 + 1);
-  unsigned long long best[2];
-  SOUP_CUDA_TRY(cudaMemcpyAsync(best, u64, 16, cudaMemcpyDeviceToHost, st));
-  SOUP_CUDA_TRY(cudaStreamSynchronize(st));
-  if (best[0] == 0) { err = "farthestEmptyCellSeed: the grid is fully occupied -- there is no empty cell to seed the periodic flood fill"; return SOUP_E_STATE; }
-  const uint32_t seed = (uint32_t)best[1];
-  const uint32_t one = 1;
-  SOUP_CUDA_TRY(cudaMemcpyAsync(vis + seed, &one, 4, cudaMemcpyHostToDevice, st));
-  SOUP_CUDA_TRY(cudaMemcpyAsync(fa, &seed, 4, cudaMemcpyHostToDevice, st));
-  SOUP_CUDA_TRY(cudaMemcpyAsync(cnt, &one, 4, cudaMemcpyHostToDevice, st));
-  uint32_t* front = fa; uint32_t* next = fb;
-  uint32_t* nfront = cnt; uint32_t* nnext = cnt + 1;
-  uint32_t level_size = 1;
-  while (level_size > 0) {
-    SOUP_CUDA_TRY(cudaMemsetAsync(nnext, 0, 4, st));
-    k_flood_level<<<nblocks(level_size), kBlock, 0, st>>>(occ, vis, g, front, nfront, next, nnext, (uint32_t)nc);
-    b.launches += 1;
-    SOUP_CUDA_TRY(cudaMemcpyAsync(&level_size, nnext, 4, cudaMemcpyDeviceToHost, st));
-    SOUP_CUDA_TRY(cudaStreamSynchronize(st));
-    std::swap(front, next);
-    std::swap(nfront, nnext);
-  }
+  const uint32_t nc32 = (uint32_t)nc;
+  k_flood_init<<<nblocks(nc), kBlock, 0, st>>>(occ, nc32, (uint32_t)g.nx, parent);
+  k_flood_union<<<nblocks(nc), kBlock, 0, st>>>(occ, nc32, g, parent);
+  k_flood_mark<<<nblocks(nc), kBlock, 0, st>>>(occ, nc32, u64 + 1, parent, vis);
   k_cell_counts<<<nblocks(nc), kBlock, 0, st>>>(occ, vis, nc, g, parcel ? parcel[0] : 0.0, parcel ? parcel[1] : 0.0,
                                                 parcel ? parcel[2] : 0.0, parcel ? parcel[3] * parcel[3] : -1.0, u64 + 2);
   if (nw) k_water<<<nblocks(nw), kBlock, 0, st>>>(b.pos, b.slot_of, off, dwat, nw, g, occ, vis, u64 + 5);
   unsigned long long res[8];
   SOUP_CUDA_TRY(cudaMemcpyAsync(res, u64, 64, cudaMemcpyDeviceToHost, st));
   SOUP_CUDA_TRY(cudaStreamSynchronize(st));
+  if (res[0] == 0) { err = "farthestEmptyCellSeed: the grid is fully occupied -- there is no empty cell to seed the periodic flood fill"; return SOUP_E_STATE; }
+  const uint32_t seed = (uint32_t)res[1];
   const double reached_empty = (double)res[4];
   const double bulk = res[4] > 0 ? (double)res[6] / (reached_empty * cell * cell * cell) : 0.0;
   const double thr = bulk > 0 ? vmin * bulk : NAN;
@@ -457,18 +483,16 @@ int run_aggregates(Batch& b, uint32_t r, const uint32_t* mem, uint32_t m, double
   g.nz = std::max(1, (int)std::floor(c.box[2] / cutoff));
   g.cell = 0;
   const uint32_t nc = (uint32_t)((uint64_t)g.nx * g.ny * g.nz);
-  Scratch S;
-  uint32_t* dmem = S.get<uint32_t>(m);
-  uint32_t* cell = S.get<uint32_t>(m);
-  uint32_t* count = S.get<uint32_t>(nc + 1);
-  uint32_t* start = S.get<uint32_t>(nc + 1);
-  uint32_t* cursor = S.get<uint32_t>(nc + 1);
-  uint32_t* sorted = S.get<uint32_t>(m);
-  uint32_t* parent = S.get<uint32_t>(m);
-  uint32_t* minidx = S.get<uint32_t>(m);
-  uint32_t* dl = S.get<uint32_t>(m);
-  uint32_t* cnt = S.get<uint32_t>(1);
-  uint32_t* tmp = S.get<uint32_t>(4 * (nc / 4096 + 64) + 256);
+  ScratchLayout L;
+  const size_t o_mem = L.add<uint32_t>(m), o_cell = L.add<uint32_t>(m), o_count = L.add<uint32_t>((size_t)nc + 1),
+               o_start = L.add<uint32_t>((size_t)nc + 1), o_cursor = L.add<uint32_t>((size_t)nc + 1), o_sorted = L.add<float4>(m),
+               o_parent = L.add<uint32_t>(m), o_min = L.add<uint32_t>(m), o_dl = L.add<uint32_t>(m), o_cnt = L.add<uint32_t>(1),
+               o_tmp = L.add<uint32_t>(4 * (size_t)(nc / 4096 + 64) + 256);
+  char* base = analysis_scratch(b, L.used);
+  auto at = [&](size_t o) { return reinterpret_cast<uint32_t*>(base + o); };
+  uint32_t *dmem = at(o_mem), *cell = at(o_cell), *count = at(o_count), *start = at(o_start), *cursor = at(o_cursor),
+           *parent = at(o_parent), *minidx = at(o_min), *dl = at(o_dl), *cnt = at(o_cnt), *tmp = at(o_tmp);
+  float4* sorted = reinterpret_cast<float4*>(base + o_sorted);
   cudaStream_t st = b.stream;
   SOUP_CUDA_TRY(cudaMemcpyAsync(dmem, mem, 4 * (size_t)m, cudaMemcpyHostToDevice, st));
   SOUP_CUDA_TRY(cudaMemsetAsync(count, 0, 4 * ((size_t)nc + 1), st));
@@ -478,11 +502,11 @@ int run_aggregates(Batch& b, uint32_t r, const uint32_t* mem, uint32_t m, double
   k_agg_bin<<<nblocks(m), kBlock, 0, st>>>(b.pos, b.slot_of, off, dmem, m, g, c.box[0] / g.nx, c.box[1] / g.ny,
                                            c.box[2] / g.nz, cell, count);
   exclusive_scan(count, start, nc, tmp, st);
-  k_agg_scatter<<<nblocks(m), kBlock, 0, st>>>(cell, m, start, cursor, sorted);
+  k_agg_scatter<<<nblocks(m), kBlock, 0, st>>>(b.pos, b.slot_of, off, dmem, cell, m, start, cursor, sorted);
   k_iota<<<nblocks(m), kBlock, 0, st>>>(parent, m);
   k_fill<<<nblocks(m), kBlock, 0, st>>>(minidx, m, NONE);
-  k_agg_union<<<nblocks(m), kBlock, 0, st>>>(b.pos, b.slot_of, off, dmem, m, g, cell, start, sorted, cutoff * cutoff,
-                                             periodic_z ? 1 : 0, parent);
+  k_agg_union<<<nblocks((uint64_t)m * 32), kBlock, 0, st>>>(sorted, m, g, c.box[0] / g.nx, c.box[1] / g.ny, c.box[2] / g.nz,
+                                                           start, cutoff * cutoff, periodic_z ? 1 : 0, parent);
   k_agg_min<<<nblocks(m), kBlock, 0, st>>>(dmem, m, parent, minidx, cnt);
   k_agg_label<<<nblocks(m), kBlock, 0, st>>>(dmem, m, parent, minidx, dl);
   SOUP_CUDA_TRY(cudaMemcpyAsync(labels, dl, 4 * (size_t)m, cudaMemcpyDeviceToHost, st));

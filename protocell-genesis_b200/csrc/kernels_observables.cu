@@ -156,7 +156,7 @@ namespace {
 // Unwrapped coordinates are rounded to f32 as the reference stores them (a Float32Array), then
 // summed in FP64 in two passes (centre, then the second moments about it), each a fixed-order block
 // reduction.  out[c]: n, centre x y z, Sxx Syy Szz Sxy Sxz Syz (per member).
-constexpr int kShapeThreads = 256;
+constexpr int kShapeThreads = 1024;   // a large aggregate is one block: its gathers' latency sets the time
 __device__ __forceinline__ double block_sum(double v, double* sh) {
   sh[threadIdx.x] = v;
   __syncthreads();
