@@ -43,10 +43,29 @@ struct ThetaAcc {
   }
 };
 
+// one particle's depth partials by the neighbour's class (its own class is fixed: an index into the nine would
+// put them in local memory)
+struct DepthAcc {
+  double c0 = 0.0, c1 = 0.0, c2 = 0.0;
+  __device__ __forceinline__ void add(uint32_t cls, double x) {
+    c0 += cls == 0u ? x : 0.0;
+    c1 += cls == 1u ? x : 0.0;
+    c2 += cls == 2u ? x : 0.0;
+  }
+  __device__ __forceinline__ void to(ThetaAcc& th, uint32_t own) const {
+#pragma unroll
+    for (int p = 0; p < 6; ++p) {
+      th.v[p] += depth_index(own, 0u) == p ? c0 : 0.0;
+      th.v[p] += depth_index(own, 1u) == p ? c1 : 0.0;
+      th.v[p] += depth_index(own, 2u) == p ? c2 : 0.0;
+    }
+  }
+};
+
 // the nonbonded pair terms of the list (pair_scalar's three terms): s, s' and the parameter partials
 template <class PP>
 __device__ __forceinline__ void pair_terms(const Shared& S, const PP& P, const PairConst& pc, float r2, int ki, int kj,
-                                           float qi, float qj, float gd, float& s, float& sp, ThetaAcc& th) {
+                                           float qi, float qj, float gd, float& s, float& sp, ThetaAcc& th, DepthAcc& dep) {
   const float rinv = rsqrtf(r2);
   const float r = r2 * rinv;
   const float rinv2 = rinv * rinv;
@@ -61,13 +80,11 @@ __device__ __forceinline__ void pair_terms(const Shared& S, const PP& P, const P
   if (r >= S.rc_attr && r <= S.rc_attr + S.wc) {   // attraction: s = -scale amp sin(2x) / r
     float scale = pc.attr;
     if (P.acid > 0.f && ((qi != 0.f) != (qj != 0.f)) && S.cls[ki] == 1u && S.cls[kj] == 1u) scale += P.acid;
-    const float x = (r - S.rc_attr) * S.attr_k;
     float sn, cs;
-    sincosf(2.0f * x, &sn, &cs);
+    sincospif((r - S.rc_attr) * (1.0f / S.wc), &sn, &cs);   // sin(2x), 2x = pi (r - rc) / wc
     s -= scale * S.attr_amp * sn * rinv;
     sp -= scale * S.attr_amp * (2.0f * S.attr_k * cs * rinv - sn * rinv2);
-    const int p = depth_index(S.cls[ki], S.cls[kj]);
-    if (p >= 0) th.v[p] += (double)(-S.attr_amp * sn * rinv) * (double)gd;
+    dep.add(S.cls[kj], (double)(-S.attr_amp * sn * rinv) * (double)gd);
   }
   const float qq = qi * qj;
   if (qq != 0.f && r < P.es_split && r < P.es_rc && P.es_A != 0.f) {   // near screened Coulomb
@@ -138,15 +155,18 @@ __device__ __forceinline__ void block_theta(const ThetaAcc& th, double* __restri
 }
 
 // (J g) of the list force (nonbonded + bonded + wall) and the parameter partials, kTpp lanes per
-// particle; jg is written (not accumulated), by original index
+// particle; jg is written (not accumulated), by original index.  gs: g in slot order, so that an entry is two
+// independent gathers.  Rows are read as far as the force reads them (list_force_end; drift: the largest
+// displacement of the frame since the lists' build): the rest is beyond the reach.  Bound: the gathers.
 __global__ void __launch_bounds__(kBlock) k_hvp(const Shared* __restrict__ Sg, const SysParams* __restrict__ sp,
                                                 const uint8_t* __restrict__ sysid, uint32_t N,
                                                 const float4* __restrict__ pos, const float* __restrict__ charge,
                                                 const uint32_t* __restrict__ slots, const uint32_t* __restrict__ center,
                                                 const uint32_t* __restrict__ id, const uint32_t* __restrict__ slot_of,
                                                 const uint32_t* __restrict__ nl, const uint32_t* __restrict__ nl_cnt,
-                                                uint32_t cap, const float4* __restrict__ g, float4* __restrict__ jg,
-                                                double* __restrict__ partial) {
+                                                const uint32_t* __restrict__ nl_shell, const uint32_t* __restrict__ drift,
+                                                uint32_t cap, const float4* __restrict__ g, const float4* __restrict__ gs,
+                                                float4* __restrict__ jg, double* __restrict__ partial) {
   __shared__ Shared S;
   for (int w = threadIdx.x; w < (int)(sizeof(Shared) / 4); w += blockDim.x)
     reinterpret_cast<uint32_t*>(&S)[w] = reinterpret_cast<const uint32_t*>(Sg)[w];
@@ -159,14 +179,19 @@ __global__ void __launch_bounds__(kBlock) k_hvp(const Shared* __restrict__ Sg, c
   float jx = 0.f, jy = 0.f, jz = 0.f;
   const bool active = k < N;
   if (active) {
-    const SysParams& Pg = sp[sysid[k]];
+    const uint32_t rs = sysid[k];
+    const SysParams& Pg = sp[rs];
     const PairP P = PairP::of(Pg);
     const float4 xi = pos[k];
     const int ki = (int)xi.w;
     const float qi = charge[k];
     const uint32_t gi = id[k];
-    const float4 gi4 = g[gi];
-    const uint32_t cnt = nl_cnt[k];
+    const float4 gi4 = gs[k];
+    const bool needq = qi != 0.f || S.cls[ki] == 1u;
+    DepthAcc dep;
+    // whole chunks of 16 (the entries of the next shells lie among those up to a shell's end)
+    const uint32_t cnt = min((list_force_end(k, nl_cnt, nl_shell, __uint_as_float(drift[rs]), Pg, list_wide(S, Pg, ki, qi)) + 15u) & ~15u,
+                             nl_cnt[k]);
     const uint32_t* row = nl + (size_t)k * cap;
     const PairConst* prow = &S.pair[ki * SOUP_KMAX];
     for (uint32_t e = (uint32_t)lane; e < cnt; e += kTpp) {
@@ -178,14 +203,15 @@ __global__ void __launch_bounds__(kBlock) k_hvp(const Shared* __restrict__ Sg, c
       const float r2 = dx * dx + dy * dy + dz * dz;
       if (r2 >= S.rmax2 || r2 < 1e-12f) continue;
       const int kj = (int)xj.w;
-      const float qj = charge[j];
+      const float qj = needq ? charge[j] : 0.f;
+      const float4 gj = gs[j];
       const float gd = gi4.x * dx + gi4.y * dy + gi4.z * dz;
       float s, spr;
-      pair_terms(S, P, prow[kj], r2, ki, kj, qi, qj, gd, s, spr, th);
+      pair_terms(S, P, prow[kj], r2, ki, kj, qi, qj, gd, s, spr, th, dep);
       if (s == 0.f && spr == 0.f) continue;
-      const float4 gj = g[id[j]];
       add_m(s, spr, rsqrtf(r2), dx, dy, dz, gi4.x - gj.x, gi4.y - gj.y, gi4.z - gj.z, jx, jy, jz);
     }
+    dep.to(th, S.cls[ki]);
     uint32_t sl[3] = {slots[3 * k], slots[3 * k + 1], slots[3 * k + 2]};
     const uint32_t owner = center[k];
     if ((sl[0] & sl[1] & sl[2] & owner) != SOUP_NONE_U32)
@@ -212,13 +238,11 @@ __global__ void __launch_bounds__(kBlock) k_hvp(const Shared* __restrict__ Sg, c
 }
 
 // the far screened-Coulomb half (split <= r < rc_es) over the head lists, a warp per head; added
-__global__ void __launch_bounds__(kBlock) k_hvp_far(const SysParams* __restrict__ sp, const uint32_t* __restrict__ head_slot,
-                                                    const uint32_t* __restrict__ head_sys, uint32_t H,
-                                                    const float4* __restrict__ pos, const float* __restrict__ charge,
-                                                    const uint32_t* __restrict__ id, const uint32_t* __restrict__ es_nl,
+__global__ void __launch_bounds__(kBlock) k_hvp_far(const SysParams* __restrict__ sp, const uint32_t* __restrict__ head_sys, uint32_t H,
+                                                    const float4* __restrict__ xq, const float4* __restrict__ gh,
+                                                    const uint32_t* __restrict__ heads, const uint32_t* __restrict__ es_nl,
                                                     const uint32_t* __restrict__ es_cnt, uint32_t cap,
-                                                    const float4* __restrict__ g, float4* __restrict__ jg,
-                                                    double* __restrict__ partial) {
+                                                    float4* __restrict__ jg, double* __restrict__ partial) {
   const uint32_t h = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const int lane = threadIdx.x & 31;
   ThetaAcc th;
@@ -228,21 +252,20 @@ __global__ void __launch_bounds__(kBlock) k_hvp_far(const SysParams* __restrict_
   bool live = false;
   if (h < H) {
     const SysParams& P = sp[head_sys[h]];
-    const uint32_t ks = head_slot[h];
-    const float qi = charge[ks];
+    const float4 xi = xq[h];
+    const float qi = xi.w;
     if (qi != 0.f && P.es_A != 0.f) {
       live = true;
-      const float4 xi = pos[ks];
-      gi = id[ks];
-      const float4 gi4 = g[gi];
+      gi = heads[h];
+      const float4 gi4 = gh[h];
       const uint32_t cnt = es_cnt[h];
       const uint32_t* row = es_nl + (size_t)h * cap;
       const float ekc = expf(-P.es_kappa * P.es_rc);
       for (uint32_t s = lane; s < cnt; s += 32) {
-        const uint32_t j = head_slot[row[s]];
-        const float qj = charge[j];
+        const uint32_t j = row[s];
+        const float4 xj = xq[j], gj = gh[j];
+        const float qj = xj.w;
         if (qj == 0.f) continue;
-        const float4 xj = pos[j];
         const float dx = fast_mi(xi.x - xj.x, P.box[0], P.inv_box[0]);
         const float dy = fast_mi(xi.y - xj.y, P.box[1], P.inv_box[1]);
         const float dz = fast_mi(xi.z - xj.z, P.box[2], P.inv_box[2]);
@@ -257,7 +280,6 @@ __global__ void __launch_bounds__(kBlock) k_hvp_far(const SysParams* __restrict_
         const float gp = -P.es_A * ek * (2.0f * rinv2 * rinv + 2.0f * P.es_kappa * rinv2 + P.es_kappa * P.es_kappa * rinv);
         const float s_ = qq * gg * rinv;
         const float sp_ = qq * (gp * rinv - gg * rinv2);
-        const float4 gj = g[id[j]];
         add_m(s_, sp_, rinv, dx, dy, dz, gi4.x - gj.x, gi4.y - gj.y, gi4.z - gj.z, jx, jy, jz);
         const double gd = (double)(gi4.x * dx + gi4.y * dy + gi4.z * dz);
         th.v[8] += (double)(qq * rinv * (-P.es_kappa * P.es_A * (ek - ekc))) * gd;
@@ -274,6 +296,51 @@ __global__ void __launch_bounds__(kBlock) k_hvp_far(const SysParams* __restrict_
     jg[gi] = make_float4(a.x + jx, a.y + jy, a.z + jz, 0.f);
   }
   block_theta(th, partial);
+}
+
+// g in slot order, and the heads' records (position, charge) and g by head index
+__global__ void k_hvp_gather(uint32_t N, const uint32_t* __restrict__ id, const float4* __restrict__ g,
+                             float4* __restrict__ gs) {
+  const uint32_t k = blockIdx.x * blockDim.x + threadIdx.x;
+  if (k < N) gs[k] = g[id[k]];
+}
+__global__ void k_hvp_heads(uint32_t H, const uint32_t* __restrict__ head_slot, const uint32_t* __restrict__ heads,
+                            const float4* __restrict__ pos, const float* __restrict__ charge,
+                            const float4* __restrict__ g, float4* __restrict__ xq, float4* __restrict__ gh) {
+  const uint32_t h = blockIdx.x * blockDim.x + threadIdx.x;
+  if (h >= H) return;
+  const uint32_t k = head_slot[h];
+  const float4 p = pos[k];
+  xq[h] = make_float4(p.x, p.y, p.z, charge[k]);
+  gh[h] = g[heads[h]];
+}
+
+// the largest squared displacement of each of blockIdx.y's frames (original order, `step` apart downwards from
+// `top`) from where the lists were built, per replica: bits[frame][replica], zeroed by the caller
+__global__ void __launch_bounds__(kBlock) k_frames_drift(const SysParams* __restrict__ sp, const uint8_t* __restrict__ sysid,
+                                                         uint32_t N, uint32_t R, const float4* __restrict__ top, size_t step,
+                                                         const uint32_t* __restrict__ id, const float4* __restrict__ pos_ref,
+                                                         uint32_t* __restrict__ bits) {
+  const uint32_t k = blockIdx.x * blockDim.x + threadIdx.x;
+  const float4* frame = top - step * blockIdx.y;
+  uint32_t d = 0, r = 0;
+  if (k < N) {
+    r = sysid[k];
+    const SysParams& P = sp[r];
+    const float4 x = frame[id[k]], p0 = pos_ref[k];
+    const float dx = ex_mi(__fsub_rn(x.x, p0.x), P.box[0]);
+    const float dy = ex_mi(__fsub_rn(x.y, p0.y), P.box[1]);
+    const float dz = ex_mi(__fsub_rn(x.z, p0.z), P.box[2]);
+    d = __float_as_uint(__fadd_rn(__fadd_rn(__fmul_rn(dx, dx), __fmul_rn(dy, dy)), __fmul_rn(dz, dz)));
+  }
+  uint32_t* b = bits + (size_t)blockIdx.y * R;
+  const uint32_t r0 = __shfl_sync(0xffffffffu, r, 0);
+  if (__all_sync(0xffffffffu, r == r0 || k >= N)) {
+    d = __reduce_max_sync(0xffffffffu, d);
+    if ((threadIdx.x & 31) == 0) atomicMax(&b[r0], d);
+  } else if (k < N) {
+    atomicMax(&b[r], d);
+  }
 }
 
 __global__ void k_unpermute(const float4* __restrict__ pos, const uint32_t* __restrict__ id, uint32_t N,
@@ -320,15 +387,27 @@ void adj_scatter_pos(Batch& b, const float4* src) {
 // (J g) at the device's current positions and lists, into jg (original order); the parameter
 // partials are added to each block's running sums in partial_dev (zeroed by the caller before the
 // first step, summed by adj_theta_sum after the last), so the reverse pass never waits on the host
-void adj_hvp(Batch& b, const float4* g, float4* jg, double* partial_dev) {
+// (scratch: the re-sort's second velocity buffer and the head-cell gather, free outside a rebuild)
+void adj_hvp(Batch& b, const uint32_t* drift, const float4* g, float4* jg, double* partial_dev) {
   const unsigned g1 = nblocks((uint64_t)b.N * kTpp, kBlock);
   const unsigned g2 = b.H ? nblocks((uint64_t)b.H * 32, kBlock) : 0;
-  b.launches += 1 + (g2 ? 1 : 0);
+  b.launches += 2 + (g2 ? 2 : 0);
+  k_hvp_gather<<<nblocks(b.N), kBlock, 0, b.stream>>>(b.N, b.id, g, b.vel2);
   k_hvp<<<g1, kBlock, 0, b.stream>>>(b.shared, b.sp, b.sysid, b.N, b.pos, b.charge, b.slots, b.center, b.id, b.slot_of,
-                                     b.nl, b.nl_cnt, b.list_stride, g, jg, partial_dev);
-  if (g2)
-    k_hvp_far<<<g2, kBlock, 0, b.stream>>>(b.sp, b.head_slot, b.head_sys, b.H, b.pos, b.charge, b.id, b.es_nl,
-                                           b.es_cnt, b.es_cap, g, jg, partial_dev + (size_t)g1 * SOUP_DIFF_NPARAM);
+                                     b.nl, b.nl_cnt, b.prune ? b.nl_shell : nullptr, drift, b.list_stride, g, b.vel2, jg,
+                                     partial_dev);
+  if (g2) {
+    k_hvp_heads<<<nblocks(b.H), kBlock, 0, b.stream>>>(b.H, b.head_slot, b.heads, b.pos, b.charge, g, b.head_xq,
+                                                       b.hsorted_xg);
+    k_hvp_far<<<g2, kBlock, 0, b.stream>>>(b.sp, b.head_sys, b.H, b.head_xq, b.hsorted_xg, b.heads, b.es_nl, b.es_cnt,
+                                           b.es_cap, jg, partial_dev + (size_t)g1 * SOUP_DIFF_NPARAM);
+  }
+}
+void adj_frames_drift(Batch& b, const float4* top, uint32_t frames, uint32_t* bits) {
+  b.launches += 1;
+  SOUP_CUDA_TRY(cudaMemsetAsync(bits, 0, 4 * (size_t)frames * b.R, b.stream));
+  k_frames_drift<<<dim3(nblocks(b.N), frames), kBlock, 0, b.stream>>>(b.sp, b.sysid, b.N, b.R, top, (size_t)b.N, b.id,
+                                                                      b.pos_ref, bits);
 }
 // theta += the blocks' sums, in block order (deterministic)
 void adj_theta_sum(Batch& b, const double* partial_dev, double* theta) {

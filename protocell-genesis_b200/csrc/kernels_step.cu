@@ -165,13 +165,23 @@ __global__ void k_max_drift(const SysParams* __restrict__ sp, const uint8_t* __r
                             const float4* __restrict__ pos, const float4* __restrict__ pos_ref,
                             uint32_t* __restrict__ drift_bits) {
   const uint32_t k = blockIdx.x * blockDim.x + threadIdx.x;
-  if (k >= N) return;
-  const SysParams& P = sp[sysid[k]];
-  const float4 x = pos[k], p0 = pos_ref[k];
-  const float dx = ex_mi(__fsub_rn(x.x, p0.x), P.box[0]);
-  const float dy = ex_mi(__fsub_rn(x.y, p0.y), P.box[1]);
-  const float dz = ex_mi(__fsub_rn(x.z, p0.z), P.box[2]);
-  atomicMax(&drift_bits[sysid[k]], __float_as_uint(__fadd_rn(__fadd_rn(__fmul_rn(dx, dx), __fmul_rn(dy, dy)), __fmul_rn(dz, dz))));
+  uint32_t d = 0, r = 0;
+  if (k < N) {
+    r = sysid[k];
+    const SysParams& P = sp[r];
+    const float4 x = pos[k], p0 = pos_ref[k];
+    const float dx = ex_mi(__fsub_rn(x.x, p0.x), P.box[0]);
+    const float dy = ex_mi(__fsub_rn(x.y, p0.y), P.box[1]);
+    const float dz = ex_mi(__fsub_rn(x.z, p0.z), P.box[2]);
+    d = __float_as_uint(__fadd_rn(__fadd_rn(__fmul_rn(dx, dx), __fmul_rn(dy, dy)), __fmul_rn(dz, dz)));
+  }
+  const uint32_t r0 = __shfl_sync(0xffffffffu, r, 0);
+  if (__all_sync(0xffffffffu, r == r0 || k >= N)) {
+    d = warp_max(d);
+    if ((threadIdx.x & 31) == 0) atomicMax(&drift_bits[r0], d);
+  } else if (k < N) {
+    atomicMax(&drift_bits[r], d);
+  }
 }
 
 // health.wgsl:52-68: components whose exponent bits are all ones (Inf or NaN), per replica

@@ -480,7 +480,7 @@ void destroy_batch(Batch* b) {
                   b->an_buf[1]};
   for (void* p : ptrs) if (p) cudaFree(p);
   for (void* p : {(void*)b->diff.frames, (void*)b->diff.A, (void*)b->diff.B, (void*)b->diff.g, (void*)b->diff.jg,
-                  (void*)b->diff.frozen_o, (void*)b->diff.partial, (void*)b->diff.all})
+                  (void*)b->diff.frozen_o, (void*)b->diff.drift, (void*)b->diff.save, (void*)b->diff.partial, (void*)b->diff.all})
     if (p) cudaFree(p);
   for (const Batch::Mark& m : b->marks) { cudaEventDestroy(m.a); cudaEventDestroy(m.b); }
   for (cudaEvent_t e : b->event_pool) cudaEventDestroy(e);
@@ -871,6 +871,53 @@ template <class T> T* dgrow(T* p, size_t& cap, size_t want) {
   cap = want;
   return q;
 }
+// The state that a window's end leaves, in the batch's original order, kept on the device (66 bytes a particle),
+// and its way back: identity order, as an upload leaves it, for the re-sort of the force pass behind it.
+struct SavedState {
+  float4 *pos, *vel;
+  float* q;
+  uint32_t *slots, *center, *held, *brng, *trng;
+  uint8_t* frozen;
+  static SavedState of(char* p, size_t n) {
+    SavedState s;
+    s.pos = reinterpret_cast<float4*>(p);
+    s.vel = s.pos + n;
+    s.q = reinterpret_cast<float*>(s.vel + n);
+    s.slots = reinterpret_cast<uint32_t*>(s.q + n);
+    s.center = s.slots + 3 * n;
+    s.held = s.center + n;
+    s.brng = s.held + n;
+    s.trng = s.brng + n;
+    s.frozen = reinterpret_cast<uint8_t*>(s.trng + n);
+    return s;
+  }
+  static SavedState live(Batch& b) {
+    return SavedState{b.pos, b.vel, b.charge, b.slots, b.center, b.held, b.brng, b.trng, b.frozen};
+  }
+};
+// save: slot k to its original index; restore: index i to slot i, with the identity maps
+__global__ void k_move_state(SavedState from, SavedState to, const uint32_t* __restrict__ id, uint32_t n, float4* force,
+                             uint32_t* id_out, uint32_t* slot_of_out) {
+  const uint32_t k = blockIdx.x * blockDim.x + threadIdx.x;
+  if (k >= n) return;
+  const uint32_t i = id ? id[k] : k;
+  to.pos[i] = from.pos[k];
+  to.vel[i] = from.vel[k];
+  to.q[i] = from.q[k];
+  for (int e = 0; e < 3; ++e) to.slots[3 * (size_t)i + e] = from.slots[3 * (size_t)k + e];
+  to.center[i] = from.center[k];
+  to.held[i] = from.held[k];
+  to.brng[i] = from.brng[k];
+  to.trng[i] = from.trng[k];
+  to.frozen[i] = from.frozen[k];
+  if (!id) {
+    force[k] = make_float4(0.f, 0.f, 0.f, 0.f);
+    id_out[k] = k;
+    slot_of_out[k] = k;
+  }
+}
+constexpr size_t kSavedBytes = 66;
+constexpr uint32_t kDriftFrames = 16;
 constexpr int kDepthPairs[6][2] = {{0, 0}, {0, 1}, {0, 2}, {1, 1}, {1, 2}, {2, 2}};
 }  // namespace
 
@@ -1651,8 +1698,10 @@ int soup_diff_forward_strided(SoupHandle* h, uint32_t steps, uint32_t checkpoint
     DiffWindow& w = b.diff;
     const uint32_t N = b.N, R = b.R;
     w.ready = false;
+    const size_t frame_bytes = 16 * (size_t)N * (steps + 1);
+    w.stored = frame_bytes <= frame_budget();
     w.charge.resize(R); w.slots.resize(R); w.center.resize(R); w.held.resize(R); w.brng.resize(R); w.frozen.resize(R);
-    for (uint32_t r = 0; r < R; ++r) {
+    for (uint32_t r = 0; r < R && !w.stored; ++r) {   // what a replay starts from
       const uint32_t n = b.cfg[r].n;
       w.charge[r].resize(n); w.slots[r].resize(3 * (size_t)n); w.center[r].resize(n); w.held[r].resize(n);
       w.brng[r].resize(n);
@@ -1672,8 +1721,6 @@ int soup_diff_forward_strided(SoupHandle* h, uint32_t steps, uint32_t checkpoint
                                                     : nullptr;
     };
     w.ck_pos.clear(); w.ck_vel.clear(); w.ck_trng.clear();
-    const size_t frame_bytes = 16 * (size_t)N * (steps + 1);
-    w.stored = frame_bytes <= frame_budget();
     if (w.stored) {   // keep every frame: the reverse pass reads them instead of replaying segments
       w.all = dgrow(w.all, w.all_cap, (size_t)N * (steps + 1));
       force_pass(b);
@@ -1696,7 +1743,16 @@ int soup_diff_forward_strided(SoupHandle* h, uint32_t steps, uint32_t checkpoint
       diff_step(b);
       if (float4* f = out_frame(t + 1)) adj_unpermute(b, f);
     }
-    diff_read(b, w.end_pos, w.end_vel, w.end_trng);
+    if (w.stored) {
+      if (!w.save) SOUP_CUDA_TRY(cudaMalloc(&w.save, kSavedBytes * (size_t)N));
+      k_move_state<<<(N + 255) / 256, 256, 0, b.stream>>>(SavedState::live(b), SavedState::of(w.save, N), b.id, N, nullptr,
+                                                          nullptr, nullptr);
+      SOUP_CUDA_TRY(cudaGetLastError());
+      w.kinds = b.kinds;
+      w.off_head_charge = b.off_head_charge;
+    } else {
+      diff_read(b, w.end_pos, w.end_vel, w.end_trng);
+    }
     w.end_step = b.step[0];
     guards(b, w.step0);
     w.ready = true;
@@ -1715,9 +1771,11 @@ int soup_diff_backward(SoupHandle* h, const float* dldx_device, double* theta_gr
       return t % S == 0 ? reinterpret_cast<const float4*>(dldx_device) + (size_t)(t / S) * N : nullptr;
     };
     // scratch
-    size_t cap1 = w.frames_cap;
-    w.frames = dgrow(w.frames, cap1, (size_t)(K + 1) * N);
-    w.frames_cap = cap1;
+    if (!w.stored) {
+      size_t cap1 = w.frames_cap;
+      w.frames = dgrow(w.frames, cap1, (size_t)(K + 1) * N);
+      w.frames_cap = cap1;
+    }
     if (!w.A) {
       SOUP_CUDA_TRY(cudaMalloc(&w.A, 16 * (size_t)N)); SOUP_CUDA_TRY(cudaMalloc(&w.B, 16 * (size_t)N));
       SOUP_CUDA_TRY(cudaMalloc(&w.g, 16 * (size_t)N)); SOUP_CUDA_TRY(cudaMalloc(&w.jg, 16 * (size_t)N));
@@ -1727,10 +1785,14 @@ int soup_diff_backward(SoupHandle* h, const float* dldx_device, double* theta_gr
     w.partial = dgrow(w.partial, cap2, adj_partial_count(b));
     w.partial_cap = cap2;
     SOUP_CUDA_TRY(cudaMemsetAsync(w.partial, 0, 8 * adj_partial_count(b), b.stream));
-    std::vector<uint8_t> fo(N, 0);   // by the batch's original index: replica r from its slot offset
-    for (uint32_t r = 0; r < b.R; ++r)
-      for (uint32_t i = 0; i < b.cfg[r].n; ++i) fo[b.hsp[r].slot_off + i] = (uint8_t)w.frozen[r][i];
-    SOUP_CUDA_TRY(cudaMemcpyAsync(w.frozen_o, fo.data(), N, cudaMemcpyHostToDevice, b.stream));
+    std::vector<uint8_t> fo(w.stored ? 0 : N, 0);   // by the batch's original index: replica r from its slot offset
+    if (w.stored) {
+      SOUP_CUDA_TRY(cudaMemcpyAsync(w.frozen_o, SavedState::of(w.save, N).frozen, N, cudaMemcpyDeviceToDevice, b.stream));
+    } else {
+      for (uint32_t r = 0; r < b.R; ++r)
+        for (uint32_t i = 0; i < b.cfg[r].n; ++i) fo[b.hsp[r].slot_off + i] = (uint8_t)w.frozen[r][i];
+      SOUP_CUDA_TRY(cudaMemcpyAsync(w.frozen_o, fo.data(), N, cudaMemcpyHostToDevice, b.stream));
+    }
     SOUP_CUDA_TRY(cudaMemcpyAsync(w.A, dldx_at(T), 16 * (size_t)N, cudaMemcpyDeviceToDevice, b.stream));
     SOUP_CUDA_TRY(cudaMemsetAsync(w.B, 0, 16 * (size_t)N, b.stream));
     SOUP_CUDA_TRY(cudaMemsetAsync(w.g, 0, 16 * (size_t)N, b.stream));
@@ -1739,18 +1801,46 @@ int soup_diff_backward(SoupHandle* h, const float* dldx_device, double* theta_gr
     double theta[SOUP_DIFF_NPARAM] = {0};
     auto set_step = [&](uint64_t s0) { for (uint32_t r = 0; r < b.R; ++r) b.step[r] = s0; };
     if (w.stored) {
-      for (uint32_t t = T; t > 0; --t) {
+      // the lists serve every frame within skin/2 of where they were built (the forward step's own test): the
+      // drifts of the next kDriftFrames frames are taken at once, so the host waits once for all of them
+      if (!w.drift) SOUP_CUDA_TRY(cudaMalloc(&w.drift, 4 * (size_t)kDriftFrames * b.R));
+      uint32_t known = 0, at = 0;          // frames the lists are known to serve; the next one's row of w.drift
+      std::vector<uint32_t> bits(kDriftFrames * (size_t)b.R);
+      for (uint32_t t = T + 1; t-- > 0;) {
+        const uint32_t* drift = b.drift_bits;
+        bool fresh = false;
+        if (known == 0) {
+          const uint32_t n = std::min(kDriftFrames, t + 1u);
+          adj_frames_drift(b, w.all + (size_t)t * N, n, w.drift);
+          SOUP_CUDA_TRY(cudaMemcpyAsync(bits.data(), w.drift, 4 * (size_t)n * b.R, cudaMemcpyDeviceToHost, b.stream));
+          SOUP_CUDA_TRY(cudaStreamSynchronize(b.stream));
+          at = 0;
+          auto serves = [&](uint32_t f) {
+            for (uint32_t r = 0; r < b.R; ++r) {
+              float d2;
+              std::memcpy(&d2, &bits[(size_t)f * b.R + r], 4);
+              if (!(d2 <= b.hsp[r].skin_half2)) return false;
+            }
+            return true;
+          };
+          while (known < n && serves(known)) ++known;
+          fresh = known == 0;
+        }
         adj_scatter_pos(b, w.all + (size_t)t * N);
-        refresh_lists(b);
-        adj_hvp(b, w.g, w.jg, w.partial);
-        const float coef = (t - 1 == 0) ? hh : hh * (1.0f + a);
-        adj_update(b, N, w.A, w.B, w.jg, dldx_at(t - 1), w.frozen_o, a, dt, coef, w.g, nullptr);
+        if (fresh) {
+          rebuild(b);
+        } else {
+          drift = w.drift + (size_t)at * b.R;
+          ++at;
+          --known;
+        }
+        if (t == 0 && dv0_device)
+          SOUP_CUDA_TRY(cudaMemcpyAsync(dv0_device, w.B, 16 * (size_t)N, cudaMemcpyDeviceToDevice, b.stream));
+        adj_hvp(b, drift, w.g, w.jg, w.partial);
+        const float coef = t == 0 ? 0.f : ((t - 1 == 0) ? hh : hh * (1.0f + a));
+        adj_update(b, N, w.A, w.B, w.jg, t == 0 ? nullptr : dldx_at(t - 1), w.frozen_o, a, dt, coef, w.g,
+                   t == 0 ? reinterpret_cast<float4*>(dx0_device) : nullptr);
       }
-      if (dv0_device) SOUP_CUDA_TRY(cudaMemcpyAsync(dv0_device, w.B, 16 * (size_t)N, cudaMemcpyDeviceToDevice, b.stream));
-      adj_scatter_pos(b, w.all);
-      refresh_lists(b);
-      adj_hvp(b, w.g, w.jg, w.partial);
-      adj_update(b, N, w.A, w.B, w.jg, nullptr, w.frozen_o, a, dt, 0.f, w.g, reinterpret_cast<float4*>(dx0_device));
     }
     const uint32_t nseg = w.stored ? 0 : (T + K - 1) / K;
     for (uint32_t seg = nseg; seg-- > 0;) {
@@ -1765,7 +1855,7 @@ int soup_diff_backward(SoupHandle* h, const float* dldx_device, double* theta_gr
       for (uint32_t t = t1; t > t0; --t) {
         adj_scatter_pos(b, w.frames + (size_t)(t - t0) * N);
         refresh_lists(b);
-        adj_hvp(b, w.g, w.jg, w.partial);
+        adj_hvp(b, b.drift_bits, w.g, w.jg, w.partial);
         const float coef = (t - 1 == 0) ? hh : hh * (1.0f + a);
         adj_update(b, N, w.A, w.B, w.jg, dldx_at(t - 1), w.frozen_o, a, dt, coef, w.g, nullptr);
       }
@@ -1773,14 +1863,23 @@ int soup_diff_backward(SoupHandle* h, const float* dldx_device, double* theta_gr
         if (dv0_device) SOUP_CUDA_TRY(cudaMemcpyAsync(dv0_device, w.B, 16 * (size_t)N, cudaMemcpyDeviceToDevice, b.stream));
         adj_scatter_pos(b, w.frames);
         refresh_lists(b);
-        adj_hvp(b, w.g, w.jg, w.partial);
+        adj_hvp(b, b.drift_bits, w.g, w.jg, w.partial);
         adj_update(b, N, w.A, w.B, w.jg, nullptr, w.frozen_o, a, dt, 0.f, w.g, reinterpret_cast<float4*>(dx0_device));
       }
     }
     // back to the end of the window
     set_step(w.end_step);
+    if (w.stored) {
+      k_move_state<<<(N + 255) / 256, 256, 0, b.stream>>>(SavedState::of(w.save, N), SavedState::live(b), nullptr, N, b.force,
+                                                          b.id, b.slot_of);
+      SOUP_CUDA_TRY(cudaGetLastError());
+      b.kinds = w.kinds;
+      b.off_head_charge = w.off_head_charge;
+      for (uint32_t r = 0; r < b.R; ++r) SOUP_CUDA_TRY(cudaMemcpyAsync(b.prot_rng_dev + r, &w.prot_rng[r], 4, cudaMemcpyHostToDevice, b.stream));
+      force_pass(b);
+    }
     adj_theta_sum(b, w.partial, theta);
-    diff_restore(b, w.end_pos, w.end_vel, w.end_trng);
+    if (!w.stored) diff_restore(b, w.end_pos, w.end_vel, w.end_trng);
     b.prot_rng = w.prot_rng;
     SOUP_CUDA_TRY(cudaStreamSynchronize(b.stream));
     for (int p = 0; p < SOUP_DIFF_NPARAM; ++p) theta_grad[p] = theta[p];

@@ -59,6 +59,10 @@ struct DiffWindow {
   size_t all_cap = 0;
   float4 *frames = nullptr, *A = nullptr, *B = nullptr, *g = nullptr, *jg = nullptr;
   uint8_t* frozen_o = nullptr;
+  uint32_t* drift = nullptr;             // kDriftFrames x R: the drifts of the frames ahead (stored windows)
+  char* save = nullptr;                  // the state at the end of a stored window, in original order
+  std::vector<std::vector<uint8_t>> kinds;
+  std::vector<uint8_t> off_head_charge;
   double* partial = nullptr;
   size_t frames_cap = 0, partial_cap = 0;
 };
@@ -233,7 +237,8 @@ uint32_t sweep_max_heads();   // heads one replica may hold for the device const
 size_t sweep_draws(const Batch& b);   // draws of every replica, in whole blocks
 void adj_unpermute(Batch& b, float4* dst);
 void adj_scatter_pos(Batch& b, const float4* src);
-void adj_hvp(Batch& b, const float4* g, float4* jg, double* partial_dev);
+void adj_hvp(Batch& b, const uint32_t* drift, const float4* g, float4* jg, double* partial_dev);
+void adj_frames_drift(Batch& b, const float4* top, uint32_t frames, uint32_t* bits);
 void adj_theta_sum(Batch& b, const double* partial_dev, double* theta);
 size_t adj_partial_count(const Batch& b);
 void adj_update(Batch& b, uint32_t n, float4* A, float4* B, const float4* jg, const float4* ldx, const uint8_t* frozen_o,
