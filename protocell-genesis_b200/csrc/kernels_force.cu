@@ -125,7 +125,7 @@ __global__ void __launch_bounds__(kForceBlock, 8) k_force(
     const uint32_t* __restrict__ center, const uint32_t* __restrict__ id, const uint32_t* __restrict__ slot_of,
     const uint32_t* __restrict__ nl, const uint32_t* __restrict__ nl_cnt, const uint32_t* __restrict__ nl_shell,
     const uint32_t* __restrict__ drift_bits, uint32_t stride, float4* __restrict__ force,
-    const uint32_t* __restrict__ sel, uint32_t nsel) {
+    const uint32_t* __restrict__ sel, uint32_t nsel, const uint32_t* __restrict__ head_of, float4* __restrict__ head_xq) {
   __shared__ PairW pw[SOUP_KMAX * SOUP_KMAX];
   for (int w = threadIdx.x; w < (int)(sizeof(pw) / 4); w += kForceBlock)
     reinterpret_cast<uint32_t*>(pw)[w] = reinterpret_cast<const uint32_t*>(Sg->pw)[w];
@@ -194,21 +194,14 @@ __global__ void __launch_bounds__(kForceBlock, 8) k_force(
       }
     }
     force[k] = make_float4(fx, fy, fz, 0.f);
+    // a head's record (x, y, z, q) by head index: the far half reads one 16-byte record per list entry instead
+    // of a slot lookup and two gathers
+    const uint32_t h = SEL ? g : (head_of ? head_of[k] : SOUP_NONE_U32);
+    if (SEL || h != SOUP_NONE_U32) head_xq[h] = make_float4(xi.x, xi.y, xi.z, qi);
   }
 }
 
 // soup/wgsl/electrostatics-long.wgsl:63-82 soup_es_force_far_main, a warp per head.
-// positions and charges of the heads by head index (x, y, z, q): the far half reads one 16-byte
-// record per list entry instead of a slot lookup followed by two gathers
-__global__ void k_gather_xq(const uint32_t* __restrict__ head_slot, uint32_t H, const float4* __restrict__ pos,
-                            const float* __restrict__ charge, float4* __restrict__ xq) {
-  const uint32_t h = blockIdx.x * blockDim.x + threadIdx.x;
-  if (h >= H) return;
-  const uint32_t k = head_slot[h];
-  const float4 p = pos[k];
-  xq[h] = make_float4(p.x, p.y, p.z, charge[k]);
-}
-
 __global__ void __launch_bounds__(256) k_es_far(const SysParams* __restrict__ sp, const uint32_t* __restrict__ head_slot,
                                                 const uint32_t* __restrict__ head_sys, uint32_t H,
                                                 const float4* __restrict__ xq, const uint32_t* __restrict__ es_nl,
@@ -221,24 +214,38 @@ __global__ void __launch_bounds__(256) k_es_far(const SysParams* __restrict__ sp
   const float4 xi = xq[h];
   const float qi = xi.w;
   if (qi == 0.f || P.es_A == 0.f) return;
+  const float bx = P.box[0], by = P.box[1], bz = P.box[2], ibx = P.inv_box[0], iby = P.inv_box[1], ibz = P.inv_box[2];
+  const float A = P.es_A, kappa = P.es_kappa, fc = P.es_fc, r0 = P.es_split, r1 = P.es_rc;
   float fx = 0.f, fy = 0.f, fz = 0.f;
   const uint32_t cnt = es_cnt[h];
   const uint32_t* row = es_nl + (size_t)h * cap;
-  auto add = [&](const float4& xj) {
-    const float qj = xj.w;
-    if (qj == 0.f) return;
-    const float dx = fast_mi(xi.x - xj.x, P.box[0], P.inv_box[0]);
-    const float dy = fast_mi(xi.y - xj.y, P.box[1], P.inv_box[1]);
-    const float dz = fast_mi(xi.z - xj.z, P.box[2], P.inv_box[2]);
-    const float r2 = dx * dx + dy * dy + dz * dz;
-    const float rinv = rsqrtf(r2);
-    const float r = r2 * rinv;
-    if (r < P.es_split || r >= P.es_rc) return;   // esForceFar (electrostatics.wgsl:87-90)
-    const float u = P.es_A * __expf(-P.es_kappa * r) * rinv;
-    const float sc = qi * qj * (u * (rinv + P.es_kappa) - P.es_fc) * rinv;
-    fx += sc * dx; fy += sc * dy; fz += sc * dz;
-  };
-  for (uint32_t s = (uint32_t)lane; s < cnt; s += 32u) add(__ldg(xq + __ldg(row + s)));
+  uint32_t j[4];
+#pragma unroll
+  for (int u = 0; u < 4; ++u) j[u] = lane + 32u * u < cnt ? __ldg(row + lane + 32u * u) : h;
+  for (uint32_t s = (uint32_t)lane; s - lane < cnt; s += 128u) {
+    float4 xj[4];
+#pragma unroll
+    for (int u = 0; u < 4; ++u) xj[u] = __ldg(xq + j[u]);
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      const uint32_t n = s + 128u + 32u * u;
+      j[u] = n < cnt ? __ldg(row + n) : h;
+    }
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      const float dx = fast_mi(xi.x - xj[u].x, bx, ibx);
+      const float dy = fast_mi(xi.y - xj[u].y, by, iby);
+      const float dz = fast_mi(xi.z - xj[u].z, bz, ibz);
+      const float r2 = dx * dx + dy * dy + dz * dz;
+      const float rinv = rsqrt_ftz(r2);
+      const float r = r2 * rinv;
+      const float w = A * __expf(-kappa * r) * rinv;
+      const float sc = qi * xj[u].w * (w * (rinv + kappa) - fc) * rinv;
+      if (s + 32u * u < cnt && xj[u].w != 0.f && r >= r0 && r < r1) {   // esForceFar (electrostatics.wgsl:87-90)
+        fx += sc * dx; fy += sc * dy; fz += sc * dz;
+      }
+    }
+  }
   for (int o = 16; o > 0; o >>= 1) {
     fx += __shfl_xor_sync(0xffffffffu, fx, o);
     fy += __shfl_xor_sync(0xffffffffu, fy, o);
@@ -317,11 +324,11 @@ void launch_force_tpp(Batch& b, bool heads) {
   if (heads)
     k_force<TPP, true><<<blocks, kForceBlock, 0, b.stream>>>(b.shared, b.sp, b.sysid, b.N, b.pos, b.charge, b.slots, b.center, b.id,
                                                      b.slot_of, b.nl, b.nl_cnt, shells, b.drift_bits, b.list_stride,
-                                                     b.force, b.head_slot, b.H);
+                                                     b.force, b.head_slot, b.H, nullptr, b.head_xq);
   else
     k_force<TPP, false><<<blocks, kForceBlock, 0, b.stream>>>(b.shared, b.sp, b.sysid, b.N, b.pos, b.charge, b.slots, b.center, b.id,
                                                       b.slot_of, b.nl, b.nl_cnt, shells, b.drift_bits, b.list_stride,
-                                                      b.force, nullptr, 0u);
+                                                      b.force, nullptr, 0u, b.H ? b.head_of : nullptr, b.head_xq);
 }
 
 }  // namespace
@@ -367,8 +374,7 @@ void launch_force_heads(Batch& b) {
 
 void launch_es_far(Batch& b) {
   if (b.H == 0) return;
-  b.launches += 2;
-  k_gather_xq<<<nblocks(b.H), kBlock, 0, b.stream>>>(b.head_slot, b.H, b.pos, b.charge, b.head_xq);
+  b.launches += 1;
   k_es_far<<<nblocks((uint64_t)b.H * 32, 256), 256, 0, b.stream>>>(b.sp, b.head_slot, b.head_sys, b.H, b.head_xq,
                                                                    b.es_nl, b.es_cnt, b.es_cap, b.force);
 }

@@ -166,9 +166,11 @@ __global__ void k_copy_back(uint32_t N, const float4* __restrict__ pos2, const f
                             const uint32_t* __restrict__ id2, float4* __restrict__ pos, float4* __restrict__ vel,
                             float4* __restrict__ force, float* __restrict__ charge, uint32_t* __restrict__ slots,
                             uint32_t* __restrict__ center, uint32_t* __restrict__ held, uint32_t* __restrict__ brng,
-                            uint32_t* __restrict__ trng, uint8_t* __restrict__ frozen, uint32_t* __restrict__ id) {
+                            uint32_t* __restrict__ trng, uint8_t* __restrict__ frozen, uint32_t* __restrict__ id,
+                            uint32_t* __restrict__ head_of) {
   const uint32_t k = blockIdx.x * blockDim.x + threadIdx.x;
   if (k >= N) return;
+  head_of[k] = SOUP_NONE_U32;   // k_head_index names the heads
   pos[k] = pos2[k]; vel[k] = vel2[k]; force[k] = force2[k]; charge[k] = charge2[k];
   slots[3 * k] = slots2[3 * k]; slots[3 * k + 1] = slots2[3 * k + 1]; slots[3 * k + 2] = slots2[3 * k + 2];
   center[k] = center2[k]; held[k] = held2[k]; brng[k] = brng2[k]; trng[k] = trng2[k]; frozen[k] = frozen2[k];
@@ -466,12 +468,14 @@ __global__ void __launch_bounds__(128) k_build_list(
 __global__ void k_head_index(const uint32_t* __restrict__ heads, const uint32_t* __restrict__ head_sys, uint32_t H,
                              const uint32_t* __restrict__ slot_of, const float4* __restrict__ pos,
                              const SysParams* __restrict__ sp, uint32_t* __restrict__ hcell_of,
-                             uint32_t* __restrict__ hcount, uint32_t* __restrict__ head_slot) {
+                             uint32_t* __restrict__ hcount, uint32_t* __restrict__ head_slot,
+                             uint32_t* __restrict__ head_of) {
   uint32_t h = blockIdx.x * blockDim.x + threadIdx.x;
   if (h >= H) return;
   const SysParams& P = sp[head_sys[h]];
   const uint32_t ks = slot_of[heads[h]];
   head_slot[h] = ks;
+  head_of[ks] = h;
   float4 p = pos[ks];
   int cx = ex_cell_axis(p.x, P.box[0], P.hdims[0]);
   int cy = ex_cell_axis(p.y, P.box[1], P.hdims[1]);
@@ -582,7 +586,7 @@ void launch_sort_and_gather(Batch& b) {
   k_copy_back<<<nblocks(b.N), kBlock, 0, b.stream>>>(b.N, b.pos2, b.vel2, b.force2, b.charge2, b.slots2, b.center2,
                                                       b.held2, b.brng2, b.trng2, b.frozen2, b.id2, b.pos, b.vel, b.force,
                                                       b.charge, b.slots, b.center, b.held, b.brng, b.trng, b.frozen,
-                                                      b.id);
+                                                      b.id, b.head_of);
   b.launches += 4 + scans;
   prof_end(b);
 }
@@ -609,7 +613,7 @@ void launch_build_es_lists(Batch& b) {
   prof_begin(b, SOUP_K_LIST);
   cudaMemsetAsync(b.hcell_count, 0, sizeof(uint32_t) * (b.nhcells + 1), b.stream);
   k_head_index<<<nblocks(b.H), kBlock, 0, b.stream>>>(b.heads, b.head_sys, b.H, b.slot_of, b.pos, b.sp, b.hcell_of,
-                                                       b.hcell_count, b.head_slot);
+                                                       b.hcell_count, b.head_slot, b.head_of);
   const uint64_t scans = exclusive_scan(b.hcell_count, b.hcell_start, b.nhcells, b.scan_tmp, b.stream);
   cudaMemsetAsync(b.hcell_cursor, 0, sizeof(uint32_t) * b.nhcells, b.stream);
   k_head_scatter<<<nblocks(b.H), kBlock, 0, b.stream>>>(b.hcell_of, b.hcell_start, b.H, b.hcell_cursor, b.hsorted);

@@ -376,7 +376,7 @@ Batch* make_batch(const SoupConfig* cfgs, const SoupInitState* inits, uint32_t R
   b.pos = dalloc<float4>(n); b.vel = dalloc<float4>(n); b.force = dalloc<float4>(n); b.pos_ref = dalloc<float4>(n);
   b.charge = dalloc<float>(n); b.slots = dalloc<uint32_t>(3 * n); b.center = dalloc<uint32_t>(n);
   b.held = dalloc<uint32_t>(n); b.brng = dalloc<uint32_t>(n); b.trng = dalloc<uint32_t>(n); b.frozen = dalloc<uint8_t>(n);
-  b.id = dalloc<uint32_t>(n); b.slot_of = dalloc<uint32_t>(n);
+  b.id = dalloc<uint32_t>(n); b.head_of = dalloc<uint32_t>(n); b.slot_of = dalloc<uint32_t>(n);
   b.pos2 = dalloc<float4>(n); b.vel2 = dalloc<float4>(n); b.force2 = dalloc<float4>(n); b.charge2 = dalloc<float>(n);
   b.slots2 = dalloc<uint32_t>(3 * n); b.center2 = dalloc<uint32_t>(n); b.held2 = dalloc<uint32_t>(n);
   b.brng2 = dalloc<uint32_t>(n); b.trng2 = dalloc<uint32_t>(n); b.frozen2 = dalloc<uint8_t>(n); b.id2 = dalloc<uint32_t>(n);
@@ -471,7 +471,7 @@ void destroy_batch(Batch* b) {
   drop_graphs(*b);
   if (b->cap_stream) cudaStreamDestroy(b->cap_stream);
   void* ptrs[] = {b->rebuild_count, b->pos, b->vel, b->force, b->pos_ref, b->charge, b->slots, b->center, b->held, b->brng, b->trng,
-                  b->frozen, b->id, b->slot_of, b->pos2, b->vel2, b->force2, b->charge2, b->slots2, b->center2,
+                  b->frozen, b->id, b->head_of, b->slot_of, b->pos2, b->vel2, b->force2, b->charge2, b->slots2, b->center2,
                   b->held2, b->brng2, b->trng2, b->frozen2, b->id2, b->cell_of_slot, b->cell_count, b->cell_start,
                   b->cell_cursor, b->perm, b->scan_tmp, b->nl, b->nl_cnt, b->nl_shell, b->heads, b->head_sys, b->es_nl,
                   b->es_cnt, b->head_slot, b->head_e, b->head_pos, b->head_xq, b->head_d, b->draw_site, b->pair_cnt, b->pair_idx, b->pair_del, b->walk_shared, b->hcell_count, b->hcell_start, b->hcell_cursor, b->hsorted, b->hsorted_xg, b->hcell_of, b->flags,

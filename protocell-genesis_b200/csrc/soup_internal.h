@@ -109,6 +109,7 @@ struct Batch {
   uint32_t* heads = nullptr;         // global original ids, per replica ascending
   uint32_t* head_sys = nullptr;      // replica of each head
   uint32_t* head_slot = nullptr;     // current slot of each head (refreshed at every rebuild)
+  uint32_t* head_of = nullptr;       // slot -> head index, or SOUP_NONE_U32 (refreshed with it)
   long long* head_e = nullptr;       // constant-pH site energy per head, fixed point 2^-40 (sweep scratch)
   float4* head_pos = nullptr;        // head positions and charges gathered for the sweep
   float4* head_xq = nullptr;         // head positions and charges by head index, for the far half
