@@ -226,7 +226,7 @@ constexpr uint32_t kWalkRuns = 128;                    // runs: two per row, (2 
 constexpr uint32_t kWalkSpan = 2048;                   // candidates whose run starts are marked at a time
 constexpr uint32_t kWalkWords = 2 * kWalkRuns + 2 * kWalkSpan / 32;   // shared words a warp's walk needs
 
-struct WalkGrid { int dims[3]; int walk; uint32_t cell_off; float range; float cell[3]; float inv_cell_x; };
+struct WalkGrid { int dims[3]; int walk, walk_x; uint32_t cell_off; float range; float cell[3]; float inv_cell_x; };
 
 __device__ __forceinline__ float sqrt_approx(float x) {   // under the walk's margins
   float y;
@@ -243,10 +243,10 @@ __device__ __forceinline__ void warp_walk(const float4& xi, const float* box, co
   uint2* mark = reinterpret_cast<uint2*>(sm + 2 * kWalkRuns);   // per 32 candidates: a bit where a run starts; the
                                                        // runs that start before them, less one
   const uint32_t lane = threadIdx.x & 31u, lt = (1u << lane) - 1u, le = lt | (1u << lane);
-  const int R = G.walk, D = 2 * R + 1;
+  const int R = G.walk, D = 2 * R + 1, Rx = G.walk_x;
   const int dx = G.dims[0], dy = G.dims[1], dz = G.dims[2];
   const int qx = ex_cell_axis(xi.x, box[0], dx), qy = ex_cell_axis(xi.y, box[1], dy), qz = ex_cell_axis(xi.z, box[2], dz);
-  const bool fx = dx < D, fy = dy < D, fz = dz < D;    // this axis is visited whole
+  const bool fx = dx < 2 * Rx + 1, fy = dy < D, fz = dz < D;    // this axis is visited whole
   const int ny = fy ? dy : D, nz = fz ? dz : D;
   const float csy = G.cell[1], csz = G.cell[2], icx = G.inv_cell_x;
   const float lrm = G.range * (1.0f + 1e-5f) + 1e-3f, lrm2 = lrm * lrm;
@@ -267,7 +267,7 @@ __device__ __forceinline__ void warp_walk(const float4& xi, const float* box, co
           l0 = start[row + (uint32_t)dx] - a0;
         } else {
           const float ext = sqrt_approx(lrm2 - g2) + 1e-3f;
-          const int xlo = max(qx - R, (int)floorf((xi.x - ext) * icx)), xhi = min(qx + R, (int)floorf((xi.x + ext) * icx));
+          const int xlo = max(qx - Rx, (int)floorf((xi.x - ext) * icx)), xhi = min(qx + Rx, (int)floorf((xi.x + ext) * icx));
           if (xlo <= xhi) {
             const AxisRange xr = span_ranges(xlo, xhi, dx);
             a0 = start[row + (uint32_t)xr.lo[0]];
@@ -363,7 +363,7 @@ __global__ void __launch_bounds__(128) k_build_list(
   const float rm = lr * (1.0f + 1e-5f) + 1e-3f;
   const bool direct = xi.x >= rm && xi.x <= box[0] - rm && xi.y >= rm && xi.y <= box[1] - rm && xi.z >= rm &&
                       xi.z <= box[2] - rm;
-  const WalkGrid G{{P.dims[0], P.dims[1], P.dims[2]}, P.walk, P.cell_off, lr, {P.cell[0], P.cell[1], P.cell[2]}, P.inv_cell[0]};
+  const WalkGrid G{{P.dims[0], P.dims[1], P.dims[2]}, P.walk, P.walk * P.fine, P.cell_off, lr, {P.cell[0], P.cell[1], P.cell[2]}, P.inv_cell[0]};
   uint32_t cnt = 0;
   // 32 candidates: the accepted ones, tagged, behind the row
   auto put = [&](auto image, uint32_t j, bool v, const float4& xj) {
@@ -535,7 +535,7 @@ __global__ void __launch_bounds__(128) k_build_es_list(const uint32_t* __restric
   const float inv[3] = {P.inv_box[0], P.inv_box[1], P.inv_box[2]};
   const float lr = P.es_list_range;
   const float lo = lr * lr * (1.0f - 1e-5f), hi = lr * lr * (1.0f + 1e-5f);
-  const WalkGrid G{{P.hdims[0], P.hdims[1], P.hdims[2]}, P.hwalk, P.hcell_off, lr, {P.hcell[0], P.hcell[1], P.hcell[2]},
+  const WalkGrid G{{P.hdims[0], P.hdims[1], P.hdims[2]}, P.hwalk, P.hwalk * P.hfine, P.hcell_off, lr, {P.hcell[0], P.hcell[1], P.hcell[2]},
                    P.inv_hcell[0]};
   uint32_t cnt = 0;
   uint32_t* row = es_nl + (size_t)h * cap;

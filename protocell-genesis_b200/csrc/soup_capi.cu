@@ -110,9 +110,16 @@ Shared make_shared(const SoupConfig& c) {
   return s;
 }
 
-void grid_of(const double box[3], double range, int walk, int dims[3]) {
+// A list grid's cells: range / walk wide, and along x, where the walk trims its rows of cells to the list
+// sphere, kFineX times finer (the returned factor) while that makes no more than kFineX cells a particle: a sparse box has
+// no rows worth trimming
+int grid_of(const double box[3], double range, int walk, uint32_t n, int dims[3]) {
   const double cell = range / walk;
-  for (int a = 0; a < 3; ++a) dims[a] = std::max(1, (int)std::floor(box[a] / cell));
+  double cells = 1;
+  for (int a = 0; a < 3; ++a) cells *= dims[a] = std::max(1, (int)std::floor(box[a] / cell));
+  if (!(cells <= n)) return 1;
+  dims[0] = std::max(1, (int)std::floor(box[0] / (cell / kFineX)));
+  return kFineX;
 }
 
 SysParams make_sys(const SoupConfig& c) {
@@ -131,9 +138,9 @@ SysParams make_sys(const SoupConfig& c) {
   p.acid = (float)c.acid_soap_scale;
   p.skin_half2 = (float)(0.25 * c.skin * c.skin);
   p.walk = 2;
-  grid_of(c.box, c.list_range, p.walk, p.dims);
+  p.fine = grid_of(c.box, c.list_range, p.walk, c.n, p.dims);
   p.hwalk = 2;
-  grid_of(c.box, es ? c.es_list_range : c.list_range, p.hwalk, p.hdims);
+  p.hfine = grid_of(c.box, es ? c.es_list_range : c.list_range, p.hwalk, c.n, p.hdims);
   p.list_cap = c.list_capacity;
   p.es_cap = c.es_list_capacity;
   // draws of a block of the walk: a round pulls, per draw, the flips among the earlier draws of its block that
@@ -988,7 +995,7 @@ void tune_plan(Batch& b, const std::vector<double>& skin, int walk) {
     const SysParams old = b.hsp[r];
     SysParams p = make_sys(c);
     p.walk = walk;
-    grid_of(c.box, c.list_range, walk, p.dims);
+    p.fine = grid_of(c.box, c.list_range, walk, c.n, p.dims);
     p.slot_off = old.slot_off; p.n = old.n; p.head_off = old.head_off; p.nheads = old.nheads;
     b.hsp[r] = p;
   }

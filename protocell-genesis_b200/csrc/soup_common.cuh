@@ -35,11 +35,13 @@ struct SysParams {
   float reach[2], shell_scale[2];
   int dims[3];               // list-build grid
   uint32_t cell_off;         // first global cell of this system
-  int walk;                  // list-build walk radius (cells)
+  int walk;                  // list-build walk radius (cells; along x `fine` times as many)
+  int fine;
   uint32_t slot_off, n;      // slot range of this system
   uint32_t head_off, nheads; // head range (ES heads)
   int hdims[3];              // head grid
-  int hwalk;                 // head-grid walk radius (cells)
+  int hwalk;                 // head-grid walk radius (cells; along x hfine times as many)
+  int hfine;
   uint32_t hcell_off;
   float cell[3], inv_cell[3], hcell[3], inv_hcell[3];   // cell sides of the two grids and their inverses
   uint32_t list_cap, es_cap; // capacities (overflow threshold)
@@ -156,6 +158,8 @@ constexpr int kShells = 8;
 __host__ __device__ __forceinline__ float list_shell_width2(float reach2, float list_range) {
   return fmaxf(list_range * list_range - reach2, 0.f) * (1.0f / (kShells - 1));
 }
+constexpr int kFineX = 4;        // grid_of
+
 // Whether a bead can take part in a term that reaches beyond the class attraction: it is charged, or a sweep
 // can charge it, or it is of the polar class.  A plain bead's force ends at rplain2.
 __device__ __forceinline__ bool list_wide(const Shared& S, const SysParams& P, int kind, float charge) {
