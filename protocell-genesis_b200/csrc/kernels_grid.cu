@@ -234,9 +234,9 @@ __device__ __forceinline__ float sqrt_approx(float x) {   // under the walk's ma
   return y;
 }
 
-// take(j0, v0, j1, v1): warp-wide, 2 x 32 candidates j (indices into the cell-ordered array; v: one of the walk's)
+// take(j0, j1): warp-wide, 2 x 32 candidates (indices into the cell-ordered array; self: the walk's own bead there)
 template <class Take>
-__device__ __forceinline__ void warp_walk(const float4& xi, const float* box, const WalkGrid& G,
+__device__ __forceinline__ void warp_walk(const float4& xi, uint32_t self, const float* box, const WalkGrid& G,
                                           const uint32_t* __restrict__ start, uint32_t* __restrict__ sm, Take&& take) {
   uint32_t* shift = sm;                                // candidate q of run s is bead q + shift[s]
   uint32_t* first = sm + kWalkRuns;                    // its first candidate
@@ -317,18 +317,20 @@ __device__ __forceinline__ void warp_walk(const float4& xi, const float* box, co
       before += __shfl_sync(0xffffffffu, incl, 31);
     }
     __syncwarp();
-    for (uint32_t c = 0; c < n; c += 64u) {
+#pragma unroll 1
+    for (uint32_t c = 0; c < n; c += 64u) {            // a place past the end stands for the walk's own bead
       const uint4 m = *reinterpret_cast<const uint4*>(&mark[c >> 5]);
-      const uint32_t q0 = w0 + c + lane, q1 = q0 + 32u, c0 = min(q0, total - 1u), c1 = min(q1, total - 1u);
-      // (a place past the end reads the last run's last candidate, which its v leaves out)
-      const uint32_t s0 = min(m.y + __popc(m.x & le), runs - 1u), s1 = min(m.w + __popc(m.z & le), runs - 1u);
-      take(shift[s0] + c0, q0 < total, shift[s1] + c1, q1 < total);
+      const uint32_t q0 = w0 + c + lane, q1 = q0 + 32u;
+      const uint32_t j0 = shift[m.y + __popc(m.x & le)] + q0, j1 = shift[m.w + __popc(m.z & le)] + q1;
+      take(q0 < total ? j0 : self, q1 < total ? j1 : self);
     }
     __syncwarp();
   }
 }
 
-constexpr uint32_t kGRegs = 16;                        // entries a lane holds while a row is grouped
+// words behind a row: the candidates on the edge of the range that the exact distance may still leave out, and
+// the 64 that overflow it
+constexpr uint32_t kRowSpare = 64, kRowSlack = kRowSpare + 64;
 
 // soup/wgsl/verlet.wgsl:53-92, a warp per particle (warp_walk).  The fast squared distance decides unless it
 // lies within 1e-5 of the range, where the reference's arithmetic decides (the minimum image cannot differ
@@ -347,7 +349,7 @@ __global__ void __launch_bounds__(128) k_build_list(
     uint32_t* __restrict__ shell_end, uint32_t* __restrict__ flags) {
   extern __shared__ __align__(16) uint32_t sm[];
   const uint32_t wib = threadIdx.x >> 5, lane = threadIdx.x & 31u, lt = (1u << lane) - 1u;
-  uint32_t* row = sm + (size_t)wib * (stride + kWalkWords);   // stride: cap rounded up to 16
+  uint32_t* row = sm + (size_t)wib * (stride + kRowSlack + kWalkWords);   // stride: cap rounded up to 16
   const uint32_t k = blockIdx.x * (blockDim.x >> 5) + wib;
   if (k >= N) return;   // whole warps
   const SysParams& P = sp[sysid[k]];
@@ -365,8 +367,9 @@ __global__ void __launch_bounds__(128) k_build_list(
                       xi.z <= box[2] - rm;
   const WalkGrid G{{P.dims[0], P.dims[1], P.dims[2]}, P.walk, P.walk * P.fine, P.cell_off, lr, {P.cell[0], P.cell[1], P.cell[2]}, P.inv_cell[0]};
   uint32_t cnt = 0;
+  bool edge = false;
   // 32 candidates: the accepted ones, tagged, behind the row
-  auto put = [&](auto image, uint32_t j, bool v, const float4& xj) {
+  auto put = [&](auto image, uint32_t j, const float4& xj) {
     float dx = xi.x - xj.x, dy = xi.y - xj.y, dz = xi.z - xj.z;
     if (decltype(image)::value) {
       dx = fast_mi(dx, box[0], inv[0]);
@@ -374,21 +377,35 @@ __global__ void __launch_bounds__(128) k_build_list(
       dz = fast_mi(dz, box[2], inv[2]);
     }
     const float r2 = dx * dx + dy * dy + dz * dz;
-    bool in = v && j != k && r2 <= lr2_hi;
-    if (in && r2 >= lr2_lo) in = ex_dist(xi, xj, box) < lr;
+    const bool in = j != k && r2 <= lr2_hi;
+    edge |= in && r2 >= lr2_lo;
     const uint32_t m = __ballot_sync(0xffffffffu, in), at = cnt + __popc(m & lt);
-    if (in && at < cap) row[at] = j | sh.tag(r2);
-    cnt = __shfl_sync(0xffffffffu, at + (in ? 1u : 0u), 31);
+    if (in) row[at] = j + sh.tag(r2);
+    cnt += __popc(m);
   };
   auto walk = [&](auto image) {
-    warp_walk(xi, box, G, start, row + stride, [&](uint32_t j0, bool v0, uint32_t j1, bool v1) {
+    warp_walk(xi, k, box, G, start, row + stride + kRowSlack, [&](uint32_t j0, uint32_t j1) {
       const float4 x0 = pos[j0], x1 = pos[j1];
-      put(image, j0, v0, x0);
-      put(image, j1, v1, x1);
+      put(image, j0, x0);
+      put(image, j1, x1);
+      cnt = min(cnt, cap + kRowSpare);                 // a row that is too long ends in the slack
     });
   };
   if (direct) walk(std::false_type{});
   else walk(std::true_type{});
+  if (__any_sync(0xffffffffu, edge)) {                 // the exact distance decides within 1e-5 of the range (rare)
+    uint32_t kept = 0;
+#pragma unroll 1
+    for (uint32_t s0 = 0; s0 < cnt; s0 += 32u) {
+      __syncwarp();
+      const uint32_t v = s0 + lane < cnt ? row[s0 + lane] : 0u;
+      const bool in = s0 + lane < cnt && ex_dist(xi, pos[v & 0x1FFFFFFFu], box) < lr;
+      const uint32_t m = __ballot_sync(0xffffffffu, in);
+      if (in) row[kept + __popc(m & lt)] = v;
+      kept += __popc(m);
+    }
+    cnt = kept;
+  }
   if (cnt > cap) {
     if (lane == 0) flags[0] = 1u;
     cnt = cap;
@@ -396,72 +413,41 @@ __global__ void __launch_bounds__(128) k_build_list(
   __syncwarp();
   // group the row by shell, keeping the walk's order inside a shell: 32 entries at a time, three ballots of the
   // shell's bits give every lane the entries of its own shell (its place among them) and lane s those of shell s
-  // (the shells' running ends).  A longer row than the registers hold (dense aggregates) goes out shell by shell.
+  // (the shells' running ends).  The loops stay rolled: unrolled, with the row in registers, the kernel outgrew the instruction cache
   uint32_t* out = nl + (size_t)k * stride;
-  const uint32_t full = (cnt + 15u) & ~15u;          // rows are padded with the particle itself
-  uint32_t e[kShells - 1];
-  if (cnt <= 32u * kGRegs) {
-    // lane l stands for shell l mod 8: a ballot of bit i xor this is ones where bit i is the shell's
-    const uint32_t y0 = (lane & 1u) - 1u, y1 = ((lane >> 1) & 1u) - 1u, y2 = ((lane >> 2) & 1u) - 1u;
-    uint32_t v[kGRegs], end = 0;
-#pragma unroll
-    for (uint32_t c = 0; c < kGRegs; ++c) {
-      if (32u * c >= cnt) break;
-      v[c] = 32u * c + lane < cnt ? row[32u * c + lane] : SOUP_NONE_U32;   // beyond the row: the last shell
-      const uint32_t b0 = __ballot_sync(0xffffffffu, v[c] & 0x20000000u), b1 = __ballot_sync(0xffffffffu, v[c] & 0x40000000u),
-                     b2 = __ballot_sync(0xffffffffu, v[c] & 0x80000000u);
-      end += __popc((b0 ^ y0) & (b1 ^ y1) & (b2 ^ y2));
-    }
-    uint32_t incl = end;                               // the shells' ends
-#pragma unroll
-    for (int o = 1; o < kShells; o <<= 1) {
-      const uint32_t y = __shfl_up_sync(0xffffffffu, incl, o);
-      if ((lane & 7u) >= (uint32_t)o) incl += y;
-    }
-    uint32_t next = incl - end;                        // the shells' next places
-#pragma unroll
-    for (uint32_t t = 0; t + 1u < (uint32_t)kShells; ++t) e[t] = __shfl_sync(0xffffffffu, incl, (int)t);
-    __syncwarp();
-#pragma unroll
-    for (uint32_t c = 0; c < kGRegs; ++c) {
-      if (32u * c >= cnt) break;
-      const uint32_t b0 = __ballot_sync(0xffffffffu, v[c] & 0x20000000u), b1 = __ballot_sync(0xffffffffu, v[c] & 0x40000000u),
-                     b2 = __ballot_sync(0xffffffffu, v[c] & 0x80000000u);
-      const uint32_t x0 = ~(uint32_t)((int)(v[c] << 2) >> 31), x1 = ~(uint32_t)((int)(v[c] << 1) >> 31),
-                     x2 = ~(uint32_t)((int)v[c] >> 31);
-      const uint32_t at = __shfl_sync(0xffffffffu, next, (int)(v[c] >> 29)) + __popc((b0 ^ x0) & (b1 ^ x1) & (b2 ^ x2) & lt);
-      if (32u * c + lane < cnt) row[at] = v[c] & 0x1FFFFFFFu;
-      next += __popc((b0 ^ y0) & (b1 ^ y1) & (b2 ^ y2));
-    }
-    if (cnt + lane < full) row[cnt + lane] = k;
-    __syncwarp();
-    for (uint32_t s = 4u * lane; s < full; s += 128u) {
-      const uint32_t c = s & ~15u, l = (s >> 2) & 3u;
-      *reinterpret_cast<uint4*>(out + s) = c + 16u <= cnt ? make_uint4(row[c + l], row[c + 4u + l], row[c + 8u + l], row[c + 12u + l])
-                                                         : *reinterpret_cast<const uint4*>(row + s);
-    }
-  } else {
-    uint32_t o = 0;
-#pragma unroll
-    for (uint32_t b = 0; b < (uint32_t)kShells; ++b) {
-      for (uint32_t s0 = 0; s0 < cnt; s0 += 32u) {
-        const uint32_t s = s0 + lane;
-        const uint32_t v = s < cnt ? row[s] : SOUP_NONE_U32;
-        const bool hit = (v >> 29) == b;
-        const uint32_t m = __ballot_sync(0xffffffffu, hit);
-        if (hit) out[o + __popc(m & lt)] = v & 0x1FFFFFFFu;
-        o += __popc(m);
-      }
-      if (b + 1u < (uint32_t)kShells) e[b] = o;
-    }
-    if (cnt + lane < full) out[cnt + lane] = k;
+  // lane l stands for shell l mod 8: a ballot of bit i xor this is ones where bit i is the shell's
+  const uint32_t y0 = (lane & 1u) - 1u, y1 = ((lane >> 1) & 1u) - 1u, y2 = ((lane >> 2) & 1u) - 1u;
+  uint32_t end = 0;
+#pragma unroll 1
+  for (uint32_t c = 0; c < cnt; c += 32u) {
+    const uint32_t v = c + lane < cnt ? row[c + lane] : SOUP_NONE_U32;   // beyond the row: the last shell
+    const uint32_t b0 = __ballot_sync(0xffffffffu, v & 0x20000000u), b1 = __ballot_sync(0xffffffffu, v & 0x40000000u),
+                   b2 = __ballot_sync(0xffffffffu, v & 0x80000000u);
+    end += __popc((b0 ^ y0) & (b1 ^ y1) & (b2 ^ y2));
   }
-  if (lane == 0) {
-    nl_cnt[k] = cnt;
-    uint4* se = reinterpret_cast<uint4*>(shell_end + (size_t)kShells * k);
-    se[0] = make_uint4(e[0], e[1], e[2], e[3]);
-    se[1] = make_uint4(e[4], e[5], e[6], cnt);
+  uint32_t incl = end;                                 // the shells' ends
+#pragma unroll
+  for (int o = 1; o < kShells; o <<= 1) {
+    const uint32_t y = __shfl_up_sync(0xffffffffu, incl, o);
+    if ((lane & 7u) >= (uint32_t)o) incl += y;
   }
+  uint32_t next = incl - end;                          // the shells' next places
+  const uint32_t whole = cnt & ~15u;
+#pragma unroll 1
+  for (uint32_t c = 0; c < cnt; c += 32u) {
+    const uint32_t v = c + lane < cnt ? row[c + lane] : SOUP_NONE_U32;
+    const uint32_t b0 = __ballot_sync(0xffffffffu, v & 0x20000000u), b1 = __ballot_sync(0xffffffffu, v & 0x40000000u),
+                   b2 = __ballot_sync(0xffffffffu, v & 0x80000000u);
+    const uint32_t x0 = ~(uint32_t)((int)(v << 2) >> 31), x1 = ~(uint32_t)((int)(v << 1) >> 31),
+                   x2 = ~(uint32_t)((int)v >> 31);
+    const uint32_t at = __shfl_sync(0xffffffffu, next, (int)(v >> 29)) + __popc((b0 ^ x0) & (b1 ^ x1) & (b2 ^ x2) & lt);
+    const uint32_t to = at < whole ? (at & ~15u) + 4u * (at & 3u) + ((at >> 2) & 3u) : at;
+    if (c + lane < cnt) out[to] = v & 0x1FFFFFFFu;
+    next += __popc((b0 ^ y0) & (b1 ^ y1) & (b2 ^ y2));
+  }
+  if (cnt + lane < ((cnt + 15u) & ~15u)) out[cnt + lane] = k;   // rows are padded with the particle itself
+  if (lane < (uint32_t)kShells) shell_end[(size_t)kShells * k + lane] = lane + 1u < (uint32_t)kShells ? incl : cnt;
+  if (lane == 0) nl_cnt[k] = cnt;
 }
 
 // heads: bin into the coarse head grid (replica-local cells), deterministic order inside a cell
@@ -520,17 +506,17 @@ __global__ void k_head_gather_sorted(const uint32_t* __restrict__ hsorted, uint3
 // neighbours' HEAD indices (head_slot maps them to slots); membership uses the exact test near the
 // range, so the set equals the reference's.
 __global__ void __launch_bounds__(128) k_build_es_list(const uint32_t* __restrict__ head_sys, uint32_t H,
-                                                       const uint32_t* __restrict__ head_slot, const float4* __restrict__ pos,
                                                        const SysParams* __restrict__ sp, const uint32_t* __restrict__ hstart,
                                                        const float4* __restrict__ hxg, uint32_t cap,
                                                        uint32_t* __restrict__ es_nl, uint32_t* __restrict__ es_cnt,
                                                        uint32_t* __restrict__ flags) {
   __shared__ __align__(16) uint32_t sm[4][kWalkWords];
   const uint32_t wib = threadIdx.x >> 5, lane = threadIdx.x & 31u, lt = (1u << lane) - 1u;
-  const uint32_t h = blockIdx.x * 4u + wib;
-  if (h >= H) return;   // whole warps
+  const uint32_t place = blockIdx.x * 4u + wib;        // in head-cell order: the warps of a block share candidates
+  if (place >= H) return;   // whole warps
+  const float4 xi = hxg[place];
+  const uint32_t h = __float_as_uint(xi.w);
   const SysParams& P = sp[head_sys[h]];
-  const float4 xi = pos[head_slot[h]];
   const float box[3] = {P.box[0], P.box[1], P.box[2]};
   const float inv[3] = {P.inv_box[0], P.inv_box[1], P.inv_box[2]};
   const float lr = P.es_list_range;
@@ -539,23 +525,23 @@ __global__ void __launch_bounds__(128) k_build_es_list(const uint32_t* __restric
                    P.inv_hcell[0]};
   uint32_t cnt = 0;
   uint32_t* row = es_nl + (size_t)h * cap;
-  auto put = [&](const float4& xj, bool v) {
+  auto put = [&](const float4& xj) {
     const uint32_t g = __float_as_uint(xj.w);
     const float dx = fast_mi(xi.x - xj.x, box[0], inv[0]);
     const float dy = fast_mi(xi.y - xj.y, box[1], inv[1]);
     const float dz = fast_mi(xi.z - xj.z, box[2], inv[2]);
     const float r2 = dx * dx + dy * dy + dz * dz;
-    bool hit = v && g != h && r2 <= hi;
+    bool hit = g != h && r2 <= hi;
     if (hit && r2 >= lo) hit = ex_dist(xi, xj, box) < lr;
     const uint32_t m = __ballot_sync(0xffffffffu, hit);
     const uint32_t at = cnt + __popc(m & lt);
     if (hit && at < cap) row[at] = g;
     cnt += __popc(m);
   };
-  warp_walk(xi, box, G, hstart, sm[wib], [&](uint32_t j0, bool v0, uint32_t j1, bool v1) {
+  warp_walk(xi, place, box, G, hstart, sm[wib], [&](uint32_t j0, uint32_t j1) {
     const float4 x0 = hxg[j0], x1 = hxg[j1];
-    put(x0, v0);
-    put(x1, v1);
+    put(x0);
+    put(x1);
   });
   if (lane == 0) {
     if (cnt > cap) { flags[1] = 1u; cnt = cap; }
@@ -595,7 +581,7 @@ void launch_build_lists(Batch& b) {
   b.launches += 1;
   prof_begin(b, SOUP_K_LIST);
   // a row of shared memory per warp: four warps per block while they fit
-  const size_t per = sizeof(uint32_t) * ((size_t)b.list_stride + kWalkWords);
+  const size_t per = sizeof(uint32_t) * ((size_t)b.list_stride + kRowSlack + kWalkWords);
   const uint32_t wpb = 4u * per <= 200u * 1024u ? 4u : 1u;
   const size_t smem = wpb * per;
   if (smem > 48u * 1024u && b.list_smem_set < smem) {
@@ -619,8 +605,7 @@ void launch_build_es_lists(Batch& b) {
   k_head_scatter<<<nblocks(b.H), kBlock, 0, b.stream>>>(b.hcell_of, b.hcell_start, b.H, b.hcell_cursor, b.hsorted);
   k_head_sort_cells<<<nblocks(b.nhcells), kBlock, 0, b.stream>>>(b.hcell_start, b.nhcells, b.hsorted);
   k_head_gather_sorted<<<nblocks(b.H), kBlock, 0, b.stream>>>(b.hsorted, b.H, b.head_slot, b.pos, b.hsorted_xg);
-  k_build_es_list<<<nblocks(b.H, 4), 128, 0, b.stream>>>(b.head_sys, b.H, b.head_slot, b.pos, b.sp, b.hcell_start,
-                                                        b.hsorted_xg, b.es_cap, b.es_nl, b.es_cnt, b.flags);
+  k_build_es_list<<<nblocks(b.H, 4), 128, 0, b.stream>>>(b.head_sys, b.H, b.sp, b.hcell_start, b.hsorted_xg, b.es_cap, b.es_nl, b.es_cnt, b.flags);
   b.launches += 6 + scans;
   prof_end(b);
 }
