@@ -38,6 +38,10 @@ __device__ __forceinline__ int match_rule(const Shared& S, float ti, float tj) {
   return -1;
 }
 
+// the claims' state: per bead by original id, `next` per item; items of one component are a list from its root's
+// head, `count` long
+struct Claims { uint32_t *parent, *head, *count, *has_item, *next; };
+
 // Phase A
 // A bead whose kind is in no rule has no candidate, draws nothing and, unless it is a catalyst or
 // tethered to one, leaves no item: its walk would change nothing (water, most of a campaign's beads).
@@ -47,12 +51,19 @@ __device__ __forceinline__ bool bond_active(const Shared& S, float ti, uint32_t 
   return in_rule || ti == S.cat_kind || centre != NONE;
 }
 
-// the active beads' slots, compacted (a warp's in one atomic); sel[0..*nsel) in no particular order
+// the active beads' slots, compacted (a warp's in one atomic); sel[0..*nsel) in no particular order.  It also
+// clears what the claims keep per bead (by original id).
 __global__ void __launch_bounds__(256) k_bond_select(const Shared* __restrict__ Sg, uint32_t N,
                                                      const float4* __restrict__ pos,
                                                      const uint32_t* __restrict__ center, uint32_t* __restrict__ sel,
-                                                     uint32_t* __restrict__ nsel) {
+                                                     uint32_t* __restrict__ nsel, Claims C) {
   const uint32_t k = blockIdx.x * blockDim.x + threadIdx.x;
+  if (k < N) {
+    C.parent[k] = k;
+    C.head[k] = NONE;
+    C.count[k] = 0;
+    C.has_item[k] = 0;
+  }
   const bool act = k < N && bond_active(*Sg, pos[k].w, center[k]);
   const uint32_t m = __ballot_sync(0xffffffffu, act);
   if (!m) return;
@@ -331,22 +342,26 @@ __device__ __forceinline__ int item_set(const uint32_t* rec, const uint32_t* cen
 // Phase B.  Every particle an item may touch runs its own desorption check in its turn, so it needs
 // an item too (proposal partners are the only ones the walk does not already cover): added here, by
 // the whole grid, before the claims.
-// nitems[1] holds the walk's item count: only the walk's items add partners (nitems[0] grows meanwhile).
+// nitems[1] holds the walk's item count: only the walk's items add partners (nitems[0] grows meanwhile).  Items whose
+// particle sets meet are joined on the way (union-find over the sets closed under centre links).
 __global__ void k_bond_partners(const uint32_t* __restrict__ center, const uint32_t* __restrict__ slot_of,
-                                uint32_t* __restrict__ items, uint32_t* __restrict__ nitems, uint32_t item_cap,
-                                uint32_t* __restrict__ has_item, uint32_t* __restrict__ flags) {
+                                uint32_t* __restrict__ items, uint32_t* __restrict__ nitems, uint32_t item_cap, Claims C,
+                                uint32_t* __restrict__ flags) {
   const uint32_t M0 = min(nitems[1], item_cap);
   uint32_t setbuf[2 * (2 + SOUP_CAND_CAP)];
   for (uint32_t t = blockIdx.x * blockDim.x + threadIdx.x; t < M0; t += gridDim.x * blockDim.x) {
     const int n = item_set(items + (size_t)t * REC, center, slot_of, setbuf);
     for (int q = 0; q < n; ++q) {
       const uint32_t x = setbuf[q];
-      if (atomicCAS(&has_item[x], 0u, 1u) == 0u) {
+      if (q) uf_union(C.parent, setbuf[0], x);
+      if (atomicCAS(&C.has_item[x], 0u, 1u) == 0u) {
         const uint32_t at = atomicAdd(nitems, 1u);
         if (at < item_cap) {
           uint32_t* nr = items + (size_t)at * REC;
           nr[0] = x; nr[1] = NONE; nr[2] = 0;
           for (int c = 0; c < SOUP_CAND_CAP; ++c) nr[3 + c] = NONE;
+          const uint32_t cx = center[slot_of[x]];
+          if (cx != NONE) uf_union(C.parent, x, cx);
         } else {
           flags[6] = 1u;
         }
@@ -355,119 +370,86 @@ __global__ void k_bond_partners(const uint32_t* __restrict__ center, const uint3
   }
 }
 
-// The claims of one replica per CTA (an item's set of particles never leaves its replica, so the
-// replicas' components are disjoint and resolve independently).  The CTA collects its items, joins the
-// items whose particle sets meet (union-find over the sets closed under centre links), and then in
-// rounds executes the minimum-id pending item of every component: the serial ascending order within
-// each component, which is all the serial order decides.
-constexpr uint32_t kClaimLocal = 8192;   // a replica's items held as a list in shared memory
-__global__ void __launch_bounds__(1024) k_bond_claims(
+// the components' lists of items, in no particular order
+__global__ void k_bond_lists(uint32_t* __restrict__ items, const uint32_t* __restrict__ nitems, uint32_t item_cap, Claims C) {
+  const uint32_t M = min(*nitems, item_cap);
+  for (uint32_t t = blockIdx.x * blockDim.x + threadIdx.x; t < M; t += gridDim.x * blockDim.x) {
+    const uint32_t root = uf_find(C.parent, items[(size_t)t * REC]);
+    items[(size_t)t * REC + 9] = root;
+    C.next[t] = atomicExch(&C.head[root], t);
+    atomicAdd(&C.count[root], 1u);
+  }
+}
+
+// Phase B, the claims: the items of a component in ascending order of their ids, which is all that the serial order
+// decides (components touch disjoint particles).  A thread runs a component of up to kClaimSerial items, its
+// list sorted first; eight threads of a warp work, so that components of unequal length hold up few others.  The
+// items of larger components are left to the last block to finish, which runs them in rounds: of every
+// component the pending item with the smallest id.
+// Bound: the chain of gathers of an item.  (One CTA a replica ran all of them: 435 us at 483k beads.)
+constexpr uint32_t kClaimSerial = 24;
+__global__ void __launch_bounds__(256) k_bond_claims(
     const Shared* __restrict__ Sg, const SysParams* __restrict__ sp, const uint8_t* __restrict__ sysid,
     const float4* __restrict__ pos, uint32_t* __restrict__ slots, uint32_t* __restrict__ center,
-    uint32_t* __restrict__ held, const uint32_t* __restrict__ slot_of, uint32_t* __restrict__ items,
-    const uint32_t* __restrict__ nitems, uint32_t item_cap, uint32_t* __restrict__ parent,
-    uint32_t* __restrict__ comp_min, uint8_t* __restrict__ done, uint32_t* __restrict__ events,
-    uint32_t* __restrict__ desorb) {
-  __shared__ Shared S;
-  __shared__ uint32_t mine[kClaimLocal];
-  __shared__ uint32_t nmine;
-  for (int w = threadIdx.x; w < (int)(sizeof(Shared) / 4); w += blockDim.x)
-    reinterpret_cast<uint32_t*>(&S)[w] = reinterpret_cast<const uint32_t*>(Sg)[w];
-  if (threadIdx.x == 0) nmine = 0;
-  __syncthreads();
-  const uint32_t r = blockIdx.x;
+    uint32_t* __restrict__ held, const uint32_t* __restrict__ slot_of, const uint32_t* __restrict__ items,
+    uint32_t* __restrict__ nitems, uint32_t item_cap, Claims C, uint32_t* __restrict__ large,
+    uint32_t* __restrict__ events, uint32_t* __restrict__ desorb) {
+  __shared__ bool last;
   const uint32_t M = min(*nitems, item_cap);
-  // this replica's items (any order: the rounds below depend on item ids, not positions); a batch of
-  // one replica takes them all as they are
-  const bool all = gridDim.x == 1;
-  if (!all) {
-    for (uint32_t t = threadIdx.x; t < M; t += blockDim.x)
-      if (sysid[slot_of[items[(size_t)t * REC]]] == r) {
-        const uint32_t at = atomicAdd(&nmine, 1u);
-        if (at < kClaimLocal) mine[at] = t;
+  St st{*Sg, sp, sysid, pos, slots, center, held, slot_of, events, desorb};
+  if ((threadIdx.x & 3u) == 0) {
+    for (uint32_t t = (blockIdx.x * blockDim.x + threadIdx.x) >> 2; t < M; t += (gridDim.x * blockDim.x) >> 2) {
+      const uint32_t* rec = items + (size_t)t * REC;
+      const uint32_t root = rec[9], n = C.count[root];
+      if (n > kClaimSerial) {
+        large[atomicAdd(&nitems[3], 1u)] = t;
+      } else if (n == 1) {
+        st.run(rec);
+      } else if (C.head[root] == t) {
+        uint32_t at[kClaimSerial], key[kClaimSerial];
+        uint32_t m = 0;
+        for (uint32_t u = t; u != NONE; u = C.next[u], ++m) {
+          const uint32_t id = items[(size_t)u * REC];
+          uint32_t p = m;
+          for (; p > 0 && key[p - 1] > id; --p) { key[p] = key[p - 1]; at[p] = at[p - 1]; }
+          key[p] = id;
+          at[p] = u;
+        }
+        for (uint32_t p = 0; p < m; ++p) st.run(items + (size_t)at[p] * REC);
       }
-  }
-  __syncthreads();
-  const bool local = !all && nmine <= kClaimLocal;
-  const uint32_t L = local ? nmine : M;
-  // item u of this CTA, or NONE for another replica's item (when the list did not fit)
-  auto item = [&](uint32_t u) -> uint32_t {
-    if (all) return u;
-    if (local) return mine[u];
-    return sysid[slot_of[items[(size_t)u * REC]]] == r ? u : NONE;
-  };
-  uint32_t setbuf[2 * (2 + SOUP_CAND_CAP)];
-  for (uint32_t u = threadIdx.x; u < L; u += blockDim.x) {
-    const uint32_t t = item(u);
-    if (t == NONE) continue;
-    const int n = item_set(items + (size_t)t * REC, center, slot_of, setbuf);
-    for (int q = 0; q < n; ++q) parent[setbuf[q]] = setbuf[q];
-    done[t] = 0;
-  }
-  __syncthreads();
-  for (uint32_t u = threadIdx.x; u < L; u += blockDim.x) {
-    const uint32_t t = item(u);
-    if (t == NONE) continue;
-    const int n = item_set(items + (size_t)t * REC, center, slot_of, setbuf);
-    for (int q = 1; q < n; ++q) uf_union(parent, setbuf[0], setbuf[q]);
-  }
-  __syncthreads();
-  for (uint32_t u = threadIdx.x; u < L; u += blockDim.x) {
-    const uint32_t t = item(u);
-    if (t == NONE) continue;
-    uint32_t* rec = items + (size_t)t * REC;
-    const uint32_t root = uf_find(parent, rec[0]);
-    rec[9] = root;
-    comp_min[root] = NONE;
-  }
-  __syncthreads();
-  St st{S, sp, sysid, pos, slots, center, held, slot_of, events, desorb};
-  // the rounds behind the first one hold a few items: with at most 32 items a thread, its pending ones are bits
-  // of a word
-  if (L <= 32u * blockDim.x) {
-    uint32_t pend = 0;
-    for (uint32_t q = 0, u = threadIdx.x; u < L; ++q, u += blockDim.x) pend |= (item(u) != NONE ? 1u : 0u) << q;
-    while (__syncthreads_or(pend != 0)) {
-      for (uint32_t m = pend; m; m &= m - 1u) {
-        const uint32_t* rec = items + (size_t)item(threadIdx.x + (uint32_t)(__ffs(m) - 1) * blockDim.x) * REC;
-        atomicMin(&comp_min[rec[9]], rec[0]);
-      }
-      __syncthreads();
-      uint32_t left = 0;
-      for (uint32_t m = pend; m; m &= m - 1u) {
-        const uint32_t* rec = items + (size_t)item(threadIdx.x + (uint32_t)(__ffs(m) - 1) * blockDim.x) * REC;
-        if (comp_min[rec[9]] == rec[0]) st.run(rec);
-        else left |= m & (0u - m);
-      }
-      __syncthreads();
-      for (uint32_t m = left; m; m &= m - 1u)
-        comp_min[items[(size_t)item(threadIdx.x + (uint32_t)(__ffs(m) - 1) * blockDim.x) * REC + 9]] = NONE;
-      pend = left;
-      __syncthreads();
     }
-    return;
   }
-  for (int round = 0;; ++round) {
+  __threadfence();
+  __syncthreads();
+  if (threadIdx.x == 0) last = atomicAdd(&nitems[4], 1u) == gridDim.x - 1u;
+  __syncthreads();
+  if (!last) return;
+  __threadfence();
+  const uint32_t L = *(volatile uint32_t*)&nitems[3];
+  volatile uint32_t* big = large;
+  volatile uint32_t* low = C.head;                       // by root: the smallest pending id
+  for (uint32_t u = threadIdx.x; u < L; u += blockDim.x) low[items[(size_t)big[u] * REC + 9]] = NONE;
+  for (;;) {
     int pending = 0;
+    __syncthreads();
     for (uint32_t u = threadIdx.x; u < L; u += blockDim.x) {
-      const uint32_t t = item(u);
-      if (t == NONE || done[t]) continue;
+      const uint32_t t = big[u];
+      if (t == NONE) continue;
       pending = 1;
-      atomicMin(&comp_min[items[(size_t)t * REC + 9]], items[(size_t)t * REC]);
+      atomicMin(&C.head[items[(size_t)t * REC + 9]], items[(size_t)t * REC]);
     }
     if (!__syncthreads_or(pending)) break;
     for (uint32_t u = threadIdx.x; u < L; u += blockDim.x) {
-      const uint32_t t = item(u);
-      if (t == NONE || done[t]) continue;
+      const uint32_t t = big[u];
+      if (t == NONE) continue;
       const uint32_t* rec = items + (size_t)t * REC;
-      if (comp_min[rec[9]] == rec[0]) { st.run(rec); done[t] = 1; }
+      if (low[rec[9]] == rec[0]) { st.run(rec); big[u] = NONE; }
     }
     __syncthreads();
     for (uint32_t u = threadIdx.x; u < L; u += blockDim.x) {
-      const uint32_t t = item(u);
-      if (t != NONE) comp_min[items[(size_t)t * REC + 9]] = NONE;
+      const uint32_t t = big[u];
+      if (t != NONE) low[items[(size_t)t * REC + 9]] = NONE;
     }
-    __syncthreads();
   }
 }
 
@@ -506,22 +488,23 @@ __global__ void k_bond_break(const Shared* __restrict__ Sg, const uint8_t* __res
 }  // namespace
 
 void launch_bonds(Batch& b) {
-  b.launches += 5;
+  b.launches += 6;
   prof_begin(b, SOUP_K_BONDS);
-  cudaMemsetAsync(b.bond_nitems, 0, 3 * sizeof(uint32_t), b.stream);
-  cudaMemsetAsync(b.has_item, 0, sizeof(uint32_t) * b.N, b.stream);
-  uint32_t* has_item = b.has_item;
+  const Claims C{b.uf_parent, b.comp_head, b.comp_count, b.has_item, b.item_next};
+  cudaMemsetAsync(b.bond_nitems, 0, 5 * sizeof(uint32_t), b.stream);
   k_bond_select<<<nblocks(b.N, 256), 256, 0, b.stream>>>(b.shared, b.N, b.pos, b.center, b.bond_sel,
-                                                         b.bond_nitems + 2);
+                                                         b.bond_nitems + 2, C);
   k_bond_walk<<<std::min(nblocks(b.N, 4), 148u * 16u), 128, 0, b.stream>>>(
       b.shared, b.sp, b.sysid, b.bond_sel, b.bond_nitems + 2, b.pos, b.charge, b.id, b.slots, b.center, b.nl, b.nl_cnt,
-      b.prune ? b.nl_shell : nullptr, b.drift_bits, b.list_stride, b.brng, b.bond_items, b.bond_nitems, has_item);
+      b.prune ? b.nl_shell : nullptr, b.drift_bits, b.list_stride, b.brng, b.bond_items, b.bond_nitems, b.has_item);
   cudaMemcpyAsync(b.bond_nitems + 1, b.bond_nitems, sizeof(uint32_t), cudaMemcpyDeviceToDevice, b.stream);
-  k_bond_partners<<<std::max(1u, std::min(nblocks(b.N, 256) / 8u, 592u)), 256, 0, b.stream>>>(
-      b.center, b.slot_of, b.bond_items, b.bond_nitems, b.N, has_item, b.flags);
-  k_bond_claims<<<b.R, 1024, 0, b.stream>>>(b.shared, b.sp, b.sysid, b.pos, b.slots, b.center, b.held, b.slot_of,
-                                            b.bond_items, b.bond_nitems, b.N, b.uf_parent, b.comp_min, b.item_done,
-                                            b.events, b.desorb);
+  const unsigned over_items = std::max(1u, std::min(nblocks(b.N, 256) / 8u, 592u));
+  k_bond_partners<<<over_items, 256, 0, b.stream>>>(b.center, b.slot_of, b.bond_items, b.bond_nitems, b.N, C, b.flags);
+  k_bond_lists<<<over_items, 256, 0, b.stream>>>(b.bond_items, b.bond_nitems, b.N, C);
+  // (the walk is over: its selection's buffer takes the large components' items)
+  k_bond_claims<<<std::min(nblocks(b.N, 256), 592u), 256, 0, b.stream>>>(
+      b.shared, b.sp, b.sysid, b.pos, b.slots, b.center, b.held, b.slot_of, b.bond_items, b.bond_nitems, b.N, C, b.bond_sel,
+      b.events, b.desorb);
   k_bond_break<<<nblocks(b.N), kBlock, 0, b.stream>>>(b.shared, b.sysid, b.N, b.pos, b.id, b.slot_of, b.slots,
                                                       b.brng, b.events);
   prof_end(b);

@@ -396,8 +396,8 @@ Batch* make_batch(const SoupConfig* cfgs, const SoupInitState* inits, uint32_t R
   b.desorb = dalloc<uint32_t>(2 * (size_t)R);
   b.drift_bits = dalloc<uint32_t>(R);
   // [0] item count, [1] the walk's count, [2] the active beads (k_bond_select)
-  b.bond_items = dalloc<uint32_t>(10 * n); b.bond_nitems = dalloc<uint32_t>(3); b.bond_sel = dalloc<uint32_t>(n);
-  b.uf_parent = dalloc<uint32_t>(n); b.comp_min = dalloc<uint32_t>(n); b.item_done = dalloc<uint8_t>(n);
+  b.bond_items = dalloc<uint32_t>(10 * n); b.bond_nitems = dalloc<uint32_t>(5); b.bond_sel = dalloc<uint32_t>(n);
+  b.uf_parent = dalloc<uint32_t>(n); b.comp_head = dalloc<uint32_t>(n); b.comp_count = dalloc<uint32_t>(n); b.item_next = dalloc<uint32_t>(n);
   b.has_item = dalloc<uint32_t>(n);
   b.prot_rng_dev = dalloc<uint32_t>(R);
   b.rebuild_count = dalloc<uint32_t>(1);
@@ -482,8 +482,8 @@ void destroy_batch(Batch* b) {
                   b->held2, b->brng2, b->trng2, b->frozen2, b->id2, b->cell_of_slot, b->cell_count, b->cell_start,
                   b->cell_cursor, b->perm, b->scan_tmp, b->nl, b->nl_cnt, b->nl_shell, b->heads, b->head_sys, b->es_nl,
                   b->es_cnt, b->head_slot, b->head_e, b->head_pos, b->head_xq, b->head_d, b->draw_site, b->pair_cnt, b->pair_idx, b->pair_del, b->walk_shared, b->hcell_count, b->hcell_start, b->hcell_cursor, b->hsorted, b->hsorted_xg, b->hcell_of, b->flags,
-                  b->events, b->desorb, b->drift_bits, b->bond_items, b->bond_nitems, b->bond_sel, b->uf_parent, b->comp_min,
-                  b->item_done, b->has_item, b->sweep_out, b->prot_rng_dev, b->sp, b->shared, b->sysid, b->an_buf[0],
+                  b->events, b->desorb, b->drift_bits, b->bond_items, b->bond_nitems, b->bond_sel, b->uf_parent, b->comp_head, b->comp_count,
+                  b->item_next, b->has_item, b->sweep_out, b->prot_rng_dev, b->sp, b->shared, b->sysid, b->an_buf[0],
                   b->an_buf[1]};
   for (void* p : ptrs) if (p) cudaFree(p);
   for (void* p : {(void*)b->diff.frames, (void*)b->diff.A, (void*)b->diff.B, (void*)b->diff.g, (void*)b->diff.jg,

@@ -141,8 +141,8 @@ struct Batch {
   uint32_t* bond_nitems = nullptr;
   uint32_t* bond_sel = nullptr;      // the active beads of a bond pass, compacted
   uint32_t* uf_parent = nullptr;     // per original id
-  uint32_t* comp_min = nullptr;      // per original id
-  uint8_t* item_done = nullptr;
+  uint32_t *comp_head = nullptr, *comp_count = nullptr;   // per original id
+  uint32_t* item_next = nullptr;
   uint32_t* has_item = nullptr;
 
   // constant-pH sweep scratch / host state
