@@ -157,7 +157,9 @@ __device__ __forceinline__ void block_theta(const ThetaAcc& th, double* __restri
 // (J g) of the list force (nonbonded + bonded + wall) and the parameter partials, kTpp lanes per
 // particle; jg is written (not accumulated), by original index.  gs: g in slot order, so that an entry is two
 // independent gathers.  Rows are read as far as the force reads them (list_force_end; drift: the largest
-// displacement of the frame since the lists' build): the rest is beyond the reach.  Bound: the gathers.
+// displacement of the frame since the lists' build): the rest is beyond the reach.
+// Bound: the gathers.  (With the depth partials indexed, so in local memory, and g gathered through the ids it took
+// 76 us at 33k beads.)
 __global__ void __launch_bounds__(kBlock) k_hvp(const Shared* __restrict__ Sg, const SysParams* __restrict__ sp,
                                                 const uint8_t* __restrict__ sysid, uint32_t N,
                                                 const float4* __restrict__ pos, const float* __restrict__ charge,

@@ -117,7 +117,10 @@ constexpr int kForceBlock = 128;
 
 // SEL: the particles are the nsel slots sel[] (the heads, after a charge sweep) instead of all N
 //
-// Bound: instruction issue and the neighbour gathers.  %FORCE%
+// Bound: the L1's wavefronts for the neighbour gathers (two thirds of its rate) and the issue of the pair maths
+// (half).  Straight-line pairs over sixteen fixed partial sums, rows read to each bead's own reach and chunks stored for the
+// lanes' order took it from 250 to 168 us right after a rebuild at 483k beads, 309 to 187 over a rebuild's steps.
+// Slower: gathers pipelined an iteration ahead (242), three or five blocks of 256 an SM (214, 244).
 template <int TPP, bool SEL>
 __global__ void __launch_bounds__(kForceBlock, 8) k_force(
     const Shared* __restrict__ Sg, const SysParams* __restrict__ sp, const uint8_t* __restrict__ sysid, uint32_t N,
@@ -201,7 +204,9 @@ __global__ void __launch_bounds__(kForceBlock, 8) k_force(
   }
 }
 
-// soup/wgsl/electrostatics-long.wgsl:63-82 soup_es_force_far_main, a warp per head.
+// soup/wgsl/electrostatics-long.wgsl:63-82 soup_es_force_far_main, a warp per head, on the records that the list
+// force wrote.  Bound: the latency of the gathers.  A lane has four in flight and the next four entries loaded (one at
+// a time: 48.9 against 39.1 us at 483k beads, 12.5 against 8.7 at 24k).
 __global__ void __launch_bounds__(256) k_es_far(const SysParams* __restrict__ sp, const uint32_t* __restrict__ head_slot,
                                                 const uint32_t* __restrict__ head_sys, uint32_t H,
                                                 const float4* __restrict__ xq, const uint32_t* __restrict__ es_nl,
@@ -345,7 +350,8 @@ void launch_force(Batch& b) {
 }
 
 // Lanes per particle: the result is the same bits, so the launch's size decides.  Few particles need the lanes
-// to cover the gathers' latency; many need the fewest instructions.  %TPP%
+// to cover the gathers' latency; many need the fewest instructions.  Measured with 4 / 8 / 16 lanes: 483k beads 241 /
+// 264 / 318 us, 121k 95 / - / 97, 24k 26.4 / 27.3 / 24.7, the 700 heads of a small system 31.6 / 22 / 13.5.
 int force_lanes(const Batch& b, uint32_t n) {
   if (b.tpp) return b.tpp <= 4 ? 4 : (b.tpp <= 8 ? 8 : 16);
   return n >= 80000u ? 4 : (n >= 40000u ? 8 : 16);

@@ -336,20 +336,21 @@ constexpr uint32_t kRowSpare = 64, kRowSlack = kRowSpare + 64;
 // lies within 1e-5 of the range, where the reference's arithmetic decides (the minimum image cannot differ
 // there: range < box/2), so the list is the reference's set.  The accepted entries are compacted into the
 // warp's shared row with ballots, then the row is grouped by build-distance shell, keeping its order inside
-// a shell, and written once, coalesced.  Every whole chunk of 16 entries is stored transposed (entry 4 e + l at
+// a shell, straight into memory.  Every whole chunk of 16 entries is stored transposed (entry 4 e + l at
 // place 4 l + e), so that the force's four lanes of a particle, which read four places each, gather four
 // successive entries at a time: beads of one run, which share cache lines.
 //
-// Bound: instruction issue (about 17 rounds of 32 candidates, some 35 instructions each, and 200 to group the
-// row).  Grouping in shared memory takes the place of a second pass that read and rewrote every row.
+// Bound: instruction issue (78% of the slots, with the shared rows holding 32 warps an SM): at a range of 4.45 sigma
+// about 600 candidates a bead, 295 of them in range.  At 483k beads a thread per bead and a second pass that grouped
+// the rows took 1533 + 411 us, this 1185; at 24k 306 and 57, at 3.3k 393 and 18.
 __global__ void __launch_bounds__(128) k_build_list(
     const Shared* __restrict__ Sg, const float4* __restrict__ pos, const float* __restrict__ charge,
     const uint8_t* __restrict__ sysid, const SysParams* __restrict__ sp, const uint32_t* __restrict__ start, uint32_t N,
-    uint32_t cap, uint32_t stride, uint32_t* __restrict__ nl, uint32_t* __restrict__ nl_cnt,
+    uint32_t cap, uint32_t held, uint32_t stride, uint32_t* __restrict__ nl, uint32_t* __restrict__ nl_cnt,
     uint32_t* __restrict__ shell_end, uint32_t* __restrict__ flags) {
   extern __shared__ __align__(16) uint32_t sm[];
   const uint32_t wib = threadIdx.x >> 5, lane = threadIdx.x & 31u, lt = (1u << lane) - 1u;
-  uint32_t* row = sm + (size_t)wib * (stride + kRowSlack + kWalkWords);   // stride: cap rounded up to 16
+  uint32_t* row = sm + (size_t)wib * (held + kRowSlack + kWalkWords);   // held: the entries it takes, cap at most
   const uint32_t k = blockIdx.x * (blockDim.x >> 5) + wib;
   if (k >= N) return;   // whole warps
   const SysParams& P = sp[sysid[k]];
@@ -384,7 +385,7 @@ __global__ void __launch_bounds__(128) k_build_list(
     cnt += __popc(m);
   };
   auto walk = [&](auto image) {
-    warp_walk(xi, k, box, G, start, row + stride + kRowSlack, [&](uint32_t j0, uint32_t j1) {
+    warp_walk(xi, k, box, G, start, row + held + kRowSlack, [&](uint32_t j0, uint32_t j1) {
       const float4 x0 = pos[j0], x1 = pos[j1];
       put(image, j0, x0);
       put(image, j1, x1);
@@ -580,16 +581,22 @@ void launch_sort_and_gather(Batch& b) {
 void launch_build_lists(Batch& b) {
   b.launches += 1;
   prof_begin(b, SOUP_K_LIST);
-  // a row of shared memory per warp: four warps per block while they fit
-  const size_t per = sizeof(uint32_t) * ((size_t)b.list_stride + kRowSlack + kWalkWords);
+  // a row of shared memory per warp: four warps per block while they fit.  A row has no more entries than
+  // its replica has beads, whatever its capacity; one of more than kRowMost (beads of one clump) is reported as too long
+  uint32_t most = 0;
+  for (uint32_t r = 0; r < b.R; ++r) most = std::max(most, b.hsp[r].n);
+  constexpr uint32_t kRowMost = 50u * 1024u;
+  const uint32_t cap = std::min(b.list_cap, std::min((most + 15u) & ~15u, kRowMost));
+  const uint32_t held = (cap + 15u) & ~15u;
+  const size_t per = sizeof(uint32_t) * ((size_t)held + kRowSlack + kWalkWords);
   const uint32_t wpb = 4u * per <= 200u * 1024u ? 4u : 1u;
   const size_t smem = wpb * per;
-  if (smem > 48u * 1024u && b.list_smem_set < smem) {
-    SOUP_CUDA_TRY(cudaFuncSetAttribute(k_build_list, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    b.list_smem_set = smem;
+  if (smem > 48u * 1024u && !b.list_smem_open) {       // to all an SM has: the setting is the device's, not this batch's
+    SOUP_CUDA_TRY(cudaFuncSetAttribute(k_build_list, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024));
+    b.list_smem_open = true;
   }
   k_build_list<<<(unsigned)((b.N + wpb - 1) / wpb), 32u * wpb, smem, b.stream>>>(
-      b.shared, b.pos, b.charge, b.sysid, b.sp, b.cell_start, b.N, b.list_cap, b.list_stride, b.nl, b.nl_cnt, b.nl_shell,
+      b.shared, b.pos, b.charge, b.sysid, b.sp, b.cell_start, b.N, cap, held, b.list_stride, b.nl, b.nl_cnt, b.nl_shell,
       b.flags);
   prof_end(b);
 }

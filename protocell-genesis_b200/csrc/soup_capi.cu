@@ -1003,6 +1003,11 @@ void tune_plan(Batch& b, const std::vector<double>& skin, int walk) {
   alloc_grids(b);
   upload_params(b);
 }
+// a tuning's lanes per particle: 8 stands for eight or the sixteen that a small launch takes by itself
+int tuned_lanes(Batch& b, uint32_t tpp) {
+  b.tpp = 0;
+  return tpp == 8 && force_lanes(b, b.N) > 8 ? 0 : (int)tpp;
+}
 template <class F> double tune_time(Batch& b, int reps, F&& f) {
   cudaEvent_t e0, e1;
   SOUP_CUDA_TRY(cudaEventCreate(&e0));
@@ -1489,7 +1494,7 @@ int soup_autotune(SoupHandle* h, uint32_t steps, SoupTuneResult* out) {
     std::vector<double> planned(b.R);
     for (uint32_t r = 0; r < b.R; ++r) planned[r] = b.cfg[r].skin;
     const int walk0 = b.hsp[0].walk;
-    const int tpp0 = force_lanes(b, b.N);
+    const int tpp0 = std::min(force_lanes(b, b.N), 8);
     auto steps_ms = [&]() { return tune_time(b, 1, [&] { step_batch(b, steps); }) / steps; };
     SoupTuneResult res{};
     if (steps) {
@@ -1498,12 +1503,12 @@ int soup_autotune(SoupHandle* h, uint32_t steps, SoupTuneResult* out) {
     }
     // block shape: lanes per particle of the list force, timed on the force alone
     double best = 1e30;
-    for (int t : {4, 8}) {
-      b.tpp = t;
+    for (uint32_t t : {4u, 8u}) {
+      b.tpp = tuned_lanes(b, t);
       const double ms = tune_time(b, 5, [&] { launch_force_list(b); });
-      if (ms < best) { best = ms; res.tpp = (uint32_t)t; }
+      if (ms < best) { best = ms; res.tpp = t; }
     }
-    b.tpp = (int)res.tpp;
+    b.tpp = tuned_lanes(b, res.tpp);
     drop_graphs(b);
     // cell size (the list-walk radius: cell = list range / walk), timed on the list build and, as the walk
     // sets the slot order the force gathers in, the ten force passes of a typical rebuild interval
@@ -1554,7 +1559,7 @@ int soup_apply_tuning(SoupHandle* h, const SoupTuneResult* t) {
     if (!(t->skin_scale > 0.0 && t->skin_scale <= 1.0)) fail(SOUP_E_ARG, "tuning: skin_scale must be in (0, 1]");
     if (t->skin_scale != 1.0 && !b.cfg[0].rebuild_on_drift)
       fail(SOUP_E_ARG, "tuning: the skin can only be scaled with drift-triggered rebuilds");
-    b.tpp = (int)t->tpp;
+    b.tpp = tuned_lanes(b, t->tpp);
     std::vector<double> sk(b.R);
     for (uint32_t r = 0; r < b.R; ++r) sk[r] = b.cfg[r].skin * t->skin_scale;
     tune_plan(b, sk, (int)t->walk);

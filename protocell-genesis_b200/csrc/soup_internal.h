@@ -101,7 +101,7 @@ struct Batch {
   uint32_t* nl = nullptr;
   uint32_t* nl_cnt = nullptr;
   uint32_t* nl_shell = nullptr;      // per slot kShells words: where the row's build-distance shells end
-  size_t list_smem_set = 0;          // dynamic shared memory k_build_list was opened to
+  bool list_smem_open = false;       // k_build_list may take more than 48 KB of shared memory
   bool prune = true;                 // force passes read only the shells the drift can have brought in range
 
   // heads / long-range electrostatics
