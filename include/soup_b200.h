@@ -315,7 +315,8 @@ int soup_set_wait_limit(SoupHandle* h, uint32_t polls);
 
 /* ---- Monte Carlo and analysis -------------------------------------------------------------- */
 /* protonationSweepDEBUG (soup/src/sim.ts): one constant-pH sweep now on the device, then the
- * rebuild + force recompute (soup/src/soup-protonation.ts:52-77). */
+ * rebuild + force recompute (soup/src/soup-protonation.ts:52-77).  With drift-triggered rebuilds the lists are
+ * rebuilt here only if the drift calls for it: they do not depend on charges. */
 int soup_protonation_sweep(SoupHandle* h, SoupSweepResult* out);
 
 /* encapsulatedWaterVolume (soup/src/water-closure.ts:271-363) on the current positions.

@@ -176,3 +176,25 @@ def test_a_window_leaves_its_end_behind():
         assert np.array_equal(a, b)
     g.step(1)
     g.dispose()
+
+
+def test_a_sweep_keeps_the_lists_while_they_serve():
+    cfg, o, g = make_pair(charged_opts(rebuild_on_drift=True, skin=0.6), relax=20)
+    g.step(3)
+
+    def force_is_right():
+        now = ob.OracleSystem(_abi, cfg, dict(positions=g.particles(), charges=g.charges(), bond_slots=g.bond_slots(),
+                                              center_link=g.center_links()))
+        return rel_rms(g.forces_no_rebuild(), now.forces64()) < FORCE_TOL
+    built = g.info()["rebuilds"]
+    g.debug_phase(_abi.PHASE_MAX_DRIFT)
+    g.protonation_sweep()
+    assert g.info()["rebuilds"] == built and force_is_right()
+    for _ in range(100):                      # kicks and drifts alone: no step looks at the drift
+        for _ in range(5):
+            g.debug_phase(_abi.PHASE_KICK_DRIFT)
+        g.protonation_sweep()
+        if g.info()["rebuilds"] > built:
+            break
+    assert g.info()["rebuilds"] == built + 1 and force_is_right()
+    g.dispose()
