@@ -68,43 +68,62 @@ __global__ void k_scan_block(const uint32_t* __restrict__ in, uint32_t* __restri
     run += v[e];
   }
 }
-__global__ void k_scan_add(uint32_t* __restrict__ out, uint32_t n, const uint32_t* __restrict__ block_offs) {
-  uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < n) out[i] += block_offs[i / 4096u];
-}
-__global__ void k_set_total(uint32_t* __restrict__ start, const uint32_t* __restrict__ count, uint32_t n) {
-  start[n] = start[n - 1] + count[n - 1];
+// The blocks' offsets added, a block of threads per scanned block, and the total behind the last.  RAW: `sums` are
+// the blocks' own totals (at most 1024), and each block of threads adds up those before it; otherwise their scan.
+template <bool RAW>
+__global__ void __launch_bounds__(1024) k_scan_add(uint32_t* __restrict__ out, uint32_t n, const uint32_t* __restrict__ sums) {
+  __shared__ uint32_t before;
+  if (threadIdx.x == 0) before = RAW ? 0u : sums[blockIdx.x];
+  __syncthreads();
+  if (RAW) {
+    const uint32_t v = __reduce_add_sync(0xffffffffu, threadIdx.x < blockIdx.x ? sums[threadIdx.x] : 0u);
+    if ((threadIdx.x & 31u) == 0 && v) atomicAdd(&before, v);
+    __syncthreads();
+  }
+  const uint32_t off = before;
+#pragma unroll
+  for (uint32_t e = 0; e < 4u; ++e) {
+    const uint32_t i = blockIdx.x * 4096u + e * 1024u + threadIdx.x;
+    if (i < n) out[i] += off;
+  }
+  if (threadIdx.x == 0 && blockIdx.x + 1u == gridDim.x) out[n] = RAW ? off + sums[blockIdx.x] : sums[gridDim.x];
 }
 
 }  // namespace
 
 // exclusive scan of in[0..n) into out[0..n), out[n] = total; tmp must hold >= 2*ceil(n/4096)+2 words.
+// One launch to 4096 words, two to 4M (a rebuild of a small system is a chain of launches of 2 us each), and
+// beyond that, where a block's offset would be a sum of more than 1024 totals, the totals are scanned first.
+// With two, five and more launches, and memsets of their own for what the sort and the lists need zeroed, a force
+// evaluation of 1,220 beads took 112 us (99 now) and ten steps of 3,277 beads 412 (398).
 // Returns the kernels it launched (no shared counter: calls from several host threads do not race).
 uint64_t exclusive_scan(const uint32_t* in, uint32_t* out, uint32_t n, uint32_t* tmp, cudaStream_t st) {
   if (n == 0) return 0;
-  uint64_t launches = 2;
-  uint32_t nb = (n + 4095) / 4096;
+  const uint32_t nb = (n + 4095) / 4096;
   if (nb == 1) {
-    k_scan_block<<<1, 1024, 0, st>>>(in, out, n, nullptr);
-  } else {
-    uint32_t* sums = tmp;
-    uint32_t* offs = tmp + nb + 1;
-    k_scan_block<<<nb, 1024, 0, st>>>(in, out, n, sums);
-    launches += exclusive_scan(sums, offs, nb, offs + nb + 1, st) + 1;
-    k_scan_add<<<nblocks(n), kBlock, 0, st>>>(out, n, offs);
+    k_scan_block<<<1, 1024, 0, st>>>(in, out, n, out + n);
+    return 1;
   }
-  k_set_total<<<1, 1, 0, st>>>(out, in, n);
-  return launches;
+  uint32_t* sums = tmp;
+  k_scan_block<<<nb, 1024, 0, st>>>(in, out, n, sums);
+  if (nb <= 1024) {
+    k_scan_add<true><<<nb, 1024, 0, st>>>(out, n, sums);
+    return 2;
+  }
+  uint32_t* offs = tmp + nb + 1;
+  const uint64_t launches = exclusive_scan(sums, offs, nb, offs + nb + 1, st);
+  k_scan_add<false><<<nb, 1024, 0, st>>>(out, n, offs);
+  return launches + 2;
 }
 
 namespace {
 
 __global__ void k_scatter(const uint32_t* __restrict__ cell_of, const uint32_t* __restrict__ start, uint32_t N,
-                          uint32_t* __restrict__ cursor, uint32_t* __restrict__ perm) {
+                          uint32_t* __restrict__ count, uint32_t* __restrict__ perm) {
   uint32_t k = blockIdx.x * blockDim.x + threadIdx.x;
   if (k >= N) return;
   uint32_t c = cell_of[k];
-  perm[start[c] + atomicAdd(&cursor[c], 1u)] = k;
+  perm[start[c] + atomicSub(&count[c], 1u) - 1u] = k;   // the counts count the places down
 }
 
 // Inside each cell, order by original index: the atomic scatter order above varies run to run, this
@@ -157,7 +176,8 @@ __global__ void k_gather(uint32_t N, const uint32_t* __restrict__ perm,
 }
 
 // the gathered arrays back into the primary buffers, so every array keeps its address across rebuilds
-// (a captured step graph holds them as kernel arguments)
+// (a captured step graph holds them as kernel arguments).  What the lists' builds behind it need zeroed is zeroed
+// here: the head cells' counts and the replicas' drifts (a memset of its own is a launch)
 __global__ void k_copy_back(uint32_t N, const float4* __restrict__ pos2, const float4* __restrict__ vel2,
                             const float4* __restrict__ force2, const float* __restrict__ charge2,
                             const uint32_t* __restrict__ slots2, const uint32_t* __restrict__ center2,
@@ -167,9 +187,12 @@ __global__ void k_copy_back(uint32_t N, const float4* __restrict__ pos2, const f
                             float4* __restrict__ force, float* __restrict__ charge, uint32_t* __restrict__ slots,
                             uint32_t* __restrict__ center, uint32_t* __restrict__ held, uint32_t* __restrict__ brng,
                             uint32_t* __restrict__ trng, uint8_t* __restrict__ frozen, uint32_t* __restrict__ id,
-                            uint32_t* __restrict__ head_of) {
+                            uint32_t* __restrict__ head_of, uint32_t nhcells, uint32_t* __restrict__ hcount, uint32_t R,
+                            uint32_t* __restrict__ drift_bits) {
   const uint32_t k = blockIdx.x * blockDim.x + threadIdx.x;
   if (k >= N) return;
+  for (uint32_t c = k; c < nhcells; c += N) hcount[c] = 0u;
+  if (k < R) drift_bits[k] = 0u;   // a replica has a bead at least
   head_of[k] = SOUP_NONE_U32;   // k_head_index names the heads
   pos[k] = pos2[k]; vel[k] = vel2[k]; force[k] = force2[k]; charge[k] = charge2[k];
   slots[3 * k] = slots2[3 * k]; slots[3 * k + 1] = slots2[3 * k + 1]; slots[3 * k + 2] = slots2[3 * k + 2];
@@ -472,11 +495,11 @@ __global__ void k_head_index(const uint32_t* __restrict__ heads, const uint32_t*
   atomicAdd(&hcount[c], 1u);
 }
 __global__ void k_head_scatter(const uint32_t* __restrict__ hcell_of, const uint32_t* __restrict__ hstart, uint32_t H,
-                               uint32_t* __restrict__ hcursor, uint32_t* __restrict__ hsorted) {
+                               uint32_t* __restrict__ hcount, uint32_t* __restrict__ hsorted) {
   uint32_t h = blockIdx.x * blockDim.x + threadIdx.x;
   if (h >= H) return;
   uint32_t c = hcell_of[h];
-  hsorted[hstart[c] + atomicAdd(&hcursor[c], 1u)] = h;
+  hsorted[hstart[c] + atomicSub(&hcount[c], 1u) - 1u] = h;
 }
 __global__ void k_head_sort_cells(const uint32_t* __restrict__ hstart, uint32_t ncells, uint32_t* __restrict__ hsorted) {
   uint32_t c = blockIdx.x * blockDim.x + threadIdx.x;
@@ -563,8 +586,7 @@ void launch_cell_index(Batch& b) {
 void launch_sort_and_gather(Batch& b) {
   prof_begin(b, SOUP_K_SORT);
   const uint64_t scans = exclusive_scan(b.cell_count, b.cell_start, b.ncells, b.scan_tmp, b.stream);
-  cudaMemsetAsync(b.cell_cursor, 0, sizeof(uint32_t) * b.ncells, b.stream);
-  k_scatter<<<nblocks(b.N), kBlock, 0, b.stream>>>(b.cell_of_slot, b.cell_start, b.N, b.cell_cursor, b.perm);
+  k_scatter<<<nblocks(b.N), kBlock, 0, b.stream>>>(b.cell_of_slot, b.cell_start, b.N, b.cell_count, b.perm);
   k_sort_cells<<<nblocks(b.ncells), kBlock, 0, b.stream>>>(b.cell_start, b.ncells, b.id, b.perm);
   k_gather<<<nblocks(b.N), kBlock, 0, b.stream>>>(b.N, b.perm, b.pos, b.vel, b.force, b.charge, b.slots, b.center,
                                                    b.held, b.brng, b.trng, b.frozen, b.id, b.pos2, b.vel2, b.force2,
@@ -573,7 +595,7 @@ void launch_sort_and_gather(Batch& b) {
   k_copy_back<<<nblocks(b.N), kBlock, 0, b.stream>>>(b.N, b.pos2, b.vel2, b.force2, b.charge2, b.slots2, b.center2,
                                                       b.held2, b.brng2, b.trng2, b.frozen2, b.id2, b.pos, b.vel, b.force,
                                                       b.charge, b.slots, b.center, b.held, b.brng, b.trng, b.frozen,
-                                                      b.id, b.head_of);
+                                                      b.id, b.head_of, b.nhcells, b.hcell_count, b.R, b.drift_bits);
   b.launches += 4 + scans;
   prof_end(b);
 }
@@ -604,12 +626,10 @@ void launch_build_lists(Batch& b) {
 void launch_build_es_lists(Batch& b) {
   if (b.H == 0) return;
   prof_begin(b, SOUP_K_LIST);
-  cudaMemsetAsync(b.hcell_count, 0, sizeof(uint32_t) * (b.nhcells + 1), b.stream);
   k_head_index<<<nblocks(b.H), kBlock, 0, b.stream>>>(b.heads, b.head_sys, b.H, b.slot_of, b.pos, b.sp, b.hcell_of,
                                                        b.hcell_count, b.head_slot, b.head_of);
   const uint64_t scans = exclusive_scan(b.hcell_count, b.hcell_start, b.nhcells, b.scan_tmp, b.stream);
-  cudaMemsetAsync(b.hcell_cursor, 0, sizeof(uint32_t) * b.nhcells, b.stream);
-  k_head_scatter<<<nblocks(b.H), kBlock, 0, b.stream>>>(b.hcell_of, b.hcell_start, b.H, b.hcell_cursor, b.hsorted);
+  k_head_scatter<<<nblocks(b.H), kBlock, 0, b.stream>>>(b.hcell_of, b.hcell_start, b.H, b.hcell_count, b.hsorted);
   k_head_sort_cells<<<nblocks(b.nhcells), kBlock, 0, b.stream>>>(b.hcell_start, b.nhcells, b.hsorted);
   k_head_gather_sorted<<<nblocks(b.H), kBlock, 0, b.stream>>>(b.hsorted, b.H, b.head_slot, b.pos, b.hsorted_xg);
   k_build_es_list<<<nblocks(b.H, 4), 128, 0, b.stream>>>(b.head_sys, b.H, b.sp, b.hcell_start, b.hsorted_xg, b.es_cap, b.es_nl, b.es_cnt, b.flags);

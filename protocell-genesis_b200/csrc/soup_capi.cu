@@ -195,8 +195,8 @@ namespace {
 
 // ---- batch construction ----------------------------------------------------------------------
 void alloc_grids(Batch& b) {
-  dfree(b.cell_count); dfree(b.cell_start); dfree(b.cell_cursor); dfree(b.scan_tmp);
-  dfree(b.hcell_count); dfree(b.hcell_start); dfree(b.hcell_cursor);
+  dfree(b.cell_count); dfree(b.cell_start); dfree(b.scan_tmp);
+  dfree(b.hcell_count); dfree(b.hcell_start);
   uint64_t nc = 0, nh = 0;
   for (uint32_t r = 0; r < b.R; ++r) {
     b.hsp[r].cell_off = (uint32_t)nc;
@@ -209,10 +209,8 @@ void alloc_grids(Batch& b) {
   b.nhcells = (uint32_t)nh;
   b.cell_count = dalloc<uint32_t>(nc + 1);
   b.cell_start = dalloc<uint32_t>(nc + 1);
-  b.cell_cursor = dalloc<uint32_t>(nc + 1);
   b.hcell_count = dalloc<uint32_t>(nh + 1);
   b.hcell_start = dalloc<uint32_t>(nh + 1);
-  b.hcell_cursor = dalloc<uint32_t>(nh + 1);
   const uint64_t m = std::max(nc, nh);
   b.scan_tmp = dalloc<uint32_t>(4 * (m / 4096 + 64) + 256);
 }
@@ -239,7 +237,6 @@ void rebuild_launches(Batch& b) {
   launch_sort_and_gather(b);
   launch_build_lists(b);
   launch_build_es_lists(b);
-  SOUP_CUDA_TRY(cudaMemsetAsync(b.drift_bits, 0, sizeof(uint32_t) * b.R, b.stream));
 }
 void rebuild(Batch& b) {
   rebuild_launches(b);
@@ -480,8 +477,8 @@ void destroy_batch(Batch* b) {
   void* ptrs[] = {b->rebuild_count, b->pos, b->vel, b->force, b->pos_ref, b->charge, b->slots, b->center, b->held, b->brng, b->trng,
                   b->frozen, b->id, b->head_of, b->slot_of, b->pos2, b->vel2, b->force2, b->charge2, b->slots2, b->center2,
                   b->held2, b->brng2, b->trng2, b->frozen2, b->id2, b->cell_of_slot, b->cell_count, b->cell_start,
-                  b->cell_cursor, b->perm, b->scan_tmp, b->nl, b->nl_cnt, b->nl_shell, b->heads, b->head_sys, b->es_nl,
-                  b->es_cnt, b->head_slot, b->head_e, b->head_pos, b->head_xq, b->head_d, b->draw_site, b->pair_cnt, b->pair_idx, b->pair_del, b->walk_shared, b->hcell_count, b->hcell_start, b->hcell_cursor, b->hsorted, b->hsorted_xg, b->hcell_of, b->flags,
+                  b->perm, b->scan_tmp, b->nl, b->nl_cnt, b->nl_shell, b->heads, b->head_sys, b->es_nl,
+                  b->es_cnt, b->head_slot, b->head_e, b->head_pos, b->head_xq, b->head_d, b->draw_site, b->pair_cnt, b->pair_idx, b->pair_del, b->walk_shared, b->hcell_count, b->hcell_start, b->hsorted, b->hsorted_xg, b->hcell_of, b->flags,
                   b->events, b->desorb, b->drift_bits, b->bond_items, b->bond_nitems, b->bond_sel, b->uf_parent, b->comp_head, b->comp_count,
                   b->item_next, b->has_item, b->sweep_out, b->prot_rng_dev, b->sp, b->shared, b->sysid, b->an_buf[0],
                   b->an_buf[1]};

@@ -93,7 +93,7 @@ struct Batch {
 
   // grid + list
   uint32_t ncells = 0;               // total list-build cells over the batch
-  uint32_t *cell_of_slot = nullptr, *cell_count = nullptr, *cell_start = nullptr, *cell_cursor = nullptr;
+  uint32_t *cell_of_slot = nullptr, *cell_count = nullptr, *cell_start = nullptr;
   uint32_t* perm = nullptr;          // new slot -> old slot
   uint32_t* scan_tmp = nullptr;
   uint32_t list_cap = 0;             // entries a row of nl may hold (max over replicas, rounded to 8)
@@ -125,7 +125,7 @@ struct Batch {
   uint32_t* es_nl = nullptr;
   uint32_t* es_cnt = nullptr;
   uint32_t nhcells = 0;
-  uint32_t *hcell_count = nullptr, *hcell_start = nullptr, *hcell_cursor = nullptr, *hsorted = nullptr;
+  uint32_t *hcell_count = nullptr, *hcell_start = nullptr, *hsorted = nullptr;
   float4* hsorted_xg = nullptr;      // the heads in head-cell order: position, head index as w bits
   uint32_t* hcell_of = nullptr;
 

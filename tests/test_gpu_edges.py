@@ -41,6 +41,25 @@ def test_lists_over_grids(box, n):
     g.dispose()
 
 
+@pytest.mark.parametrize("cells", [(16, 16, 16), (17, 16, 16), (163, 161, 161)])
+def test_lists_over_the_scans_of_their_cells(cells):
+    """4096 cells are scanned in one launch, up to 1024 blocks of them in two, more by a scan of the blocks' totals"""
+    def opts(box):
+        return cfgm.SoupOptions(box=box, seed=5, kT=1.1, start={"C": 0, "O": 0, "H": 0, "M": 1, "W": 799})
+    half = cfgm.resolve(opts([30.0] * 3), P).list_range / 2
+    cfg = cfgm.resolve(opts([(c + 0.3) * half for c in cells]), P)
+    box = np.array(cells) * half + 0.3 * half
+    rng = np.random.default_rng(5)
+    pos = ob.OracleSystem(_abi, cfg).read(ob.F_POS).reshape(-1, 4).copy()
+    at = rng.random((200, 3)) * box                      # clumps of four all over the box
+    at[:2] = [0.0, 0.0, 0.0], box - 0.5
+    pos[:, :3] = np.mod(np.repeat(at, 4, axis=0) + rng.normal(size=(800, 3)), box)
+    pos = pos.astype(np.float32).ravel()
+    o, g = ob.OracleSystem(_abi, cfg, {"positions": pos}), SoupSystem(cfg, {"positions": pos})
+    assert _lists_equal(o, g).max() >= 3
+    g.dispose()
+
+
 @pytest.mark.parametrize("n", [17, 33, 513, 700])
 def test_rows_of_any_length(n):
     """every bead in range of every other one: rows of n - 1 entries"""
