@@ -351,14 +351,78 @@ __device__ __forceinline__ void warp_walk(const float4& xi, uint32_t self, const
   }
 }
 
-// words behind a row: the candidates on the edge of the range that the exact distance may still leave out, and
-// the 64 that overflow it
-constexpr uint32_t kRowSpare = 64, kRowSlack = kRowSpare + 64;
+// words behind a row: one entry too many, and the 64 candidates behind that
+constexpr uint32_t kRowSlack = 80;
+
+// A row with more candidates than its shared words hold, or than the capacity (rare: it reports an overflow, or its
+// candidates on the edge of the range are what the exact distance leaves out).  The exact distance decides before an
+// entry counts, as the reference does, and no entry is kept in between: the row is walked twice, to count the
+// shells and to place the entries, in k_build_list's order.  Apart, so that k_build_list keeps its registers.
+__device__ __noinline__ void build_long_row(const Shared& S, const SysParams& P, const float4* __restrict__ pos, float q,
+                                            const uint32_t* __restrict__ start, uint32_t k, uint32_t cap,
+                                            uint32_t* __restrict__ sm, uint32_t* __restrict__ out,
+                                            uint32_t* __restrict__ nl_cnt, uint32_t* __restrict__ shell_end,
+                                            uint32_t* __restrict__ flags) {
+  const uint32_t lane = threadIdx.x & 31u, lt = (1u << lane) - 1u;
+  const float4 xi = pos[k];
+  const float box[3] = {P.box[0], P.box[1], P.box[2]};
+  const float inv[3] = {P.inv_box[0], P.inv_box[1], P.inv_box[2]};
+  const float lr = P.list_range, lr2_lo = lr * lr * (1.0f - 1e-5f), lr2_hi = lr * lr * (1.0f + 1e-5f);
+  const Shells sh = Shells::of(list_wide(S, P, (int)xi.w & (SOUP_KMAX - 1), q) ? S.rmax2 : S.rplain2, lr);
+  const WalkGrid G{{P.dims[0], P.dims[1], P.dims[2]}, P.walk, P.walk * P.fine, P.cell_off, lr, {P.cell[0], P.cell[1], P.cell[2]}, P.inv_cell[0]};
+  const uint32_t y0 = (lane & 1u) - 1u, y1 = ((lane >> 1) & 1u) - 1u, y2 = ((lane >> 2) & 1u) - 1u;
+  uint32_t next = 0, cnt = 0, found = 0;               // lane l: the entries, then the next place, of shell l mod 8
+#pragma unroll 1
+  for (int pass = 0; pass < 2; ++pass) {
+    const uint32_t whole = cnt & ~15u;
+    found = 0;
+    auto put = [&](uint32_t j) {
+      const float4 xj = pos[j];
+      const float dx = fast_mi(xi.x - xj.x, box[0], inv[0]);
+      const float dy = fast_mi(xi.y - xj.y, box[1], inv[1]);
+      const float dz = fast_mi(xi.z - xj.z, box[2], inv[2]);
+      const float r2 = dx * dx + dy * dy + dz * dz;
+      bool in = j != k && r2 <= lr2_hi;
+      if (in && r2 >= lr2_lo) in = ex_dist(xi, xj, box) < lr;
+      const uint32_t hits = __ballot_sync(0xffffffffu, in);
+      in = in && found + __popc(hits & lt) < cap;      // what is behind the capacity is dropped, and reported
+      found += __popc(hits);
+      const uint32_t t = in ? sh.tag(r2) >> 29 : 0u, m = __ballot_sync(0xffffffffu, in);
+      const uint32_t b0 = __ballot_sync(0xffffffffu, t & 1u), b1 = __ballot_sync(0xffffffffu, t & 2u),
+                     b2 = __ballot_sync(0xffffffffu, t & 4u);
+      if (pass == 1) {
+        const uint32_t x0 = (t & 1u) - 1u, x1 = ((t >> 1) & 1u) - 1u, x2 = ((t >> 2) & 1u) - 1u;
+        const uint32_t at = __shfl_sync(0xffffffffu, next, (int)t) + __popc(m & (b0 ^ x0) & (b1 ^ x1) & (b2 ^ x2) & lt);
+        if (in) out[at < whole ? (at & ~15u) + 4u * (at & 3u) + ((at >> 2) & 3u) : at] = j;
+      }
+      next += __popc(m & (b0 ^ y0) & (b1 ^ y1) & (b2 ^ y2));
+    };
+    warp_walk(xi, k, box, G, start, sm, [&](uint32_t j0, uint32_t j1) {
+      put(j0);
+      put(j1);
+    });
+    if (pass == 1) break;
+    cnt = min(found, cap);
+    uint32_t incl = next;                              // the shells' ends
+#pragma unroll
+    for (int o = 1; o < kShells; o <<= 1) {
+      const uint32_t y = __shfl_up_sync(0xffffffffu, incl, o);
+      if ((lane & 7u) >= (uint32_t)o) incl += y;
+    }
+    if (lane < (uint32_t)kShells) shell_end[lane] = lane + 1u < (uint32_t)kShells ? incl : cnt;
+    next = incl - next;
+  }
+  if (cnt + lane < ((cnt + 15u) & ~15u)) out[cnt + lane] = k;   // rows are padded with the particle itself
+  if (lane == 0) {
+    *nl_cnt = cnt;
+    if (found > cap) flags[0] = 1u;
+  }
+}
 
 // soup/wgsl/verlet.wgsl:53-92, a warp per particle (warp_walk).  The fast squared distance decides unless it
 // lies within 1e-5 of the range, where the reference's arithmetic decides (the minimum image cannot differ
 // there: range < box/2), so the list is the reference's set.  The accepted entries are compacted into the
-// warp's shared row with ballots, then the row is grouped by build-distance shell, keeping its order inside
+// warp's shared row with ballots (a row of more candidates than `most` is built by build_long_row), then the row is grouped by build-distance shell, keeping its order inside
 // a shell, straight into memory.  Every whole chunk of 16 entries is stored transposed (entry 4 e + l at
 // place 4 l + e), so that the force's four lanes of a particle, which read four places each, gather four
 // successive entries at a time: beads of one run, which share cache lines.
@@ -366,14 +430,15 @@ constexpr uint32_t kRowSpare = 64, kRowSlack = kRowSpare + 64;
 // Bound: instruction issue (78% of the slots, with the shared rows holding 32 warps an SM): at a range of 4.45 sigma
 // about 600 candidates a bead, 295 of them in range.  At 483k beads a thread per bead and a second pass that grouped
 // the rows took 1533 + 411 us, this 1185; at 24k 306 and 57, at 3.3k 393 and 18.
-__global__ void __launch_bounds__(128) k_build_list(
+__global__ void __launch_bounds__(128, 9) k_build_list(
     const Shared* __restrict__ Sg, const float4* __restrict__ pos, const float* __restrict__ charge,
     const uint8_t* __restrict__ sysid, const SysParams* __restrict__ sp, const uint32_t* __restrict__ start, uint32_t N,
-    uint32_t cap, uint32_t held, uint32_t stride, uint32_t* __restrict__ nl, uint32_t* __restrict__ nl_cnt,
+    uint32_t cap, uint32_t most, uint32_t stride, uint32_t* __restrict__ nl, uint32_t* __restrict__ nl_cnt,
     uint32_t* __restrict__ shell_end, uint32_t* __restrict__ flags) {
   extern __shared__ __align__(16) uint32_t sm[];
   const uint32_t wib = threadIdx.x >> 5, lane = threadIdx.x & 31u, lt = (1u << lane) - 1u;
-  uint32_t* row = sm + (size_t)wib * (held + kRowSlack + kWalkWords);   // held: the entries it takes, cap at most
+  const uint32_t held = (most + 15u) & ~15u;           // most: the candidates a shared row takes, cap at most
+  uint32_t* row = sm + (size_t)wib * (held + kRowSlack + kWalkWords);
   const uint32_t k = blockIdx.x * (blockDim.x >> 5) + wib;
   if (k >= N) return;   // whole warps
   const SysParams& P = sp[sysid[k]];
@@ -412,11 +477,17 @@ __global__ void __launch_bounds__(128) k_build_list(
       const float4 x0 = pos[j0], x1 = pos[j1];
       put(image, j0, x0);
       put(image, j1, x1);
-      cnt = min(cnt, cap + kRowSpare);                 // a row that is too long ends in the slack
+      cnt = min(cnt, most + 1u);                       // a row that is too long ends in the slack
     });
   };
   if (direct) walk(std::false_type{});
   else walk(std::true_type{});
+  uint32_t* out = nl + (size_t)k * stride;
+  if (cnt > most) {
+    build_long_row(*Sg, P, pos, charge[k], start, k, cap, row + held + kRowSlack, out, nl_cnt + k,
+                   shell_end + (size_t)kShells * k, flags);
+    return;
+  }
   if (__any_sync(0xffffffffu, edge)) {                 // the exact distance decides within 1e-5 of the range (rare)
     uint32_t kept = 0;
 #pragma unroll 1
@@ -430,15 +501,10 @@ __global__ void __launch_bounds__(128) k_build_list(
     }
     cnt = kept;
   }
-  if (cnt > cap) {
-    if (lane == 0) flags[0] = 1u;
-    cnt = cap;
-  }
   __syncwarp();
   // group the row by shell, keeping the walk's order inside a shell: 32 entries at a time, three ballots of the
   // shell's bits give every lane the entries of its own shell (its place among them) and lane s those of shell s
   // (the shells' running ends).  The loops stay rolled: unrolled, with the row in registers, the kernel outgrew the instruction cache
-  uint32_t* out = nl + (size_t)k * stride;
   // lane l stands for shell l mod 8: a ballot of bit i xor this is ones where bit i is the shell's
   const uint32_t y0 = (lane & 1u) - 1u, y1 = ((lane >> 1) & 1u) - 1u, y2 = ((lane >> 2) & 1u) - 1u;
   uint32_t end = 0;
@@ -605,11 +671,11 @@ void launch_build_lists(Batch& b) {
   prof_begin(b, SOUP_K_LIST);
   // a row of shared memory per warp: four warps per block while they fit.  A row has no more entries than
   // its replica has beads, whatever its capacity; one of more than kRowMost (beads of one clump) is reported as too long
-  uint32_t most = 0;
-  for (uint32_t r = 0; r < b.R; ++r) most = std::max(most, b.hsp[r].n);
+  uint32_t n = 0;
+  for (uint32_t r = 0; r < b.R; ++r) n = std::max(n, b.hsp[r].n);
   constexpr uint32_t kRowMost = 50u * 1024u;
-  const uint32_t cap = std::min(b.list_cap, std::min((most + 15u) & ~15u, kRowMost));
-  const uint32_t held = (cap + 15u) & ~15u;
+  const uint32_t cap = std::min(b.list_cap, kRowMost), most = std::min(cap, n);
+  const uint32_t held = (most + 15u) & ~15u;
   const size_t per = sizeof(uint32_t) * ((size_t)held + kRowSlack + kWalkWords);
   const uint32_t wpb = 4u * per <= 200u * 1024u ? 4u : 1u;
   const size_t smem = wpb * per;
@@ -618,7 +684,7 @@ void launch_build_lists(Batch& b) {
     b.list_smem_open = true;
   }
   k_build_list<<<(unsigned)((b.N + wpb - 1) / wpb), 32u * wpb, smem, b.stream>>>(
-      b.shared, b.pos, b.charge, b.sysid, b.sp, b.cell_start, b.N, cap, held, b.list_stride, b.nl, b.nl_cnt, b.nl_shell,
+      b.shared, b.pos, b.charge, b.sysid, b.sp, b.cell_start, b.N, cap, most, b.list_stride, b.nl, b.nl_cnt, b.nl_shell,
       b.flags);
   prof_end(b);
 }
