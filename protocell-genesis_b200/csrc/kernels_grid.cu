@@ -354,8 +354,8 @@ __device__ __forceinline__ void warp_walk(const float4& xi, uint32_t self, const
 // words behind a row: one entry too many, and the 64 candidates behind that
 constexpr uint32_t kRowSlack = 80;
 
-// A row with more candidates than its shared words hold, or than the capacity (rare: it reports an overflow, or its
-// candidates on the edge of the range are what the exact distance leaves out).  The exact distance decides before an
+// A row with more candidates than its shared words hold, or than the capacity (a clump, an overflow to report, or
+// candidates on the edge of the range that the exact distance leaves out).  The exact distance decides before an
 // entry counts, as the reference does, and no entry is kept in between: the row is walked twice, to count the
 // shells and to place the entries, in k_build_list's order.  Apart, so that k_build_list keeps its registers.
 __device__ __noinline__ void build_long_row(const Shared& S, const SysParams& P, const float4* __restrict__ pos, float q,
@@ -669,22 +669,28 @@ void launch_sort_and_gather(Batch& b) {
 void launch_build_lists(Batch& b) {
   b.launches += 1;
   prof_begin(b, SOUP_K_LIST);
-  // a row of shared memory per warp: four warps per block while they fit.  A row has no more entries than
-  // its replica has beads, whatever its capacity; one of more than kRowMost (beads of one clump) is reported as too long
+  // A shared row takes 1280 candidates, with which eight blocks fit an SM, or as many as twice the row a bead has in
+  // liquid (1.1 beads a sigma^3, or the replica's own density), up to 4096: two blocks an SM, behind which walking a row
+  // twice more costs less than a third block gives.  The capacity alone is no measure: sized by it, a
+  // capacity of 8192 took 1563 us at 121k beads and 6143 at 483k (382 and 1299 at 1126; lists and head lists)
+  double want = 1280.0;
   uint32_t n = 0;
-  for (uint32_t r = 0; r < b.R; ++r) n = std::max(n, b.hsp[r].n);
-  constexpr uint32_t kRowMost = 50u * 1024u;
-  const uint32_t cap = std::min(b.list_cap, kRowMost), most = std::min(cap, n);
-  const uint32_t held = (most + 15u) & ~15u;
-  const size_t per = sizeof(uint32_t) * ((size_t)held + kRowSlack + kWalkWords);
-  const uint32_t wpb = 4u * per <= 200u * 1024u ? 4u : 1u;
-  const size_t smem = wpb * per;
+  for (uint32_t r = 0; r < b.R; ++r) {
+    const SoupConfig& c = b.cfg[r];
+    n = std::max(n, c.n);
+    const double vol = c.wall_radius > 0 ? 4.18879 * c.wall_radius * c.wall_radius * c.wall_radius : c.box[0] * c.box[1] * c.box[2];
+    const double density = std::max(c.n / vol, 1.1 / (c.sigma * c.sigma * c.sigma));
+    want = std::max(want, 2.0 * density * 4.18879 * c.list_range * c.list_range * c.list_range);
+  }
+  const uint32_t most = std::min({b.list_cap, n, (uint32_t)std::min(want, 4096.0)}), held = (most + 15u) & ~15u;
+  constexpr uint32_t wpb = 4;
+  const size_t smem = wpb * sizeof(uint32_t) * ((size_t)held + kRowSlack + kWalkWords);
   if (smem > 48u * 1024u && !b.list_smem_open) {       // to all an SM has: the setting is the device's, not this batch's
     SOUP_CUDA_TRY(cudaFuncSetAttribute(k_build_list, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024));
     b.list_smem_open = true;
   }
-  k_build_list<<<(unsigned)((b.N + wpb - 1) / wpb), 32u * wpb, smem, b.stream>>>(
-      b.shared, b.pos, b.charge, b.sysid, b.sp, b.cell_start, b.N, cap, most, b.list_stride, b.nl, b.nl_cnt, b.nl_shell,
+  k_build_list<<<nblocks(b.N, wpb), 32 * wpb, smem, b.stream>>>(
+      b.shared, b.pos, b.charge, b.sysid, b.sp, b.cell_start, b.N, b.list_cap, most, b.list_stride, b.nl, b.nl_cnt, b.nl_shell,
       b.flags);
   prof_end(b);
 }

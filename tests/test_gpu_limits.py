@@ -3,8 +3,10 @@ import numpy as np
 import pytest
 
 import oracle_binding as ob
+from helpers import rel_rms
 from protocell_genesis_b200 import _abi, config as cfgm
 from protocell_genesis_b200.soup import SoupSystem
+from test_gpu_parity import FORCE_TOL
 
 pytestmark = pytest.mark.gpu
 P = cfgm.load_params()
@@ -45,3 +47,60 @@ def test_rows_beyond_the_capacity_are_reported():
     with pytest.raises(_abi.SoupError, match="listCapacity"):
         g.relax_cold_start(1, 1e-6)
     g.dispose()
+
+
+@pytest.mark.parametrize("n", [1279, 1280, 1281, 1282, 1297, 2000, 4999])
+def test_rows_longer_than_a_staged_row(n):
+    """a clump in which every bead is in range of every other: rows of n - 1 entries, of which 1280 are staged; a few
+    beads outside it keep ordinary rows"""
+    opts = cfgm.SoupOptions(box=[20] * 3, seed=1, kT=1.1, start={"C": 0, "O": 0, "H": 0, "M": 1, "W": n + 9},
+                            verlet_override={"listCapacity": 8192})
+    cfg = cfgm.resolve(opts, P)
+    pos = ob.OracleSystem(_abi, cfg).read(ob.F_POS).reshape(-1, 4).copy()
+    pos[:, :3] = np.random.default_rng(n).random((n + 10, 3)) * 1.6 + 19.0
+    pos[n:, :3] = 10.0 + 0.5 * np.arange(10)[:, None]
+    pos[:, :3] %= 20.0
+    pos = pos.astype(np.float32).ravel()
+    o, g = ob.OracleSystem(_abi, cfg, {"positions": pos}), SoupSystem(cfg, {"positions": pos})
+    oc, ol = o.verlet()
+    gc, gl = g.verlet_lists()
+    assert oc[:n].min() >= n - 1 and oc[n:].max() < 1280
+    assert np.array_equal(gc, oc)
+    assert np.array_equal(gl, ol)
+    g.dispose()
+
+
+def test_shells_of_rows_longer_than_a_staged_row(monkeypatch):
+    """a dense slab (rows of 1400 entries and more) whose inner beads move: the force read to the drift's shell is the
+    force over the whole rows, bit for bit, and the one over every pair"""
+    a, cells = 0.62, (25, 25, 15)
+    box = [25 * a, 25 * a, 40.0]
+    n = int(np.prod(cells))
+    opts = cfgm.SoupOptions(box=box, seed=1, kT=1.1, start={"C": 0, "O": 0, "H": 0, "M": 1, "W": n - 1},
+                            verlet_override={"listCapacity": 2048})
+    cfg = cfgm.resolve(opts, P)
+    cfg.dt = 1e-6                             # fast beads and short steps: the contacts' forces (1e5) hardly turn them
+    pos = ob.OracleSystem(_abi, cfg).read(ob.F_POS).reshape(-1, 4).copy()
+    at = np.stack(np.meshgrid(*[np.arange(c) for c in cells], indexing="ij"), -1).reshape(-1, 3)
+    pos[:, :3] = at * a + [0.1, 0.1, 12.0]
+    vel = np.zeros_like(pos)
+    vel[:, :3] = 2e4 * np.random.default_rng(2).normal(size=(n, 3))
+    inner = (at[:, 2] >= 5) & (at[:, 2] < 10)
+    state = {"positions": pos.astype(np.float32).ravel(), "velocities": vel.astype(np.float32).ravel(),
+             "frozen": (~inner).astype(np.uint32)}
+    runs = []
+    for full in ("0", "1"):
+        monkeypatch.setenv("SOUP_FULL_ROWS", full)
+        g = SoupSystem(cfg, state)
+        assert g.verlet_lists()[0].max() > 1400
+        seen = [g.forces_no_rebuild()]
+        for _ in range(4):
+            g.debug_phase(_abi.PHASE_KICK_DRIFT)
+            g.debug_phase(_abi.PHASE_FORCE)
+            seen.append(g.forces_no_rebuild())
+        assert 0.0 < g.info()["max_drift"] < 0.5 * cfg.skin
+        assert rel_rms(seen[-1], g.forces_brute_force()) < FORCE_TOL
+        runs.append(seen)
+        g.dispose()
+    for pruned, whole in zip(*runs):
+        assert np.array_equal(pruned, whole)
