@@ -920,6 +920,17 @@ __global__ void k_move_state(SavedState from, SavedState to, const uint32_t* __r
     slot_of_out[k] = k;
   }
 }
+// what a window holds fixed, into the slots as they are now: J.g reads the window's charges, bonds and tethers,
+// whatever the system did since
+__global__ void k_fixed_state(SavedState from, const uint32_t* __restrict__ id, uint32_t n, float* __restrict__ q,
+                              uint32_t* __restrict__ slots, uint32_t* __restrict__ center) {
+  const uint32_t k = blockIdx.x * blockDim.x + threadIdx.x;
+  if (k >= n) return;
+  const uint32_t i = id[k];
+  q[k] = from.q[i];
+  for (int e = 0; e < 3; ++e) slots[3 * (size_t)k + e] = from.slots[3 * (size_t)i + e];
+  center[k] = from.center[i];
+}
 constexpr size_t kSavedBytes = 66;
 constexpr uint32_t kDriftFrames = 16;
 constexpr int kDepthPairs[6][2] = {{0, 0}, {0, 1}, {0, 2}, {1, 1}, {1, 2}, {2, 2}};
@@ -1817,6 +1828,12 @@ int soup_diff_backward(SoupHandle* h, const float* dldx_device, double* theta_gr
       // the lists serve every frame within skin/2 of where they were built (the forward step's own test): the
       // drifts of the next kDriftFrames frames are taken at once, so the host waits once for all of them
       if (!w.drift) SOUP_CUDA_TRY(cudaMalloc(&w.drift, 4 * (size_t)kDriftFrames * b.R));
+      k_fixed_state<<<(N + 255) / 256, 256, 0, b.stream>>>(SavedState::of(w.save, N), b.id, N, b.charge, b.slots, b.center);
+      SOUP_CUDA_TRY(cudaGetLastError());
+      // a charge on another kind than the heads' is a part of how its row is grouped (list_wide): rows grouped under
+      // other charges do not serve
+      bool regroup = false;
+      for (uint32_t r = 0; r < b.R; ++r) regroup = regroup || b.off_head_charge[r] || w.off_head_charge[r];
       uint32_t known = 0, at = 0;          // frames the lists are known to serve; the next one's row of w.drift
       std::vector<uint32_t> bits(kDriftFrames * (size_t)b.R);
       for (uint32_t t = T + 1; t-- > 0;) {
@@ -1836,8 +1853,9 @@ int soup_diff_backward(SoupHandle* h, const float* dldx_device, double* theta_gr
             }
             return true;
           };
-          while (known < n && serves(known)) ++known;
+          while (!regroup && known < n && serves(known)) ++known;
           fresh = known == 0;
+          regroup = false;
         }
         adj_scatter_pos(b, w.all + (size_t)t * N);
         if (fresh) {

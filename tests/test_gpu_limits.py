@@ -1,9 +1,10 @@
-"""Calls at their limits: rows of the neighbour list at the capacity and beyond what a warp stages."""
+"""Calls at their limits and calls between others: rows of the neighbour list at the capacity and beyond what a warp
+stages, and a window's reverse pass behind other calls."""
 import numpy as np
 import pytest
 
 import oracle_binding as ob
-from helpers import rel_rms
+from helpers import oracle_bilayer_start, rel_rms
 from protocell_genesis_b200 import _abi, config as cfgm
 from protocell_genesis_b200.soup import SoupSystem
 from test_gpu_parity import FORCE_TOL
@@ -104,3 +105,47 @@ def test_shells_of_rows_longer_than_a_staged_row(monkeypatch):
         g.dispose()
     for pruned, whole in zip(*runs):
         assert np.array_equal(pruned, whole)
+
+
+@pytest.mark.parametrize("budget", [None, "0"])
+@pytest.mark.parametrize("between", ["steps", "charges", "off-head charges", "bonds"])
+def test_a_window_differentiates_its_own_charges_and_bonds(budget, between, monkeypatch):
+    """the reverse pass behind other calls gives the gradient of the window, with every frame kept and with replays.
+    Rows in another order round differently: 1e-6 a step, and 12 steps let it grow less than tenfold."""
+    import torch
+    if budget is not None:
+        monkeypatch.setenv("SOUP_DIFF_FRAME_BUDGET_MB", budget)
+    cfg, start = oracle_bilayer_start(steps=20)
+    n = cfg.n
+    assert (start["bond_slots"] != _abi.NONE).sum() > 100 and (start["charges"] != 0).sum() > 100
+    g = SoupSystem(cfg, start)
+    dldx = torch.randn((13, n, 4), generator=torch.Generator().manual_seed(1)).cuda()
+    dldx[..., 3] = 0
+    torch.cuda.synchronize()
+    grads = []
+    for other_calls in (False, True):
+        g.write_state(start)
+        g.diff_forward(12, 4)
+        if other_calls:
+            if between == "steps":
+                g.step(40)
+                g.protonation_sweep()
+            elif between == "charges":
+                g.write_charges(np.where(start["charges"] != 0, 0.0, np.where(start["positions"][3::4] == cfg.charged_kind, -1.0, 0.0)).astype(np.float32))
+            elif between == "off-head charges":
+                g.write_charges(np.full(n, 0.25, np.float32))
+            else:
+                g.write_state({"bond_slots": np.full(3 * n, _abi.NONE, np.uint32)})
+        dx0, dv0 = torch.zeros((n, 4), device="cuda"), torch.zeros((n, 4), device="cuda")
+        torch.cuda.synchronize()
+        theta = g.diff_backward(dldx.data_ptr(), dx0.data_ptr(), dv0.data_ptr())
+        torch.cuda.synchronize()
+        grads.append((theta, dx0.cpu().numpy(), dv0.cpu().numpy()))
+        assert np.array_equal(g.charges(), start["charges"]) and np.array_equal(g.bond_slots(), start["bond_slots"])
+    for a, b in zip(*grads):
+        assert np.abs(a).max() > 0
+        if a.ndim == 1:
+            assert np.all(np.abs(a - b) <= 1e-4 * np.abs(a).max()), (a, b)
+        else:
+            assert rel_rms(b, a) < 1e-4
+    g.dispose()
