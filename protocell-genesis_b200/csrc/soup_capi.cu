@@ -1580,14 +1580,16 @@ int soup_protonation_sweep(SoupHandle* h, SoupSweepResult* out) {
   return guarded(h, [&](Batch& b, uint32_t r) {
     if (!b.cfg[r].es_enabled) fail(SOUP_E_STATE, "electrostatics is not enabled on this system");
     // F(x) is stale after the charges changed.  Lists do not depend on charges: with drift-triggered rebuilds they
-    // are kept while they serve (at 483k beads a rebuild is 1.5 ms, the force pass 0.23), as inside a step
-    const bool rebuild_lists = !b.cfg[0].rebuild_on_drift || drift_exceeds(b);
+    // are kept while they serve (at 483k beads a rebuild is 1.5 ms, the force pass 0.23), as inside a step, and
+    // built before the sweep reads them when they do not
+    const bool on_drift = b.cfg[0].rebuild_on_drift;
+    if (on_drift && drift_exceeds(b)) rebuild(b);
     launch_sweep(b, r);
     std::vector<double> so(4);
     SOUP_CUDA_TRY(cudaMemcpyAsync(so.data(), b.sweep_out + 4 * r, 32, cudaMemcpyDeviceToHost, b.stream));
     SOUP_CUDA_TRY(cudaMemcpyAsync(&b.prot_rng[r], b.prot_rng_dev + r, 4, cudaMemcpyDeviceToHost, b.stream));
-    if (rebuild_lists) force_pass(b);
-    else launch_force(b);
+    if (on_drift) launch_force(b);
+    else force_pass(b);
     SOUP_CUDA_TRY(cudaStreamSynchronize(b.stream));
     if (so[0] < 0)
       fail(SOUP_E_TIMEOUT, "constant-pH sweep: a handoff between the walk's CTAs did not arrive within its "

@@ -1,13 +1,13 @@
 """Calls at their limits and calls between others: rows of the neighbour list at the capacity and beyond what a warp
-stages, and a window's reverse pass behind other calls."""
+stages, a window's reverse pass behind other calls, and a sweep on lists that no longer serve."""
 import numpy as np
 import pytest
 
 import oracle_binding as ob
-from helpers import oracle_bilayer_start, rel_rms
+from helpers import charged_opts, oracle_bilayer_start, rel_rms
 from protocell_genesis_b200 import _abi, config as cfgm
 from protocell_genesis_b200.soup import SoupSystem
-from test_gpu_parity import FORCE_TOL
+from test_gpu_parity import FORCE_TOL, make_pair
 
 pytestmark = pytest.mark.gpu
 P = cfgm.load_params()
@@ -148,4 +148,23 @@ def test_a_window_differentiates_its_own_charges_and_bonds(budget, between, monk
             assert np.all(np.abs(a - b) <= 1e-4 * np.abs(a).max()), (a, b)
         else:
             assert rel_rms(b, a) < 1e-4
+    g.dispose()
+
+
+def test_a_sweep_reads_lists_that_serve():
+    """beads that moved beyond half the skin: the sweep's decisions are the oracle's on the positions of the moment"""
+    def fixed(c):
+        c.protonation_rng = 77
+    cfg, o, g = make_pair(charged_opts(start={"C": 300, "O": 500, "H": 300, "M": 20, "W": 0}, rebuild_on_drift=True, skin=0.6,
+                                       electrostatics={"enabled": True, "pH": 4.0}), relax=20, tweak=fixed)
+    while g.info()["max_drift"] < 6.0:        # kicks and drifts alone: no step looks at the drift
+        g.debug_phase(_abi.PHASE_KICK_DRIFT)
+    now = ob.OracleSystem(_abi, cfg, dict(positions=g.particles(), charges=g.charges(), bond_slots=g.bond_slots(),
+                                          center_link=g.center_links()))
+    rg, ro = g.protonation_sweep(), now.sweep()
+    assert np.array_equal(g.charges(), now.read(ob.F_CHARGES))
+    assert g.protonation_rng_state() == int(now.read(ob.F_PROT_RNG)[0])
+    assert rg["accepted"] == ro.accepted
+    assert rg["dEsMeanKT"] == pytest.approx(ro.d_es_mean_kt, rel=1e-9, abs=1e-12)
+    assert rel_rms(g.forces_no_rebuild(), now.forces64()) < FORCE_TOL
     g.dispose()
