@@ -51,17 +51,27 @@ __device__ __forceinline__ double acid_well(const SysParams& P, double r) {
   const double c = cos((3.141592653589793 * (r - P.d_rcattr)) / (2.0 * P.d_wc));
   return -P.d_acid * P.d_eps * c * c;
 }
-// squared minimum-image distance, FP64.  The reference's image index is Math.round(d / L); here FP32 picks
-// it: it can differ only near a half-box offset, where every pair is beyond the (at most L / 2) cutoffs
-// either way.
-__device__ __forceinline__ double image(float a, float b, float inv, double L) {
+// squared minimum-image distance, FP64.  The reference's image index is Math.round(d / L).  While the cutoffs end short
+// of half the box, FP32 finds it: it can differ only near a half-box offset, where every pair is beyond them either
+// way.  A live box that has shrunk further (SysParams.image64; I64: some replica's has) takes the index from
+// d * (1 / L) in FP64, within an ulp of d / L.  With FP64 for all, a sweep at 18,659 heads takes 4% longer; with the
+// question asked in every kernel, 1%.
+template <bool I64>
+__device__ __forceinline__ double image(float a, float b, bool in64, float inv, double inv64, double L) {
   const double d = (double)a - (double)b;
-  const float n = rintf((a - b) * inv);
-  return n == 0.f ? d : d - (double)n * L;
+  if (!I64 || !in64) {
+    const float n = rintf((a - b) * inv);
+    return n == 0.f ? d : d - (double)n * L;
+  }
+  const double x = d * inv64, r = floor(x);
+  return d - (x - r >= 0.5 ? r + 1.0 : r) * L;
 }
+template <bool I64>
 __device__ __forceinline__ double dist2(const SysParams& P, const float4& a, const float4& b) {
-  const double dx = image(a.x, b.x, P.inv_box[0], P.d_box[0]), dy = image(a.y, b.y, P.inv_box[1], P.d_box[1]),
-               dz = image(a.z, b.z, P.inv_box[2], P.d_box[2]);
+  const bool in64 = I64 && P.image64 != 0;
+  const double dx = image<I64>(a.x, b.x, in64, P.inv_box[0], P.d_inv_box[0], P.d_box[0]),
+               dy = image<I64>(a.y, b.y, in64, P.inv_box[1], P.d_inv_box[1], P.d_box[1]),
+               dz = image<I64>(a.z, b.z, in64, P.inv_box[2], P.d_inv_box[2], P.d_box[2]);
   return dx * dx + dy * dy + dz * dz;
 }
 // the energy a neighbour of charge qj at squared distance r2 contributes to a site's E
@@ -119,6 +129,7 @@ __device__ __forceinline__ float fast_r2(const SysParams& P, const float4& a, co
 // screened energy per unit charge product and the well are evaluated once per pair, for E and for D (the
 // same operations in the same order as es_energy / std_delta, so the same bits).  Entries beyond both
 // cutoffs (the list's skin) are told by an FP32 distance with a wide margin.  Bound: FP64 issue.
+template <bool I64>
 __global__ void __launch_bounds__(256) k_sweep_init(const SysParams* __restrict__ sp, const uint32_t* __restrict__ head_sys,
                                                     uint32_t H, const float4* __restrict__ xq,
                                                     const uint32_t* __restrict__ es_nl, const uint32_t* __restrict__ es_cnt,
@@ -145,7 +156,7 @@ __global__ void __launch_bounds__(256) k_sweep_init(const SysParams* __restrict_
     long long d = 0;
     if (fast_r2(P, xi, xj) < screen2) {
       const float qj = xj.w;
-      const double r2 = dist2(P, xi, xj);
+      const double r2 = dist2<I64>(P, xi, xj);
       const bool es_in = r2 < cut2, ac_in = P.d_acid > 0.0 && r2 < reach2 && r2 > 0.0;
       double t1 = 0.0, t0 = 0.0;
       if (es_in || ac_in) {
@@ -271,6 +282,7 @@ constexpr uint32_t kPairDraws = 16;
 __device__ __forceinline__ size_t pidx_at(uint32_t e, uint32_t i, uint32_t W) { return ((size_t)(e >> 3) * W + i) * 8 + (e & 7u); }
 __device__ __forceinline__ uint32_t pair_count(uint32_t w) { return w & 1023u; }
 __device__ __forceinline__ int pair_same(uint32_t w) { return (int)(w >> 10) - 1; }
+template <bool I64>
 __global__ void __launch_bounds__(256) k_sweep_pairs(const SysParams* __restrict__ sp, const float4* __restrict__ xq,
                                                      const uint32_t* __restrict__ draw_site, uint32_t only,
                                                      uint32_t* __restrict__ pcnt, uint16_t* __restrict__ pidx,
@@ -315,7 +327,7 @@ __global__ void __launch_bounds__(256) k_sweep_pairs(const SysParams* __restrict
     for (uint32_t e = lane; e < n; e += 32u) {
       const uint32_t j = near[e];
       pidx[block0 * kDraws + pidx_at(e, i, W)] = (uint16_t)j;
-      pdel[block0 * kDraws + (size_t)e * W + i] = std_delta(P, dist2(P, rec[j], xi), (float)P.d_q, cut2, reach2);
+      pdel[block0 * kDraws + (size_t)e * W + i] = std_delta(P, dist2<I64>(P, rec[j], xi), (float)P.d_q, cut2, reach2);
     }
     // the last word's places beyond n name place W, which never flips
     for (uint32_t e = n + lane; e < ((n + 7u) & ~7u); e += 32u) pidx[block0 * kDraws + pidx_at(e, i, W)] = (uint16_t)W;
@@ -365,6 +377,7 @@ struct alignas(16) WalkShared {
 // Add n flips to the energies of their neighbours (global int64, reductions in L2): warp `w` of `nw` takes
 // whole flips, or parts of flips when there are more warps than flips.  Every load of a pass is in flight
 // before the first add.  (One SM adds about a lane per cycle, so the share of an SM sets the time.)
+template <bool I64>
 __device__ __forceinline__ void scatter_flips(const uint2* rec, uint32_t n, const SysParams& P, uint32_t cap,
                                               const uint32_t* __restrict__ es_nl, const long long* __restrict__ D,
                                               const float4* __restrict__ xq, long long* __restrict__ E, uint32_t w,
@@ -394,7 +407,7 @@ __device__ __forceinline__ void scatter_flips(const uint2* rec, uint32_t n, cons
         long long d = f == 0 ? dv[u] : -dv[u];
         if (f == 2) {   // a charge other than the standard one goes to 0
           const double cut2 = P.d_rc * P.d_rc, reach = P.d_rcattr + P.d_wc;
-          d = flip_delta(P, dist2(P, xq[h], xq[tv[u]]), xq[h].w, 0.f, cut2, reach * reach);
+          d = flip_delta(P, dist2<I64>(P, xq[h], xq[tv[u]]), xq[h].w, 0.f, cut2, reach * reach);
         }
         if (d != 0) atomicAdd(reinterpret_cast<unsigned long long*>(E + (tv[u] - off)), (unsigned long long)d);
       }
@@ -433,7 +446,7 @@ __device__ __forceinline__ void prefetch_rows(const SysParams& P, uint32_t cap, 
 // behind it, so no add can reach E before them), and a counter of the CTAs that are done, each release
 // ordering that CTA's reductions before it.  Every poll is bounded; one that gives up ends the walk and the
 // host reports it.
-template <uint32_t W>
+template <uint32_t W, bool I64>
 __global__ void __launch_bounds__(kWalkThreads) k_sweep_walk(
     const SysParams* __restrict__ sp, const uint32_t* __restrict__ head_slot, const float4* __restrict__ xq,
     float* __restrict__ charge, const uint32_t* __restrict__ es_nl, const uint32_t* __restrict__ es_cnt,
@@ -478,7 +491,7 @@ __global__ void __launch_bounds__(kWalkThreads) k_sweep_walk(
       const uint32_t n = s_hv & 1023u;
       if (tid < n) s_rec[tid] = __ldcg(&G.rec[tid]);
       __syncthreads();
-      scatter_flips(s_rec, n, P, cap, es_nl, D, xq, E, t >> 5, nt >> 5);
+      scatter_flips<I64>(s_rec, n, P, cap, es_nl, D, xq, E, t >> 5, nt >> 5);
       __syncthreads();
       if (tid == 0) red_add_release_gpu(&G.done, 1u);
       if (blk + 1u < blocks) prefetch_rows(P, cap, draw_site + d0 + (size_t)(blk + 1u) * W, es_nl, es_cnt, D, W, t, nt);
@@ -600,7 +613,7 @@ __global__ void __launch_bounds__(kWalkThreads) k_sweep_walk(
           const uint32_t j = px[pidx_at(q, place, W)];
           if (s_code[j] != 2) continue;
           const uint32_t sj = off + draw_site[b0 + j];
-          e += flip_delta(P, dist2(P, xq[sj], xq[off + site]), xq[sj].w, 0.f, cut2, reach2) - pd[(size_t)q * W + place];
+          e += flip_delta(P, dist2<I64>(P, xq[sj], xq[off + site]), xq[sj].w, 0.f, cut2, reach2) - pd[(size_t)q * W + place];
         }
       }
       // the charge state behind the last earlier flip of this site
@@ -638,7 +651,7 @@ __global__ void __launch_bounds__(kWalkThreads) k_sweep_walk(
     len = es_cnt[off + site];
     st = jb.a * st + jb.c;
     if (group == 1u) {
-      scatter_flips(s_rec, nf, P, cap, es_nl, D, xq, E, wid, kWalkWarps);
+      scatter_flips<I64>(s_rec, nf, P, cap, es_nl, D, xq, E, wid, kWalkWarps);
     } else if (tid == 0) {
       const uint32_t want = (group - 1u) * (blk + 1u);
       uint32_t spins = 0;
@@ -712,7 +725,7 @@ double sweep_list_entries(const Batch& b, uint32_t replica) {
   return most;
 }
 
-template <uint32_t W>
+template <uint32_t W, bool I64>
 void launch_walk(Batch& b, uint32_t replica, unsigned ry, unsigned group, size_t smem) {
   cudaLaunchConfig_t lc = {};
   lc.gridDim = dim3(ry * group);
@@ -724,7 +737,7 @@ void launch_walk(Batch& b, uint32_t replica, unsigned ry, unsigned group, size_t
   attr[0].val.cooperative = 1;
   lc.attrs = attr;
   lc.numAttrs = group > 1u ? 1 : 0;
-  SOUP_CUDA_TRY(cudaLaunchKernelEx(&lc, k_sweep_walk<W>, (const SysParams*)b.sp, (const uint32_t*)b.head_slot,
+  SOUP_CUDA_TRY(cudaLaunchKernelEx(&lc, k_sweep_walk<W, I64>, (const SysParams*)b.sp, (const uint32_t*)b.head_slot,
                                    (const float4*)b.head_pos, b.charge, (const uint32_t*)b.es_nl,
                                    (const uint32_t*)b.es_cnt, (const long long*)b.head_d, b.es_cap, b.head_e,
                                    (const uint32_t*)b.draw_site, (const uint32_t*)b.pair_cnt,
@@ -737,8 +750,10 @@ void launch_walk(Batch& b, uint32_t replica, unsigned ry, unsigned group, size_t
 void launch_sweep(Batch& b, uint32_t replica) {
   if (b.H == 0) return;
   uint32_t hmax = 0, wmax = 0;
+  bool far = false;
   for (uint32_t r = 0; r < b.R; ++r)
     if (replica == SOUP_NONE_U32 || r == replica) {
+      far = far || b.hsp[r].image64 != 0;
       hmax = std::max(hmax, b.hsp[r].nheads);
       wmax = std::max(wmax, b.hsp[r].sweep_draws);
     }
@@ -748,10 +763,10 @@ void launch_sweep(Batch& b, uint32_t replica) {
   const unsigned ry = replica == SOUP_NONE_U32 ? b.R : 1;
   const uint32_t draws = (2 * hmax + kDraws - 1) / kDraws * kDraws;   // at least every replica's whole blocks
   k_gather_heads<<<(b.H + 255) / 256, 256, 0, b.stream>>>(b.head_slot, b.H, b.pos, b.charge, b.head_pos);
-  k_sweep_init<<<(unsigned)(((uint64_t)b.H * 32 + 255) / 256), 256, 0, b.stream>>>(
+  (far ? k_sweep_init<true> : k_sweep_init<false>)<<<(unsigned)(((uint64_t)b.H * 32 + 255) / 256), 256, 0, b.stream>>>(
       b.sp, b.head_sys, b.H, b.head_pos, b.es_nl, b.es_cnt, b.es_cap, b.head_e, b.head_d, replica);
   k_sweep_draws<<<dim3((draws + 255) / 256, ry), 256, 0, b.stream>>>(b.sp, b.prot_rng_dev, replica, b.draw_site);
-  k_sweep_pairs<<<dim3(draws / kPairDraws, ry), 256, 0, b.stream>>>(
+  (far ? k_sweep_pairs<true> : k_sweep_pairs<false>)<<<dim3(draws / kPairDraws, ry), 256, 0, b.stream>>>(
       b.sp, b.head_pos, b.draw_site, replica, b.pair_cnt, b.pair_idx, b.pair_del);
   // a group of CTAs per replica, all SMs together (a cooperative launch).  The handoffs cost about 4k cycles a
   // block, in which one SM adds about 4k list entries: a replica whose blocks flip fewer than that walks alone
@@ -767,8 +782,9 @@ void launch_sweep(Batch& b, uint32_t replica) {
       any = any || ((replica == SOUP_NONE_U32 || r == replica) && b.hsp[r].nheads && b.hsp[r].sweep_draws == w);
     if (!any) continue;
     b.launches += 1;
-    if (w == 512u) launch_walk<512>(b, replica, ry, group, smem);
-    else launch_walk<256>(b, replica, ry, group, smem);
+    const auto walk = w == 512u ? (far ? launch_walk<512, true> : launch_walk<512, false>)
+                                : (far ? launch_walk<256, true> : launch_walk<256, false>);
+    walk(b, replica, ry, group, smem);
   }
   prof_end(b);
 }
@@ -781,8 +797,9 @@ size_t sweep_shared_bytes(const Batch& b) { return sizeof(WalkShared) * b.R; }
 
 void sweep_prepare(Batch& b) {
   const int most = (int)((kMaxHeads + 15) & ~15u);
-  SOUP_CUDA_TRY(cudaFuncSetAttribute(k_sweep_walk<512>, cudaFuncAttributeMaxDynamicSharedMemorySize, most));
-  SOUP_CUDA_TRY(cudaFuncSetAttribute(k_sweep_walk<256>, cudaFuncAttributeMaxDynamicSharedMemorySize, most));
+  for (const void* walk : {(const void*)k_sweep_walk<512, false>, (const void*)k_sweep_walk<512, true>,
+                           (const void*)k_sweep_walk<256, false>, (const void*)k_sweep_walk<256, true>})
+    SOUP_CUDA_TRY(cudaFuncSetAttribute(walk, cudaFuncAttributeMaxDynamicSharedMemorySize, most));
   SOUP_CUDA_TRY(cudaDeviceGetAttribute(&b.sms, cudaDevAttrMultiProcessorCount, b.device));
 }
 

@@ -153,6 +153,8 @@ SysParams make_sys(const SoupConfig& c) {
   p.d_A = es ? c.es_coeff_a : 0.0; p.d_kappa = c.es_kappa; p.d_rc = c.es_cutoff; p.d_shiftU = c.es_shift_u;
   p.d_shiftF = c.es_shift_f; p.d_pka = c.pka_intrinsic; p.d_ph = c.ph; p.d_kT = c.kT; p.d_q = c.charge_deprotonated;
   p.d_acid = c.acid_soap_scale; p.d_rcattr = c.rc_attr; p.d_wc = c.wc; p.d_eps = c.epsilon;
+  // 0.49: FP32 rounds an offset to 3e-7 of the box
+  p.image64 = std::max(c.es_cutoff, c.rc_attr + c.wc) > 0.49 * std::min({c.box[0], c.box[1], c.box[2]}) ? 1u : 0u;
   return p;
 }
 

@@ -47,6 +47,7 @@ struct SysParams {
   uint32_t list_cap, es_cap; // capacities (overflow threshold)
   uint32_t sweep_draws;      // draws of a block of the constant-pH walk: 512 or 256
   uint32_t es_on;            // electrostatics enabled
+  uint32_t image64;          // the sweep's cutoffs reach so near half the box that FP64 picks the image
   int32_t charged_kind;
   // FP64 host-style numbers for the constant-pH sweep
   double d_box[3], d_inv_box[3];

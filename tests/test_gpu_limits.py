@@ -1,5 +1,6 @@
 """Calls at their limits and calls between others: rows of the neighbour list at the capacity and beyond what a warp
-stages, a window's reverse pass behind other calls, and a sweep on lists that no longer serve."""
+stages, a window's reverse pass behind other calls, a sweep on lists that no longer
+serve, and one in a box below twice its cutoff."""
 import numpy as np
 import pytest
 
@@ -167,4 +168,36 @@ def test_a_sweep_reads_lists_that_serve():
     assert rg["accepted"] == ro.accepted
     assert rg["dEsMeanKT"] == pytest.approx(ro.d_es_mean_kt, rel=1e-9, abs=1e-12)
     assert rel_rms(g.forces_no_rebuild(), now.forces64()) < FORCE_TOL
+    g.dispose()
+
+
+def test_site_energies_at_half_a_box():
+    """a box below twice the cutoff, as a live box can shrink to, with heads half a box and up to 4e-7 apart: FP32
+    rounds the offset to a half and takes the image on the other side.  The mean energy is FP64's to its fixed point."""
+    opts = cfgm.SoupOptions(box=[20] * 3, seed=1, kT=1.1, start={"C": 0, "O": 100, "H": 0, "M": 1, "W": 0},
+                            electrostatics={"enabled": True, "pH": 5.0, "ionicStrengthMolar": 0.01})
+    cfg = cfgm.resolve(opts, P)
+    cfg.box[0] = cfg.box[1] = cfg.box[2] = 16.0
+    cfg.protonation_rng = 5
+    cfg.es_list_capacity = 128
+    assert cfg.es_cutoff > 8.5
+    rng = np.random.default_rng(1)
+    pos = ob.OracleSystem(_abi, cfg).read(ob.F_POS).reshape(-1, 4).copy()
+    heads = np.nonzero(pos[:, 3] == cfg.charged_kind)[0]
+    pos[:, :3] = rng.random((cfg.n, 3)) * [0.0, 3.0, 3.0]
+    pos[heads[:50], 0] = np.float32(8.3)
+    near = np.float32(8.3) - np.float32(8.0)
+    pos[heads[50:], 0] = near - np.float32(2.0 ** -25) * rng.integers(1, 13, 50)
+    pos = pos.astype(np.float32)
+    apart = pos[heads[:1], 0].astype(np.float64) - pos[heads[50:], 0].astype(np.float64)
+    assert np.all(apart > 8.0) and np.all((pos[heads[0], 0] - pos[heads[50:], 0]) == np.float32(8.0))
+    q = np.zeros(cfg.n, np.float32)
+    q[heads[::2]] = -1.0
+    state = {"positions": pos.ravel(), "charges": q}
+    o, g = ob.OracleSystem(_abi, cfg, state), SoupSystem(cfg, state)
+    for k in range(3):
+        rg, ro = g.protonation_sweep(), o.sweep()
+        assert np.array_equal(g.charges(), o.read(ob.F_CHARGES)), k
+        assert rg["accepted"] == ro.accepted > 0, k
+        assert rg["dEsMeanKT"] == pytest.approx(ro.d_es_mean_kt, rel=1e-10, abs=1e-11), k
     g.dispose()
