@@ -263,26 +263,30 @@ __global__ void k_agg_bin(const float4* __restrict__ pos, const uint32_t* __rest
   cell[k] = c;
   atomicAdd(&count[c], 1u);
 }
+constexpr uint32_t kFar = 1u << 31;   // with a member's index: its coordinates are far outside the box, or not numbers
 __global__ void k_agg_scatter(const float4* __restrict__ pos, const uint32_t* __restrict__ slot_of, uint32_t off,
                               const uint32_t* __restrict__ mem, const uint32_t* __restrict__ cell, uint32_t m,
-                              const uint32_t* __restrict__ start, uint32_t* __restrict__ cursor,
+                              const uint32_t* __restrict__ start, uint32_t* __restrict__ cursor, Grid g,
                               float4* __restrict__ sorted) {
   const uint32_t k = blockIdx.x * blockDim.x + threadIdx.x;
   if (k >= m) return;
   const uint32_t c = cell[k];
   const float4 p = pos[slot_of[off + mem[k]]];
-  sorted[start[c] + atomicAdd(&cursor[c], 1u)] = make_float4(p.x, p.y, p.z, __uint_as_float(k));   // w: the member
+  const bool in = fabs(p.x - 0.5 * g.box[0]) <= g.box[0] && fabs(p.y - 0.5 * g.box[1]) <= g.box[1] &&
+                  fabs(p.z - 0.5 * g.box[2]) <= g.box[2];
+  sorted[start[c] + atomicAdd(&cursor[c], 1u)] = make_float4(p.x, p.y, p.z, __uint_as_float(in ? k : k | kFar));   // w: the member
 }
 // A warp per member, over the members in cell order: a run of candidates per (y, z) row and wrapped x piece, a
 // lane each.  The reference's FP64 test decides only where the FP32 distance lies within a margin of the
-// cutoff ten times its error (roundings of coordinates and box: a few 1e-7 of the box).  (A thread per member, with three dependent loads and three FP64
-// divisions a candidate: 826 us at 16,500 members.)
+// cutoff: its error is a few roundings of the separation as stored, which is at most two boxes (4e-7 of the box, and
+// the margin more than twice that), or the member is marked (kFar) and FP64 decides.  (A thread per member, with three dependent loads and three FP64 divisions a candidate: 826 us at 16,500
+// members.)
 __global__ void k_agg_union(const float4* __restrict__ sorted, uint32_t m, Grid g, double wx, double wy, double wz,
                             const uint32_t* __restrict__ start, double c2, int periodic_z, uint32_t* __restrict__ parent) {
   const uint32_t w = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31u;
   if (w >= m) return;   // whole warps
   const float4 pi = sorted[w];
-  const uint32_t k = __float_as_uint(pi.w);
+  const uint32_t wk = __float_as_uint(pi.w), k = wk & (kFar - 1u);
   const float lx = (float)g.box[0], ly = (float)g.box[1], lz = (float)g.box[2];
   const float c = sqrtf((float)c2), margin = 1e-4f * c + 1e-6f * fmaxf(lx, fmaxf(ly, lz));
   const float lo = c > margin ? (c - margin) * (c - margin) : 0.f, hi = (c + margin) * (c + margin);
@@ -296,15 +300,16 @@ __global__ void k_agg_union(const float4* __restrict__ sorted, uint32_t m, Grid 
   auto scan = [&](uint32_t a, uint32_t e) {
     for (uint32_t t = a + lane; t < e; t += 32u) {
       const float4 pj = sorted[t];
-      const uint32_t l = __float_as_uint(pj.w);
+      const uint32_t wl = __float_as_uint(pj.w), l = wl & (kFar - 1u);
       if (l <= k) continue;
       float dx = pi.x - pj.x, dy = pi.y - pj.y, dz = pi.z - pj.z;
       dx -= rintf(dx / lx) * lx;
       dy -= rintf(dy / ly) * ly;
       if (periodic_z) dz -= rintf(dz / lz) * lz;
       const float r2 = dx * dx + dy * dy + dz * dz;
-      if (r2 > hi) continue;
-      if (r2 >= lo) {
+      const bool far = (wl | wk) >= kFar;
+      if (!far && r2 > hi) continue;
+      if (far || r2 >= lo) {
         const double ddx = mi1(__dsub_rn((double)pi.x, (double)pj.x), g.box[0]);
         const double ddy = mi1(__dsub_rn((double)pi.y, (double)pj.y), g.box[1]);
         const double rz = __dsub_rn((double)pi.z, (double)pj.z);
@@ -502,7 +507,7 @@ int run_aggregates(Batch& b, uint32_t r, const uint32_t* mem, uint32_t m, double
   k_agg_bin<<<nblocks(m), kBlock, 0, st>>>(b.pos, b.slot_of, off, dmem, m, g, c.box[0] / g.nx, c.box[1] / g.ny,
                                            c.box[2] / g.nz, cell, count);
   exclusive_scan(count, start, nc, tmp, st);
-  k_agg_scatter<<<nblocks(m), kBlock, 0, st>>>(b.pos, b.slot_of, off, dmem, cell, m, start, cursor, sorted);
+  k_agg_scatter<<<nblocks(m), kBlock, 0, st>>>(b.pos, b.slot_of, off, dmem, cell, m, start, cursor, g, sorted);
   k_iota<<<nblocks(m), kBlock, 0, st>>>(parent, m);
   k_fill<<<nblocks(m), kBlock, 0, st>>>(minidx, m, NONE);
   k_agg_union<<<nblocks((uint64_t)m * 32), kBlock, 0, st>>>(sorted, m, g, c.box[0] / g.nx, c.box[1] / g.ny, c.box[2] / g.nz,

@@ -1,6 +1,7 @@
 """Calls at their limits and calls between others: rows of the neighbour list at the capacity and beyond what a warp
 stages, a window's reverse pass behind other calls, a sweep on lists that no longer
-serve, and one in a box below twice its cutoff."""
+serve, one in a box below twice its cutoff, and
+aggregates of coordinates far outside the box."""
 import numpy as np
 import pytest
 
@@ -200,4 +201,25 @@ def test_site_energies_at_half_a_box():
         assert np.array_equal(g.charges(), o.read(ob.F_CHARGES)), k
         assert rg["accepted"] == ro.accepted > 0, k
         assert rg["dEsMeanKT"] == pytest.approx(ro.d_es_mean_kt, rel=1e-10, abs=1e-11), k
+    g.dispose()
+
+
+@pytest.mark.parametrize("boxes", [0, 3, 200, 50000])
+@pytest.mark.parametrize("cutoff", [1.3, 4.0])
+def test_aggregates_of_unwrapped_coordinates(boxes, cutoff):
+    """coordinates written up to `boxes` boxes away: the reference takes the image in FP64"""
+    side = 15.3
+    opts = cfgm.SoupOptions(box=[side] * 3, seed=7, kT=1.1, start={"C": 600, "O": 0, "H": 0, "M": 1, "W": 0})
+    cfg = cfgm.resolve(opts, P)
+    rng = np.random.default_rng(boxes)
+    pos = ob.OracleSystem(_abi, cfg).read(ob.F_POS).reshape(-1, 4).astype(np.float64)
+    pos[:, :3] = rng.random((cfg.n, 3)) * side + side * rng.integers(-boxes, boxes + 1, (cfg.n, 3))
+    pos = pos.astype(np.float32).ravel()
+    g = SoupSystem(cfg, {"positions": pos})
+    members = np.arange(0, cfg.n, 2 if cutoff < 2 else 29, dtype=np.uint32)
+    n_o, lab_o = ob.aggregates(_abi, pos, members, cfg.box, cutoff)
+    for labels in (g.aggregate_labels, g.aggregate_labels_noalloc):
+        n_g, lab_g = labels(members, cutoff)
+        assert n_g == n_o and np.array_equal(lab_g, lab_o)
+    assert 1 < n_o < len(members)
     g.dispose()
