@@ -26,6 +26,11 @@ __device__ __forceinline__ double js_round(double x) {
   return (__dsub_rn(x, r) >= 0.5) ? r + 1.0 : r;
 }
 __device__ __forceinline__ double wrap1(double v, double L) { return __dsub_rn(v, __dmul_rn(floor(__ddiv_rn(v, L)), L)); }
+// the cell of a coordinate on one axis of n cells of width w; the first where it is no number, or where the wrap of
+// an unwrapped one rounds to just below 0
+__device__ __forceinline__ int cell1(double v, double L, double w, int n) {
+  return max(0, min(n - 1, (int)floor(__ddiv_rn(wrap1(v, L), w))));
+}
 __device__ __forceinline__ double mi1(double d, double L) { return __dsub_rn(d, __dmul_rn(js_round(__ddiv_rn(d, L)), L)); }
 __device__ __forceinline__ double sq3(double a, double b, double c) {
   return __dadd_rn(__dadd_rn(__dmul_rn(a, a), __dmul_rn(b, b)), __dmul_rn(c, c));
@@ -194,9 +199,9 @@ __global__ void k_water(const float4* __restrict__ pos, const uint32_t* __restri
   const uint32_t k = blockIdx.x * blockDim.x + threadIdx.x;
   const bool mine = k < nw;
   const float4 p = pos[mine ? slot_of[off + wat[k]] : off];
-  const int gx = min(g.nx - 1, (int)floor(__ddiv_rn(wrap1((double)p.x, g.box[0]), g.cell)));
-  const int gy = min(g.ny - 1, (int)floor(__ddiv_rn(wrap1((double)p.y, g.box[1]), g.cell)));
-  const int gz = min(g.nz - 1, (int)floor(__ddiv_rn(wrap1((double)p.z, g.box[2]), g.cell)));
+  const int gx = cell1(p.x, g.box[0], g.cell, g.nx);
+  const int gy = cell1(p.y, g.box[1], g.cell, g.ny);
+  const int gz = cell1(p.z, g.box[2], g.cell, g.nz);
   const size_t c = (size_t)gx + (size_t)g.nx * ((size_t)gy + (size_t)g.ny * gz);
   const bool in = mine && !occ[c];
   add_counts(in && !vis[c], in && vis[c], 0, out);
@@ -256,9 +261,9 @@ __global__ void k_agg_bin(const float4* __restrict__ pos, const uint32_t* __rest
   const uint32_t k = blockIdx.x * blockDim.x + threadIdx.x;
   if (k >= m) return;
   const float4 p = pos[slot_of[off + mem[k]]];
-  const int cx = min(g.nx - 1, (int)floor(__ddiv_rn(wrap1((double)p.x, g.box[0]), wx)));
-  const int cy = min(g.ny - 1, (int)floor(__ddiv_rn(wrap1((double)p.y, g.box[1]), wy)));
-  const int cz = min(g.nz - 1, (int)floor(__ddiv_rn(wrap1((double)p.z, g.box[2]), wz)));
+  const int cx = cell1(p.x, g.box[0], wx, g.nx);
+  const int cy = cell1(p.y, g.box[1], wy, g.ny);
+  const int cz = cell1(p.z, g.box[2], wz, g.nz);
   const uint32_t c = (uint32_t)cx + (uint32_t)g.nx * ((uint32_t)cy + (uint32_t)g.ny * cz);
   cell[k] = c;
   atomicAdd(&count[c], 1u);
@@ -290,9 +295,9 @@ __global__ void k_agg_union(const float4* __restrict__ sorted, uint32_t m, Grid 
   const float lx = (float)g.box[0], ly = (float)g.box[1], lz = (float)g.box[2];
   const float c = sqrtf((float)c2), margin = 1e-4f * c + 1e-6f * fmaxf(lx, fmaxf(ly, lz));
   const float lo = c > margin ? (c - margin) * (c - margin) : 0.f, hi = (c + margin) * (c + margin);
-  const int cx = min(g.nx - 1, (int)floor(__ddiv_rn(wrap1((double)pi.x, g.box[0]), wx)));
-  const int cy = min(g.ny - 1, (int)floor(__ddiv_rn(wrap1((double)pi.y, g.box[1]), wy)));
-  const int cz = min(g.nz - 1, (int)floor(__ddiv_rn(wrap1((double)pi.z, g.box[2]), wz)));
+  const int cx = cell1(pi.x, g.box[0], wx, g.nx);
+  const int cy = cell1(pi.y, g.box[1], wy, g.ny);
+  const int cz = cell1(pi.z, g.box[2], wz, g.nz);
   // x - 1 .. x + 1 as at most two pieces of a row; axes of up to three cells are visited whole
   const int x0 = g.nx <= 3 ? 0 : cx - 1, x1 = g.nx <= 3 ? g.nx - 1 : cx + 1;
   const int ylo = g.ny <= 3 ? 0 : cy - 1, yhi = g.ny <= 3 ? g.ny - 1 : cy + 1;
@@ -544,7 +549,7 @@ struct PGrid {
 };
 
 __device__ __forceinline__ int pcell_axis(double x, const PGrid& g, int a) {
-  return min(g.n[a] - 1, (int)floor(__ddiv_rn(wrap1(x, g.box[a]), g.w[a])));
+  return cell1(x, g.box[a], g.w[a], g.n[a]);
 }
 
 // the distinct cells among c-1, c, c+1 (periodic) on an axis of n cells

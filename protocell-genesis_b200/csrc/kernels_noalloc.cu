@@ -52,6 +52,10 @@ __device__ __forceinline__ double js_round(double x) {
   return (__dsub_rn(x, r) >= 0.5) ? r + 1.0 : r;
 }
 __device__ __forceinline__ double wrap1(double v, double L) { return __dsub_rn(v, __dmul_rn(floor(__ddiv_rn(v, L)), L)); }
+// the cell of a coordinate on one axis; the first where it is no number or rounds to just below 0
+__device__ __forceinline__ int cell1(double v, double L, double w, int n) {
+  return max(0, min(n - 1, (int)floor(__ddiv_rn(wrap1(v, L), w))));
+}
 __device__ __forceinline__ double mi1(double d, double L) { return __dsub_rn(d, __dmul_rn(js_round(__ddiv_rn(d, L)), L)); }
 
 struct AggGrid {
@@ -82,9 +86,9 @@ __global__ void k_nf_bin(const float4* __restrict__ pos, const uint32_t* __restr
   const uint32_t k = blockIdx.x * blockDim.x + threadIdx.x;
   if (k >= m) return;
   const float4 p = pos[slot_of[off + s[kOffMem + k]]];
-  const int cx = min(g.nx - 1, (int)floor(__ddiv_rn(wrap1((double)p.x, g.box[0]), g.w[0])));
-  const int cy = min(g.ny - 1, (int)floor(__ddiv_rn(wrap1((double)p.y, g.box[1]), g.w[1])));
-  const int cz = min(g.nz - 1, (int)floor(__ddiv_rn(wrap1((double)p.z, g.box[2]), g.w[2])));
+  const int cx = cell1(p.x, g.box[0], g.w[0], g.nx);
+  const int cy = cell1(p.y, g.box[1], g.w[1], g.ny);
+  const int cz = cell1(p.z, g.box[2], g.w[2], g.nz);
   const uint32_t c = (uint32_t)cx + (uint32_t)g.nx * ((uint32_t)cy + (uint32_t)g.ny * cz);
   s[kOffCell + k] = c;
   s[kOffParent + k] = k;

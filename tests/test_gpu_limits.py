@@ -223,3 +223,25 @@ def test_aggregates_of_unwrapped_coordinates(boxes, cutoff):
         assert n_g == n_o and np.array_equal(lab_g, lab_o)
     assert 1 < n_o < len(members)
     g.dispose()
+
+
+def test_analysis_of_coordinates_that_are_no_numbers():
+    """beads at infinity or at no number at all are aggregates of their own and leave the others' labels; a closure
+    with some among its members and its water comes back"""
+    opts = cfgm.SoupOptions(box=[15] * 3, seed=7, kT=1.1, start={"C": 300, "O": 0, "H": 0, "M": 1, "W": 0})
+    cfg = cfgm.resolve(opts, P)
+    pos = ob.OracleSystem(_abi, cfg).read(ob.F_POS).reshape(-1, 4).copy()
+    pos[:, :3] = np.random.default_rng(3).random((cfg.n, 3)) * 15.0
+    lost = np.array([0, 7, 150, 299])
+    pos[lost, [0, 1, 2, 0]] = np.array([np.nan, np.inf, -np.inf, np.nan], np.float32)
+    pos = pos.astype(np.float32)
+    g = SoupSystem(cfg, {"positions": pos.ravel()})
+    members = np.arange(cfg.n, dtype=np.uint32)
+    kept = np.setdiff1d(members, lost).astype(np.uint32)
+    n_o, lab_o = ob.aggregates(_abi, pos.ravel(), kept, cfg.box, 1.3)
+    for labels in (g.aggregate_labels, g.aggregate_labels_noalloc):
+        n_g, lab_g = labels(members, 1.3)
+        assert n_g == n_o + len(lost) and np.array_equal(lab_g[kept], lab_o) and np.array_equal(lab_g[lost], lost)
+    r = g.closure(members[:150], members[150:], [7.5, 7.5, 7.5], 0.5, 1.0, 0.5)
+    assert r["totalEmptyCells"] > 0
+    g.dispose()
