@@ -94,7 +94,7 @@ __global__ void __launch_bounds__(1024) k_scan_add(uint32_t* __restrict__ out, u
 // exclusive scan of in[0..n) into out[0..n), out[n] = total; tmp must hold >= 2*ceil(n/4096)+2 words.
 // One launch to 4096 words, two to 4M (a rebuild of a small system is a chain of launches of 2 us each), and
 // beyond that, where a block's offset would be a sum of more than 1024 totals, the totals are scanned first.
-// With two, five and more launches, and memsets of their own for what the sort and the lists need zeroed, a force
+// With two, five and more launches, and memsets of their own for the cursors and the head cells, a force
 // evaluation of 1,220 beads took 112 us (99 now) and ten steps of 3,277 beads 412 (398).
 // Returns the kernels it launched (no shared counter: calls from several host threads do not race).
 uint64_t exclusive_scan(const uint32_t* in, uint32_t* out, uint32_t n, uint32_t* tmp, cudaStream_t st) {
@@ -176,8 +176,8 @@ __global__ void k_gather(uint32_t N, const uint32_t* __restrict__ perm,
 }
 
 // the gathered arrays back into the primary buffers, so every array keeps its address across rebuilds
-// (a captured step graph holds them as kernel arguments).  What the lists' builds behind it need zeroed is zeroed
-// here: the head cells' counts and the replicas' drifts (a memset of its own is a launch)
+// (a captured step graph holds them as kernel arguments).  The replicas' drifts are zeroed here (a memset of its own
+// is a launch)
 __global__ void k_copy_back(uint32_t N, const float4* __restrict__ pos2, const float4* __restrict__ vel2,
                             const float4* __restrict__ force2, const float* __restrict__ charge2,
                             const uint32_t* __restrict__ slots2, const uint32_t* __restrict__ center2,
@@ -187,11 +187,9 @@ __global__ void k_copy_back(uint32_t N, const float4* __restrict__ pos2, const f
                             float4* __restrict__ force, float* __restrict__ charge, uint32_t* __restrict__ slots,
                             uint32_t* __restrict__ center, uint32_t* __restrict__ held, uint32_t* __restrict__ brng,
                             uint32_t* __restrict__ trng, uint8_t* __restrict__ frozen, uint32_t* __restrict__ id,
-                            uint32_t* __restrict__ head_of, uint32_t nhcells, uint32_t* __restrict__ hcount, uint32_t R,
-                            uint32_t* __restrict__ drift_bits) {
+                            uint32_t* __restrict__ head_of, uint32_t R, uint32_t* __restrict__ drift_bits) {
   const uint32_t k = blockIdx.x * blockDim.x + threadIdx.x;
   if (k >= N) return;
-  for (uint32_t c = k; c < nhcells; c += N) hcount[c] = 0u;
   if (k < R) drift_bits[k] = 0u;   // a replica has a bead at least
   head_of[k] = SOUP_NONE_U32;   // k_head_index names the heads
   pos[k] = pos2[k]; vel[k] = vel2[k]; force[k] = force2[k]; charge[k] = charge2[k];
@@ -540,7 +538,8 @@ __global__ void __launch_bounds__(128, 9) k_build_list(
   if (lane == 0) nl_cnt[k] = cnt;
 }
 
-// heads: bin into the coarse head grid (replica-local cells), deterministic order inside a cell
+// heads: bin into the coarse head grid (replica-local cells), deterministic order inside a cell.  The cells' counts
+// are zero before and after: k_head_scatter counts them down
 __global__ void k_head_index(const uint32_t* __restrict__ heads, const uint32_t* __restrict__ head_sys, uint32_t H,
                              const uint32_t* __restrict__ slot_of, const float4* __restrict__ pos,
                              const SysParams* __restrict__ sp, uint32_t* __restrict__ hcell_of,
@@ -661,7 +660,7 @@ void launch_sort_and_gather(Batch& b) {
   k_copy_back<<<nblocks(b.N), kBlock, 0, b.stream>>>(b.N, b.pos2, b.vel2, b.force2, b.charge2, b.slots2, b.center2,
                                                       b.held2, b.brng2, b.trng2, b.frozen2, b.id2, b.pos, b.vel, b.force,
                                                       b.charge, b.slots, b.center, b.held, b.brng, b.trng, b.frozen,
-                                                      b.id, b.head_of, b.nhcells, b.hcell_count, b.R, b.drift_bits);
+                                                      b.id, b.head_of, b.R, b.drift_bits);
   b.launches += 4 + scans;
   prof_end(b);
 }

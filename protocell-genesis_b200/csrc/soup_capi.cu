@@ -212,6 +212,7 @@ void alloc_grids(Batch& b) {
   b.cell_count = dalloc<uint32_t>(nc + 1);
   b.cell_start = dalloc<uint32_t>(nc + 1);
   b.hcell_count = dalloc<uint32_t>(nh + 1);
+  SOUP_CUDA_TRY(cudaMemsetAsync(b.hcell_count, 0, 4 * (size_t)(nh + 1), b.stream));   // every rebuild leaves it at zero
   b.hcell_start = dalloc<uint32_t>(nh + 1);
   const uint64_t m = std::max(nc, nh);
   b.scan_tmp = dalloc<uint32_t>(4 * (m / 4096 + 64) + 256);

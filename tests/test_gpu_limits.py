@@ -1,7 +1,6 @@
 """Calls at their limits and calls between others: rows of the neighbour list at the capacity and beyond what a warp
-stages, a window's reverse pass behind other calls, a sweep on lists that no longer
-serve, one in a box below twice its cutoff, and
-aggregates of coordinates far outside the box."""
+stages, rebuilds of a box of many more cells than beads, a window's reverse pass behind other calls, a sweep on lists
+that no longer serve, one in a box below twice its cutoff, aggregates of coordinates far outside the box."""
 import numpy as np
 import pytest
 
@@ -244,4 +243,27 @@ def test_analysis_of_coordinates_that_are_no_numbers():
         assert n_g == n_o + len(lost) and np.array_equal(lab_g[kept], lab_o) and np.array_equal(lab_g[lost], lost)
     r = g.closure(members[:150], members[150:], [7.5, 7.5, 7.5], 0.5, 1.0, 0.5)
     assert r["totalEmptyCells"] > 0
+    g.dispose()
+
+
+def test_head_lists_of_a_sparse_box_over_rebuilds():
+    """a million head cells for 200 heads, rebuilt over and over, and again after the grids were made anew: the cells'
+    counts start at zero every time"""
+    opts = cfgm.SoupOptions(box=[170] * 3, seed=2, kT=1.1, start={"C": 0, "O": 200, "H": 0, "M": 1, "W": 99},
+                            electrostatics={"enabled": True, "pH": 7.0, "ionicStrengthMolar": 1.0}, rebuild_on_drift=True, skin=0.5)
+    cfg = cfgm.resolve(opts, P)
+    assert (170.0 / (cfg.es_list_range / 2)) ** 3 > 1e6
+    rng = np.random.default_rng(2)
+    pos = ob.OracleSystem(_abi, cfg).read(ob.F_POS).reshape(-1, 4).copy()
+    pos[:, :3] = np.mod(np.repeat(rng.random((75, 3)) * 170.0, 4, axis=0) + rng.normal(size=(300, 3)), 170.0)
+    pos = pos.astype(np.float32).ravel()
+    g = SoupSystem(cfg, {"positions": pos})
+    for again in range(4):
+        if again == 2:
+            g.set_box([170.0] * 3)
+        g.debug_phase(_abi.PHASE_REBUILD)
+        o = ob.OracleSystem(_abi, cfg, {"positions": g.particles()})
+        for a, b in zip(g.es_lists(), o.es_lists()):
+            assert np.array_equal(a, b)
+    assert g.es_lists()[0].max() >= 2
     g.dispose()
