@@ -350,18 +350,24 @@ void launch_force(Batch& b) {
 }
 
 // Lanes per particle: the result is the same bits, so the launch's size decides.  Few particles need the lanes
-// to cover the gathers' latency; many need the fewest instructions.  Measured with 4 / 8 / 16 lanes: 483k beads 241 /
-// 264 / 318 us, 121k 95 / - / 97, 24k 26.4 / 27.3 / 24.7, the 700 heads of a small system 31.6 / 22 / 13.5.
-int force_lanes(const Batch& b, uint32_t n) {
-  if (b.tpp) return b.tpp <= 4 ? 4 : (b.tpp <= 8 ? 8 : 16);
-  return n >= 80000u ? 4 : (n >= 40000u ? 8 : 16);
+// to cover the gathers' latency; many need the fewest instructions, and rows of a chunk or two leave most lanes idle.
+// Measured with 4 / 8 / 16 lanes, us: 6k beads 16.1 / 14.0 / 12.3, 10k 16.8 / 15.5 / 16.3, 24k 22.0 / 21.7 / 22.5, 30k
+// 23.9 / 23.9 / 26.2, 40k 30.1 / 28.1 / 31.0, 60k 36.8 / 35.4 / 41.6, 80k 43.3 / 41.9 / 52.7, 100k 52.8 / 53.8 / 65.7,
+// 121k 57.7 / 64.0 / 81.8 (another mix of kinds: 80k 40.5 / 41.4 / 46.4); rows of 24 entries: 20k 11.3 / 12.3 / 12.9,
+// of 5: 60k 12.5 / 15.4 / 24.4, 3k 9.5 / 9.3 / 9.9; the 700 heads of a small system 31.6 / 22 / 13.5.
+int force_lanes(const Batch& b, bool heads) {
+  const int set = heads ? b.tpp_heads : b.tpp;
+  const uint32_t n = heads ? b.H : b.N;
+  if (set) return set <= 4 ? 4 : (set <= 8 ? 8 : 16);
+  if (n >= 8192u && b.mean_row < 32.0) return 4;
+  return n >= 80000u ? 4 : (n >= 28000u ? 8 : 16);
 }
 
 void launch_force_list(Batch& b, bool heads) {
   const uint32_t n = heads ? b.H : b.N;
   if (n == 0) return;
   b.launches += 1;
-  switch (force_lanes(b, n)) {
+  switch (force_lanes(b, heads)) {
     case 4: launch_force_tpp<4>(b, heads); break;
     case 8: launch_force_tpp<8>(b, heads); break;
     default: launch_force_tpp<16>(b, heads); break;

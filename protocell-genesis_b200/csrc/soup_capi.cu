@@ -218,9 +218,17 @@ void alloc_grids(Batch& b) {
   b.scan_tmp = dalloc<uint32_t>(4 * (m / 4096 + 64) + 256);
 }
 
+// the sphere of the wall, or the box
+double volume_of(const SoupConfig& c) {
+  return c.wall_radius > 0 ? 4.18879 * c.wall_radius * c.wall_radius * c.wall_radius : c.box[0] * c.box[1] * c.box[2];
+}
+
 void upload_params(Batch& b) {
+  b.mean_row = 0.0;
   for (uint32_t r = 0; r < b.R; ++r) {
     SysParams& p = b.hsp[r];
+    const SoupConfig& c = b.cfg[r];
+    b.mean_row += (double)c.n / b.N * c.n / volume_of(c) * 4.18879 * c.list_range * c.list_range * c.list_range;
     for (int a = 0; a < 3; ++a) {
       p.cell[a] = p.box[a] / (float)p.dims[a]; p.inv_cell[a] = (float)p.dims[a] / p.box[a];
       p.hcell[a] = p.box[a] / (float)p.hdims[a]; p.inv_hcell[a] = (float)p.hdims[a] / p.box[a];
@@ -456,7 +464,7 @@ Batch* make_batch(const SoupConfig* cfgs, const SoupInitState* inits, uint32_t R
   upload_params(b);
   // lanes per particle in the list force by the launch's size (force_lanes); SOUP_TPP in the environment
   // overrides it (up to 4: 4, up to 8: 8, else 16)
-  if (const char* e = std::getenv("SOUP_TPP")) b.tpp = std::atoi(e);
+  if (const char* e = std::getenv("SOUP_TPP")) b.tpp = b.tpp_heads = std::atoi(e);
   if (const char* e = std::getenv("SOUP_FULL_ROWS")) b.prune = std::atoi(e) == 0;
   force_pass(b);   // priming pass (soup/src/sim.ts:396-408)
   SOUP_CUDA_TRY(cudaStreamSynchronize(b.stream));
@@ -1014,10 +1022,10 @@ void tune_plan(Batch& b, const std::vector<double>& skin, int walk) {
   alloc_grids(b);
   upload_params(b);
 }
-// a tuning's lanes per particle: 8 stands for eight or the sixteen that a small launch takes by itself
+// a tuning's lanes per particle, of whole passes: 8 stands for eight or the sixteen that a small launch takes by itself
 int tuned_lanes(Batch& b, uint32_t tpp) {
   b.tpp = 0;
-  return tpp == 8 && force_lanes(b, b.N) > 8 ? 0 : (int)tpp;
+  return tpp == 8 && force_lanes(b) > 8 ? 0 : (int)tpp;
 }
 template <class F> double tune_time(Batch& b, int reps, F&& f) {
   cudaEvent_t e0, e1;
@@ -1505,7 +1513,7 @@ int soup_autotune(SoupHandle* h, uint32_t steps, SoupTuneResult* out) {
     std::vector<double> planned(b.R);
     for (uint32_t r = 0; r < b.R; ++r) planned[r] = b.cfg[r].skin;
     const int walk0 = b.hsp[0].walk;
-    const int tpp0 = std::min(force_lanes(b, b.N), 8);
+    const int tpp0 = std::min(force_lanes(b), 8);
     auto steps_ms = [&]() { return tune_time(b, 1, [&] { step_batch(b, steps); }) / steps; };
     SoupTuneResult res{};
     if (steps) {

@@ -163,7 +163,9 @@ struct Batch {
   std::vector<uint64_t> next_sweep;
   uint64_t rebuilds = 0, sweeps = 0;
   bool force_fresh = false;          // force array matches positions+charges+lists
-  int tpp = 0;                       // threads per particle in the list force (0: by the launch's size)
+  int tpp = 0;                       // threads per particle in a whole pass of the list force (0: by force_lanes)
+  int tpp_heads = 0;                 // the same in a pass over the heads alone
+  double mean_row = 0.0;             // list entries a bead has if the beads fill their boxes (or parcels) evenly
   uint32_t wait_limit = 0;           // polls of a bounded device-side handoff before it gives up (0: default)
   DiffWindow diff;
   // captured step chunks (CUDA graphs), keyed by length and schedule phase; the drift-triggered
@@ -219,7 +221,7 @@ void launch_build_lists(Batch& b);
 void launch_build_es_lists(Batch& b);
 void launch_force(Batch& b);       // list force, then the far electrostatics half
 void launch_force_list(Batch& b, bool heads = false);
-int force_lanes(const Batch& b, uint32_t n);   // lanes per particle for n particles
+int force_lanes(const Batch& b, bool heads = false);   // lanes per particle of a pass
 void launch_force_heads(Batch& b);  // the heads' list force and far half only (after a charge sweep)
 void launch_es_far(Batch& b);
 void launch_force_brute(Batch& b);

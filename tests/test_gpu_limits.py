@@ -1,14 +1,15 @@
 """Calls at their limits and calls between others: rows of the neighbour list at the capacity and beyond what a warp
 stages, rebuilds of a box of many more cells than beads, a window's reverse pass behind other calls, a sweep on lists
-that no longer serve, one in a box below twice its cutoff, aggregates of coordinates far outside the box."""
+that no longer serve, one in a box below twice its cutoff, aggregates of coordinates far outside the box, and the lanes of
+the list force."""
 import numpy as np
 import pytest
 
 import oracle_binding as ob
-from helpers import charged_opts, oracle_bilayer_start, rel_rms
+from helpers import charged_opts, confined_opts, oracle_bilayer_start, rel_rms
 from protocell_genesis_b200 import _abi, config as cfgm
-from protocell_genesis_b200.soup import SoupSystem
-from test_gpu_parity import FORCE_TOL, make_pair
+from protocell_genesis_b200.soup import SoupBatch, SoupSystem
+from test_gpu_parity import FORCE_TOL, make_pair, oracle_state
 
 pytestmark = pytest.mark.gpu
 P = cfgm.load_params()
@@ -267,3 +268,49 @@ def test_head_lists_of_a_sparse_box_over_rebuilds():
             assert np.array_equal(a, b)
     assert g.es_lists()[0].max() >= 2
     g.dispose()
+
+
+@pytest.mark.parametrize("maker", ["replicas", "confined"])
+def test_lanes_per_bead_change_no_bit_of_batches_and_parcels(maker, monkeypatch):
+    """warps that span two replicas (bead counts that leave a remainder by every group), a parcel behind its wall, and
+    the pass over the heads alone behind a sweep"""
+    sched = dict(rebuild_on_drift=True, skin=1.0, sweep_every=4, chunk_steps=4)
+    if maker == "replicas":
+        start = {"C": 611, "O": 103, "H": 500, "M": 21, "W": 0}
+        opts = [charged_opts(**sched), charged_opts(start=start, seed=8, **sched), charged_opts(seed=9, **sched)]
+    else:
+        opts = [confined_opts(**sched)]
+    cfgs = [cfgm.resolve(o, P) for o in opts]
+    states = []
+    for cfg in cfgs:
+        o = ob.OracleSystem(_abi, cfg)
+        o.relax(20, 0.1)
+        states.append(oracle_state(o))
+    runs = []
+    for lanes in ("4", "8", "16", "0"):
+        monkeypatch.setenv("SOUP_TPP", lanes)
+        b = SoupBatch(cfgs, states)
+        b.step(8)                             # two sweeps
+        runs.append([a for r in b.replicas for a in (r.particles(), r.velocities(), r.charges(), r.forces_no_rebuild())])
+        for r in b.replicas:
+            assert rel_rms(r.forces_no_rebuild(), r.forces_brute_force()) < FORCE_TOL
+        b.dispose()
+    for other in runs[1:]:
+        for x, y in zip(runs[0], other):
+            assert np.array_equal(x, y)
+
+
+@pytest.mark.parametrize("n", [8191, 8200])
+def test_a_dilute_system_steps_the_same_with_any_lanes(n, monkeypatch):
+    """rows of a few entries on either side of the line from which they take four lanes"""
+    opts = cfgm.SoupOptions(box=[70] * 3, seed=5, kT=1.1, start={"C": 0, "O": 0, "H": 0, "M": 1, "W": n - 1})
+    cfg = cfgm.resolve(opts, P)
+    pos = ob.OracleSystem(_abi, cfg).read(ob.F_POS)
+    runs = []
+    for lanes in ("0", "16"):
+        monkeypatch.setenv("SOUP_TPP", lanes)
+        g = SoupSystem(cfg, {"positions": pos})
+        g.step(10)
+        runs.append((g.particles(), g.forces_no_rebuild()))
+        g.dispose()
+    assert all(np.array_equal(a, b) for a, b in zip(*runs))
