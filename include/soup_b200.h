@@ -316,7 +316,9 @@ int soup_set_wait_limit(SoupHandle* h, uint32_t polls);
 /* ---- Monte Carlo and analysis -------------------------------------------------------------- */
 /* protonationSweepDEBUG (soup/src/sim.ts): one constant-pH sweep now on the device, then the
  * rebuild + force recompute (soup/src/soup-protonation.ts:52-77).  With drift-triggered rebuilds the lists are
- * rebuilt here only if the drift calls for it: they do not depend on charges. */
+ * rebuilt before it only if the drift calls for it: they do not depend on charges.  What the sweep keeps on the
+ * device beside the lists is made with the system: 8 bytes per entry of the head lists' capacity, and 5.3 KB per
+ * titratable bead (per replica, rounded up to 655 KB or 1.3 MB) for the pairs of draws near one another. */
 int soup_protonation_sweep(SoupHandle* h, SoupSweepResult* out);
 
 /* encapsulatedWaterVolume (soup/src/water-closure.ts:271-363) on the current positions.

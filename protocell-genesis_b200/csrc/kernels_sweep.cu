@@ -245,13 +245,9 @@ __device__ __forceinline__ void red_add_release_gpu(uint32_t* p, uint32_t v) {
   asm volatile("red.release.gpu.add.u32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
 }
 
-// Replica r's draws start here: whole blocks, and room for the 2 H draws a sweep consumes at most (an attempt
-// takes a site draw and at most one acceptance draw).
-__host__ __device__ __forceinline__ size_t draws_before(size_t heads_before, size_t replicas_before) {
-  return ((2 * heads_before + kDraws - 1) / kDraws + 2 * replicas_before) * kDraws;
-}
-__device__ __forceinline__ size_t draw0(const SysParams& P, uint32_t r) { return draws_before(P.head_off, r); }
-__device__ __forceinline__ uint32_t draw_blocks(const SysParams& P) { return (2 * P.nheads + P.sweep_draws - 1) / P.sweep_draws; }
+// whole blocks for the 2 H draws a sweep consumes at most (an attempt takes a site draw and at most one acceptance draw)
+__host__ __device__ __forceinline__ uint32_t blocks_of(uint32_t heads, uint32_t W) { return (2 * heads + W - 1) / W; }
+__device__ __forceinline__ uint32_t draw_blocks(const SysParams& P) { return blocks_of(P.nheads, P.sweep_draws); }
 // the reference's min(H - 1, floor(u H)) for u = bits / 2^32: u H = bits H / 2^32 is exact in FP64
 // (bits H < 2^52), so its floor is the high word of the 64-bit product, always below H
 __device__ __forceinline__ uint32_t site_of(uint32_t bits, uint32_t H) {
@@ -268,18 +264,37 @@ __global__ void k_sweep_draws(const SysParams* __restrict__ sp, const uint32_t* 
   const uint32_t d = blockIdx.x * blockDim.x + threadIdx.x;
   if (d >= draw_blocks(P) * P.sweep_draws) return;
   const Lcg j = lcg_pow(d + 1u);
-  draw_site[draw0(P, r) + d] = site_of(pcg_bits(j.a * rng_io[r] + j.c), H);
+  draw_site[P.draw_off + d] = site_of(pcg_bits(j.a * rng_io[r] + j.c), H);
 }
 
 // The pairs of draws within a block whose sites are near one another.  For place i of a block: entry e names
 // an earlier place j (ascending) and the change of i's site energy when j's site deprotonates (std_delta, the
 // value the D rows hold).  A place's word in pcnt packs the entry count and, from bit 10 on, 1 + the last
 // earlier place of the same site (0: none; a flip changes its own site's state and not its energy).  The
-// walk's threads read their entries a place each: pidx [block][e / 8][place][e % 8], pdel [block][e][place].
+// walk's threads read their entries a place each, eight entries (a group g = e / 8) to a word of pidx, in 256 columns:
+// pidx [block][group][column][e % 8], pdel [block][group][e % 8][column].  A place has no more entries than there are
+// places before it, so of a block of 512 places 256 + c and 255 - c share column c, the one's groups from the top down,
+// the other's from the bottom up, 65 in all; a block of 256 has a column a place (folded, its sweep took 1% longer).
+// 10 bytes an entry, 5.3 KB a head.
 // A block of threads stages the sites' records and takes kPairDraws draws, a warp per draw at a time: it
 // screens 32 earlier draws at a time and evaluates the near ones packed.
 constexpr uint32_t kPairDraws = 16;
-__device__ __forceinline__ size_t pidx_at(uint32_t e, uint32_t i, uint32_t W) { return ((size_t)(e >> 3) * W + i) * 8 + (e & 7u); }
+constexpr uint32_t kPairCols = 256;
+__host__ __device__ __forceinline__ uint32_t pair_block(uint32_t W) { return kPairCols * (W == 512u ? 8u * 65u : W); }   // entries
+// place i's column and first group, and the way to its next
+__device__ __forceinline__ bool pair_up(uint32_t i, uint32_t W) { return W == 512u && i < kPairCols; }
+__device__ __forceinline__ uint32_t pair_column(uint32_t i, uint32_t W) { return pair_up(i, W) ? 255u - i : i % kPairCols; }
+__device__ __forceinline__ uint32_t pair_first(uint32_t i, uint32_t W) { return pair_up(i, W) ? 64u : 0u; }
+__device__ __forceinline__ int pair_step(uint32_t i, uint32_t W) { return pair_up(i, W) ? -1 : 1; }
+__device__ __forceinline__ uint32_t pair_group(uint32_t e, uint32_t i, uint32_t W) {
+  return pair_first(i, W) + (e >> 3) * (uint32_t)pair_step(i, W);
+}
+__device__ __forceinline__ uint32_t pidx_at(uint32_t e, uint32_t i, uint32_t W) {
+  return (pair_group(e, i, W) * kPairCols + pair_column(i, W)) * 8u + (e & 7u);
+}
+__device__ __forceinline__ uint32_t pdel_at(uint32_t e, uint32_t i, uint32_t W) {
+  return (pair_group(e, i, W) * 8u + (e & 7u)) * kPairCols + pair_column(i, W);
+}
 __device__ __forceinline__ uint32_t pair_count(uint32_t w) { return w & 1023u; }
 __device__ __forceinline__ int pair_same(uint32_t w) { return (int)(w >> 10) - 1; }
 template <bool I64>
@@ -296,7 +311,7 @@ __global__ void __launch_bounds__(256) k_sweep_pairs(const SysParams* __restrict
   const uint32_t W = P.sweep_draws, first = blockIdx.x * kPairDraws;   // W is a multiple of kPairDraws
   if (first >= draw_blocks(P) * W) return;
   const uint32_t lane = threadIdx.x & 31u, wid = threadIdx.x >> 5;
-  const size_t block0 = draw0(P, r) + (first / W) * W;
+  const size_t block0 = P.draw_off + (first / W) * W, pair0 = P.pair_off + (size_t)(first / W) * pair_block(W);
   const uint32_t i0 = first % W;
   const uint32_t* ds = draw_site + block0;
   const float4* hx = xq + P.head_off;
@@ -326,11 +341,11 @@ __global__ void __launch_bounds__(256) k_sweep_pairs(const SysParams* __restrict
     __syncwarp();
     for (uint32_t e = lane; e < n; e += 32u) {
       const uint32_t j = near[e];
-      pidx[block0 * kDraws + pidx_at(e, i, W)] = (uint16_t)j;
-      pdel[block0 * kDraws + (size_t)e * W + i] = std_delta(P, dist2<I64>(P, rec[j], xi), (float)P.d_q, cut2, reach2);
+      pidx[pair0 + pidx_at(e, i, W)] = (uint16_t)j;
+      pdel[pair0 + pdel_at(e, i, W)] = std_delta(P, dist2<I64>(P, rec[j], xi), (float)P.d_q, cut2, reach2);
     }
     // the last word's places beyond n name place W, which never flips
-    for (uint32_t e = n + lane; e < ((n + 7u) & ~7u); e += 32u) pidx[block0 * kDraws + pidx_at(e, i, W)] = (uint16_t)W;
+    for (uint32_t e = n + lane; e < ((n + 7u) & ~7u); e += 32u) pidx[pair0 + pidx_at(e, i, W)] = (uint16_t)W;
     if (lane == 0) pcnt[block0 + i] = n | (same << 10);
     __syncwarp();
   }
@@ -470,7 +485,7 @@ __global__ void __launch_bounds__(kWalkThreads) k_sweep_walk(
   WalkShared& G = shared[r];
   const uint32_t off = P.head_off, tid = threadIdx.x, lane = tid & 31u, wid = tid >> 5;
   long long* E = Eg + off;
-  const size_t d0 = draw0(P, r);
+  const size_t d0 = P.draw_off;
   const uint32_t blocks = draw_blocks(P);
 
   if (rank != 0) {
@@ -516,6 +531,8 @@ __global__ void __launch_bounds__(kWalkThreads) k_sweep_walk(
   constexpr uint32_t parts = kWalkThreads / W, warps = W / 32u;
   const uint32_t place = tid % W, part = tid / W;
   const bool first = part == 0;        // these threads decide (whole warps)
+  const uint32_t column = pair_column(place, W);
+  const int step = pair_step(place, W);
   uint32_t st;                         // the stream's state behind this thread's draw
   {
     const Lcg j = lcg_pow(place + 1u);
@@ -529,11 +546,12 @@ __global__ void __launch_bounds__(kWalkThreads) k_sweep_walk(
   for (uint32_t blk = 0; !over; ++blk) {
     const size_t b0 = d0 + (size_t)blk * W;
     // this draw's near draws: places eight to a word, changes one by one
-    const uint16_t* px = pidx + b0 * kDraws;
-    const long long* pd = pdel + b0 * kDraws;
+    const size_t p0 = P.pair_off + (size_t)blk * pair_block(W);
+    const uint16_t* px = pidx + p0;
+    const long long* pd = pdel + p0;
     const uint32_t np = pair_count(word);
-    const uint4* pi = reinterpret_cast<const uint4*>(px) + place;
-    const uint4 idx0 = 8u * part < np ? __ldg(pi + (size_t)part * W) : make_uint4(0u, 0u, 0u, 0u);
+    const uint4* pi = reinterpret_cast<const uint4*>(px) + (pair_first(place, W) + part * (uint32_t)step) * kPairCols + column;
+    const uint4 idx0 = 8u * part < np ? __ldg(pi) : make_uint4(0u, 0u, 0u, 0u);
     const uint32_t v_acc = pcg_bits(st * 747796405u + 2891336453u);   // the next draw of the stream
     const long long e_base = (long long)__ldcg(reinterpret_cast<const unsigned long long*>(E + site));
     const uint32_t f_base = flag[site];
@@ -583,16 +601,21 @@ __global__ void __launch_bounds__(kWalkThreads) k_sweep_walk(
       }
       long long sum = 0;
       uint4 nxt = idx0;
-      const long long* pv = pd + (size_t)(8u * part) * W + place;
-      for (uint32_t q = 8u * part; q < np; q += 8u * parts, pv += (size_t)(8u * parts) * W) {
+      const uint4* pw = pi;
+      const long long* pv = pd + (pair_first(place, W) + part * (uint32_t)step) * (8u * kPairCols) + column;
+      for (uint32_t q = 8u * part; q < np; q += 8u * parts, pv += step * (int)(8u * kPairCols * parts)) {
         const uint32_t jw[4] = {nxt.x, nxt.y, nxt.z, nxt.w};
-        if (q + 8u * parts < np) nxt = __ldg(pi + (size_t)((q >> 3) + parts) * W);
+        // the next word: stepped to with 256 draws a block (counted from the first, a sweep of 4,665 heads took 441 us and
+        // not 424), counted from the first with 512 (18,659 heads, 995 and not 1013)
+        if (W == 512u) pw = pi + step * (int)((q / 8u - part + parts) * kPairCols);
+        else pw += kPairCols * parts;
+        if (q + 8u * parts < np) nxt = __ldg(pw);
         int c[8];
         long long v[8];
 #pragma unroll
         for (int u = 0; u < 8; ++u) {
           c[u] = s_code[u & 1 ? jw[u >> 1] >> 16 : jw[u >> 1] & 0xFFFFu];
-          v[u] = c[u] != 0 ? __ldg(pv + (size_t)u * W) : 0;
+          v[u] = c[u] != 0 ? __ldg(pv + u * kPairCols) : 0;
         }
 #pragma unroll
         for (int u = 0; u < 8; ++u) {  // c v for c = 0, 1, -1
@@ -613,7 +636,7 @@ __global__ void __launch_bounds__(kWalkThreads) k_sweep_walk(
           const uint32_t j = px[pidx_at(q, place, W)];
           if (s_code[j] != 2) continue;
           const uint32_t sj = off + draw_site[b0 + j];
-          e += flip_delta(P, dist2<I64>(P, xq[sj], xq[off + site]), xq[sj].w, 0.f, cut2, reach2) - pd[(size_t)q * W + place];
+          e += flip_delta(P, dist2<I64>(P, xq[sj], xq[off + site]), xq[sj].w, 0.f, cut2, reach2) - pd[pdel_at(q, place, W)];
         }
       }
       // the charge state behind the last earlier flip of this site
@@ -790,8 +813,16 @@ void launch_sweep(Batch& b, uint32_t replica) {
 }
 
 uint32_t sweep_max_heads() { return kMaxHeads; }
-size_t sweep_draws(const Batch& b) { return b.H ? draws_before(b.H, b.R) : 0; }
-size_t sweep_pairs(const Batch& b) { return sweep_draws(b) * kDraws; }
+void sweep_layout(Batch& b, size_t& draws, size_t& pairs) {
+  draws = pairs = 0;
+  for (SysParams& p : b.hsp) {
+    const uint32_t W = p.sweep_most = p.sweep_draws, blocks = blocks_of(p.nheads, W);
+    p.draw_off = (uint32_t)draws;
+    p.pair_off = pairs;
+    draws += (size_t)blocks * W;
+    pairs += (size_t)blocks * pair_block(W);
+  }
+}
 
 size_t sweep_shared_bytes(const Batch& b) { return sizeof(WalkShared) * b.R; }
 

@@ -158,6 +158,15 @@ SysParams make_sys(const SoupConfig& c) {
   return p;
 }
 
+// a replica's parameters made anew (a live box, another skin): its places in the batch's arrays stay
+SysParams remake_sys(const SoupConfig& c, const SysParams& old) {
+  SysParams p = make_sys(c);
+  p.slot_off = old.slot_off; p.n = old.n; p.head_off = old.head_off; p.nheads = old.nheads;
+  p.sweep_most = old.sweep_most; p.draw_off = old.draw_off; p.pair_off = old.pair_off;
+  p.sweep_draws = std::min(p.sweep_draws, p.sweep_most);   // the smaller blocks fit what the larger were laid out for
+  return p;
+}
+
 uint64_t cells_of(const int d[3]) { return (uint64_t)d[0] * d[1] * d[2]; }
 
 }  // namespace
@@ -449,9 +458,11 @@ Batch* make_batch(const SoupConfig* cfgs, const SoupInitState* inits, uint32_t R
   b.head_e = dalloc<long long>(b.H);
   b.head_pos = dalloc<float4>(b.H);
   b.head_xq = dalloc<float4>(b.H);
-  b.draw_site = dalloc<uint32_t>(sweep_draws(b)); b.pair_cnt = dalloc<uint32_t>(sweep_draws(b));
+  size_t draws, pairs;
+  sweep_layout(b, draws, pairs);
+  b.draw_site = dalloc<uint32_t>(draws); b.pair_cnt = dalloc<uint32_t>(draws);
   b.walk_shared = dalloc<char>(sweep_shared_bytes(b));
-  b.pair_idx = dalloc<uint16_t>(sweep_pairs(b)); b.pair_del = dalloc<long long>(sweep_pairs(b));
+  b.pair_idx = dalloc<uint16_t>(pairs); b.pair_del = dalloc<long long>(pairs);
   sweep_prepare(b);
   b.es_nl = dalloc<uint32_t>((size_t)b.H * std::max<uint32_t>(b.es_cap, 1)); b.es_cnt = dalloc<uint32_t>(b.H);
   b.head_d = dalloc<long long>((size_t)b.H * std::max<uint32_t>(b.es_cap, 1));
@@ -1011,11 +1022,9 @@ void tune_plan(Batch& b, const std::vector<double>& skin, int walk) {
     c.list_range += ds;
     if (c.es_enabled) c.es_list_range += ds;
     c.skin = skin[r];
-    const SysParams old = b.hsp[r];
-    SysParams p = make_sys(c);
+    SysParams p = remake_sys(c, b.hsp[r]);
     p.walk = walk;
     p.fine = grid_of(c.box, c.list_range, walk, c.n, p.dims);
-    p.slot_off = old.slot_off; p.n = old.n; p.head_off = old.head_off; p.nheads = old.nheads;
     b.hsp[r] = p;
   }
   drop_graphs(b);
@@ -1405,10 +1414,7 @@ void apply_box(Batch& b, uint32_t r, const double box[3]) {
   check_box(b.cfg[r], box);
   for (int a = 0; a < 3; ++a) b.cfg[r].box[a] = box[a];
   if (b.wall_r0[r] > 0) b.cfg[r].wall_radius = b.wall_r0[r] * (box[0] / b.wall_box0[r]);
-  const SysParams old = b.hsp[r];
-  SysParams p = make_sys(b.cfg[r]);
-  p.slot_off = old.slot_off; p.n = old.n; p.head_off = old.head_off; p.nheads = old.nheads;
-  b.hsp[r] = p;
+  b.hsp[r] = remake_sys(b.cfg[r], b.hsp[r]);
   drop_graphs(b);
   alloc_grids(b);
   upload_params(b);

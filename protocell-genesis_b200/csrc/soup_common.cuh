@@ -45,7 +45,10 @@ struct SysParams {
   uint32_t hcell_off;
   float cell[3], inv_cell[3], hcell[3], inv_hcell[3];   // cell sides of the two grids and their inverses
   uint32_t list_cap, es_cap; // capacities (overflow threshold)
-  uint32_t sweep_draws;      // draws of a block of the constant-pH walk: 512 or 256
+  uint32_t sweep_draws;      // draws of a block of the constant-pH walk: 512 or 256, sweep_most at most
+  uint32_t sweep_most;       // what the arrays of its draws and pairs are laid out for (sweep_layout)
+  uint32_t draw_off;         // first draw of this replica in them
+  uint64_t pair_off;         // first entry of its pairs
   uint32_t es_on;            // electrostatics enabled
   uint32_t image64;          // the sweep's cutoffs reach so near half the box that FP64 picks the image
   int32_t charged_kind;

@@ -117,8 +117,8 @@ struct Batch {
                                      // deprotonates, fixed point 2^-40 (sweep scratch)
   uint32_t* draw_site = nullptr;     // the site each draw of a sweep's stream selects (sweep scratch)
   uint32_t* pair_cnt = nullptr;      // per draw: the earlier draws of its block with a site near its own
-  uint16_t* pair_idx = nullptr;      // [block][entry][place] which (k_sweep_pairs)
-  long long* pair_del = nullptr;     // [block][entry][place] the change of the draw's site energy when that one flips
+  uint16_t* pair_idx = nullptr;      // per block, entry and place: which (k_sweep_pairs)
+  long long* pair_del = nullptr;     // the same: the change of the draw's site energy when that one flips
   void* walk_shared = nullptr;       // per replica: what the CTAs of a walk share (WalkShared)
   int sms = 0;                       // of the device
   uint32_t es_cap = 0;
@@ -235,9 +235,9 @@ void launch_relax_step(Batch& b, float d);
 void launch_bonds(Batch& b);
 void launch_sweep(Batch& b, uint32_t replica);
 size_t sweep_shared_bytes(const Batch& b);
-size_t sweep_pairs(const Batch& b);   // entries of the sweep's pair arrays
+// lays the sweep's arrays out by the replicas' heads and block sizes: their draws and pair entries
+void sweep_layout(Batch& b, size_t& draws, size_t& pairs);
 uint32_t sweep_max_heads();   // heads one replica may hold for the device constant-pH sweep
-size_t sweep_draws(const Batch& b);   // draws of every replica, in whole blocks
 void adj_unpermute(Batch& b, float4* dst);
 void adj_scatter_pos(Batch& b, const float4* src);
 void adj_hvp(Batch& b, const uint32_t* drift, const float4* g, float4* jg, double* partial_dev);

@@ -1,7 +1,7 @@
 """Calls at their limits and calls between others: rows of the neighbour list at the capacity and beyond what a warp
 stages, rebuilds of a box of many more cells than beads, a window's reverse pass behind other calls, a sweep on lists
-that no longer serve, one in a box below twice its cutoff, aggregates of coordinates far outside the box, and the lanes of
-the list force."""
+that no longer serve, one in a box below twice its cutoff, aggregates of coordinates far outside the box, the lanes of
+the list force, and the sweep's arrays in live boxes and many replicas."""
 import numpy as np
 import pytest
 
@@ -314,3 +314,51 @@ def test_a_dilute_system_steps_the_same_with_any_lanes(n, monkeypatch):
         runs.append((g.particles(), g.forces_no_rebuild()))
         g.dispose()
     assert all(np.array_equal(a, b) for a, b in zip(*runs))
+
+
+def _sweeps_are_the_oracles(g, cfg, sweeps=2):
+    cfg.protonation_rng = g.protonation_rng_state()
+    o = ob.OracleSystem(_abi, cfg, {"positions": g.particles(), "charges": g.charges()})
+    for k in range(sweeps):
+        rg, ro = g.protonation_sweep(), o.sweep()
+        assert np.array_equal(g.charges(), o.read(ob.F_CHARGES)), k
+        assert g.protonation_rng_state() == int(o.read(ob.F_PROT_RNG)[0]), k
+        assert rg["accepted"] == ro.accepted > 0, k
+
+
+@pytest.mark.parametrize("sides", [(40.0, 16.0, 40.0), (16.0, 40.0, 17.0)])
+@pytest.mark.parametrize("heads", [100, 300, 1100])
+def test_sweeps_in_a_live_box(sides, heads):
+    """boxes in which the walk takes 512 and 256 draws a block, one after the other, in arrays laid out for the first"""
+    cfg = cfgm.resolve(cfgm.SoupOptions(box=[sides[0]] * 3, seed=heads, kT=1.1, start={"C": 0, "O": heads, "H": 0, "M": 1, "W": 400},
+                                        electrostatics={"enabled": True, "pH": 4.5, "ionicStrengthMolar": 0.1}), P)
+    share = [cfg.es_cutoff ** 3 * 4.18879 / s ** 3 for s in sides]
+    assert (min(share) < 0.06 < max(share)) and cfg.es_cutoff < 0.45 * 16
+    cfg.protonation_rng = 3
+    cfg.es_list_capacity = heads
+    pos = ob.OracleSystem(_abi, cfg).read(ob.F_POS).reshape(-1, 4).copy()
+    pos[:, :3] = np.random.default_rng(heads).random((cfg.n, 3)) * 15.9
+    g = SoupSystem(cfg, {"positions": pos.astype(np.float32).ravel()})
+    for k, side in enumerate(sides):
+        if k:
+            g.set_box([side] * 3)
+            cfg.box[0] = cfg.box[1] = cfg.box[2] = side
+        _sweeps_are_the_oracles(g, cfg)
+    g.dispose()
+
+
+def test_the_memory_of_many_small_replicas():
+    """the sweep's arrays follow the replicas' own heads: 255 replicas of 20 heads took 1.3 GB for pairs that cannot be"""
+    import torch
+    cfgs = []
+    for r in range(255):
+        cfg = cfgm.resolve(cfgm.SoupOptions(box=[15] * 3, seed=r, kT=1.1, start={"C": 0, "O": 20, "H": 0, "M": 1, "W": 43},
+                                            electrostatics={"enabled": True, "pH": 7.0, "ionicStrengthMolar": 0.1}), P)
+        cfgs.append(cfg)
+    torch.cuda.synchronize()
+    before = torch.cuda.mem_get_info()[0]
+    b = SoupBatch(cfgs)
+    held = before - torch.cuda.mem_get_info()[0]
+    b.replicas[254].protonation_sweep()
+    b.dispose()
+    assert held < 300e6, held
