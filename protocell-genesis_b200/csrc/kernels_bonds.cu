@@ -9,14 +9,15 @@
 // The reference resolves slot and centre claims by CAS races between threads, so its outcome varies
 // with scheduling.  The canonical semantics here (and in the CPU oracle) are the serial execution of
 // the formation pass in ascending particle order.  It is computed in parallel, exactly:
-//   Phase A (one thread per particle): the candidate walk and both Metropolis draws.  Neither
+//   Phase A (a warp per particle that can react): the candidate walk and both Metropolis draws.  Neither
 //     depends on claim outcomes (a pair i<j is only ever formed by i; draws consume the particle's
 //     own stream), so accept decisions and the final RNG state are computed here, in parallel.
-//   Phase B (one CTA): every particle with an accepted proposal, every catalyst, every particle
+//   Phase B (all SMs): every particle with an accepted proposal, every catalyst, every particle
 //     holding a centre link, and every proposal partner becomes an "item".  Items whose particle
 //     sets (self, partners, the catalyst found, and their current centre links) intersect are
 //     joined by union-find; different components touch disjoint state, so they commute.  Inside a
-//     component the items run in ascending index order, one per round.
+//     component the items run in ascending index order: a thread runs a whole component, and the last block
+//     to finish the large ones, an item of each per round.
 //   Breaking is race-free in the reference (only the lower index of a bond draws for it) and runs
 //     one thread per particle.
 #include "soup_internal.h"
@@ -386,7 +387,8 @@ __global__ void k_bond_lists(uint32_t* __restrict__ items, const uint32_t* __res
 // list sorted first; eight threads of a warp work, so that components of unequal length hold up few others.  The
 // items of larger components are left to the last block to finish, which runs them in rounds: of every
 // component the pending item with the smallest id.
-// Bound: the chain of gathers of an item.  (One CTA a replica ran all of them: 435 us at 483k beads.)
+// Bound: the chain of gathers of an item.  (One CTA a replica ran all of them: 549 us at 483k beads, 31 now and 6 for
+// the lists.)
 constexpr uint32_t kClaimSerial = 24;
 __global__ void __launch_bounds__(256) k_bond_claims(
     const Shared* __restrict__ Sg, const SysParams* __restrict__ sp, const uint8_t* __restrict__ sysid,

@@ -112,7 +112,8 @@ __device__ __forceinline__ void list_sum(uint32_t k, int lane, uint32_t end, con
 }
 
 // eight 128-thread blocks per SM (64 registers): small blocks even out rows of unequal length (256 threads: 192
-// against 183 us at 483k beads); fewer registers spill, fewer blocks hide less of the gathers' latency
+// against 183 us at 483k beads).  At 64 the four-lane forms spill 36 bytes a thread and the heads' eight-lane one 24;
+// fewer registers spill more, fewer blocks hide less of the gathers' latency
 constexpr int kForceBlock = 128;
 
 // SEL: the particles are the nsel slots sel[] (the heads, after a charge sweep) instead of all N

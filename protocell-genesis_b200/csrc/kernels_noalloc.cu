@@ -1,8 +1,8 @@
 // kernels_noalloc.cu -- aggregate labels without any device allocation.
 //
-// soup_aggregate_labels (kernels_analysis.cu) allocates its scratch (cell bins, union-find parents,
-// component minima) with cudaMalloc on every call and frees it with cudaFree.  Some callers cannot
-// do that: a host process whose GPU memory is already reserved by another allocator (a framework's
+// soup_aggregate_labels (kernels_analysis.cu) keeps its scratch (cell bins, union-find parents,
+// component minima) with the system, and grows it with cudaMalloc and cudaFree when a request is larger than any
+// before.  Some callers cannot do that: a host process whose GPU memory is already reserved by another allocator (a framework's
 // caching allocator that holds the whole device) can see cudaMalloc fail with out-of-memory even
 // though the job has room, and cudaFree synchronises the whole device, stalling the MD stream that
 // shares the GPU.  This file gives them soup_aggregate_labels_noalloc: the same labels, computed

@@ -24,9 +24,10 @@
 //                 ones alone, so what stands is the sequential chain's result, and draw d stands after at
 //                 most d rounds (3 rounds a block at 18,659 heads, 4 to 5 where the cutoff spans the box).
 //                 Then the other CTAs add the block's flips to E from the D rows.
-//   What bounds the walk: latency.  One warp that resolved windows of 32 draws took 3.99 ms a sweep at 18,659
-//   heads (1,075 windows of handoffs and dependent loads); blocks of 512 take 0.91 ms, 14k cycles for each of
-//   66: 3 rounds of 1.5k, 2 pulls of 2k, 2k to commit, 7k for the handoff, the adds and the way back.
+//   What bounds the walk: latency.  One warp that resolved windows of 32 draws took 4.1 ms a sweep at 18,659
+//   heads (1,075 windows of handoffs and dependent loads); blocks of 512 take 0.76 ms, some 22k cycles for each of
+//   66.  By clock stamps (which add a tenth): 3 rounds of 3.5k to decide and scan, 2 pulls of 1.5k, 1.7k to commit, and
+//   7.5k until the other CTAs have added the flips: 3k for the adds, 4k to 5k for the handoff there and back.
 // E and D are fixed point (2^-40 kT, int64): integer adds commute, so E does not depend on the
 // order the updates land in and every run is reproducible.  E_h is the FP64 sum rounded once, each
 // D_ht is rounded once, so the energies agree with the reference's FP64 sums to about 1e-11 kT (the
@@ -791,8 +792,8 @@ void launch_sweep(Batch& b, uint32_t replica) {
   k_sweep_draws<<<dim3((draws + 255) / 256, ry), 256, 0, b.stream>>>(b.sp, b.prot_rng_dev, replica, b.draw_site);
   (far ? k_sweep_pairs<true> : k_sweep_pairs<false>)<<<dim3(draws / kPairDraws, ry), 256, 0, b.stream>>>(
       b.sp, b.head_pos, b.draw_site, replica, b.pair_cnt, b.pair_idx, b.pair_del);
-  // a group of CTAs per replica, all SMs together (a cooperative launch).  The handoffs cost about 4k cycles a
-  // block, in which one SM adds about 4k list entries: a replica whose blocks flip fewer than that walks alone
+  // a group of CTAs per replica, all SMs together (a cooperative launch).  A handoff there and back costs 4k to 5k cycles
+  // a block, in which one SM adds about 4k list entries: a replica whose blocks flip fewer than that walks alone
   // (a fifth of the draws flips; a list holds the heads within the range, at most all of them).
   const unsigned each = std::max(1u, (unsigned)b.sms / ry);
   const double entries = 0.2 * std::min(2u * hmax, wmax) * std::min<double>(hmax, sweep_list_entries(b, replica));
